@@ -119,8 +119,8 @@ typedef struct {
   int32_t gate_kind;  /* TOPS_GATE_* */
   int32_t impl;       /* TOPS_IMPL_* */
   float scale;
-  const int32_t* cu_seqlens; /* device int32 [N+1] or NULL */
-  const int32_t* cu_seqlens_host; /* the same values in host memory (needed when cu_seqlens != NULL) */
+  const int32_t* cu_seqlens; /* device int32 [N+1]; only the generic kernels read it, may be NULL otherwise */
+  const int32_t* cu_seqlens_host; /* packed batches: sequence boundaries [N+1] in host memory; NULL: dense */
   int32_t N;                 /* sequences when packed; else ignored (N = B) */
 } tops_chunk_problem;
 
@@ -177,7 +177,7 @@ typedef struct {
   float* A_out;
   void* h_out;
   /* Optional scratch kept for the backward call of the same problem:
-   * B*NT*H*K*V elements of the input dtype.  Its content is private to the
+   * tops_b200_chunk_saved_bytes of it.  Its content is private to the
    * kernel family that ran (the tcgen05 kernels store pre-scaled bf16 states);
    * hand it to tops_b200_chunk_gla_bwd as `h_saved` only when
    * tops_b200_chunk_selected_impl reports TOPS_IMPL_SM100 for the problem. */
@@ -189,6 +189,8 @@ typedef struct {
 } tops_chunk_fwd_params;
 /* Which kernel family TOPS_IMPL_AUTO resolves to for this problem on the current device. */
 int tops_b200_chunk_selected_impl(const tops_chunk_problem* pb);
+/* Bytes of the `saved_out` scratch of this problem; 0 when the kernel family that serves it keeps none. */
+size_t tops_b200_chunk_saved_bytes(const tops_chunk_problem* pb);
 size_t tops_b200_chunk_fwd_workspace_bytes(const tops_chunk_fwd_params* p);
 int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* workspace, size_t workspace_bytes,
                             void* stream);

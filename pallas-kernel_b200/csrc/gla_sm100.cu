@@ -2,8 +2,10 @@
 // in shared memory by TMA, contractions issued with tcgen05.mma into tensor
 // memory, fp32 accumulation, gates and state kept in fp32.
 //
-// Shapes taken here: bf16 q/k/v/g, K = V = 128, chunk 64, T a multiple of 64,
-// dense batch, per-channel gates.  Everything else runs on the generic kernels.
+// Shapes taken here: bf16 q/k/v/g, chunk 64.  The plain form of the kernels: K = V = 128, T a
+// multiple of 64, dense batch, per-channel or scalar gates.  The general form: packed batches, any T,
+// 32 <= K <= 128, 32 <= V <= 1024 (multiples of 8), also constant or no gates.  Everything else runs on
+// the generic kernels.
 //
 // Data layout.  Activations stay in the caller's [B,T,H,D] layout; a chunk of
 // one head is a 64 x 128 tile whose rows are H*D elements apart, fetched as two
@@ -35,8 +37,11 @@
 // a warp may only touch the 32 tensor-memory lanes (warp & 3) * 32 .. + 31, so
 // the thread owns accumulator row `col` and splits the accumulator columns
 // with the three other warps of its lane quarter by `seg`.
+#include <algorithm>
 #include <atomic>
+#include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "gla_sm100.cuh"
 #include "sm100_host.cuh"
@@ -49,12 +54,89 @@ namespace sm100 {
 namespace {
 
 // ===========================================================================
+// Where the chunks of a call live
+// ===========================================================================
+// Every kernel exists in two forms.  The plain one (GEN = false) takes dense batches of whole chunks with
+// K = V = 128.  The general one (GEN = true) takes packed batches, sequences of any length, K <= 128 and any V
+// (multiples of 8):
+//   * the last chunk of a sequence may be short.  Its tile fetch reads on into the next sequence (or past the end
+//     of the tensor, where TMA fills zeros); the rows that are not its own are overwritten with zeros in shared
+//     memory before a product reads them, so nothing of another sequence, not even an infinity, gets in: zero
+//     gates repeat the last cumulative gate, zero q, k, v, do add nothing.  Only short chunks pay for it.
+//   * channels beyond K or V are zero-filled by TMA; the state tiles in scratch are always 128 x 128.
+//   * V > 128 runs as VS slices of 128 value channels that share q, k and g.
+//   * packed batches find their segments and chunks in tables that k_plan writes.
+struct __align__(16) SegEntry {   // a run of chunks of one sequence, walked by one block (per head and value slice)
+  int row, end;      // first token of the run; end of its sequence (token rows of the flattened [B*T] axis)
+  int slot, nch;     // index of its first chunk among all chunks; number of chunks
+  int id;            // index of the run in sequence order (the table itself is sorted by length, longest first)
+  int seq, cnt, pad; // its sequence; number of runs that sequence is cut into
+};
+struct ChunkEntry { int row, end; };
+struct Geo {
+  const SegEntry* segs;       // packed batches; null: dense, cps chunks per segment
+  const ChunkEntry* chunks;   // packed batches; null: dense
+  int K, V, VS;
+  int cps, nseg;              // dense: chunks per segment, segments per sequence
+  int NTseq;                  // dense: chunks per sequence
+};
+// the block's position: blocks are numbered (segment, head, value slice), slice fastest
+// cnt: runs its sequence is cut into.  A sequence of one run starts from and ends in the caller's states (index
+// seqh); the runs of a longer one start from the states that k_join_segments_gen leaves (index sidx).
+struct BlockPos { int h, vs, row, end, slot, nch, cnt; size_t sidx, seqh; };
+__device__ __forceinline__ BlockPos block_pos(const Geo& g, int T, int H, int blk) {
+  BlockPos q;
+  q.vs = blk % g.VS;
+  const int sh = blk / g.VS;
+  q.h = sh % H;
+  const int s = sh / H;
+  int id;
+  if (g.segs) {
+    const SegEntry e = g.segs[s];
+    q.row = e.row; q.end = e.end; q.slot = e.slot; q.nch = e.nch; id = e.id;
+    q.cnt = e.cnt; q.seqh = (size_t)e.seq * H + q.h;
+  } else {
+    const int b = s / g.nseg, sg = s - b * g.nseg;
+    q.row = b * T + sg * g.cps * C; q.end = (b + 1) * T;
+    q.slot = b * g.NTseq + sg * g.cps;
+    q.nch = min(g.cps, g.NTseq - sg * g.cps);
+    q.cnt = g.nseg; q.seqh = (size_t)b * H + q.h;
+    id = s;
+  }
+  q.sidx = (size_t)id * H + q.h;
+  return q;
+}
+// overwrites rows [len, 64) of a 64 x 128 tile with zeros (threads t0, t0 + nt, ...)
+__device__ __forceinline__ void zero_rows(uint8_t* tile, int len, int t0, int nt) {
+  for (int i = t0; i < (64 - len) * 16; i += nt) {
+    const int r = len + (i >> 4), piece = i & 15;
+    *reinterpret_cast<uint4*>(tile + (piece >> 3) * SLAB64 + r * 128 + (piece & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// 32 values of row `row` of a state [.., K, V], columns c0 .. c0 + 31 (zero outside K x V)
+__device__ __forceinline__ void load_state32(float (&S)[32], const float* base, int row, int c0, int K, int V) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (base && row < K && c0 + j < V) x = *reinterpret_cast<const float4*>(base + (size_t)row * V + c0 + j);
+    S[j] = x.x; S[j + 1] = x.y; S[j + 2] = x.z; S[j + 3] = x.w;
+  }
+}
+__device__ __forceinline__ void store_state32(float* base, const float (&S)[32], int row, int c0, int K, int V) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    if (row < K && c0 + j < V)
+      *reinterpret_cast<float4*>(base + (size_t)row * V + c0 + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
+}
+
+// ===========================================================================
 // State scans
 // ===========================================================================
 struct ScanParams {
   CUtensorMap mx, mg, my;  // x: k (fwd) / q (bwd); y: v / do
   CUtensorMap mst;         // the states tensor as [B*NT*H*128, 128] (TMA stores)
   const float* s0;         // state each block starts from: [B,H,nseg,K,V] or null (zero)
+  const float* s0_seg;     // GEN: the same for the runs of a sequence that is cut into several
   __nv_bfloat16* states;   // h' / dh'  [B,T/64,H,K,V]; null: keep no chunk-start states (summary pass)
   float* s_final;          // state each block ends with: [B,H,nseg,K,V] or null
   float* gsum;             // summed log-gates of each block's chunks [B,H,nseg,K] or null
@@ -62,6 +144,8 @@ struct ScanParams {
   int nseg;                // time segments per sequence, one block each
   float scale;
   const __nv_bfloat16* gscalar;   // scalar gates [B,T,H] (SCALAR kernels; mg is unused then)
+  const float* gamma;      // constant gates [H] (SCALAR GEN kernels; gscalar is null then; both null: no gate)
+  Geo geo;                 // GEN kernels
   int skip_xy;             // test hook: the x/y tile load of this chunk is never issued (-1: none), so that the
                            // bounded wait for it runs out and the kernel leaves through its error path
 };
@@ -97,7 +181,7 @@ struct ScanShared {
 // the chunk before it but the running sum R, the chain product -> register update -> next product is gone and a
 // chunk costs its gating and its products.  The chunks are walked from the far end (forward scan: last chunk
 // first; reverse scan: first chunk first), so that R is known when a chunk is gated.
-template <bool BWD, bool SCALAR, bool SUM>
+template <bool BWD, bool SCALAR, bool SUM, bool GEN>
 __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant__ ScanParams p) {
   // every shared object is carved from the dynamic allocation, whose start is 1024-byte aligned when the
   // kernel has no static shared memory (checked below: the swizzled tiles need that alignment)
@@ -112,9 +196,21 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool driver = warp >= 16;   // warp 16 issues the products, warp 17 the copies
   const int q4 = warp & 3, seg = (warp >> 2) & 3, col = q4 * 32 + lane;
-  const int blk = blockIdx.x, sg = blk % p.nseg, bh = blk / p.nseg, b = bh / p.H, h = bh % p.H;
-  const int NT = p.NT;
+  BlockPos bp;
+  if constexpr (GEN) {
+    bp = block_pos(p.geo, p.T, p.H, blockIdx.x);
+  } else {
+    const int sg = blockIdx.x % p.nseg, bh = blockIdx.x / p.nseg, b = bh / p.H;
+    bp.h = bh % p.H; bp.vs = 0; bp.row = b * p.T + sg * p.NT * C; bp.end = (b + 1) * p.T;
+    bp.slot = b * (p.T / C) + sg * p.NT; bp.nch = p.NT; bp.sidx = bp.seqh = blockIdx.x; bp.cnt = 1;
+  }
+  const int h = bp.h, NT = bp.nch;
+  const int VS = GEN ? p.geo.VS : 1, K = GEN ? p.geo.K : D, V = GEN ? p.geo.V : D;
+  const int yc = bp.vs * D;   // first value channel of this block's slice
+  const float* const start_state = (GEN && !SUM && bp.cnt > 1) ? p.s0_seg + bp.sidx * K * V
+                                                       : (p.s0 ? p.s0 + bp.seqh * K * V : nullptr);
   const bool keep_states = p.states != nullptr;
+  if (GEN && SUM && p.geo.segs && bp.cnt == 1) return;   // a packed sequence that is not cut needs no summary
   // tensor-memory columns: two exponent tiles, two state-product accumulators
   constexpr uint32_t cE = 0, cS = 256;
   if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
@@ -122,8 +218,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     return;
   }
 
-  // chunk pp of this block (in the order the block walks them) within its sequence
-  auto chunk_of = [&](int pp) { return sg * NT + ((BWD != SUM) ? NT - 1 - pp : pp); };
+  // chunk pp of this block (in the order the block walks them) within its run of chunks
+  auto chunk_of = [&](int pp) { return (BWD != SUM) ? NT - 1 - pp : pp; };
   // SUM: summed gates of the chunks already done, per channel (two copies, written for the next chunk while the
   // current one is read; in the place of e0, which a summary pass does not use) or, for scalar gates, in a
   // register of every thread
@@ -136,7 +232,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   auto y_stage = [&](int pp) { const int st = pp % NXY; return st < 3 ? ys + st * TILE64 : hst + (st - 3) * 2 * TILE64 + TILE64; };
   auto xy_bar = [&](int pp) { return &sh.fullxy[pp % NXY]; };
   auto xy_parity = [&](int pp) { return (uint32_t)((pp / NXY) & 1); };
-  auto chunk_row = [&](int pp) { return b * p.T + chunk_of(pp) * C; };
+  auto chunk_row = [&](int pp) { return bp.row + chunk_of(pp) * C; };
+  auto chunk_len = [&](int pp) { return GEN ? min(C, bp.end - chunk_row(pp)) : C; };   // rows that are the sequence's own
   auto issue_g = [&](int pp) {
     uint8_t* dst = gs + (pp % 3) * TILE64;
     mbar_expect_tx(&sh.fullg[pp % 3], TILE64);
@@ -149,8 +246,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     mbar_expect_tx(bar, 2 * TILE64);
     tma_load_3d(xd, &p.mx, bar, 0, h, chunk_row(pp));
     tma_load_3d(xd + SLAB64, &p.mx, bar, 64, h, chunk_row(pp));
-    tma_load_3d(yd, &p.my, bar, 0, h, chunk_row(pp));
-    tma_load_3d(yd + SLAB64, &p.my, bar, 64, h, chunk_row(pp));
+    tma_load_3d(yd, &p.my, bar, yc, h, chunk_row(pp));
+    tma_load_3d(yd + SLAB64, &p.my, bar, yc + 64, h, chunk_row(pp));
   };
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&sh.fullg[i], 1);
@@ -173,7 +270,13 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   const long long gidx0 = (long long)(chunk_row(0) + lane) * p.H + h;
   const long long gstep = (long long)(chunk_row(NT > 1 ? 1 : 0) - chunk_row(0)) * p.H;   // +-64 H elements per chunk
   auto gate_index = [&](int c) { return (size_t)(gidx0 + c * gstep); };
-  auto load_gates = [&](int c) { gring.prefetch(p.gscalar, c < NT, c < NT ? gate_index(c) : 0, (size_t)32 * p.H, c, lane); };
+  const float gconst = (GEN && SCALAR && p.gamma) ? p.gamma[h] : 0.f;   // GEN: a constant decay, or none
+  auto load_gates = [&](int c) {
+    const int len = c < NT ? chunk_len(c) : 0;
+    const bool stored = !GEN || p.gscalar;
+    gring.prefetch(p.gscalar, stored && lane < len, stored && lane + 32 < len, c < NT ? gate_index(c) : 0, (size_t)32 * p.H, c,
+                   lane);
+  };
   if (SCALAR) {
     if (!driver) {
       gring.init(gs + warp * GateRing::kBytesPerWarp);
@@ -193,8 +296,16 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   const uint32_t lane_base = q4 * 32;
 
   // exponents E = pattern . g of chunk pp: [time (repeated to 128 lanes)][channel]; row 63 is G_n
+  // (called by the whole product warp: a short chunk's foreign gate rows are zeroed first)
   auto issue_gate_mma = [&](int pp) {
     if (SCALAR) return;
+    if (GEN && chunk_len(pp) < C) {
+      if (!mbar_wait(&sh.fullg[pp % 3], (pp / 3) & 1)) { *abort_flag = 1; fail(1); }
+      zero_rows(gs + (pp % 3) * TILE64, chunk_len(pp), lane, 32);
+      fence_async_smem();
+      __syncwarp();
+    }
+    if (lane != 0) return;
     if (!mbar_wait(&sh.fullg[pp % 3], (pp / 3) & 1)) { *abort_flag = 1; fail(1); }
     tc_fence_after();
     const uint32_t ga = smem_u32(gs + (pp % 3) * TILE64);
@@ -225,9 +336,21 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     tc_fence_after();
     const int i = (q4 * 32 + lane) & 63;          // time row of this thread
     const int cg = (q4 >> 1) * 4 + seg;           // its 16 channels
+    const int len = chunk_len(pp);
+    const bool mine = !GEN || i < len;            // (a short chunk's foreign rows become zero)
+    if (GEN && !mine) {
+      uint8_t* yt = y_stage(pp) + (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        *reinterpret_cast<uint4*>(yt + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u) = make_uint4(0u, 0u, 0u, 0u);
+    }
     if (SCALAR) {
       float g_lo, g_hi;
       gring.take(gate_index(pp), pp, lane, g_lo, g_hi);
+      if (GEN) {
+        g_lo = lane < len ? (p.gscalar ? g_lo : gconst) : 0.f;
+        g_hi = lane + 32 < len ? (p.gscalar ? g_hi : gconst) : 0.f;
+      }
       const WarpGates w = warp_cumulate(g_lo, g_hi, lane);
       const float Gi = (q4 & 1) ? w.hi : w.lo;
       gn_next = w.gn;
@@ -239,7 +362,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-        *reinterpret_cast<uint4*>(xt + off) = scale8_by(*reinterpret_cast<const uint4*>(xt + off), f);
+        *reinterpret_cast<uint4*>(xt + off) =
+            mine ? scale8_by(*reinterpret_cast<const uint4*>(xt + off), f) : make_uint4(0u, 0u, 0u, 0u);
       }
       fence_async_smem();
       tc_fence_before();
@@ -274,7 +398,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-      *reinterpret_cast<uint4*>(xt + off) = scale8(*reinterpret_cast<const uint4*>(xt + off), e + 8 * u);
+      *reinterpret_cast<uint4*>(xt + off) =
+          mine ? scale8(*reinterpret_cast<const uint4*>(xt + off), e + 8 * u) : make_uint4(0u, 0u, 0u, 0u);
     }
     fence_async_smem();
     tc_fence_before();
@@ -292,23 +417,21 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     // The two issuing threads run the same barriers as the compute warps and never wait for one another: the
     // product thread's time is the tensor core's (an issue takes about as long as the product before it runs),
     // the copy thread's is spent waiting for products to release tiles.
-    if (lane == 0) {
-      issue_gate_mma(0);
-      if (NT > 1) issue_gate_mma(1);
-    }
+    issue_gate_mma(0);
+    if (NT > 1) issue_gate_mma(1);
+    __syncwarp();
     bool ok = !__syncthreads_or(*abort_flag);   // chunk 0 is gated
-    if (ok && lane == 0) {
-      issue_state_mma(0);
+    if (ok) {
+      if (lane == 0) issue_state_mma(0);
       if (NT > 2) issue_gate_mma(2);
+      __syncwarp();
     }
     for (int pp = 0; ok && pp < NT; ++pp) {
       // h'_pp is staged, chunk pp+1 is gated; every thread of the block sees the same verdict, so
       // all of them leave the loop at the same barrier
       if (__syncthreads_or(*abort_flag)) break;
-      if (lane == 0) {
-        if (pp + 1 < NT) issue_state_mma(pp + 1);
-        if (pp + 3 < NT) issue_gate_mma(pp + 3);   // its exponent slot was read by the gating of chunk pp+1
-      }
+      if (lane == 0 && pp + 1 < NT) issue_state_mma(pp + 1);
+      if (pp + 3 < NT) issue_gate_mma(pp + 3);   // its exponent slot was read by the gating of chunk pp+1
       __syncwarp();
     }
   } else if (warp == 17) {
@@ -322,7 +445,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
       if (__syncthreads_or(*abort_flag)) break;
       if (lane == 0) {
         if (keep_states) {
-          const int hrow = ((b * (p.T / C) + chunk_of(pp)) * p.H + h) * D;
+          const int hrow = (((bp.slot + chunk_of(pp)) * p.H + h) * VS + bp.vs) * D;
           tma_store_2d(&p.mst, hst + (pp & 1) * TILE128, 0, hrow);
           tma_store_2d(&p.mst, hst + (pp & 1) * TILE128 + TILE128 / 2, 64, hrow);
           tma_store_commit();
@@ -340,14 +463,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     // ------------------------------------------------------------------ state in registers
     // fp32 state: row k = col, columns 32 seg .. + 31
     float S[32];
-    {
-      const float* src = p.s0 ? p.s0 + ((size_t)blk * D + col) * D + seg * 32 : nullptr;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        float4 x = src ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        S[j] = x.x; S[j + 1] = x.y; S[j + 2] = x.z; S[j + 3] = x.w;
-      }
-    }
+    load_state32(S, start_state, col, yc + seg * 32, K, V);
     float gtot = 0.f;   // summed log-gates of this thread's channel over the block's chunks
     gate_chunk(0);
     if (SCALAR) load_gates(3);
@@ -399,12 +515,10 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
       tmem_ld32(tmem_addr(tm, lane_base, cS + seg * 32), S);
       tc_fence_before();
     }
-    if (ok && p.s_final) {
-      float* dst = p.s_final + ((size_t)blk * D + col) * D + seg * 32;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
-    }
-    if (ok && p.gsum && seg == 0) p.gsum[(size_t)blk * D + col] = gtot;
+    // (SUM: what the join needs, per run; otherwise the join has written the final state of a sequence cut into runs)
+    if (ok && p.s_final && (SUM || bp.cnt == 1))
+      store_state32(p.s_final + (SUM ? bp.sidx : bp.seqh) * K * V, S, col, yc + seg * 32, K, V);
+    if (ok && p.gsum && seg == 0 && bp.vs == 0) p.gsum[bp.sidx * D + col] = gtot;
     // (a loop left early may leave gate copies of this thread in flight: they land before the block ends)
     if (SCALAR) asm volatile("cp.async.wait_all;" ::: "memory");
   }
@@ -412,9 +526,9 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && sh.abort_flag) {
-    if (p.states) poison(p.states + ((size_t)(b * (p.T / C) + chunk_of(0)) * p.H + h) * D * D);
-    if (p.s_final) poison(p.s_final + (size_t)blk * D * D);
-    if (p.gsum) poison(p.gsum + (size_t)blk * D);
+    if (p.states) poison(p.states + ((size_t)((bp.slot + chunk_of(0)) * p.H + h) * VS + bp.vs) * D * D);
+    if (p.s_final && (SUM || bp.cnt == 1)) poison(p.s_final + (SUM ? bp.sidx : bp.seqh) * K * V + yc);
+    if (p.gsum) poison(p.gsum + bp.sidx * D);
   }
 }
 
@@ -445,6 +559,51 @@ __global__ void k_join_segments(const float* __restrict__ first, const float* __
   }
 }
 
+// The same for the general form: states are [K, V] per (sequence, head), segments of sequence n are
+// [seg0[n], seg0[n+1]) (packed) or n * nseg .. (dense).  Sequences of one segment need no join.
+template <bool REVERSE>
+__global__ void k_join_segments_gen(const float* __restrict__ first, const float* __restrict__ P, const float* __restrict__ S,
+                                    float* __restrict__ start, float* __restrict__ last, const int* __restrict__ seg0, int nseg,
+                                    int H, int K, int V) {
+  const int n = blockIdx.x / H, h = blockIdx.x - n * H;
+  const int s0 = seg0 ? seg0[n] : n * nseg, cnt = seg0 ? seg0[n + 1] - s0 : nseg;
+  if (cnt == 1) return;
+  const size_t KV = (size_t)K * V;
+  for (size_t e = (blockIdx.y * blockDim.x + threadIdx.x) * 4; e < KV; e += (size_t)gridDim.y * blockDim.x * 4) {
+    const int k = (int)(e / V);
+    float4 cur = first ? *reinterpret_cast<const float4*>(first + (size_t)blockIdx.x * KV + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int i = 0; i < cnt; ++i) {
+      const size_t r = (size_t)(s0 + (REVERSE ? cnt - 1 - i : i)) * H + h;
+      *reinterpret_cast<float4*>(start + r * KV + e) = cur;
+      const float w = __expf(P[r * D + k]);
+      const float4 add = *reinterpret_cast<const float4*>(S + r * KV + e);
+      cur = make_float4(fmaf(cur.x, w, add.x), fmaf(cur.y, w, add.y), fmaf(cur.z, w, add.z), fmaf(cur.w, w, add.w));
+    }
+    if (last) *reinterpret_cast<float4*>(last + (size_t)blockIdx.x * KV + e) = cur;
+  }
+}
+
+// Tables of a packed batch, written from the kernel's own parameters: no host buffer has to outlive the call and
+// nothing goes through the copy engine.  The words start with (first token, end, first chunk slot) of every
+// sequence; when all of them are in this launch (N > 0) it also writes the chunk table.
+template <int W> struct PlanWords { int w[W]; };
+constexpr int kPlanSmall = 1000, kPlanLarge = 8000;   // kernel parameters hold 4 KB cheaply, 32764 bytes at most
+__device__ __forceinline__ void plan_chunks(const int* seqs, int N, ChunkEntry* chunks) {
+  for (int n = blockIdx.x; n < N; n += gridDim.x) {
+    const int row = seqs[3 * n], end = seqs[3 * n + 1], slot = seqs[3 * n + 2];
+    for (int c = threadIdx.x; row + c * C < end; c += blockDim.x) chunks[slot + c] = ChunkEntry{row + c * C, end};
+  }
+}
+template <int W>
+__global__ void k_plan(const __grid_constant__ PlanWords<W> src, int* dst, int n, int N, ChunkEntry* chunks) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src.w[i];
+  plan_chunks(src.w, N, chunks);
+}
+__global__ void k_plan_chunks(const int* __restrict__ seqs, int N, ChunkEntry* __restrict__ chunks) {
+  plan_chunks(seqs, N, chunks);
+}
+
 // ===========================================================================
 // Forward output
 // ===========================================================================
@@ -454,18 +613,20 @@ struct FwdOParams {
   __nv_bfloat16* o;
   int T, H, NT;
   float scale;
+  const float* gamma;             // constant gates [H] (SCALAR GEN kernel)
+  Geo geo;                        // GEN kernel
 };
 
 // SCALAR: no gate tile and no exponent product; every warp cumulates the chunk's 64 gates in registers.
-template <bool SCALAR>
+template <bool SCALAR, bool GEN>
 __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ FwdOParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* qs = smem;                 // q -> q~ in place
   uint8_t* ks = qs + TILE64;          // k -> k~ in place
   uint8_t* gs = ks + TILE64;          // g; later the bf16 intra matrix (first 8 KB)
-  uint8_t* vs = gs + TILE64;
-  uint8_t* hs = vs + TILE64;          // h_c exp(mid) scale, 128 x 128 (scaled by the scan kernel)
+  uint8_t* vt = gs + TILE64;
+  uint8_t* hs = vt + TILE64;          // h_c exp(mid) scale, 128 x 128 (scaled by the scan kernel)
   uint8_t* mt = hs + TILE128;         // TRI_MID pattern, 64 x 64
   __shared__ uint64_t bar_load, bar_e, bar_a, bar_o;
   __shared__ uint32_t tmem_slot;
@@ -473,8 +634,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   const int q4 = warp & 3, seg = warp >> 2;
   // heads vary fastest over the blocks in flight: together they read whole token rows of the
   // [B,T,H,D] activations (all heads of a time step are contiguous in memory)
-  const int h = blockIdx.x, ci = blockIdx.y, b = blockIdx.z;
-  const int row = b * p.T + ci * C;
+  // (grid: heads x value slices, chunks of a sequence, sequences; packed: heads x value slices, all chunks, 1)
+  const int VS = GEN ? p.geo.VS : 1, V = GEN ? p.geo.V : D;
+  const int h = GEN ? blockIdx.x / VS : blockIdx.x, vs = GEN ? blockIdx.x % VS : 0, ci = blockIdx.y, b = blockIdx.z;
+  const int slot = b * p.NT + ci;
+  int row = b * p.T + ci * C, end = (b + 1) * p.T;
+  if (GEN && p.geo.chunks) { const ChunkEntry e = p.geo.chunks[slot]; row = e.row; end = e.end; }
+  const int len = GEN ? min(C, end - row) : C;
   constexpr uint32_t cO = 0, cE = 0, cA = 128;   // E is consumed before O is produced
 
   if (tid == 0) {
@@ -484,17 +650,19 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     if (!SCALAR) { tma_load_3d(gs, &p.mg, &bar_load, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, &bar_load, 64, h, row); }
     tma_load_3d(qs, &p.mq, &bar_load, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, &bar_load, 64, h, row);
     tma_load_3d(ks, &p.mk, &bar_load, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, &bar_load, 64, h, row);
-    tma_load_3d(vs, &p.mv, &bar_load, 0, h, row); tma_load_3d(vs + SLAB64, &p.mv, &bar_load, 64, h, row);
-    const int hrow = ((b * p.NT + ci) * p.H + h) * D;
+    tma_load_3d(vt, &p.mv, &bar_load, vs * D, h, row); tma_load_3d(vt + SLAB64, &p.mv, &bar_load, vs * D + 64, h, row);
+    const int hrow = ((slot * p.H + h) * VS + vs) * D;
     tma_load_2d(hs, &p.mh, &bar_load, 0, hrow); tma_load_2d(hs + TILE128 / 2, &p.mh, &bar_load, 64, hrow);
   }
   __syncwarp();
   if (warp == 0) { tmem_alloc(&tmem_slot, 256); tmem_relinquish(); }
   __nv_bfloat16 greg_lo = __float2bfloat16(0.f), greg_hi = greg_lo;   // SCALAR: the gates of time steps lane and lane + 32
   if (SCALAR) {   // (one chunk per block: the loads have the whole tile fetch to land)
-    const __nv_bfloat16* src = p.gscalar + (size_t)(row + lane) * p.H + h;
-    greg_lo = src[0];
-    greg_hi = src[(size_t)32 * p.H];
+    if (!GEN || p.gscalar) {
+      const __nv_bfloat16* src = p.gscalar + (size_t)(row + lane) * p.H + h;
+      if (!GEN || lane < len) greg_lo = src[0];
+      if (!GEN || lane + 32 < len) greg_hi = src[(size_t)32 * p.H];
+    }
   } else {
     build_tri_tile(mt, 64, TRI_MID);
   }
@@ -506,6 +674,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   const uint32_t lane_base = q4 * 32;
   bool ok = __syncthreads_and(mbar_wait(&bar_load, 0));
   if (!ok) fail(3);
+  if (GEN && len < C) {   // (uniform over the block)
+    if (!SCALAR) zero_rows(gs, len, tid, NTHREADS);
+    zero_rows(vt, len, tid, NTHREADS);
+    zero_rows(qs, len, tid, NTHREADS);
+    zero_rows(ks, len, tid, NTHREADS);
+    fence_async_smem();
+    __syncthreads();
+  }
   if (!SCALAR && ok && tid == 0) {
     tc_fence_after();
     const uint32_t ga = smem_u32(gs), ma = smem_u32(mt);
@@ -522,7 +698,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   if (SCALAR && ok) {
     // thread (q4, lane < 16, seg) gates 32 channels of time row 16 q4 + lane, whose cumulative gate sits in
     // lane (16 q4 + lane) mod 32 of the warp
-    const WarpGates w = warp_cumulate(__bfloat162float(greg_lo), __bfloat162float(greg_hi), lane);
+    float g_lo = __bfloat162float(greg_lo), g_hi = __bfloat162float(greg_hi);
+    if (GEN && p.gamma) {
+      g_lo = lane < len ? p.gamma[h] : 0.f;
+      g_hi = lane + 32 < len ? p.gamma[h] : 0.f;
+    }
+    const WarpGates w = warp_cumulate(g_lo, g_hi, lane);
     const int i = 16 * q4 + (lane & 15);
     const float E = __shfl_sync(0xffffffffu, (q4 >> 1) ? w.hi : w.lo, i & 31) - w.mid();
     const float f = fast_exp(E), r = fast_exp(-E);
@@ -587,7 +768,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   __syncthreads();
   if (ok && tid == 0) {
     tc_fence_after();
-    const uint32_t pa = smem_u32(gs), va = smem_u32(vs);
+    const uint32_t pa = smem_u32(gs), va = smem_u32(vt);
 #pragma unroll
     for (int k0 = 0; k0 < C; k0 += 16)   // o += A v
       umma_bf16(tm + cO, desc_kmajor(pa, 64, 0, k0), desc_mnmajor(va, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
@@ -601,20 +782,21 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   if (ok) {
     tc_fence_after();
     const int i = 16 * q4 + lane;
-    __nv_bfloat16* dst = p.o + ((size_t)(row + i) * p.H + h) * D + seg * 32;
+    const int vc = vs * D + seg * 32;
+    __nv_bfloat16* dst = p.o + ((size_t)(row + i) * p.H + h) * V + vc;
     float a[32];
     tmem_ld32(tmem_addr(tm, lane_base, cO + seg * 32), a);
-    if (lane < 16) {
+    if (lane < 16 && (!GEN || i < len)) {
 #pragma unroll
       for (int t = 0; t < 32; t += 8)
-        *reinterpret_cast<uint4*>(dst + t) = make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]),
+        if (!GEN || vc + t < V) *reinterpret_cast<uint4*>(dst + t) = make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]),
                                                         pack_bf16(a[t + 4], a[t + 5]), pack_bf16(a[t + 6], a[t + 7]));
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
-  if (tid == 0 && !ok) poison(p.o + ((size_t)row * p.H + h) * D);
+  if (tid == 0 && !ok) poison(p.o + ((size_t)row * p.H + h) * V + vs * D);
 }
 
 // ===========================================================================
@@ -635,6 +817,7 @@ struct FusedParams {
   CUtensorMap mq, mk, mg, mv;
   CUtensorMap mst;         // the states tensor as [B*NT*H*128, 128] (TMA stores); unused when states == nullptr
   const float* s0;         // state each block starts from: [B,H,nseg,K,V] or null (zero)
+  const float* s0_seg;     // GEN: the same for the runs of a sequence that is cut into several
   __nv_bfloat16* states;   // h' [B,T/64,H,K,V] or null
   float* s_final;          // state each block ends with: [B,H,nseg,K,V] or null
   __nv_bfloat16* o;        // [B,T,H,V]
@@ -642,6 +825,8 @@ struct FusedParams {
   int T, H, NT;            // T: tokens per sequence; NT: chunks per block (T / 64 / nseg)
   int nseg;                // time segments per sequence, one block each
   float scale;
+  const float* gamma;      // constant gates [H] (SCALAR GEN kernel)
+  Geo geo;                 // GEN kernel
 };
 struct FusedShared {
   uint64_t fullin[2], ebar, abar, sbar, obar;
@@ -653,7 +838,7 @@ constexpr size_t FUSED_SMEM = 2 * FUSED_STAGE + 2 * TILE128 + 2 * SLAB64 + 2048 
 
 // SCALAR: no gate tile is fetched and no exponent product issued; every compute warp cumulates the chunk's 64
 // gates in registers (warp_cumulate), which gives its threads E of their time row, G_n and mid directly.
-template <bool SCALAR>
+template <bool SCALAR, bool GEN>
 __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_constant__ FusedParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* in = smem;                         // 2 stages x (q, k, g, v)
@@ -666,9 +851,20 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool driver = warp == 16;
   const int q4 = warp & 3, seg = (warp >> 2) & 3, col = q4 * 32 + lane;
-  const int blk = blockIdx.x, sg = blk % p.nseg, bh = blk / p.nseg, b = bh / p.H, h = bh % p.H;
-  const int NT = p.NT;
-  const int c0 = sg * NT;   // first chunk of this block within its sequence
+  BlockPos bp;
+  if constexpr (GEN) {
+    bp = block_pos(p.geo, p.T, p.H, blockIdx.x);
+  } else {
+    const int sg = blockIdx.x % p.nseg, bh = blockIdx.x / p.nseg, b = bh / p.H;
+    bp.h = bh % p.H; bp.vs = 0; bp.row = b * p.T + sg * p.NT * C; bp.end = (b + 1) * p.T;
+    bp.slot = b * (p.T / C) + sg * p.NT; bp.nch = p.NT; bp.sidx = bp.seqh = blockIdx.x; bp.cnt = 1;
+  }
+  const int h = bp.h, NT = bp.nch;
+  const int VS = GEN ? p.geo.VS : 1, K = GEN ? p.geo.K : D, V = GEN ? p.geo.V : D;
+  const int yc = bp.vs * D;   // first value channel of this block's slice
+  const float* const start_state = (GEN && bp.cnt > 1) ? p.s0_seg + bp.sidx * K * V
+                                                       : (p.s0 ? p.s0 + bp.seqh * K * V : nullptr);
+  auto chunk_len = [&](int pp) { return GEN ? min(C, bp.end - (bp.row + pp * C)) : C; };
   constexpr uint32_t cE = 0, cD = 128, cO = 256, cA = 384, cW = 448;
   if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
     if (tid == 0) fail(12);
@@ -678,12 +874,12 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
     uint8_t* qs = in + (pp & 1) * FUSED_STAGE;
     uint8_t *ks = qs + TILE64, *gs = ks + TILE64, *vs = gs + TILE64;
     uint64_t* bar = &sh.fullin[pp & 1];
-    const int row = b * p.T + (c0 + pp) * C;
+    const int row = bp.row + pp * C;
     mbar_expect_tx(bar, SCALAR ? 3 * TILE64 : FUSED_STAGE);
     if (!SCALAR) { tma_load_3d(gs, &p.mg, bar, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, bar, 64, h, row); }
     tma_load_3d(qs, &p.mq, bar, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, bar, 64, h, row);
     tma_load_3d(ks, &p.mk, bar, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, bar, 64, h, row);
-    tma_load_3d(vs, &p.mv, bar, 0, h, row); tma_load_3d(vs + SLAB64, &p.mv, bar, 64, h, row);
+    tma_load_3d(vs, &p.mv, bar, yc, h, row); tma_load_3d(vs + SLAB64, &p.mv, bar, yc + 64, h, row);
   };
   if (tid == 0) {
     mbar_init(&sh.fullin[0], 1); mbar_init(&sh.fullin[1], 1);
@@ -703,10 +899,12 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
   // GateRing instead)
   __nv_bfloat16 greg_lo = __float2bfloat16(0.f), greg_hi = greg_lo;
   auto load_gates = [&](int c) {
-    const __nv_bfloat16* src = p.gscalar + (size_t)(b * p.T + (c0 + c) * C + lane) * p.H + h;
-    greg_lo = src[0];
-    greg_hi = src[(size_t)32 * p.H];
+    if (GEN && !p.gscalar) return;
+    const __nv_bfloat16* src = p.gscalar + (size_t)(bp.row + c * C + lane) * p.H + h;
+    if (!GEN || lane < chunk_len(c)) greg_lo = src[0];
+    if (!GEN || lane + 32 < chunk_len(c)) greg_hi = src[(size_t)32 * p.H];
   };
+  const float gconst = (GEN && SCALAR && p.gamma) ? p.gamma[h] : 0.f;   // GEN: a constant decay, or none
   if (SCALAR) {
     if (!driver) load_gates(0);
   } else {
@@ -722,8 +920,16 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
 
   if (driver) {
     // ------------------------------------------------------------------ products and copies
+    // (called by the whole driver warp: a short chunk's foreign gate rows are zeroed first)
     auto issue_exponents = [&](int pp) {
       if (SCALAR) return;
+      if (GEN && chunk_len(pp) < C) {
+        if (!mbar_wait(&sh.fullin[pp & 1], (pp >> 1) & 1)) { *abort_flag = 1; fail(3); }
+        zero_rows(in + (pp & 1) * FUSED_STAGE + 2 * TILE64, chunk_len(pp), lane, 32);
+        fence_async_smem();
+        __syncwarp();
+      }
+      if (lane != 0) return;
       if (!mbar_wait(&sh.fullin[pp & 1], (pp >> 1) & 1)) { *abort_flag = 1; fail(3); }
       tc_fence_after();
       const uint32_t ga = smem_u32(in + (pp & 1) * FUSED_STAGE + 2 * TILE64), ma = smem_u32(mt), wa = smem_u32(wt);
@@ -735,7 +941,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         umma_bf16(tm + cW, desc_mnmajor(ga, 64, j0, 0), desc_kmajor(wa, 16, 0, j0), umma_idesc(128, 16, 1, 0), j0 > 0);
       umma_commit(&sh.ebar);
     };
-    if (lane == 0) issue_exponents(0);
+    issue_exponents(0);
     __syncwarp();
     for (int pp = 0; pp < NT; ++pp) {
       const uint32_t ph = pp & 1;
@@ -762,7 +968,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         for (int k0 = 0; k0 < D; k0 += 16)   // o = q~ h'
           umma_bf16(tm + cO, desc_kmajor(qa, 64, 0, k0), desc_mnmajor(ha, 128, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
         if (p.states) {
-          const int hrow = ((b * (p.T / C) + c0 + pp) * p.H + h) * D;
+          const int hrow = (((bp.slot + pp) * p.H + h) * VS + bp.vs) * D;
           tma_store_2d(&p.mst, ht, 0, hrow);
           tma_store_2d(&p.mst, ht + TILE128 / 2, 64, hrow);
           tma_store_commit();
@@ -777,13 +983,13 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         for (int k0 = 0; k0 < C; k0 += 16)   // o += tril(A) scale v
           umma_bf16(tm + cO, desc_kmajor(pa, 64, 0, k0), desc_mnmajor(va, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
         umma_commit(&sh.obar);
-        // exponents of the next chunk (E and W of this one were read before B1)
-        if (pp + 1 < NT) issue_exponents(pp + 1);
-        // every tile of this stage is dead once its products are complete
-        if (pp + 2 < NT) {
-          if (!mbar_wait(&sh.obar, ph)) { *abort_flag = 1; fail(5); }
-          issue_load(pp + 2);
-        }
+      }
+      // exponents of the next chunk (E and W of this one were read before B1)
+      if (pp + 1 < NT) issue_exponents(pp + 1);
+      // every tile of this stage is dead once its products are complete
+      if (lane == 0 && pp + 2 < NT) {
+        if (!mbar_wait(&sh.obar, ph)) { *abort_flag = 1; fail(5); }
+        issue_load(pp + 2);
       }
       __syncwarp();
     }
@@ -792,14 +998,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
   } else {
     // ------------------------------------------------------------------ state in registers
     float S[32];
-    {
-      const float* src = p.s0 ? p.s0 + ((size_t)blk * D + col) * D + seg * 32 : nullptr;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        float4 x = src ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        S[j] = x.x; S[j + 1] = x.y; S[j + 2] = x.z; S[j + 3] = x.w;
-      }
-    }
+    load_state32(S, start_state, col, yc + seg * 32, K, V);
     // Outputs leave in two steps: the accumulator rows (an M = 64 accumulator keeps 16 rows in the first
     // 16 lanes of each warp) are packed to bf16 in a shared tile; after the next block-wide barrier every
     // thread copies 32 contiguous bytes of it, so that a warp writes whole 256-byte rows.
@@ -807,11 +1006,12 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       const int r = tid >> 3, piece = tid & 7;   // 64 rows x 8 pieces of 16 channels
       // 16-byte pieces of a row are stored XOR-permuted by the row number (bank conflicts of the writers)
       const uint8_t* rowp = ost + r * 256;
-      uint4* dst = reinterpret_cast<uint4*>(p.o + ((size_t)(b * p.T + (c0 + pp) * C + r) * p.H + h) * D + piece * 16);
+      uint4* dst = reinterpret_cast<uint4*>(p.o + ((size_t)(bp.row + pp * C + r) * p.H + h) * V + yc + piece * 16);
       const uint4 x = *reinterpret_cast<const uint4*>(rowp + (((2 * piece) ^ r) & 15) * 16);
       const uint4 y = *reinterpret_cast<const uint4*>(rowp + (((2 * piece + 1) ^ r) & 15) * 16);
-      __stcs(dst, x);
-      __stcs(dst + 1, y);
+      if (GEN && r >= chunk_len(pp)) return;
+      if (!GEN || yc + piece * 16 < V) __stcs(dst, x);
+      if (!GEN || yc + piece * 16 + 8 < V) __stcs(dst + 1, y);
     };
     bool ok = true;
     for (int pp = 0; ok && pp < NT; ++pp) {
@@ -821,9 +1021,15 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       uint8_t* ht = hst + (pp & 1) * TILE128;
       if (!mbar_wait(&sh.fullin[pp & 1], (pp >> 1) & 1) || (!SCALAR && !mbar_wait(&sh.ebar, ph))) { *abort_flag = 1; fail(9); }
       tc_fence_after();
+      const int len = chunk_len(pp);
       WarpGates wg;
       if (SCALAR) {
-        wg = warp_cumulate(__bfloat162float(greg_lo), __bfloat162float(greg_hi), lane);
+        float g_lo = __bfloat162float(greg_lo), g_hi = __bfloat162float(greg_hi);
+        if (GEN) {
+          g_lo = lane < len ? (p.gscalar ? g_lo : gconst) : 0.f;
+          g_hi = lane + 32 < len ? (p.gscalar ? g_hi : gconst) : 0.f;
+        }
+        wg = warp_cumulate(g_lo, g_hi, lane);
       }
       // per-channel factors of this thread's state row
       float decay, c2;
@@ -848,7 +1054,17 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
                          pack_bf16(S[j + 4] * hscale, S[j + 5] * hscale), pack_bf16(S[j + 6] * hscale, S[j + 7] * hscale));
       }
       // gate q, k: thread (q4, lane, seg) owns time row (32 q4 + lane) mod 64 and 16 channels
-      if (SCALAR) {
+      if (GEN && ((q4 * 32 + lane) & 63) >= len) {   // a short chunk's foreign rows of q, k, v become zero
+        const int i = (q4 * 32 + lane) & 63, cg = (q4 >> 1) * 4 + seg;
+        const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
+          *reinterpret_cast<uint4*>(qs + off) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(ks + off) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(gs + TILE64 + off) = make_uint4(0u, 0u, 0u, 0u);   // v
+        }
+      } else if (SCALAR) {
         const int i = (q4 * 32 + lane) & 63;
         const int cg = (q4 >> 1) * 4 + seg;
         const float E = ((q4 & 1) ? wg.hi : wg.lo) - wg.mid();
@@ -921,18 +1137,14 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
     }
     __syncthreads();   // the outputs of the last chunk are staged
     if (ok) copy_out(NT - 1);
-    if (ok && p.s_final) {
-      float* dst = p.s_final + ((size_t)blk * D + col) * D + seg * 32;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
-    }
+    if (ok && p.s_final && bp.cnt == 1) store_state32(p.s_final + bp.seqh * K * V, S, col, yc + seg * 32, K, V);
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && sh.abort_flag) {
-    poison(p.o + ((size_t)(b * p.T + c0 * C) * p.H + h) * D);
-    if (p.s_final) poison(p.s_final + (size_t)blk * D * D);
+    poison(p.o + ((size_t)bp.row * p.H + h) * V + yc);
+    if (p.s_final && bp.cnt == 1) poison(p.s_final + bp.seqh * K * V + yc);
   }
 }
 
@@ -948,6 +1160,12 @@ struct BwdParams {
   const __nv_bfloat16* gscalar;   // scalar gates [B,T,H] (SCALAR kernels; mg is unused then)
   int T, H, NT, total;   // total = B * H * NT chunks
   float scale;
+  const float* gamma;    // constant gates [H] (SCALAR GEN kernels)
+  Geo geo;               // GEN kernels
+  // GEN, V > 128: one launch per value slice.  dq, dk and dg are sums over the slices: every launch but the last
+  // writes fp32 partial sums, every launch but the first adds the partial sums of the one before.
+  int vs;
+  const float *add_dq, *add_dk, *add_dg;   // null: nothing to add
 };
 
 // Warp roles: warps 0-15 gate q and k of the next chunk and write the gradients of a chunk out of
@@ -965,7 +1183,7 @@ constexpr int BWD_EPI_THREADS = 512, BWD_GATE_THREADS = 128;
 // issued: every write-out warp cumulates the 64 gates of a chunk in registers (warp_cumulate) and hands the
 // factors exp(+-(G - mid)) of the time steps around by shuffles.  dg is summed over the key channels inside
 // the kernel and written as fp32 [B,T,H] (the scalar gate's gradient is the sum of the channels').
-template <typename TG, typename TD, bool SCALAR>
+template <typename TG, typename TD, bool SCALAR, bool GEN>
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_constant__ BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -994,14 +1212,32 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   constexpr uint32_t cEm = 0, cA = 0, cdA = 64, cET = 128, cdq = 256, cdk1 = 320, cdk2 = 384, cdv = 448;
   const int nit = (p.total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
-  auto chunk_rows = [&](int it, int& h, int& row, int& hrow) {
+  const int K = GEN ? p.geo.K : D, V = GEN ? p.geo.V : D;
+  const int yc = GEN ? p.vs * D : 0;   // first value channel of this launch's slice
+  // returns how many of the chunk's rows are the sequence's own
+  auto chunk_rows = [&](int it, int& h, int& row, int& hrow) -> int {
     // heads vary fastest over the chunks in flight: together the blocks read and write whole
     // token rows of the [B,T,H,D] activations
     const int cid = blockIdx.x + it * gridDim.x;
-    const int ci = (cid / p.H) % p.NT, b = cid / (p.H * p.NT);
     h = cid % p.H;
-    row = b * p.T + ci * C;
-    hrow = ((b * p.NT + ci) * p.H + h) * D;
+    if constexpr (GEN) {
+      const int slot = cid / p.H;
+      hrow = (cid * p.geo.VS + p.vs) * D;
+      int end;
+      if (p.geo.chunks) {
+        const ChunkEntry e = p.geo.chunks[slot];
+        row = e.row; end = e.end;
+      } else {
+        const int b = slot / p.NT;
+        row = b * p.T + (slot - b * p.NT) * C; end = (b + 1) * p.T;
+      }
+      return min(C, end - row);
+    } else {
+      const int ci = (cid / p.H) % p.NT, b = cid / (p.H * p.NT);
+      row = b * p.T + ci * C;
+      hrow = ((b * p.NT + ci) * p.H + h) * D;
+      return C;
+    }
   };
   // bounded wait that also gives up when another role has failed
   auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
@@ -1039,7 +1275,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     const int q4 = warp & 3, seg = warp >> 2, col = q4 * 32 + lane;
     const uint32_t lane_base = q4 * 32;
     const ColAddr ca = col_prep(64, col);
-    const size_t ostride = (size_t)p.H * D;
+    const size_t ostride = (size_t)p.H * K, vstride = (size_t)p.H * V;
+    const bool has_k = !GEN || col < K, has_v = !GEN || yc + col < V;
     TG* const dq_out = reinterpret_cast<TG*>(p.dq);
     TG* const dk_out = reinterpret_cast<TG*>(p.dk);
     TD* const dg_out = reinterpret_cast<TD*>(p.dg);
@@ -1050,12 +1287,18 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     // (in registers, loaded a chunk ahead: see the note in k_fwd_fused)
     __nv_bfloat16 greg_lo = __float2bfloat16(0.f), greg_hi = greg_lo;
     float fw_next = 1.f, rw_next = 1.f;
+    float gconst = 0.f;
+    int glen = C;
     auto load_gates = [&](int it) {
       int h, row, hrow;
-      chunk_rows(it, h, row, hrow);
+      glen = chunk_rows(it, h, row, hrow);
+      if (GEN && !p.gscalar) {
+        gconst = p.gamma ? p.gamma[h] : 0.f;
+        return;
+      }
       const __nv_bfloat16* src = p.gscalar + (size_t)(row + lane) * p.H + h;
-      greg_lo = src[0];
-      greg_hi = src[(size_t)32 * p.H];
+      if (!GEN || lane < glen) greg_lo = src[0];
+      if (!GEN || lane + 32 < glen) greg_hi = src[(size_t)32 * p.H];
     };
     if (SCALAR && nit > 0) load_gates(0);
     auto gate_chunk = [&](int it) -> bool {
@@ -1066,8 +1309,18 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       tc_fence_after();
       const int i = (q4 * 32 + lane) & 63;
       const int cg = (q4 >> 1) * 4 + seg;
+      bool mine = true;   // GEN: a short chunk's foreign rows become zero
+      if (GEN) {
+        int h_, row_, hrow_;
+        mine = i < chunk_rows(it, h_, row_, hrow_);
+      }
       if (SCALAR) {
-        const WarpGates w = warp_cumulate(__bfloat162float(greg_lo), __bfloat162float(greg_hi), lane);
+        float g_lo = __bfloat162float(greg_lo), g_hi = __bfloat162float(greg_hi);
+        if (GEN) {
+          g_lo = lane < glen ? (p.gscalar ? g_lo : gconst) : 0.f;
+          g_hi = lane + 32 < glen ? (p.gscalar ? g_hi : gconst) : 0.f;
+        }
+        const WarpGates w = warp_cumulate(g_lo, g_hi, lane);
         const float mid = w.mid();
         const float f_lo = fast_exp(w.lo - mid), r_lo = fast_exp(mid - w.lo);
         const float f_hi = fast_exp(w.hi - mid), r_hi = fast_exp(mid - w.hi);
@@ -1078,8 +1331,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-          *reinterpret_cast<uint4*>(qs + off) = scale8_by(*reinterpret_cast<const uint4*>(qs + off), f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8_by(*reinterpret_cast<const uint4*>(ks + off), r);
+          *reinterpret_cast<uint4*>(qs + off) =
+              mine ? scale8_by(*reinterpret_cast<const uint4*>(qs + off), f) : make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(ks + off) =
+              mine ? scale8_by(*reinterpret_cast<const uint4*>(ks + off), r) : make_uint4(0u, 0u, 0u, 0u);
         }
         fence_async_smem();
         tc_fence_before();
@@ -1098,8 +1353,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           f[t] = fast_exp(em[8 * u + t]);
           r[t] = fast_exp(-em[8 * u + t]);
         }
-        *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), f);
-        *reinterpret_cast<uint4*>(ks + off) = scale8(*reinterpret_cast<const uint4*>(ks + off), r);
+        *reinterpret_cast<uint4*>(qs + off) =
+            mine ? scale8(*reinterpret_cast<const uint4*>(qs + off), f) : make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(ks + off) =
+            mine ? scale8(*reinterpret_cast<const uint4*>(ks + off), r) : make_uint4(0u, 0u, 0u, 0u);
       }
       fence_async_smem();
       tc_fence_before();
@@ -1111,7 +1368,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     for (int it = 0; live && it < nit; ++it) {
       const int sl = it & 1;
       int h, row, hrow;
-      chunk_rows(it, h, row, hrow);
+      const int len = chunk_rows(it, h, row, hrow);
       const float fw = fw_next, rw = rw_next;   // (SCALAR) of this chunk
       // the next chunk's gating runs while the tensor core works on this chunk's gradient products
       if (it + 1 < nit && !gate_chunk(it + 1)) break;
@@ -1122,7 +1379,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       tc_fence_after();
       const uint8_t* qt = qs + sl * TILE64;
       const uint8_t* kt = ks + sl * TILE64;
-      const size_t obase = ((size_t)(row + seg * SEG) * p.H + h) * D + col;
+      const size_t obase = ((size_t)(row + seg * SEG) * p.H + h) * K + col;
+      const size_t vbase = ((size_t)(row + seg * SEG) * p.H + h) * V + yc + col;
       const size_t obase4 = obase - (lane & 3) + (size_t)(lane & 3) * ostride;   // channel group, own time row
       float dgl[SEG];
       float run = 0.f, tail = 0.f;
@@ -1149,9 +1407,20 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           run += qv * dqs - kv * dks;                     // q dq - k dk
           tail = fmaf(dki, kv, tail);                     // dk_inter k
           dgl[t] = run;
-          st_out(p.dv, obase + t * ostride, dv[u]);
-          st_out(dq_out, obase + t * ostride, e * dqs);
-          st_out(dk_out, obase + t * ostride, r * dks);
+          if constexpr (GEN) {
+            if (seg * SEG + t < len) {
+              if (has_v) st_out(p.dv, vbase + t * vstride, dv[u]);
+              if (has_k) {
+                const size_t o = obase + t * ostride;
+                st_out(dq_out, o, p.add_dq ? fmaf(e, dqs, p.add_dq[o]) : e * dqs);
+                st_out(dk_out, o, p.add_dk ? fmaf(r, dks, p.add_dk[o]) : r * dks);
+              }
+            }
+          } else {
+            st_out(p.dv, vbase + t * vstride, dv[u]);
+            st_out(dq_out, obase + t * ostride, e * dqs);
+            st_out(dk_out, obase + t * ostride, r * dks);
+          }
         }
       }
       sufsum[sl][seg][col] = run;
@@ -1173,7 +1442,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         if (lane < SEG) atomicAdd(&dgk_s[sl][seg * SEG + lane], mine);
         asm volatile("bar.sync 1, %0;" ::"n"(BWD_EPI_THREADS) : "memory");
         if (tid < C) {
-          if (p.dg) reinterpret_cast<float*>(p.dg)[(size_t)(row + tid) * p.H + h] = dgk_s[sl][tid];
+          if (p.dg && (!GEN || tid < len)) {
+            const size_t o = (size_t)(row + tid) * p.H + h;
+            reinterpret_cast<float*>(p.dg)[o] = dgk_s[sl][tid] + ((GEN && p.add_dg) ? p.add_dg[o] : 0.f);
+          }
           dgk_s[sl][tid] = 0.f;   // (this slot is used again two chunks on, two barriers later)
         }
       } else if (p.dg) {
@@ -1182,7 +1454,18 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
 #pragma unroll
         for (int t = 0; t < SEG; t += 4) {
           float w[4] = {dgl[t] + cst, dgl[t + 1] + cst, dgl[t + 2] + cst, dgl[t + 3] + cst};
-          st_transposed4(dg_out, obase4 + t * ostride, w, lane);
+          if constexpr (GEN) {
+            // (every lane takes part in the exchange; K is a multiple of 8, so a group of four is inside or outside)
+            const bool in = has_k && seg * SEG + t + (lane & 3) < len;
+            if (p.add_dg) {
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (has_k && seg * SEG + t + u < len) w[u] += p.add_dg[obase + (t + u) * ostride];
+            }
+            st_transposed4(dg_out, obase4 + t * ostride, w, lane, in);
+          } else {
+            st_transposed4(dg_out, obase4 + t * ostride, w, lane);
+          }
         }
       }
     }
@@ -1230,10 +1513,25 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     }
   } else if (warp == 20) {
     // ------------------------------------------------------------------ tensor-core issue
-    if (lane == 0) {
+    // GEN: the whole warp walks the chunks, because a short chunk's foreign rows of g, v, do are zeroed here before
+    // a product reads them; products are issued by one thread
+    if (GEN || lane == 0) {
       const uint32_t ga = smem_u32(gs), mma = smem_u32(mtm), va = smem_u32(vs), doa = smem_u32(dos), ha = smem_u32(hs),
                      dha = smem_u32(dhs), pa = smem_u32(Ps), daa = smem_u32(dAs);
+      auto zero_foreign = [&](int it, uint8_t* t0, uint8_t* t1) {
+        int h_, row_, hrow_;
+        const int len = chunk_rows(it, h_, row_, hrow_);
+        if (len == C) return;
+        zero_rows(t0, len, lane, 32);
+        if (t1) zero_rows(t1, len, lane, 32);
+        fence_async_smem();
+        __syncwarp();
+      };
       auto issue_gate = [&](int it) {
+        if (GEN) {
+          zero_foreign(it, gs, nullptr);
+          if (lane != 0) return;
+        }
 #pragma unroll
         for (int j0 = 0; j0 < C; j0 += 16)   // G - mid, [time (repeated)][channel]
           umma_bf16(tm + cEm, desc_kmajor(mma, 128, 0, j0), desc_mnmajor(ga, 64, j0, 0), umma_idesc(128, 128, 0, 1), j0 > 0);
@@ -1244,12 +1542,17 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         umma_commit(&bar_gate);
       };
       auto issue_A = [&](int it) {
+        if (GEN && lane != 0) return;
         const uint32_t qta = smem_u32(qs + (it & 1) * TILE64), kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // A[i][j] = q~ k~^T
           umma_bf16(tm + cA, desc_kmajor(qta, 64, 0, k0), desc_kmajor(kta, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
       };
-      auto issue_dA = [&]() {
+      auto issue_dA = [&](int it) {
+        if (GEN) {
+          zero_foreign(it, vs, dos);
+          if (lane != 0) return;
+        }
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // dA[i][j] = do v^T
           umma_bf16(tm + cdA, desc_kmajor(doa, 64, 0, k0), desc_kmajor(va, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
@@ -1259,6 +1562,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       // the chunk's tiles have landed, while the conversion warps still work on A and dA; after it dh'
       // and v are dead and the next chunk's are fetched.  The second group needs the converted operands.
       auto issue_inter = [&](int it) {
+        if (GEN && lane != 0) return;
         const uint32_t kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // dq_inter^T[k][i] = h' do^T
@@ -1272,6 +1576,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         umma_commit(&bar_r2);
       };
       auto issue_intra = [&](int it) {
+        if (GEN && lane != 0) return;
         const uint32_t qta = smem_u32(qs + (it & 1) * TILE64), kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 16)   // dv^T[v][j] += sum_i do[i][v] A[i][j]
@@ -1285,38 +1590,44 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           umma_bf16(tm + cdk1, desc_mnmajor(qta, 64, k0, 0), desc_mnmajor(daa, 64, k0, 0), umma_idesc(128, 64, 1, 1), k0 > 0);
         umma_commit(&bar_main);
       };
-      bool ok = SCALAR || wait(&full_g, 0, 6);
+      // (GEN: all lanes take the same path, also when a wait gives up)
+      auto waitw = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+        const bool r = wait(bar, parity, code);
+        return GEN ? (bool)__all_sync(0xffffffffu, r) : r;
+      };
+      bool ok = SCALAR || waitw(&full_g, 0, 6);
       if (ok) {
         tc_fence_after();
         if (!SCALAR) issue_gate(0);
-        ok = wait(&gated, 0, 12);
+        ok = waitw(&gated, 0, 12);
       }
       if (ok) {
         tc_fence_after();
         issue_A(0);
-        ok = wait(&full_hdo, 0, 6) && wait(&full_dhv, 0, 6);
+        ok = waitw(&full_hdo, 0, 6) && waitw(&full_dhv, 0, 6);
       }
-      if (ok) issue_dA();
+      if (ok) issue_dA(0);
       for (int it = 0; ok && it < nit; ++it) {
         // A and dA of this chunk are issued; the previous chunk has left tensor memory
-        if (it >= 1 && !wait(&e_done[(it - 1) & 1], ((it - 1) >> 1) & 1, 14)) break;
+        if (it >= 1 && !waitw(&e_done[(it - 1) & 1], ((it - 1) >> 1) & 1, 14)) break;
         tc_fence_after();
         issue_inter(it);
-        if (!wait(&conv_done, it & 1, 13)) break;   // A and dA of this chunk are in shared memory
+        if (!waitw(&conv_done, it & 1, 13)) break;   // A and dA of this chunk are in shared memory
         tc_fence_after();
         const bool more = it + 1 < nit;
         if (more && !SCALAR) {   // the next chunk's exponents take the place of A and dA in tensor memory
-          if (!wait(&full_g, (it + 1) & 1, 6)) break;
+          if (!waitw(&full_g, (it + 1) & 1, 6)) break;
           issue_gate(it + 1);
         }
         issue_intra(it);
         if (more) {
-          if (!wait(&gated, (it + 1) & 1, 12)) break;
+          if (!waitw(&gated, (it + 1) & 1, 12)) break;
           tc_fence_after();
           issue_A(it + 1);
-          if (!wait(&full_hdo, (it + 1) & 1, 6) || !wait(&full_dhv, (it + 1) & 1, 6)) break;
-          issue_dA();
+          if (!waitw(&full_hdo, (it + 1) & 1, 6) || !waitw(&full_dhv, (it + 1) & 1, 6)) break;
+          issue_dA(it + 1);
         }
+        if (GEN) __syncwarp();
       }
     }
   } else {
@@ -1342,14 +1653,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         int h, row, hrow;
         chunk_rows(it, h, row, hrow);
         mbar_expect_tx(&full_hdo, TILE128 + TILE64);
-        tma_load_3d(dos, &p.mdo, &full_hdo, 0, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &full_hdo, 64, h, row);
+        tma_load_3d(dos, &p.mdo, &full_hdo, yc, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &full_hdo, yc + 64, h, row);
         tma_load_2d(hs, &p.mh, &full_hdo, 0, hrow); tma_load_2d(hs + TILE128 / 2, &p.mh, &full_hdo, 64, hrow);
       };
       auto load_dhv = [&](int it) {
         int h, row, hrow;
         chunk_rows(it, h, row, hrow);
         mbar_expect_tx(&full_dhv, TILE128 + TILE64);
-        tma_load_3d(vs, &p.mv, &full_dhv, 0, h, row); tma_load_3d(vs + SLAB64, &p.mv, &full_dhv, 64, h, row);
+        tma_load_3d(vs, &p.mv, &full_dhv, yc, h, row); tma_load_3d(vs + SLAB64, &p.mv, &full_dhv, yc + 64, h, row);
         tma_load_2d(dhs, &p.mdh, &full_dhv, 0, hrow); tma_load_2d(dhs + TILE128 / 2, &p.mdh, &full_dhv, 64, hrow);
       };
       if (!SCALAR) load_g(0);
@@ -1388,8 +1699,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   if (tid == 0 && abort_flag && nit > 0) {
     int h, row, hrow;
     chunk_rows(0, h, row, hrow);
-    poison(reinterpret_cast<TG*>(p.dq) + ((size_t)row * p.H + h) * D);
-    poison(p.dv + ((size_t)row * p.H + h) * D);
+    poison(reinterpret_cast<TG*>(p.dq) + ((size_t)row * p.H + h) * K);
+    poison(p.dv + ((size_t)row * p.H + h) * V + yc);
   }
 }
 
@@ -1432,12 +1743,12 @@ int run_scan(bool bwd, const tops_chunk_problem& pb, int nseg, const void* x, co
   const bool sum = !states && !s0;
   if (bwd) {
     const char* label = states ? "sm100_bwd_dh" : "sm100_bwd_dh_summary";
-    if (sum) return scalar ? launch(k_scan<true, true, true>, label) : launch(k_scan<true, false, true>, label);
-    return scalar ? launch(k_scan<true, true, false>, label) : launch(k_scan<true, false, false>, label);
+    if (sum) return scalar ? launch(k_scan<true, true, true, false>, label) : launch(k_scan<true, false, true, false>, label);
+    return scalar ? launch(k_scan<true, true, false, false>, label) : launch(k_scan<true, false, false, false>, label);
   }
   const char* label = states ? "sm100_fwd_h" : "sm100_fwd_h_summary";
-  if (sum) return scalar ? launch(k_scan<false, true, true>, label) : launch(k_scan<false, false, true>, label);
-  return scalar ? launch(k_scan<false, true, false>, label) : launch(k_scan<false, false, false>, label);
+  if (sum) return scalar ? launch(k_scan<false, true, true, false>, label) : launch(k_scan<false, false, true, false>, label);
+  return scalar ? launch(k_scan<false, true, false, false>, label) : launch(k_scan<false, false, false, false>, label);
 }
 
 // Time segments per sequence.  The scans walk a sequence chunk by chunk with one block; when there are
@@ -1484,7 +1795,7 @@ int segment_starts(bool bwd, const tops_chunk_problem& pb, int nseg, const void*
 bool supported(const tops_chunk_problem& pb) {
   if (pb.dtype != TOPS_BF16 || pb.gate_dtype != TOPS_BF16) return false;
   if (pb.gate_kind != TOPS_GATE_PER_CHANNEL && pb.gate_kind != TOPS_GATE_SCALAR) return false;
-  if (pb.K != D || pb.V != D || pb.chunk != C || pb.T % C != 0 || pb.cu_seqlens) return false;
+  if (pb.K != D || pb.V != D || pb.chunk != C || pb.T % C != 0 || pb.cu_seqlens || pb.cu_seqlens_host) return false;
   if (!(pb.scale > 0.f) || !(pb.scale < 1e30f)) return false;   // states are stored multiplied by scale
   if ((size_t)pb.B * pb.T >= (1u << 31)) return false;
   return device_is_sm100() && encode_fn() != nullptr;
@@ -1545,10 +1856,10 @@ int chunk_fwd(const tops_chunk_fwd_params& p, void* ws, size_t, cudaStream_t st)
     }
     up.s0 = start; up.s_final = last; up.o = reinterpret_cast<__nv_bfloat16*>(p.o);
     up.T = pb.T; up.H = pb.H; up.NT = NT / nseg; up.nseg = nseg; up.scale = pb.scale;
-    if ((rc = opt_in_smem(k_fwd_fused<true>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false>, FUSED_SMEM))) return rc;
+    if ((rc = opt_in_smem(k_fwd_fused<true, false>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false, false>, FUSED_SMEM))) return rc;
     KernelScope ks("sm100_fwd_fused", st);
-    if (scalar) k_fwd_fused<true><<<pb.B * pb.H * nseg, FUSED_THREADS, FUSED_SMEM, st>>>(up);
-    else k_fwd_fused<false><<<pb.B * pb.H * nseg, FUSED_THREADS, FUSED_SMEM, st>>>(up);
+    if (scalar) k_fwd_fused<true, false><<<pb.B * pb.H * nseg, FUSED_THREADS, FUSED_SMEM, st>>>(up);
+    else k_fwd_fused<false, false><<<pb.B * pb.H * nseg, FUSED_THREADS, FUSED_SMEM, st>>>(up);
     return post_launch();
   }
   rc = run_scan(false, pb, nseg, p.k, p.g, p.v, start, h, last, nullptr, st);
@@ -1560,10 +1871,10 @@ int chunk_fwd(const tops_chunk_fwd_params& p, void* ws, size_t, cudaStream_t st)
   if (!scalar && (rc = act_map(&fp.mg, p.g, BT, pb.H))) return rc;
   fp.gscalar = reinterpret_cast<const __nv_bfloat16*>(p.g);
   fp.o = reinterpret_cast<__nv_bfloat16*>(p.o); fp.T = pb.T; fp.H = pb.H; fp.NT = NT; fp.scale = pb.scale;
-  if ((rc = opt_in_smem(k_fwd_o<true>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false>, FWD_O_SMEM))) return rc;
+  if ((rc = opt_in_smem(k_fwd_o<true, false>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false, false>, FWD_O_SMEM))) return rc;
   KernelScope ks("sm100_fwd_o", st);
-  if (scalar) k_fwd_o<true><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
-  else k_fwd_o<false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
+  if (scalar) k_fwd_o<true, false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
+  else k_fwd_o<false, false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
   return post_launch();
 }
 
@@ -1572,19 +1883,19 @@ size_t bwd_workspace_bytes(const tops_chunk_bwd_params& p) {
 }
 
 bool bwd_dtypes_ok(const tops_chunk_bwd_params& p) {
-  if (p.pb.gate_kind == TOPS_GATE_SCALAR)   // dg is the scalar gate's gradient, fp32 [B,T,H]
+  if (p.pb.gate_kind != TOPS_GATE_PER_CHANNEL)   // dg is the scalar gate's gradient, fp32 [B,T,H]
     return (p.grad_dtype == TOPS_F32 || p.grad_dtype == TOPS_BF16) && p.dg_dtype == TOPS_F32;
   return (p.grad_dtype == TOPS_F32 && p.dg_dtype == TOPS_F32) ||
          (p.grad_dtype == TOPS_BF16 && (p.dg_dtype == TOPS_F32 || p.dg_dtype == TOPS_BF16));
 }
 
-template <typename TG, typename TD, bool SCALAR = false>
+template <typename TG, typename TD, bool SCALAR = false, bool GEN = false>
 int launch_bwd_main(const BwdParams& bp, cudaStream_t st) {
-  int rc = opt_in_smem(k_bwd_main<TG, TD, SCALAR>, BWD_SMEM);
+  int rc = opt_in_smem(k_bwd_main<TG, TD, SCALAR, GEN>, BWD_SMEM);
   if (rc) return rc;
   const int grid = bp.total < sm_count() ? bp.total : sm_count();
   KernelScope ks("sm100_bwd_main", st);
-  k_bwd_main<TG, TD, SCALAR><<<grid, BWD_THREADS, BWD_SMEM, st>>>(bp);
+  k_bwd_main<TG, TD, SCALAR, GEN><<<grid, BWD_THREADS, BWD_SMEM, st>>>(bp);
   return post_launch();
 }
 
@@ -1642,6 +1953,346 @@ int chunk_bwd(const tops_chunk_bwd_params& p, void* ws, size_t, cudaStream_t st)
   if (p.grad_dtype == TOPS_F32) return launch_bwd_main<float, float>(bp, st);
   if (p.dg_dtype == TOPS_F32) return launch_bwd_main<__nv_bfloat16, float>(bp, st);
   return launch_bwd_main<__nv_bfloat16, __nv_bfloat16>(bp, st);
+}
+
+// ---------------------------------------------------------------------------
+// the general form: packed batches, any T, K <= 128, V in slices of 128, constant or no gate
+// ---------------------------------------------------------------------------
+namespace {
+
+// Time of a pass over runs of at most `cps` chunks, in chunks of the fused forward, with one block per SM: when
+// there are more blocks than SMs they follow one another, longest first, and the last ones to finish leave about
+// half a run of imbalance.
+struct RunCost { long long chunks = 0; int blocks = 0, longest = 0; };
+double pass_time(const RunCost& r, int sms) {
+  if (r.blocks <= sms) return r.longest;
+  const double even = (double)r.chunks / sms;
+  return r.longest > even + 0.5 * r.longest ? r.longest : even + 0.5 * r.longest;
+}
+
+// Everything the launches of one call need to know about where chunks live.
+struct GenPlan {
+  Geo geo{};
+  int N = 0, HV = 0, total_chunks = 0, runs = 0;
+  bool cut = false;             // some sequence is walked as several runs
+  std::vector<int> nch;         // packed: chunks per sequence
+  int cps = 0;
+
+  explicit GenPlan(const tops_chunk_problem& pb) {
+    geo.K = pb.K; geo.V = pb.V; geo.VS = cdiv(pb.V, D);
+    HV = pb.H * geo.VS;
+    int longest = 0;
+    if (pb.cu_seqlens_host) {
+      N = pb.N;
+      nch.resize(N);
+      for (int n = 0; n < N; ++n) {
+        nch[n] = cdiv(pb.cu_seqlens_host[n + 1] - pb.cu_seqlens_host[n], C);
+        total_chunks += nch[n];
+        longest = nch[n] > longest ? nch[n] : longest;
+      }
+    } else {
+      N = pb.B;
+      longest = geo.NTseq = cdiv(pb.T, C);
+      total_chunks = N * longest;
+    }
+    // Cutting sequences into runs costs a summary pass (about 0.45 of the main pass per chunk) and a join (about
+    // two chunks' time); it pays when whole sequences would leave SMs idle.  Every candidate length is priced.
+    const int sms = sm_count();
+    cps = longest;
+    double best = 1e30;
+    for (int c = longest; c >= 4; c = c > 64 ? c * 3 / 4 : c - (c > 16 ? 2 : 1)) {
+      RunCost all, sum;
+      for (int n = 0; n < (nch.empty() ? 1 : N); ++n) {
+        const int k = nch.empty() ? longest : nch[n], cnt = cdiv(k, c), mult = (nch.empty() ? N : 1) * HV;
+        const int len = cdiv(k, cnt);
+        all.chunks += (long long)k * mult; all.blocks += cnt * mult;
+        if (len > all.longest) all.longest = len;
+        if (cnt > 1) {
+          sum.chunks += (long long)k * mult; sum.blocks += cnt * mult;
+          if (len > sum.longest) sum.longest = len;
+        }
+      }
+      const double t = pass_time(all, sms) + (sum.blocks ? 0.45 * pass_time(sum, sms) + 2.0 : 0.0);
+      if (t < best - 1e-9) { best = t; cps = c; }
+    }
+    if (nch.empty()) {
+      geo.nseg = cdiv(longest, cps);
+      geo.cps = cdiv(longest, geo.nseg);
+      geo.nseg = cdiv(longest, geo.cps);
+      runs = N * geo.nseg;
+      cut = geo.nseg > 1;
+    } else {
+      geo.nseg = 1; geo.cps = longest;
+      for (int n = 0; n < N; ++n) { const int c = count(n); runs += c; cut = cut || c > 1; }
+    }
+  }
+  // runs of sequence n (packed): as even as whole chunks allow, none empty
+  int run_len(int n) const { return cdiv(nch[n], cdiv(nch[n], cps)); }
+  int count(int n) const { return cdiv(nch[n], run_len(n)); }
+  int blocks() const { return runs * HV; }
+  // (the chunk-parallel output kernel numbers chunks in a 16-bit grid dimension)
+  bool fused() const { return blocks() >= kFusedMinBlocks || total_chunks > 65535; }
+  size_t words() const { return nch.empty() ? 0 : 3 * (size_t)N + (size_t)align_up(N + 1, 4) + (3 * (size_t)N % 4 ? 4 - 3 * (size_t)N % 4 : 0) + 8 * (size_t)runs; }
+  size_t table_bytes() const { return nch.empty() ? 0 : align_up(words() * 4) + align_up((size_t)total_chunks * sizeof(ChunkEntry)); }
+  size_t state_bytes() const { return align_up((size_t)total_chunks * HV * D * D * 2); }
+  size_t seg_state() const { return (size_t)runs * (HV / geo.VS) * geo.K * geo.V; }
+  // end states, entry states, summed gates of the runs
+  size_t seg_bytes() const { return cut ? align_up((2 * seg_state() + (size_t)runs * (HV / geo.VS) * D) * sizeof(float)) : 0; }
+
+  const int* seg0 = nullptr;   // device: first run of every sequence
+  // writes the tables into `ws` (table_bytes() of it)
+  int upload(const tops_chunk_problem& pb, void* ws, cudaStream_t st) {
+    if (nch.empty()) return TOPS_OK;
+    int* dst = reinterpret_cast<int*>(ws);
+    ChunkEntry* chunks = reinterpret_cast<ChunkEntry*>(reinterpret_cast<char*>(ws) + align_up(words() * 4));
+    std::vector<int> w(words(), 0);
+    const size_t seg0_at = align_up(3 * (size_t)N, 4), seg_at = seg0_at + align_up(N + 1, 4);
+    std::vector<SegEntry> e;
+    e.reserve(runs);
+    int slot = 0, id = 0;
+    for (int n = 0; n < N; ++n) {
+      const int row = pb.cu_seqlens_host[n], end = pb.cu_seqlens_host[n + 1], len = run_len(n), cnt = count(n);
+      w[3 * n] = row; w[3 * n + 1] = end; w[3 * n + 2] = slot;
+      w[seg0_at + n] = id;
+      for (int i = 0; i < cnt; ++i, ++id) {
+        const int c0 = i * len;
+        e.push_back(SegEntry{row + c0 * C, end, slot + c0, nch[n] - c0 < len ? nch[n] - c0 : len, id, n, cnt, 0});
+      }
+      slot += nch[n];
+    }
+    w[seg0_at + N] = id;
+    std::stable_sort(e.begin(), e.end(), [](const SegEntry& a, const SegEntry& b) { return a.nch > b.nch; });
+    memcpy(w.data() + seg_at, e.data(), e.size() * sizeof(SegEntry));
+    geo.segs = reinterpret_cast<const SegEntry*>(dst + seg_at);
+    geo.chunks = chunks;
+    seg0 = dst + seg0_at;
+    KernelScope ks("sm100_plan", st);
+    if (w.size() <= kPlanSmall) {
+      PlanWords<kPlanSmall> pw;
+      memcpy(pw.w, w.data(), w.size() * 4);
+      k_plan<kPlanSmall><<<N < 64 ? N : 64, 128, 0, st>>>(pw, dst, (int)w.size(), N, chunks);
+      return post_launch();
+    }
+    static_assert(sizeof(PlanWords<kPlanLarge>) + 64 <= 32764, "kernel parameter space");
+    for (size_t at = 0; at < w.size(); at += kPlanLarge) {
+      PlanWords<kPlanLarge> pw;
+      const size_t n = w.size() - at < kPlanLarge ? w.size() - at : kPlanLarge;
+      memcpy(pw.w, w.data() + at, n * 4);
+      k_plan<kPlanLarge><<<32, 128, 0, st>>>(pw, dst + at, (int)n, 0, chunks);
+      const int rc = post_launch();
+      if (rc) return rc;
+    }
+    k_plan_chunks<<<N < 512 ? N : 512, 128, 0, st>>>(dst, N, chunks);
+    return post_launch();
+  }
+};
+struct GenSegs {
+  float *ends, *starts, *gsum;
+  GenSegs(void* base, const GenPlan& g) {
+    ends = reinterpret_cast<float*>(base); starts = ends + g.seg_state(); gsum = starts + g.seg_state();
+  }
+};
+bool scalar_kind(int kind) { return kind != TOPS_GATE_PER_CHANNEL; }
+
+int run_scan_gen(bool bwd, bool sum, const tops_chunk_problem& pb, const GenPlan& g, const void* x, const void* gate, const void* y,
+                 const float* s0, const float* s0_seg, void* states, float* s_final, float* gsum, cudaStream_t st) {
+  ScanParams sp;
+  const int BT = pb.B * pb.T;
+  const bool scalar = scalar_kind(pb.gate_kind);
+  int rc;
+  if ((rc = act_map(&sp.mx, x, BT, pb.H, pb.K)) || (rc = act_map(&sp.my, y, BT, pb.H, pb.V))) return rc;
+  if (!scalar && (rc = act_map(&sp.mg, gate, BT, pb.H, pb.K))) return rc;
+  sp.gscalar = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(gate) : nullptr;
+  sp.gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(gate) : nullptr;
+  if (states && (rc = state_map(&sp.mst, states, (size_t)g.total_chunks * g.HV * D))) return rc;
+  sp.s0 = s0; sp.s0_seg = s0_seg; sp.states = reinterpret_cast<__nv_bfloat16*>(states); sp.s_final = s_final; sp.gsum = gsum;
+  sp.T = pb.T; sp.H = pb.H; sp.NT = 0; sp.nseg = 1; sp.scale = pb.scale; sp.geo = g.geo; sp.skip_xy = -1;
+  auto launch = [&](auto kernel, const char* label) {
+    if ((rc = opt_in_smem(kernel, SCAN_SMEM))) return rc;
+    KernelScope ks(label, st);
+    kernel<<<g.blocks(), SCAN_THREADS, SCAN_SMEM, st>>>(sp);
+    return post_launch();
+  };
+  if (bwd) {
+    const char* label = sum ? "sm100_bwd_dh_summary" : "sm100_bwd_dh";
+    if (sum) return scalar ? launch(k_scan<true, true, true, true>, label) : launch(k_scan<true, false, true, true>, label);
+    return scalar ? launch(k_scan<true, true, false, true>, label) : launch(k_scan<true, false, false, true>, label);
+  }
+  const char* label = sum ? "sm100_fwd_h_summary" : "sm100_fwd_h";
+  if (sum) return scalar ? launch(k_scan<false, true, true, true>, label) : launch(k_scan<false, false, true, true>, label);
+  return scalar ? launch(k_scan<false, true, false, true>, label) : launch(k_scan<false, false, false, true>, label);
+}
+
+// summary pass + join for the sequences that are cut into runs
+int gen_starts(bool bwd, const tops_chunk_problem& pb, const GenPlan& g, const void* x, const void* gate, const void* y,
+               const float* first, float* last, const GenSegs& sc, cudaStream_t st) {
+  if (!g.cut) return TOPS_OK;
+  int rc = run_scan_gen(bwd, true, pb, g, x, gate, y, nullptr, nullptr, nullptr, sc.ends, sc.gsum, st);
+  if (rc) return rc;
+  KernelScope ks("sm100_join_segments", st);
+  const int slices = cdiv(pb.K * pb.V, 1024);
+  const dim3 grid(g.N * pb.H, slices < 16 ? slices : 16);
+  if (bwd) k_join_segments_gen<true><<<grid, 256, 0, st>>>(first, sc.gsum, sc.ends, sc.starts, last, g.seg0, g.geo.nseg, pb.H, pb.K, pb.V);
+  else k_join_segments_gen<false><<<grid, 256, 0, st>>>(first, sc.gsum, sc.ends, sc.starts, last, g.seg0, g.geo.nseg, pb.H, pb.K, pb.V);
+  return post_launch();
+}
+}  // namespace
+
+// What TOPS_IMPL_AUTO gives to the general form.  K, V below 32 leave most of a 128-wide tile empty: those stay on
+// the CUDA-core kernels.  An odd number of scalar gates would make a 4-byte gate fetch straddle the tensor's end.
+bool supported_gen(const tops_chunk_problem& pb) {
+  if (pb.dtype != TOPS_BF16 || pb.chunk != C) return false;
+  const bool stored_gate = pb.gate_kind == TOPS_GATE_PER_CHANNEL || pb.gate_kind == TOPS_GATE_SCALAR;
+  if (stored_gate && pb.gate_dtype != TOPS_BF16) return false;
+  if (pb.K < 32 || pb.K > D || pb.K % 8 != 0 || pb.V < 32 || pb.V > 8 * D || pb.V % 8 != 0) return false;
+  if (!(pb.scale > 0.f) || !(pb.scale < 1e30f)) return false;
+  if (pb.gate_kind == TOPS_GATE_SCALAR && ((size_t)pb.B * pb.T * pb.H) % 2 != 0) return false;
+  if ((size_t)pb.B * pb.T >= (1u << 31) - 64) return false;
+  const size_t chunk_rows = ((size_t)pb.B * pb.T / C + pb.B + (pb.cu_seqlens_host ? pb.N : 0)) * pb.H * cdiv(pb.V, D);
+  if (chunk_rows * D >= (1u << 31)) return false;   // rows of the state map are 32-bit coordinates
+  return device_is_sm100() && encode_fn() != nullptr;
+}
+
+// The plain form cuts a sequence only where whole runs of equal length come out; with few (batch, head) pairs and an
+// awkward chunk count (a prime, say) it would leave most SMs idle where the general form does not.
+bool prefer_gen(const tops_chunk_problem& pb) {
+  if (!supported(pb)) return supported_gen(pb);
+  const int nseg = pick_segments(pb), bh = pb.B * pb.H, nt = pb.T / C;
+  if (2 * bh > sm_count() || nt < 8) return false;
+  const int want = sm_count() / bh < nt / 4 ? sm_count() / bh : nt / 4;
+  return 4 * nseg < 3 * want && supported_gen(pb);
+}
+
+size_t gen_saved_bytes(const tops_chunk_problem& pb) { return GenPlan(pb).state_bytes(); }
+
+size_t gen_fwd_workspace_bytes(const tops_chunk_fwd_params& p) {
+  const GenPlan g(p.pb);
+  return g.table_bytes() + (p.saved_out || g.fused() ? 0 : g.state_bytes()) + g.seg_bytes() + 256;
+}
+
+int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
+  const tops_chunk_problem& pb = p.pb;
+  const bool scalar = scalar_kind(pb.gate_kind);
+  if (!aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || (pb.gate_kind != TOPS_GATE_GAMMA && !aligned16(p.g)) ||
+      !aligned16(p.o) || !aligned16(p.h0) || !aligned16(p.ht) || !aligned16(p.saved_out) || !aligned16(ws))
+    return TOPS_E_ALIGN;
+  GenPlan g(pb);
+  char* wsp = reinterpret_cast<char*>(ws);
+  int rc = g.upload(pb, wsp, st);
+  if (rc) return rc;
+  wsp += g.table_bytes();
+  const bool fused = g.fused();
+  void* h = p.saved_out;
+  if (!h && !fused) { h = wsp; wsp += g.state_bytes(); }
+  const GenSegs sc(wsp, g);
+  if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, p.h0, p.ht, sc, st))) return rc;
+  const int BT = pb.B * pb.T;
+  const __nv_bfloat16* gs = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(p.g) : nullptr;
+  const float* gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(p.g) : nullptr;
+  const size_t state_rows = (size_t)g.total_chunks * g.HV * D;
+  if (fused) {
+    FusedParams up;
+    if ((rc = act_map(&up.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&up.mk, p.k, BT, pb.H, pb.K)) ||
+        (rc = act_map(&up.mv, p.v, BT, pb.H, pb.V)))
+      return rc;
+    if (!scalar && (rc = act_map(&up.mg, p.g, BT, pb.H, pb.K))) return rc;
+    up.gscalar = gs; up.gamma = gamma; up.states = nullptr;
+    if (h) {
+      if ((rc = state_map(&up.mst, h, state_rows))) return rc;
+      up.states = reinterpret_cast<__nv_bfloat16*>(h);
+    }
+    up.s0 = p.h0; up.s0_seg = sc.starts; up.s_final = p.ht; up.o = reinterpret_cast<__nv_bfloat16*>(p.o);
+    up.T = pb.T; up.H = pb.H; up.NT = 0; up.nseg = 1; up.scale = pb.scale; up.geo = g.geo;
+    if ((rc = opt_in_smem(k_fwd_fused<true, true>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false, true>, FUSED_SMEM))) return rc;
+    KernelScope ks("sm100_fwd_fused", st);
+    if (scalar) k_fwd_fused<true, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
+    else k_fwd_fused<false, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
+    return post_launch();
+  }
+  if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, p.h0, sc.starts, h, p.ht, nullptr, st))) return rc;
+  FwdOParams fp;
+  if ((rc = act_map(&fp.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&fp.mk, p.k, BT, pb.H, pb.K)) ||
+      (rc = act_map(&fp.mv, p.v, BT, pb.H, pb.V)) || (rc = state_map(&fp.mh, h, state_rows)))
+    return rc;
+  if (!scalar && (rc = act_map(&fp.mg, p.g, BT, pb.H, pb.K))) return rc;
+  fp.gscalar = gs; fp.gamma = gamma; fp.geo = g.geo;
+  fp.o = reinterpret_cast<__nv_bfloat16*>(p.o); fp.T = pb.T; fp.H = pb.H; fp.scale = pb.scale;
+  const bool packed = !g.nch.empty();
+  fp.NT = packed ? g.total_chunks : g.geo.NTseq;
+  if ((rc = opt_in_smem(k_fwd_o<true, true>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false, true>, FWD_O_SMEM))) return rc;
+  const dim3 grid(g.HV, fp.NT, packed ? 1 : pb.B);
+  KernelScope ks("sm100_fwd_o", st);
+  if (scalar) k_fwd_o<true, true><<<grid, NTHREADS, FWD_O_SMEM, st>>>(fp);
+  else k_fwd_o<false, true><<<grid, NTHREADS, FWD_O_SMEM, st>>>(fp);
+  return post_launch();
+}
+
+// fp32 partial sums of dq, dk and dg over the value slices
+static size_t gen_partial_floats(const tops_chunk_bwd_params& p) {
+  if (p.pb.V <= D) return 0;
+  const size_t n = (size_t)p.pb.B * p.pb.T * p.pb.H;
+  return n * p.pb.K * 2 + (p.dg ? n * (scalar_kind(p.pb.gate_kind) ? 1 : p.pb.K) : 0);
+}
+
+size_t gen_bwd_workspace_bytes(const tops_chunk_bwd_params& p) {
+  const GenPlan g(p.pb);
+  return g.table_bytes() + (p.h_saved ? 1 : 2) * g.state_bytes() + g.seg_bytes() + align_up(gen_partial_floats(p) * sizeof(float)) + 256;
+}
+
+int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
+  const tops_chunk_problem& pb = p.pb;
+  if (!bwd_dtypes_ok(p)) return TOPS_E_UNSUPPORTED;
+  if (!aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || (pb.gate_kind != TOPS_GATE_GAMMA && !aligned16(p.g)) ||
+      !aligned16(p.do_) || !aligned16(p.h0) || !aligned16(p.dht) || !aligned16(p.dh0) || !aligned16(p.dq) || !aligned16(p.dk) ||
+      !aligned16(p.dv) || !aligned16(p.dg) || !aligned16(p.h_saved) || !aligned16(ws))
+    return TOPS_E_ALIGN;
+  GenPlan g(pb);
+  char* wsp = reinterpret_cast<char*>(ws);
+  int rc = g.upload(pb, wsp, st);
+  if (rc) return rc;
+  wsp += g.table_bytes();
+  char* dh = wsp; wsp += g.state_bytes();
+  const char* h = reinterpret_cast<const char*>(p.h_saved);
+  char* hw = nullptr;
+  if (!h) { hw = wsp; wsp += g.state_bytes(); }
+  const GenSegs sc(wsp, g); wsp += g.seg_bytes();
+  float* part = reinterpret_cast<float*>(wsp);
+  if (!h) {
+    if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, p.h0, nullptr, sc, st))) return rc;
+    if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, p.h0, sc.starts, hw, nullptr, nullptr, st))) return rc;
+    h = hw;
+  }
+  if ((rc = gen_starts(true, pb, g, p.q, p.g, p.do_, p.dht, p.dh0, sc, st))) return rc;
+  if ((rc = run_scan_gen(true, false, pb, g, p.q, p.g, p.do_, p.dht, sc.starts, dh, p.dh0, nullptr, st))) return rc;
+  BwdParams bp;
+  const int BT = pb.B * pb.T;
+  const size_t rows = (size_t)g.total_chunks * g.HV * D;
+  const bool scalar = scalar_kind(pb.gate_kind);
+  if ((rc = act_map(&bp.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&bp.mk, p.k, BT, pb.H, pb.K)) ||
+      (rc = act_map(&bp.mv, p.v, BT, pb.H, pb.V)) || (rc = act_map(&bp.mdo, p.do_, BT, pb.H, pb.V)) ||
+      (rc = state_map(&bp.mh, h, rows)) || (rc = state_map(&bp.mdh, dh, rows)))
+    return rc;
+  if (!scalar && (rc = act_map(&bp.mg, p.g, BT, pb.H, pb.K))) return rc;
+  bp.gscalar = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(p.g) : nullptr;
+  bp.gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(p.g) : nullptr;
+  bp.dv = reinterpret_cast<__nv_bfloat16*>(p.dv);
+  bp.T = pb.T; bp.H = pb.H; bp.NT = g.nch.empty() ? g.geo.NTseq : g.total_chunks; bp.scale = pb.scale; bp.geo = g.geo;
+  bp.total = g.total_chunks * pb.H;
+  const size_t n = (size_t)BT * pb.H;
+  float *pdq = part, *pdk = part + n * pb.K, *pdg = p.dg ? part + 2 * n * pb.K : nullptr;
+  for (int vs = 0; vs < g.geo.VS; ++vs) {
+    const bool last = vs == g.geo.VS - 1;
+    bp.vs = vs;
+    bp.dq = last ? p.dq : pdq; bp.dk = last ? p.dk : pdk; bp.dg = last ? p.dg : pdg;
+    bp.add_dq = vs ? pdq : nullptr; bp.add_dk = vs ? pdk : nullptr; bp.add_dg = vs ? pdg : nullptr;
+    if (scalar) rc = (!last || p.grad_dtype == TOPS_F32) ? launch_bwd_main<float, float, true, true>(bp, st)
+                                                         : launch_bwd_main<__nv_bfloat16, float, true, true>(bp, st);
+    else if (!last || p.grad_dtype == TOPS_F32) rc = launch_bwd_main<float, float, false, true>(bp, st);
+    else if (p.dg_dtype == TOPS_F32) rc = launch_bwd_main<__nv_bfloat16, float, false, true>(bp, st);
+    else rc = launch_bwd_main<__nv_bfloat16, __nv_bfloat16, false, true>(bp, st);
+    if (rc) return rc;
+  }
+  return TOPS_OK;
 }
 
 // The summary of one time shard for the state exchange between ranks: the state after the shard from a

@@ -13,6 +13,14 @@ int chunk_fwd(const tops_chunk_fwd_params& p, void* ws, size_t ws_bytes, cudaStr
 bool bwd_dtypes_ok(const tops_chunk_bwd_params& p);
 size_t bwd_workspace_bytes(const tops_chunk_bwd_params& p);
 int chunk_bwd(const tops_chunk_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
+// The general form: packed batches, sequences of any length, K <= 128, V in slices of 128, constant or no gates.
+bool supported_gen(const tops_chunk_problem& pb);
+bool prefer_gen(const tops_chunk_problem& pb);   // whether TOPS_IMPL_AUTO takes the general form
+size_t gen_saved_bytes(const tops_chunk_problem& pb);
+size_t gen_fwd_workspace_bytes(const tops_chunk_fwd_params& p);
+int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st);
+size_t gen_bwd_workspace_bytes(const tops_chunk_bwd_params& p);
+int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st);
 // Shard summary for the state exchange of a time-sharded sequence (see tops_b200_chunk_state_exchange_pack).
 size_t summary_workspace_bytes(const tops_chunk_problem& pb);
 int state_summary(const tops_chunk_problem& pb, bool reverse, const void* x, const void* g, const void* y,

@@ -66,11 +66,12 @@ inline int cached_map(CUtensorMap* m, int kind, const void* ptr, uint64_t a, uin
   return TOPS_OK;
 }
 
-// [B*T, H, 128] bf16 activations: box = 64 channels x 1 head x 64 tokens
-inline int act_map(CUtensorMap* m, const void* ptr, int BT, int H) {
-  return cached_map(m, 0, ptr, (uint64_t)BT, (uint64_t)H, [&](CUtensorMap* out) {
-    cuuint64_t dims[3] = {(cuuint64_t)kHeadDim, (cuuint64_t)H, (cuuint64_t)BT};
-    cuuint64_t strides[2] = {(cuuint64_t)kHeadDim * 2, (cuuint64_t)H * kHeadDim * 2};
+// [B*T, H, W] bf16 activations (W a multiple of 8): box = 64 channels x 1 head x 64 tokens; what a box covers
+// beyond the tensor is filled with zeros
+inline int act_map(CUtensorMap* m, const void* ptr, int BT, int H, int W = kHeadDim) {
+  return cached_map(m, 0, ptr, (uint64_t)BT, (uint64_t)H | ((uint64_t)W << 32), [&](CUtensorMap* out) {
+    cuuint64_t dims[3] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)BT};
+    cuuint64_t strides[2] = {(cuuint64_t)W * 2, (cuuint64_t)H * W * 2};
     cuuint32_t box[3] = {64, 1, 64};
     cuuint32_t es[3] = {1, 1, 1};
     return encode_fn()(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es,

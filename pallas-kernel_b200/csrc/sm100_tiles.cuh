@@ -104,13 +104,14 @@ struct GateRing {
   __device__ __forceinline__ void init(uint8_t* warp_area) { base = smem_u32(warp_area); }
   // idx: element index of the gate of time step `lane` of chunk c in the [B,T,H] tensor; hi_off: elements to
   // time step lane + 32 (an even number)
-  __device__ __forceinline__ void prefetch(const __nv_bfloat16* g, bool valid, size_t idx, size_t hi_off, int c, int lane) {
-    if (valid) {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(g);
-      const uint32_t dst = base + (uint32_t)(((c & 3) * 64 + lane) * 4);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(w + (idx >> 1)) : "memory");
+  // (valid_lo, valid_hi: whether this lane's two time steps exist; a step that does not is not fetched)
+  __device__ __forceinline__ void prefetch(const __nv_bfloat16* g, bool valid_lo, bool valid_hi, size_t idx, size_t hi_off, int c,
+                                           int lane) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(g);
+    const uint32_t dst = base + (uint32_t)(((c & 3) * 64 + lane) * 4);
+    if (valid_lo) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(w + (idx >> 1)) : "memory");
+    if (valid_hi)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 128u), "l"(w + ((idx + hi_off) >> 1)) : "memory");
-    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   __device__ __forceinline__ void take(size_t idx, int c, int lane, float& lo, float& hi) {
@@ -213,18 +214,18 @@ __device__ __forceinline__ void transpose4(float (&v)[4], int lane) {
 }
 // The same exchange followed by a store of the four neighbouring channels of time step
 // t0 + (lane & 3) at p[i]; the bf16 form rounds after the first stage and moves packed pairs.
-__device__ __forceinline__ void st_transposed4(float* p, size_t i, float (&v)[4], int lane) {
+__device__ __forceinline__ void st_transposed4(float* p, size_t i, float (&v)[4], int lane, bool store = true) {
   transpose4(v, lane);
-  __stcs(reinterpret_cast<float4*>(p + i), make_float4(v[0], v[1], v[2], v[3]));
+  if (store) __stcs(reinterpret_cast<float4*>(p + i), make_float4(v[0], v[1], v[2], v[3]));
 }
-__device__ __forceinline__ void st_transposed4(__nv_bfloat16* p, size_t i, const float (&v)[4], int lane) {
+__device__ __forceinline__ void st_transposed4(__nv_bfloat16* p, size_t i, const float (&v)[4], int lane, bool store = true) {
   const bool odd = lane & 1, hi = lane & 2;
   const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 1);
   const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[2] : v[3], 1);
   const uint32_t pa = odd ? pack_bf16(r0, v[1]) : pack_bf16(v[0], r0);
   const uint32_t pb = odd ? pack_bf16(r1, v[3]) : pack_bf16(v[2], r1);
   const uint32_t u = __shfl_xor_sync(0xffffffffu, hi ? pa : pb, 2);
-  __stcs(reinterpret_cast<uint2*>(p + i), hi ? make_uint2(u, pb) : make_uint2(pa, u));
+  if (store) __stcs(reinterpret_cast<uint2*>(p + i), hi ? make_uint2(u, pb) : make_uint2(pa, u));
 }
 // gradients are written once and not read again by these kernels: streaming stores
 __device__ __forceinline__ void st_out(float* p, size_t i, float x) { __stcs(p + i, x); }

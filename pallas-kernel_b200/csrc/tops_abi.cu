@@ -65,13 +65,15 @@ struct Carver {
 
 bool valid_dtype(int dt) { return dt == TOPS_F32 || dt == TOPS_BF16 || dt == TOPS_F16; }
 
+bool packed(const tops_chunk_problem& pb) { return pb.cu_seqlens || pb.cu_seqlens_host; }
+
 int check_problem(const tops_chunk_problem& pb) {
   if (pb.B < 1 || pb.T < 1 || pb.H < 1 || pb.K < 1 || pb.V < 1) return TOPS_E_BAD_SHAPE;
   if (pb.chunk != 16 && pb.chunk != 32 && pb.chunk != 64) return TOPS_E_BAD_SHAPE;
   if (!valid_dtype(pb.dtype) || !valid_dtype(pb.gate_dtype)) return TOPS_E_BAD_DTYPE;
   if (pb.gate_kind < TOPS_GATE_NONE || pb.gate_kind > TOPS_GATE_GAMMA) return TOPS_E_BAD_SHAPE;
   if (pb.gate_kind == TOPS_GATE_GAMMA && pb.gate_dtype != TOPS_F32) return TOPS_E_BAD_DTYPE;
-  if (pb.cu_seqlens) {
+  if (packed(pb)) {
     if (pb.B != 1 || pb.N < 1 || pb.cu_seqlens_host == nullptr) return TOPS_E_BAD_SHAPE;
     if (pb.cu_seqlens_host[0] != 0 || pb.cu_seqlens_host[pb.N] != pb.T) return TOPS_E_BAD_SHAPE;
     for (int n = 0; n < pb.N; ++n)
@@ -81,7 +83,7 @@ int check_problem(const tops_chunk_problem& pb) {
 }
 
 int count_chunks(const tops_chunk_problem& pb) {
-  if (!pb.cu_seqlens) return pb.B * cdiv(pb.T, pb.chunk);
+  if (!packed(pb)) return pb.B * cdiv(pb.T, pb.chunk);
   int tot = 0;
   for (int n = 0; n < pb.N; ++n) tot += cdiv(pb.cu_seqlens_host[n + 1] - pb.cu_seqlens_host[n], pb.chunk);
   return tot;
@@ -100,7 +102,8 @@ int make_problem(const tops_chunk_problem& in, Carver& cv, cudaStream_t st, Prob
   pb.H = in.H; pb.K = in.K; pb.V = in.V; pb.dtype = in.dtype; pb.gate_kind = in.gate_kind; pb.scale = in.scale;
   pb.total_chunks = count_chunks(in);
   pb.m.T = in.T; pb.m.C = in.chunk;
-  if (in.cu_seqlens) {
+  if (packed(in)) {
+    if (launch && !in.cu_seqlens) return TOPS_E_NULL;   // these kernels read the boundaries from the device
     int32_t* cs = cv.take<int32_t>(in.N + 1);
     int32_t* chunk_seq = cv.take<int32_t>(pb.total_chunks);
     pb.m.cu = in.cu_seqlens; pb.m.cs = cs; pb.m.chunk_seq = chunk_seq; pb.m.N = in.N; pb.m.NT = pb.total_chunks;
@@ -119,9 +122,22 @@ size_t state_elems(const tops_chunk_problem& pb) {
   return (size_t)count_chunks(pb) * pb.H * pb.K * pb.V;
 }
 
-bool use_sm100(const tops_chunk_problem& pb) {
-  if (pb.impl == TOPS_IMPL_GENERIC) return false;
-  return sm100::supported(pb);
+// Which kernels serve a problem: the tcgen05 kernels in their plain or their general form, or the generic ones.
+// An explicit TOPS_IMPL_SM100 asks for the plain form.
+enum Family { FAMILY_GENERIC, FAMILY_PLAIN, FAMILY_GENERAL };
+Family family(const tops_chunk_problem& pb, bool plain_only = false) {
+  if (pb.impl == TOPS_IMPL_GENERIC) return FAMILY_GENERIC;
+  if (pb.impl != TOPS_IMPL_SM100 && !plain_only && sm100::prefer_gen(pb)) return FAMILY_GENERAL;
+  return sm100::supported(pb) ? FAMILY_PLAIN : FAMILY_GENERIC;
+}
+// optional outputs only the generic kernels write; segment summaries only the plain form takes
+Family family(const tops_chunk_fwd_params& p) {
+  if (p.g_cumsum_out || p.A_out || p.h_out) return FAMILY_GENERIC;
+  return family(p.pb, p.segments != nullptr);
+}
+Family family(const tops_chunk_bwd_params& p) {
+  if (!sm100::bwd_dtypes_ok(p)) return FAMILY_GENERIC;
+  return family(p.pb, p.rev_segments != nullptr);
 }
 
 }  // namespace
@@ -155,7 +171,12 @@ extern "C" int tops_b200_last_cuda_error(char* buf, size_t cap) {
 
 extern "C" int tops_b200_chunk_selected_impl(const tops_chunk_problem* pb) {
   if (!pb || check_problem(*pb)) return TOPS_IMPL_GENERIC;
-  return use_sm100(*pb) ? TOPS_IMPL_SM100 : TOPS_IMPL_GENERIC;
+  return family(*pb) == FAMILY_GENERIC ? TOPS_IMPL_GENERIC : TOPS_IMPL_SM100;
+}
+
+extern "C" size_t tops_b200_chunk_saved_bytes(const tops_chunk_problem* pb) {
+  if (!pb || check_problem(*pb) || family(*pb) == FAMILY_GENERIC) return 0;
+  return sm100::gen_saved_bytes(*pb);   // (the two forms keep the same tiles)
 }
 
 extern "C" int tops_b200_device_error(int* out) {
@@ -225,7 +246,7 @@ extern "C" int tops_b200_chunk_fwd_h(const tops_fwd_h_params* p, void* stream) {
   if (!p || !p->k || !p->v) return TOPS_E_NULL;
   int rc = check_problem(p->pb);
   if (rc) return rc;
-  if (p->pb.cu_seqlens) return TOPS_E_UNSUPPORTED;
+  if (packed(p->pb)) return TOPS_E_UNSUPPORTED;
   if (p->pb.gate_kind != TOPS_GATE_NONE && !p->g_cumsum) return TOPS_E_NULL;
   if (p->h && p->h_dtype != TOPS_F32 && p->h_dtype != p->pb.dtype) return TOPS_E_BAD_DTYPE;
   Carver cv(nullptr);
@@ -240,7 +261,7 @@ extern "C" int tops_b200_chunk_bwd_dh(const tops_bwd_dh_params* p, void* stream)
   if (!p || !p->q || !p->do_) return TOPS_E_NULL;
   int rc = check_problem(p->pb);
   if (rc) return rc;
-  if (p->pb.cu_seqlens) return TOPS_E_UNSUPPORTED;
+  if (packed(p->pb)) return TOPS_E_UNSUPPORTED;
   if (p->pb.gate_kind != TOPS_GATE_NONE && !p->g_cumsum) return TOPS_E_NULL;
   Carver cv(nullptr);
   Problem pb;
@@ -267,7 +288,9 @@ static size_t fwd_layout(const tops_chunk_fwd_params* p, void* ws, cudaStream_t 
 
 extern "C" size_t tops_b200_chunk_fwd_workspace_bytes(const tops_chunk_fwd_params* p) {
   if (!p || check_problem(p->pb)) return 0;
-  if (use_sm100(p->pb) && !p->g_cumsum_out && !p->A_out && !p->h_out) return sm100::fwd_workspace_bytes(*p);
+  const Family f = family(*p);
+  if (f == FAMILY_PLAIN) return sm100::fwd_workspace_bytes(*p);
+  if (f == FAMILY_GENERAL) return sm100::gen_fwd_workspace_bytes(*p);
   Problem pb;
   return fwd_layout(p, nullptr, nullptr, false, &pb, nullptr, nullptr, nullptr) + 256;
 }
@@ -281,7 +304,9 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
   if (p->pb.impl == TOPS_IMPL_SM100 && !sm100::supported(p->pb)) return TOPS_E_UNSUPPORTED;
   if (!workspace || workspace_bytes < tops_b200_chunk_fwd_workspace_bytes(p)) return TOPS_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  if (use_sm100(p->pb) && !p->g_cumsum_out && !p->A_out && !p->h_out) return sm100::chunk_fwd(*p, workspace, workspace_bytes, st);
+  const Family f = family(*p);
+  if (f == FAMILY_PLAIN) return sm100::chunk_fwd(*p, workspace, workspace_bytes, st);
+  if (f == FAMILY_GENERAL) return sm100::gen_chunk_fwd(*p, workspace, st);
 
   Problem pb;
   float* gcum = nullptr;
@@ -370,7 +395,9 @@ static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t 
 
 extern "C" size_t tops_b200_chunk_bwd_workspace_bytes(const tops_chunk_bwd_params* p) {
   if (!p || check_problem(p->pb)) return 0;
-  if (use_sm100(p->pb) && sm100::bwd_dtypes_ok(*p)) return sm100::bwd_workspace_bytes(*p);
+  const Family f = family(*p);
+  if (f == FAMILY_PLAIN) return sm100::bwd_workspace_bytes(*p);
+  if (f == FAMILY_GENERAL) return sm100::gen_bwd_workspace_bytes(*p);
   Problem pb;
   return bwd_layout(p, nullptr, nullptr, false, &pb, nullptr, nullptr) + 256;
 }
@@ -385,7 +412,9 @@ extern "C" int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* wor
   if (p->pb.impl == TOPS_IMPL_SM100 && !sm100::supported(p->pb)) return TOPS_E_UNSUPPORTED;
   if (!workspace || workspace_bytes < tops_b200_chunk_bwd_workspace_bytes(p)) return TOPS_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  if (use_sm100(p->pb) && sm100::bwd_dtypes_ok(*p)) return sm100::chunk_bwd(*p, workspace, workspace_bytes, st);
+  const Family f = family(*p);
+  if (f == FAMILY_PLAIN) return sm100::chunk_bwd(*p, workspace, workspace_bytes, st);
+  if (f == FAMILY_GENERAL) return sm100::gen_chunk_bwd(*p, workspace, st);
   if (p->dg_dtype != TOPS_F32) return TOPS_E_UNSUPPORTED;   // the generic kernels write fp32 dg per gate element
 
   Problem pb;

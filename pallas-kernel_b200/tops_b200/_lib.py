@@ -140,6 +140,8 @@ lib.tops_b200_launch_count.restype = C.c_int64
 lib.tops_b200_launch_count.argtypes = []
 lib.tops_b200_chunk_selected_impl.restype = C.c_int
 lib.tops_b200_chunk_selected_impl.argtypes = [C.POINTER(ChunkProblem)]
+lib.tops_b200_chunk_saved_bytes.restype = _sz
+lib.tops_b200_chunk_saved_bytes.argtypes = [C.POINTER(ChunkProblem)]
 lib.tops_b200_device_error.restype = C.c_int
 lib.tops_b200_device_error.argtypes = [C.POINTER(C.c_int)]
 lib.tops_b200_device_error_reset.restype = C.c_int

@@ -7,7 +7,15 @@ import ctypes as C
 import torch
 
 from .. import _lib as L
-from .common import make_problem, total_chunks
+from .common import device_boundaries, make_problem, total_chunks
+
+
+def tensor_core_shape(q, v, gate, gate_kind):
+    """Whether the tcgen05 kernels take tensors like these (with chunks of 64, whatever T and the packing)."""
+    K, V = q.shape[-1], v.shape[-1]
+    return (q.dtype == torch.bfloat16
+            and (gate_kind in (L.GATE_NONE, L.GATE_GAMMA) or gate.dtype == torch.bfloat16)
+            and 32 <= K <= 128 and K % 8 == 0 and 32 <= V <= 1024 and V % 8 == 0)
 
 
 @L.on_tensor_device
@@ -42,12 +50,15 @@ def chunk_fwd_call(q, k, v, gate, gate_kind, scale, h0, want_ht, chunk, cu_seqle
                         cu_seqlens, keep)
     p.q, p.k, p.v, p.g, p.h0, p.o, p.ht = L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(gate), L.ptr(h0), L.ptr(o), L.ptr(ht)
     p.g_cumsum_out, p.A_out, p.h_out = L.ptr(gcum), L.ptr(A), L.ptr(hs)
-    if want_saved and not (want_gcum or want_A or want_h) \
-            and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100:
-        hs = torch.empty(B, nch // B, H, K, V, dtype=k.dtype, device=dev)
+    extra = want_gcum or want_A or want_h
+    fast = not extra and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100
+    if fast and want_saved:
+        hs = torch.empty(L.lib.tops_b200_chunk_saved_bytes(C.byref(p.pb)) // 2, dtype=k.dtype, device=dev)
         p.saved_out = L.ptr(hs)
-    if segments is not None and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100:
+    if fast and segments is not None:
         p.segments = L.ptr(segments)
+    if cu_seqlens is not None and not fast:
+        device_boundaries(p.pb, cu_seqlens, keep)
     ws = L.workspace(L.lib.tops_b200_chunk_fwd_workspace_bytes(C.byref(p)), dev)
     L.check(L.lib.tops_b200_chunk_gla_fwd(C.byref(p), ws.data_ptr(), ws.numel(), L.stream_ptr(dev)),
             "chunk_gla_fwd")
@@ -81,10 +92,14 @@ def chunk_bwd_call(q, k, v, gate, gate_kind, scale, h0, do, dht, chunk, grad_dty
                         L.F32 if gate is None else L.dtype_code(gate.dtype), gate_kind, scale, impl,
                         cu_seqlens, keep)
     dg_dtype = torch.float32
-    direct = primal_dtypes and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100
+    fast = L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100
+    direct = primal_dtypes and fast
     if direct:
         grad_dtype = q.dtype
-        dg_dtype = torch.float32 if gate_kind == L.GATE_SCALAR else gate.dtype   # a scalar gate's dg is always fp32
+        if gate_kind == L.GATE_PER_CHANNEL:   # (a scalar gate's dg is always fp32)
+            dg_dtype = gate.dtype
+    if cu_seqlens is not None and not fast:
+        device_boundaries(p.pb, cu_seqlens, keep)
     dq = torch.empty(B, T, H, K, dtype=grad_dtype, device=dev)
     dk = torch.empty(B, T, H, K, dtype=grad_dtype, device=dev)
     dv = torch.empty(B, T, H, V, dtype=do.dtype, device=dev)
@@ -100,9 +115,9 @@ def chunk_bwd_call(q, k, v, gate, gate_kind, scale, h0, do, dht, chunk, grad_dty
     p.grad_dtype = L.dtype_code(grad_dtype)
     p.dg_dtype = L.dtype_code(dg_dtype)
     if h_saved is not None:
-        assert h_saved.dtype == q.dtype and h_saved.shape[-3:] == (H, K, V)
+        assert h_saved.dtype == q.dtype
         p.h_saved = L.ptr(h_saved)
-    if rev_segments is not None and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100:
+    if rev_segments is not None and fast:
         p.rev_segments = L.ptr(rev_segments)
     ws = L.workspace(L.lib.tops_b200_chunk_bwd_workspace_bytes(C.byref(p)), dev)
     L.check(L.lib.tops_b200_chunk_gla_bwd(C.byref(p), ws.data_ptr(), ws.numel(), L.stream_ptr(dev)),

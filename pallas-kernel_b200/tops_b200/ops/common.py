@@ -22,18 +22,24 @@ def _is_pow2(x: int) -> bool:
 def make_problem(B, T, H, K, V, chunk, dtype, gate_dtype, gate_kind, scale, impl=L.IMPL_AUTO,
                  cu_seqlens=None, keep=None):
     """Fill a ChunkProblem.  `cu_seqlens` may be a list / CPU tensor / CUDA
-    tensor; both a device and a host copy are handed to the library and are
-    kept alive through `keep`."""
+    tensor; a host copy is handed to the library and kept alive through `keep`
+    (`device_boundaries` adds the device copy the generic kernels read)."""
     pb = L.ChunkProblem()
     pb.B, pb.T, pb.H, pb.K, pb.V, pb.chunk = B, T, H, K, V, chunk
     pb.dtype, pb.gate_dtype, pb.gate_kind, pb.impl = dtype, gate_dtype, gate_kind, impl
     pb.scale = float(scale)
     if cu_seqlens is not None:
-        host = torch.as_tensor(cu_seqlens).to("cpu", torch.int32).contiguous()
-        dev = host.to(torch.device("cuda", torch.cuda.current_device()))
-        keep.extend([host, dev])
-        pb.cu_seqlens, pb.cu_seqlens_host, pb.N = dev.data_ptr(), host.data_ptr(), host.numel() - 1
+        cu = cu_seqlens if isinstance(cu_seqlens, list) else [int(x) for x in cu_seqlens]
+        host = (C.c_int32 * len(cu))(*cu)
+        keep.append(host)
+        pb.cu_seqlens_host, pb.N = C.addressof(host), len(cu) - 1
     return pb
+
+
+def device_boundaries(pb, cu_seqlens, keep):
+    dev = torch.tensor(list(cu_seqlens), dtype=torch.int32, device=torch.device("cuda", torch.cuda.current_device()))
+    keep.append(dev)
+    pb.cu_seqlens = dev.data_ptr()
 
 
 def total_chunks(B, T, chunk, cu_seqlens=None) -> int:

@@ -16,7 +16,7 @@ import ctypes as C
 import torch
 
 from .. import _lib as L
-from ._chunk import chunk_bwd_call, chunk_fwd_call
+from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
 
 
 def _check_qkvg(q, k, v, g, initial_state, cu_seqlens):
@@ -76,13 +76,12 @@ def chunk_gla_bwd(q, k, v, g, g_cumsum, scale, initial_state, h, A, do, dht, chu
 def _kernel_chunk(q, v, g, cu_seqlens, chunk_size):
     """Chunk length the kernels use for the differentiable op.  The op's results (o, final state,
     gradients) do not depend on the chunk length beyond where bf16 roundings fall, so a problem the
-    tcgen05 kernels can take (bf16, K = V = 128, dense, T a multiple of 64) runs with their chunk of
+    tcgen05 kernels can take (bf16, K <= 128) runs with their chunk of
     64 whatever `chunk_size` asks for (the reference's default is 16); everything else keeps the
     requested length.  The orchestrators that return per-chunk intermediates never change it."""
     assert chunk_size >= 1 and (chunk_size & (chunk_size - 1)) == 0, \
         f"chunk_size must be a power of 2, got {chunk_size}"   # tops/ops/common/cumsum.py:506-508
-    if (g is not None and cu_seqlens is None and q.dtype == torch.bfloat16 and g.dtype == torch.bfloat16
-            and q.shape[-1] == 128 and v.shape[-1] == 128 and q.shape[1] % 64 == 0):
+    if tensor_core_shape(q, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL):
         return 64
     # the kernels hold chunks of 16, 32 or 64 time steps; longer (or shorter) powers of two give the
     # same results computed with the nearest length they hold

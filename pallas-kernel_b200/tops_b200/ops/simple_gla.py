@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib as L
-from ._chunk import chunk_bwd_call, chunk_fwd_call
+from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
 from .gla import fused_recurrent_gla
 
 
@@ -65,6 +65,8 @@ def _fwd(q, k, v, g, g_gamma, scale, initial_state, output_final_state, chunk_si
     _check(q, k, v, g, g_gamma, initial_state, cu_seqlens)
     gate, kind = _gate(g, g_gamma)
     chunk_size = _kernel_chunk(chunk_size)
+    if tensor_core_shape(q, v, gate, kind):
+        chunk_size = 64
     o, ht, _, _, saved = chunk_fwd_call(q, k, v, gate, kind, scale, initial_state, output_final_state, chunk_size,
                                         _cu(cu_seqlens), want_saved=want_saved)
     return o, ht, saved
@@ -86,7 +88,10 @@ def chunk_simple_gla_bwd(q, k, v, g, g_gamma, initial_state, do, dht, scale, chu
     forward kept (None recomputes them, as the reference does)."""
     _check(q, k, v, g, g_gamma, initial_state, cu_seqlens)
     gate, kind = _gate(g, g_gamma)
-    return chunk_bwd_call(q, k, v, gate, kind, scale, initial_state, do, dht, _kernel_chunk(chunk_size), q.dtype,
+    chunk_size = _kernel_chunk(chunk_size)
+    if tensor_core_shape(q, v, gate, kind):
+        chunk_size = 64
+    return chunk_bwd_call(q, k, v, gate, kind, scale, initial_state, do, dht, chunk_size, q.dtype,
                           g is not None, initial_state is not None, _cu(cu_seqlens), h_saved=h_saved)
 
 

@@ -136,7 +136,7 @@ def cuda_ops(kind: str = "simple_gla", chunk_size: int = 64) -> LocalOps:
     def pack_problem(x, y, g):
         B, T, H, K = x.shape
         pb = common.make_problem(B, T, H, K, y.shape[-1], C, L.dtype_code(x.dtype), L.dtype_code(g.dtype),
-                                 L.GATE_PER_CHANNEL if g.ndim == 4 else L.GATE_SCALAR, 1.0)
+                                 L.GATE_PER_CHANNEL if g.ndim == 4 else L.GATE_SCALAR, 1.0, L.IMPL_SM100)
         ok = (x.dtype == torch.bfloat16 and g.dtype == torch.bfloat16
               and L.lib.tops_b200_chunk_selected_impl(C_.byref(pb)) == L.IMPL_SM100)
         return pb if ok else None
