@@ -63,6 +63,10 @@ namespace {
 //     of the tensor, where TMA fills zeros); the rows that are not its own are overwritten with zeros in shared
 //     memory before a product reads them, so nothing of another sequence, not even an infinity, gets in: zero
 //     gates repeat the last cumulative gate, zero q, k, v, do add nothing.  Only short chunks pay for it.
+//   * the diagonal of the intra-chunk matrix, q_i . k_i, has no gates in it and is summed in fp32 from the raw q and k
+//     while they are gated (the products of the gated bf16 operands lose about 2^-9 |q| |k|, which is all there is of a
+//     diagonal entry where q_i and k_i are nearly orthogonal; the output of a sequence's first token is that entry
+//     times v, and an output norm divides by it).
 //   * channels beyond K or V are zero-filled by TMA; the state tiles in scratch are always 128 x 128.
 //   * V > 128 runs as VS slices of 128 value channels that share q, k and g.
 //   * packed batches find their segments and chunks in tables that k_plan writes.
@@ -112,6 +116,24 @@ __device__ __forceinline__ void zero_rows(uint8_t* tile, int len, int t0, int nt
     const int r = len + (i >> 4), piece = i & 15;
     *reinterpret_cast<uint4*>(tile + (piece >> 3) * SLAB64 + r * 128 + (piece & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
+}
+// the part of q_i . k_i of 16 channels (two packed vectors of 8 of each)
+__device__ __forceinline__ float dot8(uint4 a, uint4 b, float s) {
+  const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&a), *y = reinterpret_cast<const __nv_bfloat162*>(&b);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float2 u = __bfloat1622float2(x[t]), v = __bfloat1622float2(y[t]);
+    s = fmaf(u.x, v.x, s);
+    s = fmaf(u.y, v.y, s);
+  }
+  return s;
+}
+// puts the sum of `n` partial dot products part[.][i] into a[j], j = i - j0 (row i's diagonal entry)
+__device__ __forceinline__ void set_diagonal(float (&a)[16], const float* part, int n, int i, int j) {
+  float d = 0.f;
+  for (int c = 0; c < n; ++c) d += part[c * C + i];
+#pragma unroll
+  for (int t = 0; t < 16; ++t) a[t] = t == j ? d : a[t];
 }
 // 32 values of row `row` of a state [.., K, V], columns c0 .. c0 + 31 (zero outside K x V)
 __device__ __forceinline__ void load_state32(float (&S)[32], const float* base, int row, int c0, int K, int V) {
@@ -628,6 +650,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   uint8_t* vt = gs + TILE64;
   uint8_t* hs = vt + TILE64;          // h_c exp(mid) scale, 128 x 128 (scaled by the scan kernel)
   uint8_t* mt = hs + TILE128;         // TRI_MID pattern, 64 x 64
+  float* diag = reinterpret_cast<float*>(gs + SLAB64);   // GEN: partial q_i . k_i [4][64] (the gates are consumed by then)
   __shared__ uint64_t bar_load, bar_e, bar_a, bar_o;
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -708,13 +731,17 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     const float E = __shfl_sync(0xffffffffu, (q4 >> 1) ? w.hi : w.lo, i & 31) - w.mid();
     const float f = fast_exp(E), r = fast_exp(-E);
     if (lane < 16) {
+      float dot = 0.f;
       const uint32_t rowoff = (uint32_t)(seg >> 1) * SLAB64 + (uint32_t)i * 128u;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t off = rowoff + (((uint32_t)((seg & 1) * 4 + u) ^ (uint32_t)i) & 7u) * 16u;
-        *reinterpret_cast<uint4*>(qs + off) = scale8_by(*reinterpret_cast<const uint4*>(qs + off), f);
-        *reinterpret_cast<uint4*>(ks + off) = scale8_by(*reinterpret_cast<const uint4*>(ks + off), r);
+        const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+        if (GEN) dot = dot8(qr, kr, dot);
+        *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
+        *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
       }
+      if (GEN) diag[seg * C + i] = dot;
     }
     fence_async_smem();
     tc_fence_before();
@@ -725,6 +752,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), e);
     if (lane < 16) {   // rows of an M = 64 accumulator sit in lanes 0..15 of each 32-lane quarter
       const int i = 16 * q4 + lane;
+      float dot = 0.f;
       const uint32_t rowoff = (uint32_t)(seg >> 1) * SLAB64 + (uint32_t)i * 128u;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -732,9 +760,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
         float f[8], r[8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) { f[t] = fast_exp(e[8 * u + t]); r[t] = fast_exp(-e[8 * u + t]); }
-        *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), f);
-        *reinterpret_cast<uint4*>(ks + off) = scale8(*reinterpret_cast<const uint4*>(ks + off), r);
+        const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+        if (GEN) dot = dot8(qr, kr, dot);
+        *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
+        *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
       }
+      if (GEN) diag[seg * C + i] = dot;
     }
     fence_async_smem();
     tc_fence_before();
@@ -761,6 +792,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     const int i = 16 * q4 + lane;
     float a[16];
     tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
+    if (GEN && lane < 16 && seg == q4) set_diagonal(a, diag, 4, i, lane);
     if (lane < 16) store_tril16(gs, i, seg * 16, a, p.scale);
     fence_async_smem();
     tc_fence_before();
@@ -1019,6 +1051,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       uint8_t* qs = in + (pp & 1) * FUSED_STAGE;
       uint8_t *ks = qs + TILE64, *gs = ks + TILE64;
       uint8_t* ht = hst + (pp & 1) * TILE128;
+      float* diag = reinterpret_cast<float*>(gs + SLAB64);   // GEN: partial q_i . k_i [8][64], in the consumed gate tile
       if (!mbar_wait(&sh.fullin[pp & 1], (pp >> 1) & 1) || (!SCALAR && !mbar_wait(&sh.ebar, ph))) { *abort_flag = 1; fail(9); }
       tc_fence_after();
       const int len = chunk_len(pp);
@@ -1069,14 +1102,19 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         const int cg = (q4 >> 1) * 4 + seg;
         const float E = ((q4 & 1) ? wg.hi : wg.lo) - wg.mid();
         const float f = fast_exp(E), r = fast_exp(-E);
+        float dot = 0.f;
         const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-          *reinterpret_cast<uint4*>(qs + off) = scale8_by(*reinterpret_cast<const uint4*>(qs + off), f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8_by(*reinterpret_cast<const uint4*>(ks + off), r);
+          const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+          if (GEN) dot = dot8(qr, kr, dot);
+          *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
+          *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
         }
+        if (GEN) diag[cg * C + i] = dot;
       } else {
+        float dot = 0.f;
         const int i = (q4 * 32 + lane) & 63;
         const int cg = (q4 >> 1) * 4 + seg;
         const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
@@ -1089,9 +1127,12 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
             f[t] = fast_exp(em[8 * u + t]);
             r[t] = fast_exp(-em[8 * u + t]);
           }
-          *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8(*reinterpret_cast<const uint4*>(ks + off), r);
+          const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+          if (GEN) dot = dot8(qr, kr, dot);
+          *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
+          *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
         }
+        if (GEN) diag[cg * C + i] = dot;
       }
       fence_async_smem();
       tc_fence_before();
@@ -1105,6 +1146,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         const int i = 16 * q4 + lane;   // rows of an M = 64 accumulator sit in lanes 0..15 of each quarter
         float a[16];
         tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
+        if (GEN && lane < 16 && seg == q4) set_diagonal(a, diag, 8, i, lane);
         if (lane < 16) store_tril16(gs, i, seg * 16, a, p.scale);
       }
       fence_async_smem();
@@ -1206,6 +1248,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   __shared__ float tails[2][4][D];    // per-segment sum_i dk_inter k
   __shared__ float hdh_s[2][D];       // sum_v h' dh'
   __shared__ float dgk_s[2][C];       // SCALAR: dg of a chunk summed over the channels
+  __shared__ float diag[2][GEN ? 8 * C : 1];   // GEN: partial q_i . k_i [8][64] of a chunk
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // tensor-memory columns: the exponent tile E_mid is consumed by the gating before A and dA take its place
@@ -1309,6 +1352,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       tc_fence_after();
       const int i = (q4 * 32 + lane) & 63;
       const int cg = (q4 >> 1) * 4 + seg;
+      float dot = 0.f;
       bool mine = true;   // GEN: a short chunk's foreign rows become zero
       if (GEN) {
         int h_, row_, hrow_;
@@ -1331,11 +1375,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-          *reinterpret_cast<uint4*>(qs + off) =
-              mine ? scale8_by(*reinterpret_cast<const uint4*>(qs + off), f) : make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(ks + off) =
-              mine ? scale8_by(*reinterpret_cast<const uint4*>(ks + off), r) : make_uint4(0u, 0u, 0u, 0u);
+          const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+          if (GEN) dot = dot8(qr, kr, dot);
+          *reinterpret_cast<uint4*>(qs + off) = mine ? scale8_by(qr, f) : make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(ks + off) = mine ? scale8_by(kr, r) : make_uint4(0u, 0u, 0u, 0u);
         }
+        if (GEN) diag[sl][cg * C + i] = mine ? dot : 0.f;
         fence_async_smem();
         tc_fence_before();
         mbar_arrive(&gated);
@@ -1353,11 +1398,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           f[t] = fast_exp(em[8 * u + t]);
           r[t] = fast_exp(-em[8 * u + t]);
         }
-        *reinterpret_cast<uint4*>(qs + off) =
-            mine ? scale8(*reinterpret_cast<const uint4*>(qs + off), f) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(ks + off) =
-            mine ? scale8(*reinterpret_cast<const uint4*>(ks + off), r) : make_uint4(0u, 0u, 0u, 0u);
+        const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
+        if (GEN) dot = dot8(qr, kr, dot);
+        *reinterpret_cast<uint4*>(qs + off) = mine ? scale8(qr, f) : make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(ks + off) = mine ? scale8(kr, r) : make_uint4(0u, 0u, 0u, 0u);
       }
+      if (GEN) diag[sl][cg * C + i] = mine ? dot : 0.f;
       fence_async_smem();
       tc_fence_before();
       mbar_arrive(&gated);
@@ -1482,6 +1528,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       for (int sg = 0; sg < 4; ++sg) {
         float a[16];
         tmem_ld16(tmem_addr(tm, lane_base, cA + sg * 16), a);
+        if (GEN && lane < 16 && sg == g4) set_diagonal(a, diag[it & 1], 8, ri, lane);
         if (lane < 16) store_tril16(Ps, ri, sg * 16, a, p.scale);
         tmem_ld16(tmem_addr(tm, lane_base, cdA + sg * 16), a);
         if (lane < 16) store_tril16(dAs, ri, sg * 16, a, p.scale);

@@ -1,0 +1,52 @@
+"""The gate and norm kernels at the sizes where their thread layouts change: vectors of four and of eight elements, rows
+shared by 1 to 32 lanes, several vectors per lane, one row, more columns than a block has threads."""
+import pytest
+import torch
+
+from oracle import aux as O
+from tests.util import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _grads(fn, inputs, dy):
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    y = fn(*leaves)
+    return [y.detach(), *torch.autograd.grad(y, leaves, dy.to(y.dtype))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,D", [(1, 4), (3, 8), (65, 12), (7, 72), (33, 136), (5, 260), (9, 516), (2, 1000), (31, 1024)])
+def test_row_kernels(dtype, rows, D):
+    from tops_b200.ops.norm import l2norm, rmsnorm_gated
+    gen = torch.Generator().manual_seed(rows * D)
+    x, g, dy = (torch.randn(rows, D, generator=gen).to(dtype) for _ in range(3))
+    w = 1 + 0.1 * torch.randn(D, generator=gen)
+    for f, ref, args in ((l2norm, O.l2norm, (x,)), (rmsnorm_gated, O.rmsnorm_gated, (x, g, w))):
+        want = _grads(ref, args, dy)
+        got = _grads(f, [t.cuda() for t in args], dy.cuda())
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert_close(f"{f.__name__} {i}", a.float().cpu(), b.float(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lower_bound", [None, -5.0])
+@pytest.mark.parametrize("rows,H,K", [(1, 1, 4), (5, 3, 12), (700, 2, 40), (3, 5, 512), (1300, 1, 8)])
+def test_gate_kernels(dtype, lower_bound, rows, H, K):
+    from tops_b200.ops.gate import gla_gate, kda_gate_fwd
+    gen = torch.Generator().manual_seed(rows + H * K)
+    # (up to +-20: both tails of the softplus)
+    g = (8 * torch.randn(rows, H, K, generator=gen)).clamp(-20, 20).to(dtype)
+    dy = torch.randn(rows, H, K, generator=gen)
+    A, bias = 0.5 * torch.randn(H, generator=gen), torch.randn(H * K, generator=gen)
+    want = _grads(lambda a, b, c: O.kda_gate_fwd(a, b, c, lower_bound), (g, A, bias), dy)
+    got = _grads(lambda a, b, c: kda_gate_fwd(a, b, c, lower_bound), (g.cuda(), A.cuda(), bias.cuda()), dy.cuda())
+    assert_close("y", got[0].cpu(), want[0], torch.float32)
+    assert_close("dg", got[1].float().cpu(), want[1].float(), dtype)
+    for name, a, r in (("dA_log", got[2], want[2]), ("dbias", got[3], want[3])):   # sums over rows: relative bar
+        assert ((a.cpu() - r).norm() / r.norm()).item() <= (1e-4 if dtype == torch.float32 else 1e-2), name
+    if lower_bound is None:
+        want = _grads(lambda a: O.gla_gate(a, 16.0, None), (g,), dy)
+        got = _grads(lambda a: gla_gate(a, 16.0, None), (g.cuda(),), dy.cuda())
+        for a, b in zip(got, want):
+            assert_close("gla_gate", a.float().cpu(), b.float(), dtype)
