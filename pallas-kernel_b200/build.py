@@ -2,7 +2,8 @@
 
 Usage: python pallas-kernel_b200/build.py [--force]
 Objects go to pallas-kernel_b200/build/, the shared library next to the
-Python package (tops_b200/libtops_b200.so) so that it travels with the tree.
+Python package (tops_b200/libtops_b200.so) so that it travels with the tree;
+the host path of the differentiable ops (torch_ext/torch_ops.cpp) beside it.
 """
 from __future__ import annotations
 
@@ -15,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "tops_b200", "libtops_b200.so")
+EXT = os.path.join(HERE, "tops_b200", "_torch_ops.so")
 OBJ = os.path.join(HERE, "build")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -35,6 +37,35 @@ def _deps_mtime():
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    lib = build_kernels(force, verbose)
+    build_torch_ops(force)
+    return lib
+
+
+def build_torch_ops(force: bool = False) -> str:
+    """_torch_ops.so: tensors -> C ABI and the autograd nodes, compiled against the installed torch."""
+    src = os.path.join(HERE, "torch_ext", "torch_ops.cpp")
+    deps = max(os.path.getmtime(src), os.path.getmtime(os.path.join(ROOT, "include", "tops_b200.h")))
+    if not force and os.path.exists(EXT) and os.path.getmtime(EXT) >= deps:
+        return EXT
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    inc = [os.path.join(ROOT, "include"), os.path.join(base, "include"),
+           os.path.join(base, "include", "torch", "csrc", "api", "include"), "/usr/local/cuda/include",
+           sysconfig.get_paths()["include"]]
+    libs = ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_torch_ops",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in inc), src, "-o", EXT,
+           "-L" + os.path.dirname(OUT), "-l:libtops_b200.so", "-L" + os.path.join(base, "lib"), *libs, "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    return EXT
+
+
+def build_kernels(force: bool = False, verbose: bool = False) -> str:
     if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= _deps_mtime():
         return OUT
     os.makedirs(OBJ, exist_ok=True)
@@ -68,7 +99,7 @@ def build_jax_shim() -> str | None:
     except Exception as exc:
         print(f"jax not found ({type(exc).__name__}: {exc}) - the jax.ffi shim is skipped")
         return None
-    lib = build()
+    lib = build_kernels()
     out = os.path.join(HERE, "tops_b200", "libtops_b200_jax.so")
     cmd = [NVCC, "-std=c++17", "-O2", "-shared", "-Xcompiler", "-fPIC", "-I" + inc, "-I" + os.path.join(ROOT, "include"),
            os.path.join(HERE, "jax_ffi", "jax_ffi_shim.cc"), "-o", out, "-L" + os.path.dirname(lib), "-l:libtops_b200.so",

@@ -2007,14 +2007,17 @@ int chunk_bwd(const tops_chunk_bwd_params& p, void* ws, size_t, cudaStream_t st)
 // ---------------------------------------------------------------------------
 namespace {
 
-// Time of a pass over runs of at most `cps` chunks, in chunks of the fused forward, with one block per SM: when
-// there are more blocks than SMs they follow one another, longest first, and the last ones to finish leave about
-// half a run of imbalance.
+// Time (us) of a pass over runs of chunks, one block per SM: a block costs `fixed` (its first loads, tensor memory, the
+// states in and out) plus `per` a chunk; when there are more blocks than SMs they follow one another, longest first,
+// and the last ones to finish leave some imbalance.  Measured: fused forward 28 us for runs of 6 chunks, 212 us for 64;
+// summary scan 18 us for 6, 1.1 us a chunk.
 struct RunCost { long long chunks = 0; int blocks = 0, longest = 0; };
-double pass_time(const RunCost& r, int sms) {
-  if (r.blocks <= sms) return r.longest;
-  const double even = (double)r.chunks / sms;
-  return r.longest > even + 0.5 * r.longest ? r.longest : even + 0.5 * r.longest;
+double pass_time(const RunCost& r, int sms, double fixed, double per) {
+  if (!r.blocks) return 0.0;
+  const double longest = fixed + per * r.longest;
+  if (r.blocks <= sms) return longest;
+  const double even = (fixed * r.blocks + per * r.chunks) / sms + 0.3 * longest;
+  return longest > even ? longest : even;
 }
 
 // Everything the launches of one call need to know about where chunks live.
@@ -2042,8 +2045,8 @@ struct GenPlan {
       longest = geo.NTseq = cdiv(pb.T, C);
       total_chunks = N * longest;
     }
-    // Cutting sequences into runs costs a summary pass (about 0.45 of the main pass per chunk) and a join (about
-    // two chunks' time); it pays when whole sequences would leave SMs idle.  Every candidate length is priced.
+    // Cutting sequences into runs costs a summary pass and a join (which moves three states per run); it pays when whole
+    // sequences would leave SMs idle.  Every candidate length is priced.
     const int sms = sm_count();
     cps = longest;
     double best = 1e30;
@@ -2059,7 +2062,8 @@ struct GenPlan {
           if (len > sum.longest) sum.longest = len;
         }
       }
-      const double t = pass_time(all, sms) + (sum.blocks ? 0.45 * pass_time(sum, sms) + 2.0 : 0.0);
+      const double join = sum.blocks ? 8.0 + 12.0 * sum.blocks / geo.VS * pb.K * pb.V / 4e6 : 0.0;
+      const double t = pass_time(all, sms, 9.0, 3.2) + pass_time(sum, sms, 11.0, 1.1) + join;
       if (t < best - 1e-9) { best = t; cps = c; }
     }
     if (nch.empty()) {

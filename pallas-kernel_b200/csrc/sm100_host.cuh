@@ -2,6 +2,7 @@
 // tensor maps of the two tensor shapes the kernels fetch, and per-device properties.
 #pragma once
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "sm100_prims.cuh"
@@ -126,10 +127,24 @@ inline DeviceInfo device_info() {
 inline int sm_count() { return device_info().sms; }
 inline bool device_is_sm100() { return device_info().sm100; }
 
+// Lets a kernel use `bytes` of dynamic shared memory, asked of the runtime once per kernel and device (about 1 us each
+// time otherwise, in front of every launch).
 template <class F>
 inline int opt_in_smem(F f, size_t bytes) {
+  struct Seen { const void* f; int dev; size_t bytes; };
+  static std::mutex mu;
+  static std::vector<Seen> seen;   // (one entry per kernel and device: a few dozen at most)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return TOPS_E_CUDA; }
+  const void* key = reinterpret_cast<const void*>(f);
+  std::lock_guard<std::mutex> lk(mu);
+  for (const Seen& s : seen)
+    if (s.f == key && s.dev == dev && s.bytes == bytes) return TOPS_OK;
   const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) return TOPS_OK;
+  if (e == cudaSuccess) {
+    seen.push_back(Seen{key, dev, bytes});
+    return TOPS_OK;
+  }
   record_cuda_error((int)e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
   return TOPS_E_CUDA;
 }

@@ -18,6 +18,11 @@ if not os.path.exists(_PATH):
         f"{_PATH} is missing: build it with `python pallas-kernel_b200/build.py` "
         "(tops_b200 has no CPU or eager fallback)")
 lib = C.CDLL(_PATH)
+try:
+    from . import _torch_ops as ops_ext   # the host path of the differentiable ops
+except ImportError as exc:
+    raise ImportError("tops_b200/_torch_ops.so is missing or does not load: build it with "
+                      f"`python pallas-kernel_b200/build.py` ({exc})") from exc
 
 F32, BF16, F16 = 0, 1, 2
 GATE_NONE, GATE_PER_CHANNEL, GATE_SCALAR, GATE_GAMMA = 0, 1, 2, 3
@@ -273,6 +278,7 @@ def raise_on_device_error(what: str = "tops_b200") -> None:
 # TOPS_B200_CHECK_DEVICE=1 makes every differentiable op check the device error word after its
 # backward pass (one synchronisation per step); off by default, the word stays readable at any time.
 CHECK_DEVICE = os.environ.get("TOPS_B200_CHECK_DEVICE", "0") not in ("", "0")
+ops_ext.configure(TopsError, CHECK_DEVICE)
 
 
 def on_tensor_device(fn):

@@ -7,7 +7,7 @@
 * `gla_gate`: `log_sigmoid(g) / normalizer` with an optional lower clip, the gate of the GLA
   layer (`tops/layers/gla.py:277-279`).
 
-All are differentiable (torch.autograd.Function over one forward and one backward kernel); `g` is
+All are differentiable (one forward and one backward kernel each); `g` is
 `[..., H, K]`, `A_log` `[H]`, `dt_bias` `[H*K]`.
 """
 from __future__ import annotations
@@ -17,6 +17,7 @@ import ctypes as C
 import torch
 
 from .. import _lib as L
+from .._lib import ops_ext as X
 
 
 def _fill(p, g, H, K, kind, A_log, dt_bias, lower_bound, normalizer, clamp_min, out_dtype):
@@ -29,35 +30,31 @@ def _fill(p, g, H, K, kind, A_log, dt_bias, lower_bound, normalizer, clamp_min, 
     p.has_clamp_min = int(clamp_min is not None)
 
 
-def _expand(A_log, dt_bias, H, K):
-    """Head-wise parameters of fewer heads are repeated (`tops/cpu/ops/kda/gate.py:20-57`)."""
+def _check_gate(g):
+    assert g.ndim >= 2, f"g must have at least 2 dims, got shape {tuple(g.shape)}"
+    assert g.shape[-1] % 4 == 0, "K must be a multiple of 4"
+
+
+def _check_params(A_log, dt_bias, H, K):
     assert A_log.ndim == 1, f"A_log must be 1D, got shape {tuple(A_log.shape)}"
     base = A_log.shape[0]
     assert H % base == 0, f"Effective heads {H} must be divisible by A_log heads {base}"
+    assert dt_bias is None or dt_bias.ndim == 1 and dt_bias.shape[0] in (base * K, H * K), \
+        f"dt_bias shape {tuple(dt_bias.shape)} incompatible with (base={base * K}, expanded={H * K})"
+    return base
+
+
+def _expand(A_log, dt_bias, H, K):
+    """Head-wise parameters of fewer heads are repeated (`tops/cpu/ops/kda/gate.py:20-57`)."""
+    base = _check_params(A_log, dt_bias, H, K)
     A = A_log.float().repeat_interleave(H // base).contiguous()
     b = None
     if dt_bias is not None:
-        assert dt_bias.ndim == 1 and dt_bias.shape[0] in (base * K, H * K), \
-            f"dt_bias shape {tuple(dt_bias.shape)} incompatible with (base={base * K}, expanded={H * K})"
         b = dt_bias.float()
         if b.shape[0] != H * K:
             b = b.reshape(base, K).repeat_interleave(H // base, dim=0).reshape(-1)
         b = b.contiguous()
     return A, b
-
-
-@L.on_tensor_device
-def _gate_fwd_call(g, kind, A, b, lower_bound, normalizer, clamp_min, out_dtype):
-    assert g.ndim >= 2, f"g must have at least 2 dims, got shape {tuple(g.shape)}"
-    H, K = g.shape[-2:]
-    assert K % 4 == 0, "K must be a multiple of 4"
-    g = g.contiguous()
-    out = torch.empty(g.shape, dtype=out_dtype, device=g.device)
-    p = L.GateActParams()
-    _fill(p, g, H, K, kind, A, b, lower_bound, normalizer, clamp_min, out_dtype)
-    p.out = L.ptr(out)
-    L.check(L.lib.tops_b200_gate_act_fwd(C.byref(p), L.stream_ptr(g.device)), "gate_act_fwd")
-    return out
 
 
 @L.on_tensor_device
@@ -95,25 +92,12 @@ def kda_gate_bwd(g, A_log, dt_bias=None, dyg=None, lower_bound=None):
     return dg, dA, db
 
 
-class _KdaGate(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, g, A_log, dt_bias, lower_bound, out_dtype):
-        H, K = g.shape[-2:]
-        A, b = _expand(A_log, dt_bias, H, K)
-        ctx.save_for_backward(g, A_log, dt_bias)
-        ctx.lower_bound = lower_bound
-        return _gate_fwd_call(g, _kind(lower_bound), A, b, lower_bound, 1.0, None, out_dtype)
-
-    @staticmethod
-    def backward(ctx, dy):
-        g, A_log, dt_bias = ctx.saved_tensors
-        dg, dA, db = kda_gate_bwd(g, A_log, dt_bias, dy, ctx.lower_bound)
-        return dg, dA, db, None, None
-
-
 def kda_gate_fwd(g, A_log, dt_bias=None, lower_bound=None, output_dtype=torch.float32):
     """KDA gate activation (`tops/cpu/ops/kda/gate.py:60-126`); differentiable in g, A_log, dt_bias."""
-    return _KdaGate.apply(g, A_log, dt_bias, lower_bound, output_dtype)
+    _check_gate(g)
+    H, K = g.shape[-2:]
+    _check_params(A_log, dt_bias, H, K)
+    return X.gate(g, A_log, dt_bias, _kind(lower_bound), 0.0 if lower_bound is None else float(lower_bound), 1.0, None, output_dtype)
 
 
 fused_kda_gate = kda_gate_fwd
@@ -131,21 +115,8 @@ def kda_gate_chunk_cumsum(g, A_log, chunk_size, scale=None, dt_bias=None, cu_seq
     return out.to(output_dtype)
 
 
-class _GlaGate(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, g, normalizer, clamp_min):
-        ctx.save_for_backward(g)
-        ctx.normalizer, ctx.clamp_min = normalizer, clamp_min
-        return _gate_fwd_call(g, L.GATE_ACT_LOG_SIGMOID, None, None, None, normalizer, clamp_min, g.dtype)
-
-    @staticmethod
-    def backward(ctx, dy):
-        (g,) = ctx.saved_tensors
-        dg, _, _ = _gate_bwd_call(g, dy, L.GATE_ACT_LOG_SIGMOID, None, None, None, ctx.normalizer, ctx.clamp_min, False)
-        return dg, None, None
-
-
 def gla_gate(g, gate_logit_normalizer=16.0, clamp_min=None):
     """`log_sigmoid(g) / gate_logit_normalizer`, clipped from below by `clamp_min` when given: the gate
     of the GLA layer (`tops/layers/gla.py:277-279`), in g's dtype.  Differentiable."""
-    return _GlaGate.apply(g, float(gate_logit_normalizer), clamp_min)
+    _check_gate(g)
+    return X.gate(g, None, None, L.GATE_ACT_LOG_SIGMOID, 0.0, float(gate_logit_normalizer), clamp_min, None)

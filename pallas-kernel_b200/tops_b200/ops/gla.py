@@ -5,7 +5,7 @@
 
 Tensors are CUDA tensors `[B, T, H, D]`; states `[N, H, K, V]` fp32.  The
 public `chunk_gla` / `fused_chunk_gla` / `fused_recurrent_gla` are
-differentiable (torch.autograd.Function standing where the reference's JAX ops
+differentiable (autograd nodes of the torch extension standing where the reference's JAX ops
 use / would use `custom_vjp`); the explicit `*_bwd` functions return the
 oracle's dtypes (dq, dk, dg fp32; dv in do.dtype).
 """
@@ -16,17 +16,19 @@ import ctypes as C
 import torch
 
 from .. import _lib as L
+from .._lib import ops_ext as X
 from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
 
 
 def _check_qkvg(q, k, v, g, initial_state, cu_seqlens):
-    assert q.ndim == 4, f"q must be [B,T,H,K], got {tuple(q.shape)}"
-    B, T, H, K = q.shape
-    assert k.shape == q.shape, f"k shape {tuple(k.shape)} != q shape {tuple(q.shape)}"
-    assert v.ndim == 4 and v.shape[:3] == q.shape[:3], f"v shape {tuple(v.shape)} incompatible with q"
+    shape, vshape = q.shape, v.shape
+    assert len(shape) == 4, f"q must be [B,T,H,K], got {tuple(shape)}"
+    B, T, H, K = shape
+    assert k.shape == shape, f"k shape {tuple(k.shape)} != q shape {tuple(shape)}"
+    assert len(vshape) == 4 and vshape[:3] == shape[:3], f"v shape {tuple(vshape)} incompatible with q"
     assert k.dtype == q.dtype and v.dtype == q.dtype, "q, k, v must share a dtype"
-    V = v.shape[-1]
-    assert g is None or g.shape == q.shape, f"g shape {tuple(g.shape)} != q shape {tuple(q.shape)}"
+    V = vshape[3]
+    assert g is None or g.shape == shape, f"g shape {tuple(g.shape)} != q shape {tuple(shape)}"
     N = B
     if cu_seqlens is not None:
         assert B == 1, f"B must be 1 for varlen, got {B}"
@@ -88,30 +90,6 @@ def _kernel_chunk(q, v, g, cu_seqlens, chunk_size):
     return min(max(chunk_size, 16), 64)
 
 
-class _ChunkGLA(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, g, initial_state, scale, output_final_state, cu, chunk_size):
-        # the tcgen05 forward keeps its chunk-start states for the backward (one bf16 [B,NT,H,K,V] tensor)
-        keep = any(t is not None and t.requires_grad for t in (q, k, v, g, initial_state))
-        o, ht, _, _, hs = chunk_fwd_call(q, k, v, g, L.GATE_PER_CHANNEL if g is not None else L.GATE_NONE,
-                                         scale, initial_state, output_final_state, chunk_size, cu, want_saved=keep)
-        ctx.save_for_backward(q, k, v, g, initial_state, hs)
-        ctx.scale, ctx.cu, ctx.chunk = scale, cu, chunk_size
-        return o, ht
-
-    @staticmethod
-    def backward(ctx, do, dht):
-        q, k, v, g, h0, hs = ctx.saved_tensors
-        kind = L.GATE_PER_CHANNEL if g is not None else L.GATE_NONE
-        # cotangents take the primal's dtype at this boundary
-        dq, dk, dv, dg, dh0 = chunk_bwd_call(q, k, v, g, kind, ctx.scale, h0, do.to(q.dtype), dht, ctx.chunk,
-                                             torch.float32, g is not None, h0 is not None, ctx.cu, h_saved=hs,
-                                             primal_dtypes=True)
-        if L.CHECK_DEVICE:
-            L.raise_on_device_error("chunk_gla backward")
-        return (dq, dk, dv, dg, None if h0 is None else dh0.to(h0.dtype), None, None, None, None)
-
-
 def chunk_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, output_final_state=False,
               cu_seqlens=None, chunk_size=16):
     """Chunked GLA (reference `tops/cpu/ops/gla/chunk.py:648-709`; the
@@ -128,11 +106,8 @@ def chunk_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, out
         gg = g_gamma.to(torch.float32)
         gg = gg.view(1, 1, H, 1) if gg.ndim == 1 and gg.shape[0] == H else gg
         g = torch.broadcast_to(gg, (B, T, H, K)).contiguous()
-    if initial_state is not None:
-        initial_state = initial_state.to(torch.float32)
-    o, ht = _ChunkGLA.apply(q, k, v, g, initial_state, float(scale), bool(output_final_state),
-                            _cu_list(cu_seqlens), int(_kernel_chunk(q, v, g, cu_seqlens, chunk_size)))
-    return o, (ht if output_final_state else None)
+    return X.chunk(q, k, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL, initial_state, float(scale),
+                   bool(output_final_state), _cu_list(cu_seqlens) or [], _kernel_chunk(q, v, g, cu_seqlens, chunk_size))
 
 
 def fused_chunk_gla(q, k, v, g=None, scale=None, initial_state=None, output_final_state=False,
@@ -173,13 +148,14 @@ def _rec_fwd_call(q, k, v, gk, gv, scale, initial_state, want_state, reverse, cu
 
 
 def _check_rec(q, k, v, gk, gv, initial_state, cu_seqlens):
-    B, T, H, K = q.shape
-    V = v.shape[-1]
+    shape, vshape = q.shape, v.shape
+    B, T, H, K = shape
+    V = vshape[-1]
     N = len(cu_seqlens) - 1 if cu_seqlens is not None else B
-    assert k.shape == (B, T, H, K), f"k shape {tuple(k.shape)} != expected {(B, T, H, K)}"
-    assert v.shape[:3] == (B, T, H), f"v shape {tuple(v.shape)} incompatible with q"
-    assert gk is None or gk.shape == (B, T, H, K), f"gk shape {tuple(gk.shape)} != expected {(B, T, H, K)}"
-    assert gv is None or gv.shape == (B, T, H, V), f"gv shape {tuple(gv.shape)} != expected {(B, T, H, V)}"
+    assert k.shape == shape, f"k shape {tuple(k.shape)} != expected {(B, T, H, K)}"
+    assert vshape[:3] == shape[:3], f"v shape {tuple(vshape)} incompatible with q"
+    assert gk is None or gk.shape == shape, f"gk shape {tuple(gk.shape)} != expected {(B, T, H, K)}"
+    assert gv is None or gv.shape == vshape, f"gv shape {tuple(gv.shape)} != expected {(B, T, H, V)}"
     assert initial_state is None or initial_state.shape == (N, H, K, V), \
         f"initial_state shape {tuple(initial_state.shape)} != expected {(N, H, K, V)}"
     assert cu_seqlens is None or B == 1, f"cu_seqlens requires B=1, got B={B}"
@@ -240,23 +216,6 @@ def fused_recurrent_bwd(q, k, v, gk=None, gv=None, o=None, do=None, dht=None, sc
     return dq, dk, dv, dgk, dgv, dh0
 
 
-class _FusedRecurrentGLA(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, gk, gv, initial_state, scale, output_final_state, reverse, cu):
-        o32, ht = _rec_fwd_call(q, k, v, gk, gv, scale, initial_state, output_final_state, reverse, cu,
-                                torch.float32)
-        ctx.save_for_backward(q, k, v, gk, gv, initial_state, o32 if gv is not None else None)
-        ctx.scale, ctx.reverse, ctx.cu = scale, reverse, cu
-        return o32.to(q.dtype), ht
-
-    @staticmethod
-    def backward(ctx, do, dht):
-        q, k, v, gk, gv, h0, o32 = ctx.saved_tensors
-        dq, dk, dv, dgk, dgv, dh0 = fused_recurrent_bwd(q, k, v, gk, gv, o32, do, dht, ctx.scale, h0,
-                                                        ctx.reverse, ctx.cu)
-        return dq, dk, dv, dgk, dgv, dh0, None, None, None, None
-
-
 def fused_recurrent_gla(q, k, v, gk=None, gv=None, scale=None, initial_state=None,
                         output_final_state=False, reverse=False, cu_seqlens=None):
     """Recurrent GLA (reference `tops/cpu/ops/gla/fused_recurrent.py:362-422`):
@@ -264,9 +223,9 @@ def fused_recurrent_gla(q, k, v, gk=None, gv=None, scale=None, initial_state=Non
     K = _check_rec(q, k, v, gk, gv, initial_state, cu_seqlens)
     if scale is None:
         scale = K ** -0.5
-    o, ht = _FusedRecurrentGLA.apply(q, k, v, gk, gv, initial_state, float(scale), bool(output_final_state),
-                                     bool(reverse), _cu_list(cu_seqlens))
-    return o, (ht if output_final_state else None)
+    assert gk is None or gv is None or gk.dtype == gv.dtype
+    return X.recurrent(q, k, v, gk, gv, float(scale), initial_state, bool(output_final_state), bool(reverse),
+                       _cu_list(cu_seqlens) or [])
 
 
 def fused_recurrent_gla_decode_(q, k, v, gk, state, scale=None, gv=None):
@@ -277,5 +236,4 @@ def fused_recurrent_gla_decode_(q, k, v, gk, state, scale=None, gv=None):
     assert state.dtype == torch.float32 and state.is_contiguous()
     if scale is None:
         scale = K ** -0.5
-    o, _ = _rec_fwd_call(q, k, v, gk, gv, scale, state, True, False, None, q.dtype, state_out=state)
-    return o
+    return X.recurrent_decode(q, k, v, gk, gv, float(scale), state)

@@ -17,17 +17,19 @@ import ctypes as C
 import torch
 
 from .. import _lib as L
+from .._lib import ops_ext as X
 
 
 def _check(q, k, v, g, beta, initial_state):
-    assert q.ndim == 4, f"q must be 4D [B,T,H,K], got {q.ndim}D"
-    B, T, H, K = q.shape
-    assert k.shape == q.shape, f"k shape {tuple(k.shape)} != q shape {tuple(q.shape)}"
-    assert v.ndim == 4 and v.shape[:3] == q.shape[:3], f"v shape {tuple(v.shape)} incompatible with q"
-    assert g.ndim == 4 and g.shape == q.shape, f"g shape {tuple(g.shape)} != q shape {tuple(q.shape)}"
-    assert beta.ndim == 3 and beta.shape == q.shape[:3], f"beta shape {tuple(beta.shape)} != {tuple(q.shape[:3])}"
+    shape, vshape = q.shape, v.shape
+    assert len(shape) == 4, f"q must be 4D [B,T,H,K], got {len(shape)}D"
+    B, T, H, K = shape
+    assert k.shape == shape, f"k shape {tuple(k.shape)} != q shape {tuple(shape)}"
+    assert len(vshape) == 4 and vshape[:3] == shape[:3], f"v shape {tuple(vshape)} incompatible with q"
+    assert g.shape == shape, f"g shape {tuple(g.shape)} != q shape {tuple(shape)}"
+    assert beta.shape == shape[:3], f"beta shape {tuple(beta.shape)} != {tuple(shape[:3])}"
     assert k.dtype == q.dtype and v.dtype == q.dtype, "q, k, v must share a dtype"
-    V = v.shape[-1]
+    V = vshape[3]
     assert K <= 256, "K <= 256 (reference: tops/ops/common/chunk_delta_h.py:952)"
     if initial_state is not None:
         assert initial_state.shape == (B, H, K, V), \
@@ -218,42 +220,12 @@ def chunk_kda_bwd(q, k, v, g, beta, do, scale=None, initial_state=None, dht=None
     return dq, dk, dv, dbeta, dg, dh0
 
 
-class _KDA(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, g, beta, initial_state, scale, output_final_state, chunked):
-        saved = None
-        if chunked:
-            keep = any(t is not None and t.requires_grad for t in (q, k, v, g, beta, initial_state))
-            o, ht, _, _, saved = _chunk_fwd_call(q, k, v, g, beta, scale, initial_state, output_final_state, 64, False,
-                                                 keep)
-        else:
-            o, ht = kda_fwd(q, k, v, g, beta, scale, initial_state, output_final_state)
-        ctx.save_for_backward(q, k, v, g, beta, initial_state, *(saved or ()))
-        ctx.scale, ctx.chunked = scale, saved is not None
-        return o, ht
-
-    @staticmethod
-    def backward(ctx, do, dht):
-        q, k, v, g, beta, h0 = ctx.saved_tensors[:6]
-        if ctx.chunked:
-            # cotangents take the primal's dtype at this boundary
-            dq, dk, dv, dg, dbeta, dh0 = _chunk_bwd_call(q, k, v, g, beta, do, ctx.scale, dht, ctx.saved_tensors[6:],
-                                                         h0 is not None, q.dtype)
-            if L.CHECK_DEVICE:
-                L.raise_on_device_error("chunk_kda backward")
-            return (dq, dk, dv, dg.to(g.dtype), dbeta.to(beta.dtype), None if h0 is None else dh0.to(h0.dtype),
-                    None, None, None)
-        dq, dk, dv, dg, dbeta, dh0 = kda_bwd(q, k, v, g, beta, do, ctx.scale, h0, dht)
-        return dq, dk, dv, dg, dbeta, None if h0 is None else dh0.to(h0.dtype), None, None, None
-
-
 def fused_recurrent_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False):
     """Token-serial KDA (reference `tops/ops/kda/fused_recurrent.py:19-105`)."""
     B, T, H, K, V = _check(q, k, v, g, beta, initial_state)
     if scale is None:
         scale = K ** -0.5
-    o, ht = _KDA.apply(q, k, v, g, beta, initial_state, float(scale), bool(output_final_state), False)
-    return o, (ht if output_final_state else None)
+    return X.kda(q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), False)
 
 
 def fused_recurrent_kda_decode_(q, k, v, g, beta, state, scale=None):
@@ -263,9 +235,7 @@ def fused_recurrent_kda_decode_(q, k, v, g, beta, state, scale=None):
     assert state.dtype == torch.float32 and state.is_contiguous()
     if scale is None:
         scale = K ** -0.5
-    with torch.no_grad():
-        o, _ = kda_fwd(q, k, v, g, beta, float(scale), state, True, state_out=state)
-    return o
+    return X.kda_decode(q, k, v, g, beta, float(scale), state)
 
 
 def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None,
@@ -280,6 +250,4 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
         scale = K ** -0.5
     # the result does not depend on the chunk length beyond where roundings fall: a problem the
     # tensor-core kernels take runs with their chunk of 64
-    chunked = T % 64 == 0 and chunk_kernels_take(q, k, v, g, beta, 64)
-    o, ht = _KDA.apply(q, k, v, g, beta, initial_state, float(scale), bool(output_final_state), chunked)
-    return o, (ht if output_final_state else None)
+    return X.kda(q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), True)

@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib as L
+from .._lib import ops_ext as X
 from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
 from .gla import fused_recurrent_gla
 
@@ -95,28 +96,6 @@ def chunk_simple_gla_bwd(q, k, v, g, g_gamma, initial_state, do, dht, scale, chu
                           g is not None, initial_state is not None, _cu(cu_seqlens), h_saved=h_saved)
 
 
-class _ChunkSimpleGLA(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, g, g_gamma, initial_state, scale, output_final_state, cu, chunk_size):
-        keep = any(t is not None and t.requires_grad for t in (q, k, v, g, initial_state))
-        o, ht, hs = _fwd(q, k, v, g, g_gamma, scale, initial_state, output_final_state, chunk_size, cu, keep)
-        ctx.save_for_backward(q, k, v, g, g_gamma, initial_state, hs)
-        ctx.scale, ctx.cu, ctx.chunk = scale, cu, chunk_size
-        return o, ht
-
-    @staticmethod
-    def backward(ctx, do, dht):
-        q, k, v, g, g_gamma, h0, hs = ctx.saved_tensors
-        dq, dk, dv, dg, dh0 = chunk_simple_gla_bwd(q, k, v, g, g_gamma, h0, do.to(q.dtype), dht, ctx.scale, ctx.chunk,
-                                                   ctx.cu, h_saved=hs)
-        # a constant decay gets a zero cotangent, as in the reference (tops/ops/simple_gla/chunk.py:764)
-        if L.CHECK_DEVICE:
-            L.raise_on_device_error("chunk_simple_gla backward")
-        dgamma = None if g_gamma is None else torch.zeros_like(g_gamma)
-        return (dq, dk, dv, None if g is None else dg.to(g.dtype), dgamma,
-                None if h0 is None else dh0.to(h0.dtype), None, None, None, None)
-
-
 def chunk_simple_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, output_final_state=False,
                      cu_seqlens=None, chunk_size=64):
     """Chunked simple_gla (reference `tops/cpu/ops/simple_gla/chunk.py:796-889`;
@@ -125,12 +104,11 @@ def chunk_simple_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=No
     K = _check(q, k, v, g, g_gamma, initial_state, cu_seqlens)
     if scale is None:
         scale = K ** -0.5
-    if initial_state is not None:
-        initial_state = initial_state.to(torch.float32)
+    gate, kind = _gate(g, g_gamma)
     chunk_size = _kernel_chunk(chunk_size)
-    o, ht = _ChunkSimpleGLA.apply(q, k, v, g, g_gamma, initial_state, float(scale), bool(output_final_state),
-                                  _cu(cu_seqlens), int(chunk_size))
-    return o, (ht if output_final_state else None)
+    if tensor_core_shape(q, v, gate, kind):
+        chunk_size = 64
+    return X.chunk(q, k, v, gate, kind, initial_state, float(scale), bool(output_final_state), _cu(cu_seqlens) or [], chunk_size)
 
 
 def fused_chunk_simple_gla(q, k, v, g_gamma=None, initial_state=None, scale=None, output_final_state=False,
