@@ -204,6 +204,96 @@ __global__ void __launch_bounds__(NTH) k_state_scan(ScanArgs<T> a) {
 }
 
 // ===========================================================================
+// The same states, chunk-parallel: every chunk's own contribution x~^T y first, then a running sum over the chunks
+// ===========================================================================
+// The serial scan above walks a sequence with K/64 x V/64 blocks per (sequence, head) and pays a full load latency and
+// two barriers per chunk (3.6 us at C = 16): with few heads most of the GPU idles.  Here k_chunk_products computes all
+// chunks at once and k_chunk_states adds them up, one thread per four state elements, its loads independent of the sum.
+// It costs two more passes over the states, so it serves the problems whose serial scan would not fill the GPU.
+// fp32, B = 2, T = 512, H = 4, K = V = 64, C = 16: 117 -> PAR_US us for both kernels.
+template <class T, int C, bool BWD>
+__global__ void __launch_bounds__(NTH) k_chunk_products(ScanArgs<T> a, float* __restrict__ D, float* __restrict__ decay) {
+  __shared__ float xs[C * LD];
+  __shared__ float ys[C * LD];
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int tilesV = (a.V + BT - 1) / BT;
+  const int k0 = (blockIdx.y / tilesV) * BT, v0 = (blockIdx.y % tilesV) * BT, h = blockIdx.z;
+  const ChunkPos p = chunk_global(a.m, blockIdx.x);
+  const bool per_ch = a.gate.kind == TOPS_GATE_PER_CHANNEL;
+  for (int idx = tid; idx < C * BT; idx += NTH) {
+    const int i = idx / BT, c = idx % BT;
+    float xv = 0.f, yv = 0.f;
+    const size_t tok = (size_t)p.batch * a.m.T + p.t0 + i;
+    if (i < p.len) {
+      if (k0 + c < a.K) {
+        const float raw = to_f(a.x[(tok * a.H + h) * a.K + k0 + c]);
+        const float gi = a.gate.at(p, a.m.T, h, i, k0 + c);
+        if (!BWD) xv = per_ch ? round_to<T>(raw * expf(a.gate.at(p, a.m.T, h, C - 1, k0 + c) - gi)) : raw;
+        else xv = per_ch ? round_to<T>(raw * a.scale * expf(gi)) : round_to<T>(round_to<T>(raw * a.scale) * expf(gi));
+      }
+      if (v0 + c < a.V) {
+        float raw = to_f(a.y[(tok * a.H + h) * a.V + v0 + c]);
+        if (!BWD && !per_ch && a.gate.kind != TOPS_GATE_NONE) {
+          const float gi = a.gate.at(p, a.m.T, h, i, 0);
+          raw = round_to<T>(raw * expf(a.gate.at(p, a.m.T, h, C - 1, 0) - gi));
+        }
+        yv = raw;
+      }
+    }
+    xs[i * LD + c] = xv;
+    ys[i * LD + c] = yv;
+  }
+  const size_t slot = ((size_t)p.batch * a.m.NT + p.slot) * a.H + h;
+  if (v0 == 0 && tid < BT && k0 + tid < a.K) decay[slot * a.K + k0 + tid] = expf(a.gate.at(p, a.m.T, h, C - 1, k0 + tid));
+  __syncthreads();
+  float acc[4][4];
+  zero(acc);
+  tile_mma<4, 4>(acc, C, [&](int r, int i) { return xs[i * LD + r]; }, [&](int i, int c) { return ys[i * LD + c]; });
+  float* dst = D + slot * a.K * (size_t)a.V;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int kk = k0 + ty + 16 * i, vv = v0 + tx + 16 * j;
+      if (kk < a.K && vv < a.V) dst[(size_t)kk * a.V + vv] = acc[i][j];
+    }
+}
+
+// D may be the states' own memory (fp32 states): a thread reads its element of a chunk before it writes it.
+template <class T, bool BWD>
+__global__ void __launch_bounds__(NTH) k_chunk_states(ScanArgs<T> a, const float* D, const float* __restrict__ decay) {
+  constexpr int U = 8;   // chunks whose loads are in flight together
+  const int n = blockIdx.y / a.H, h = blockIdx.y % a.H;
+  const int e = blockIdx.x * NTH + threadIdx.x, KV = a.K * a.V;
+  if (e >= KV) return;
+  const int k = e / a.V, nch = chunks_in_seq(a.m, n);
+  float S = a.s0 ? a.s0[((size_t)n * a.H + h) * KV + e] : 0.f;
+  const ChunkPos p0 = chunk_in_seq(a.m, n, 0);
+  const size_t base = ((size_t)p0.batch * a.m.NT + p0.slot) * a.H + h;   // chunks of a sequence are H slots apart
+  for (int s0 = 0; s0 < nch; s0 += U) {
+    float d[U], w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s0 + u < nch) {
+        const size_t slot = base + (size_t)(BWD ? nch - 1 - s0 - u : s0 + u) * a.H;
+        d[u] = D[slot * KV + e];
+        w[u] = decay[slot * a.K + k];
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s0 + u < nch) {
+        const size_t slot = base + (size_t)(BWD ? nch - 1 - s0 - u : s0 + u) * a.H;
+        if (a.states) {
+          if (a.states_f32) reinterpret_cast<float*>(a.states)[slot * KV + e] = S;
+          else reinterpret_cast<T*>(a.states)[slot * KV + e] = from_f<T>(S);
+        }
+        S = fmaf(S, w[u], d[u]);
+      }
+  }
+  if (a.s_final) a.s_final[((size_t)n * a.H + h) * KV + e] = S;
+}
+
+// ===========================================================================
 // Forward output: A = tril(q~ k~^T) * scale, o = scale * qg h + A v
 // ===========================================================================
 template <class T>
@@ -651,14 +741,45 @@ int launch_prepare_chunks(const int32_t* cu, int N, int C, int32_t* cs, int32_t*
   return post_launch();
 }
 
+// Whether the states of a problem are computed chunk-parallel: more than a few chunks to walk and a serial scan that
+// would leave SMs idle.
+bool parallel_scan(const Problem& pb) {
+  return pb.total_chunks >= 4 * pb.m.N && cdiv(pb.K, BT) * cdiv(pb.V, BT) * pb.m.N * pb.H < 2 * 148 &&
+         pb.m.N * (long long)pb.H <= 65535 && pb.H <= 65535;
+}
+size_t scan_scratch_floats(const Problem& pb, bool states_f32) {
+  if (!parallel_scan(pb)) return 0;
+  const size_t n = (size_t)pb.total_chunks * pb.H * pb.K;
+  return align_up(n * 4) / 4 + (states_f32 ? 0 : n * pb.V);
+}
+
 template <class T, int C>
 static int scan_T(const Problem& pb, bool bwd, const void* x, const void* y, const float* s0, void* states,
-                  int states_f32, float* s_final, cudaStream_t st) {
+                  int states_f32, float* s_final, float* scratch, cudaStream_t st) {
   ScanArgs<T> a;
   a.m = pb.m; a.gate = Gate{pb.gcum, pb.gate_kind, pb.H, pb.K}; a.H = pb.H; a.K = pb.K; a.V = pb.V;
   a.x = (const T*)x; a.y = (const T*)y; a.s0 = s0; a.states = states; a.states_f32 = states_f32;
   a.s_final = s_final; a.scale = pb.scale;
-  dim3 grid(cdiv(pb.K, BT) * cdiv(pb.V, BT), pb.m.N * pb.H);
+  const int tiles = cdiv(pb.K, BT) * cdiv(pb.V, BT);
+  if (scratch && parallel_scan(pb)) {
+    float* decay = scratch;
+    float* D = (states && states_f32) ? reinterpret_cast<float*>(states)
+                                      : scratch + align_up((size_t)pb.total_chunks * pb.H * pb.K * 4) / 4;
+    {
+      KernelScope ks(bwd ? "generic_chunk_products_dh" : "generic_chunk_products_h", st);
+      const dim3 grid(pb.total_chunks, tiles, pb.H);
+      if (bwd) k_chunk_products<T, C, true><<<grid, NTH, 0, st>>>(a, D, decay);
+      else k_chunk_products<T, C, false><<<grid, NTH, 0, st>>>(a, D, decay);
+      const int rc = post_launch();
+      if (rc) return rc;
+    }
+    KernelScope ks(bwd ? "generic_chunk_states_dh" : "generic_chunk_states_h", st);
+    const dim3 grid(cdiv(pb.K * pb.V, NTH), pb.m.N * pb.H);
+    if (bwd) k_chunk_states<T, true><<<grid, NTH, 0, st>>>(a, D, decay);
+    else k_chunk_states<T, false><<<grid, NTH, 0, st>>>(a, D, decay);
+    return post_launch();
+  }
+  dim3 grid(tiles, pb.m.N * pb.H);
   KernelScope ks(bwd ? "generic_scan_dh" : "generic_scan_h", st);
   if (bwd) k_state_scan<T, C, true><<<grid, NTH, 0, st>>>(a);
   else k_state_scan<T, C, false><<<grid, NTH, 0, st>>>(a);
@@ -740,8 +861,8 @@ static int bwd_T(const Problem& pb, const BwdBuffers& b, cudaStream_t st) {
   } while (0)
 
 int launch_scan(const Problem& pb, bool bwd, const void* x, const void* y, const float* s0, void* states,
-                int states_f32, float* s_final, cudaStream_t st) {
-  DISPATCH_T_C(pb, (scan_T<T, C>(pb, bwd, x, y, s0, states, states_f32, s_final, st)));
+                int states_f32, float* s_final, float* scratch, cudaStream_t st) {
+  DISPATCH_T_C(pb, (scan_T<T, C>(pb, bwd, x, y, s0, states, states_f32, s_final, scratch, st)));
 }
 
 int launch_fwd_o(const Problem& pb, const void* q, const void* k, const void* v, const void* h, int h_f32,

@@ -31,8 +31,10 @@ int launch_cumsum(const SeqMap& m, int H, int D, int dtype, int reverse, const v
 int launch_prepare_chunks(const int32_t* cu, int N, int C, int32_t* cs, int32_t* chunk_seq, cudaStream_t st);
 // forward (bwd=false): x=k, y=v, s0=h0, states=h, s_final=ht
 // reverse (bwd=true):  x=q, y=do, s0=dht, states=dh, s_final=dh0
+// scratch: scan_scratch_floats() of it, or null (then the chunks are walked one after another)
+size_t scan_scratch_floats(const Problem& pb, bool states_f32);
 int launch_scan(const Problem& pb, bool bwd, const void* x, const void* y, const float* s0, void* states,
-                int states_f32, float* s_final, cudaStream_t st);
+                int states_f32, float* s_final, float* scratch, cudaStream_t st);
 int launch_fwd_o(const Problem& pb, const void* q, const void* k, const void* v, const void* h, int h_f32,
                  void* o, float* A_out, int round_A, cudaStream_t st);
 int launch_bwd(const Problem& pb, const BwdBuffers& b, cudaStream_t st);

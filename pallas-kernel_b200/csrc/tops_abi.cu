@@ -253,7 +253,7 @@ extern "C" int tops_b200_chunk_fwd_h(const tops_fwd_h_params* p, void* stream) {
   Problem pb;
   if ((rc = make_problem(p->pb, cv, (cudaStream_t)stream, &pb, true))) return rc;
   pb.gcum = p->g_cumsum;
-  return generic::launch_scan(pb, false, p->k, p->v, p->h0, p->h, p->h_dtype == TOPS_F32, p->ht,
+  return generic::launch_scan(pb, false, p->k, p->v, p->h0, p->h, p->h_dtype == TOPS_F32, p->ht, nullptr,
                               (cudaStream_t)stream);
 }
 
@@ -267,12 +267,12 @@ extern "C" int tops_b200_chunk_bwd_dh(const tops_bwd_dh_params* p, void* stream)
   Problem pb;
   if ((rc = make_problem(p->pb, cv, (cudaStream_t)stream, &pb, true))) return rc;
   pb.gcum = p->g_cumsum;
-  return generic::launch_scan(pb, true, p->q, p->do_, p->dht, p->dh, 1, p->dh0, (cudaStream_t)stream);
+  return generic::launch_scan(pb, true, p->q, p->do_, p->dht, p->dh, 1, p->dh0, nullptr, (cudaStream_t)stream);
 }
 
 // ---- forward ----------------------------------------------------------------
 static size_t fwd_layout(const tops_chunk_fwd_params* p, void* ws, cudaStream_t st, bool launch, Problem* pb,
-                         float** gcum, void** h, int* rc_out) {
+                         float** gcum, void** h, float** scratch, int* rc_out) {
   Carver cv(ws);
   int rc = make_problem(p->pb, cv, st, pb, launch);
   if (rc_out) *rc_out = rc;
@@ -281,8 +281,10 @@ static size_t fwd_layout(const tops_chunk_fwd_params* p, void* ws, cudaStream_t 
   if (p->g_cumsum_out == nullptr && ge != 0 && ws == nullptr) g = nullptr;
   char* hh = p->h_out ? reinterpret_cast<char*>(p->h_out)
                       : reinterpret_cast<char*>(cv.take<char>(state_elems(p->pb) * dtype_size(p->pb.dtype)));
+  float* sc = cv.take<float>(generic::scan_scratch_floats(*pb, p->pb.dtype == TOPS_F32));
   if (gcum) *gcum = g;
   if (h) *h = hh;
+  if (scratch) *scratch = sc;
   return cv.off;
 }
 
@@ -292,7 +294,7 @@ extern "C" size_t tops_b200_chunk_fwd_workspace_bytes(const tops_chunk_fwd_param
   if (f == FAMILY_PLAIN) return sm100::fwd_workspace_bytes(*p);
   if (f == FAMILY_GENERAL) return sm100::gen_fwd_workspace_bytes(*p);
   Problem pb;
-  return fwd_layout(p, nullptr, nullptr, false, &pb, nullptr, nullptr, nullptr) + 256;
+  return fwd_layout(p, nullptr, nullptr, false, &pb, nullptr, nullptr, nullptr, nullptr) + 256;
 }
 
 extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* workspace, size_t workspace_bytes,
@@ -311,7 +313,8 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
   Problem pb;
   float* gcum = nullptr;
   void* h = nullptr;
-  fwd_layout(p, workspace, st, true, &pb, &gcum, &h, &rc);
+  float* scratch = nullptr;
+  fwd_layout(p, workspace, st, true, &pb, &gcum, &h, &scratch, &rc);
   if (rc) return rc;
   if (p->pb.gate_kind == TOPS_GATE_PER_CHANNEL || p->pb.gate_kind == TOPS_GATE_SCALAR) {
     int D = p->pb.gate_kind == TOPS_GATE_PER_CHANNEL ? p->pb.K : 1;
@@ -320,7 +323,7 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
   } else if (p->pb.gate_kind == TOPS_GATE_GAMMA) {
     pb.gcum = reinterpret_cast<const float*>(p->g);
   }
-  if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, h, 0, p->ht, st))) return rc;
+  if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, h, p->pb.dtype == TOPS_F32, p->ht, scratch, st))) return rc;
   int round_A = p->pb.gate_kind == TOPS_GATE_PER_CHANNEL || p->pb.gate_kind == TOPS_GATE_NONE;
   return generic::launch_fwd_o(pb, p->q, p->k, p->v, h, 0, p->o, p->A_out, round_A, st);
 }
@@ -370,6 +373,7 @@ struct BwdLayout {
   float *gcum, *h, *dh, *A, *dA, *dg_part;
   size_t dg_stride;
   int tilesK;
+  float* scratch;
 };
 
 static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t st, bool launch, Problem* pb,
@@ -389,6 +393,7 @@ static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t 
   l.tilesK = cdiv(p->pb.K, 64);
   l.dg_stride = (size_t)p->pb.B * p->pb.T * p->pb.H;
   l.dg_part = p->pb.gate_kind == TOPS_GATE_SCALAR ? cv.take<float>(l.dg_stride * l.tilesK) : nullptr;
+  l.scratch = cv.take<float>(generic::scan_scratch_floats(*pb, true));
   if (L) *L = l;
   return cv.off;
 }
@@ -429,8 +434,8 @@ extern "C" int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* wor
   } else if (kind == TOPS_GATE_GAMMA) {
     pb.gcum = reinterpret_cast<const float*>(p->g);
   }
-  if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, L.h, 1, nullptr, st))) return rc;
-  if ((rc = generic::launch_scan(pb, true, p->q, p->do_, p->dht, L.dh, 1, p->dh0, st))) return rc;
+  if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, L.h, 1, nullptr, L.scratch, st))) return rc;
+  if ((rc = generic::launch_scan(pb, true, p->q, p->do_, p->dht, L.dh, 1, p->dh0, L.scratch, st))) return rc;
   BwdBuffers b{};
   b.q = p->q; b.k = p->k; b.v = p->v; b.do_ = p->do_; b.A = L.A; b.dA = L.dA; b.h = L.h; b.dh = L.dh;
   b.dq = p->dq; b.dk = p->dk; b.dv = p->dv; b.grad_dtype = p->grad_dtype;
