@@ -186,6 +186,10 @@ typedef struct {
    * call (reverse = 0) on this same problem left behind.  It holds the time segments' summaries, so the
    * forward skips its own summary scan and only chains the segments from `h0`.  NULL otherwise. */
   void* segments;
+  /* Optional: elements between consecutive tokens of q, k and v when they are column ranges of one wider matrix (the
+   * output of one projection); 0: contiguous tensors.  tcgen05 kernels only (TOPS_E_UNSUPPORTED otherwise); a multiple
+   * of 8, every pointer 16-byte aligned. */
+  int64_t pitch;
 } tops_chunk_fwd_params;
 /* Which kernel family TOPS_IMPL_AUTO resolves to for this problem on the current device. */
 int tops_b200_chunk_selected_impl(const tops_chunk_problem* pb);
@@ -263,6 +267,8 @@ typedef struct {
   /* The same for the reverse scan: the workspace of a `tops_b200_chunk_state_exchange_pack` call with
    * reverse = 1 (x = q, y = do, the same scale) on this problem.  NULL otherwise. */
   void* rev_segments;
+  int64_t pitch;      /* of q, k, v: see tops_chunk_fwd_params */
+  int64_t grad_pitch; /* the same for dq, dk and dv */
 } tops_chunk_bwd_params;
 size_t tops_b200_chunk_bwd_workspace_bytes(const tops_chunk_bwd_params* p);
 int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* workspace, size_t workspace_bytes,
@@ -289,6 +295,7 @@ typedef struct {
   void* o;
   const int32_t* cu_seqlens;
   int32_t N;
+  int64_t pitch; /* elements between consecutive tokens of q, k and v (column ranges of one matrix); 0: contiguous */
 } tops_recurrent_fwd_params;
 int tops_b200_fused_recurrent_gla_fwd(const tops_recurrent_fwd_params* p, void* stream);
 
@@ -494,9 +501,36 @@ typedef struct {
   int32_t dy_dtype;
   void* dg;                 /* [rows,H,K] in fwd.dtype */
   float* dA_log;            /* [H] or NULL */
-  float* dbias;             /* [H*K] or NULL */
+  float* dbias;             /* [H*K] or NULL; every kind: the column sums of dg */
 } tops_gate_act_bwd_params;
 int tops_b200_gate_act_fwd(const tops_gate_act_params* p, void* stream);
+/* The low-rank gate of the GLA layer (`tops/layers/gla.py:153-156,277-279`) in one pass: x = low W^T + bias (fp32
+ * sums, rounded to the dtype), y = log_sigmoid(x) / normalizer, optionally clipped.  low [rows, R] with `low_pitch`
+ * elements between rows, W [N, R], bias [N], x and y [rows, N] (x may be NULL); all of one dtype; R <= 64, R and N
+ * multiples of 8. */
+typedef struct {
+  int64_t rows, low_pitch;
+  int32_t R, N, dtype;
+  const void *low, *W, *bias;
+  float normalizer, clamp_min;
+  int32_t has_clamp_min;
+  void *x, *y;
+} tops_lowrank_gate_params;
+int tops_b200_lowrank_gate_fwd(const tops_lowrank_gate_params* p, void* stream);
+/* Linear projections of at most 64 rows: y_m = x W_m^T for `count` weight matrices [N_m, K] (bf16, contiguous, fp32
+ * accumulation), x [rows, K] with `x_pitch` elements between rows, y_m [rows, N_m] with y_pitch[m].  K a multiple of
+ * 32; x and W_m 16-byte aligned.  The projections around one decode step of the layer (`tops/layers/gla.py:190-345`). */
+#define TOPS_SKINNY_MAX 6
+typedef struct {
+  int32_t rows, K, count;
+  int64_t x_pitch;
+  const void* x;
+  const void* W[TOPS_SKINNY_MAX];
+  void* y[TOPS_SKINNY_MAX];
+  int32_t N[TOPS_SKINNY_MAX];
+  int64_t y_pitch[TOPS_SKINNY_MAX];
+} tops_skinny_linear_params;
+int tops_b200_skinny_linear(const tops_skinny_linear_params* p, void* stream);
 size_t tops_b200_gate_act_bwd_workspace_bytes(const tops_gate_act_bwd_params* p);
 int tops_b200_gate_act_bwd(const tops_gate_act_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream);
 
@@ -522,6 +556,11 @@ typedef struct {
   void* dx;             /* backward */
   void* dgate;          /* rmsnorm_gated backward */
   float* dweight;       /* rmsnorm_gated backward, may be NULL */
+  /* rmsnorm_gated: the gate (and dgate) may be column ranges of a wider matrix: row r is head r % heads of token
+   * r / heads, at token * pitch + head * D.  0: contiguous. */
+  int64_t gate_pitch, dgate_pitch;
+  int32_t heads;
+  int32_t weight_dtype; /* of weight: TOPS_F32 (0) or any other */
 } tops_norm_params;
 int tops_b200_l2norm_fwd(const tops_norm_params* p, void* stream);
 int tops_b200_l2norm_bwd(const tops_norm_params* p, void* stream);

@@ -44,8 +44,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 def build_torch_ops(force: bool = False) -> str:
     """_torch_ops.so: tensors -> C ABI and the autograd nodes, compiled against the installed torch."""
-    src = os.path.join(HERE, "torch_ext", "torch_ops.cpp")
-    deps = max(os.path.getmtime(src), os.path.getmtime(os.path.join(ROOT, "include", "tops_b200.h")))
+    ext = os.path.join(HERE, "torch_ext")
+    srcs = sorted(f for f in os.listdir(ext) if f.endswith(".cpp"))
+    deps = max(os.path.getmtime(f) for f in [os.path.join(ROOT, "include", "tops_b200.h"),
+                                             *(os.path.join(ext, f) for f in os.listdir(ext))])
     if not force and os.path.exists(EXT) and os.path.getmtime(EXT) >= deps:
         return EXT
     import sysconfig
@@ -56,12 +58,24 @@ def build_torch_ops(force: bool = False) -> str:
            os.path.join(base, "include", "torch", "csrc", "api", "include"), "/usr/local/cuda/include",
            sysconfig.get_paths()["include"]]
     libs = ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_torch_ops",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in inc), src, "-o", EXT,
-           "-L" + os.path.dirname(OUT), "-l:libtops_b200.so", "-L" + os.path.join(base, "lib"), *libs, "-Wl,-rpath,$ORIGIN"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    os.makedirs(OBJ, exist_ok=True)
+
+    def run(cmd):
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed:\n{r.stdout}\n{r.stderr}")
+
+    def compile_one(src):
+        obj = os.path.join(OBJ, "torch_" + src[:-4] + ".o")
+        run(["g++", "-O2", "-std=c++17", "-fPIC", "-DTORCH_EXTENSION_NAME=_torch_ops",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in inc), "-c",
+             os.path.join(ext, src), "-o", obj])
+        return obj
+
+    with ThreadPoolExecutor(max_workers=4) as ex:
+        objs = list(ex.map(compile_one, srcs))
+    run(["g++", "-shared", "-o", EXT, *objs, "-L" + os.path.dirname(OUT), "-l:libtops_b200.so",
+         "-L" + os.path.join(base, "lib"), *libs, "-Wl,-rpath,$ORIGIN"])
     return EXT
 
 

@@ -83,6 +83,11 @@ template <class T, int VW> struct HalfVec {
       v[2 * i] = a.x; v[2 * i + 1] = a.y;
     }
   }
+  static __device__ __forceinline__ void load(const T* p, float (&v)[VW]) {
+    Raw r;
+    load(p, r);
+    widen(r, v);
+  }
   static __device__ __forceinline__ void store(T* p, const float (&v)[VW]) {
     if constexpr (VW == 8)
       *reinterpret_cast<uint4*>(p) = make_uint4(Pair<T>::put(v[0], v[1]), Pair<T>::put(v[2], v[3]), Pair<T>::put(v[4], v[5]),
@@ -430,11 +435,32 @@ __global__ void __launch_bounds__(256) k_l2norm_bwd(const T* __restrict__ x, con
   }
 }
 
+// the gate's rows: contiguous (pitch 0), or heads of tokens `pitch` elements apart
+struct RowPitch {
+  long long pitch;
+  int heads;
+  __device__ __forceinline__ size_t at(size_t row, int D) const {
+    if (!pitch) return row * D;
+    const unsigned r = (unsigned)row, tok = r / (unsigned)heads;
+    return (size_t)tok * pitch + (size_t)(r - tok * heads) * D;
+  }
+};
+struct NormWeight {
+  const void* p;
+  int dtype;
+  template <int VW> __device__ __forceinline__ void load(int c, float (&v)[VW]) const {
+    if (dtype == TOPS_F32) Vec<float, VW>::load(reinterpret_cast<const float*>(p) + c, v);
+    else
+#pragma unroll
+      for (int t = 0; t < VW; ++t) v[t] = load_any(p, dtype, c + t);
+  }
+};
+
 // gated RMS norm: y = x rsqrt(mean(x^2) + eps) w silu(g)
 template <class T, int VW, int NV, int LG>
 __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__ x, const T* __restrict__ g,
-                                                           const float* __restrict__ w, T* __restrict__ y, size_t rows, int D,
-                                                           float eps) {
+                                                           NormWeight w, T* __restrict__ y, size_t rows, int D, float eps,
+                                                           RowPitch gp) {
   constexpr int U = rows_in_flight2<NV>();
   constexpr int LPR = 1 << LG, per = 256 / LPR;
   const int lr = threadIdx.x & (LPR - 1);
@@ -448,7 +474,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__
       Vec<T, VW>::clear(rx[u][n]);
       if (r0 + u * per < rows && c < D) {
         Vec<T, VW>::load(x + (r0 + u * per) * D + c, rx[u][n]);
-        Vec<T, VW>::load(g + (r0 + u * per) * D + c, rg[u][n]);
+        Vec<T, VW>::load(g + gp.at(r0 + u * per, D) + c, rg[u][n]);
       }
     }
   const float invD = 1.f / (float)D;
@@ -473,7 +499,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__
           Vec<T, VW>::widen(rg[u][n], gv);
 #pragma unroll
           for (int t = 0; t < VW; ++t) wv[t] = 1.f;
-          if (w) Vec<float, VW>::load(w + c, wv);
+          if (w.p) w.load<VW>(c, wv);
 #pragma unroll
           for (int t = 0; t < VW; ++t) o[t] = v[n][t] * r * wv[t] * (gv[t] * sigmoidf(gv[t]));
           Vec<T, VW>::store(y + row * D + c, o);
@@ -487,9 +513,9 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__
 // a block adds its threads' in order and leaves one partial row in part_w[block][D].
 template <class T, int VW, int NV, int LG>
 __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__ x, const T* __restrict__ g,
-                                                           const float* __restrict__ w, const T* __restrict__ dy,
-                                                           T* __restrict__ dx, T* __restrict__ dg, float* __restrict__ part_w,
-                                                           size_t rows, int D, float eps) {
+                                                           NormWeight w, const T* __restrict__ dy, T* __restrict__ dx,
+                                                           T* __restrict__ dg, float* __restrict__ part_w, size_t rows, int D,
+                                                           float eps, RowPitch gp, RowPitch dgp) {
   extern __shared__ float dw_sm[];   // [256 / LPR][D]
   constexpr int LPR = 1 << LG, per = 256 / LPR;
   const int lr = threadIdx.x & (LPR - 1), grp = threadIdx.x / LPR;
@@ -511,7 +537,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__
       Vec<T, VW>::clear(rd[n]);
       if (row < rows && c < D) {
         Vec<T, VW>::load(x + row * D + c, rx[n]);
-        Vec<T, VW>::load(g + row * D + c, rg[n]);
+        Vec<T, VW>::load(g + gp.at(row, D) + c, rg[n]);
         Vec<T, VW>::load(dy + row * D + c, rd[n]);
       }
     }
@@ -533,7 +559,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__
       Vec<T, VW>::widen(rg[n], gv);
 #pragma unroll
       for (int t = 0; t < VW; ++t) wv[t] = 1.f;
-      if (w && c < D) Vec<float, VW>::load(w + c, wv);
+      if (w.p && c < D) w.load<VW>(c, wv);
 #pragma unroll
       for (int t = 0; t < VW; ++t) {
         const float gg = gv[t], s = sigmoidf(gg), silu = gg * s, xn = v[n][t] * r, dwv = dv[n][t] * wv[t];
@@ -542,7 +568,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__
         dv[n][t] = dwv * silu;                              // d(normalised x)
         dot = fmaf(dv[n][t], xn, dot);
       }
-      if (row < rows && c < D) Vec<T, VW>::store(dg + row * D + c, og);
+      if (row < rows && c < D) Vec<T, VW>::store(dg + dgp.at(row, D) + c, og);
     }
     dot = row_sum<LG>(dot) * invD;
     if (row < rows) {
@@ -691,7 +717,7 @@ int gate_bwd(const tops_gate_act_bwd_params& p, void* ws, cudaStream_t st) {
   const GateGrid gg = gate_grid(HK, f.K, (size_t)f.rows, 1);
   const int nblk = gg.grid.x;
   const bool kda = f.kind != TOPS_GATE_ACT_LOG_SIGMOID;
-  float* part_bias = (kda && p.dbias) ? reinterpret_cast<float*>(ws) : nullptr;
+  float* part_bias = p.dbias ? reinterpret_cast<float*>(ws) : nullptr;
   float* part_A = (kda && p.dA_log) ? reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + align_up((size_t)nblk * HK * sizeof(float)))
                                     : nullptr;
   const GateConst c = gate_const(f);
@@ -729,7 +755,108 @@ int gate_bwd(const tops_gate_act_bwd_params& p, void* ws, cudaStream_t st) {
   return TOPS_OK;
 }
 
+// A block owns 512 columns, two per thread, and walks the tokens, eight at a time through shared memory; with R = 16
+// (the layer's rank) a thread's two rows of W stay in registers.  8192 tokens, N = 512: 10 us (16 MB written).
+template <class T, int R_>   // R_: the rank, or 0: any multiple of 8 up to 64
+__global__ void __launch_bounds__(256) k_lowrank_gate(tops_lowrank_gate_params p) {
+  constexpr int TOK = 8;
+  __shared__ __align__(16) float lo[64][TOK];
+  const int R = R_ ? R_ : p.R, n = blockIdx.y * 512 + threadIdx.x * 2;
+  const bool on = n < p.N;   // (N is a multiple of 8)
+  const T *low = reinterpret_cast<const T*>(p.low), *W = reinterpret_cast<const T*>(p.W);
+  const float inv = 1.f / p.normalizer;
+  float bias[2] = {0.f, 0.f}, w[2][R_ ? R_ : 8];
+  if (on) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      bias[j] = to_f(reinterpret_cast<const T*>(p.bias)[n + j]);
+      if (R_) {
+#pragma unroll
+        for (int c = 0; c < R_; c += 8) {
+          float t[8];
+          Vec<T, 8>::load(W + (size_t)(n + j) * R + c, t);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) w[j][c + i] = t[i];
+        }
+      }
+    }
+  }
+  for (size_t r0 = (size_t)blockIdx.x * TOK; r0 < (size_t)p.rows; r0 += (size_t)gridDim.x * TOK) {
+    for (int i = threadIdx.x; i < TOK * R; i += 256) {
+      const int t = i / R, c = i - t * R;
+      lo[c][t] = r0 + t < (size_t)p.rows ? to_f(low[(r0 + t) * p.low_pitch + c]) : 0.f;
+    }
+    __syncthreads();
+    if (on) {
+      float acc[2][TOK];
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) { acc[0][t] = bias[0]; acc[1][t] = bias[1]; }
+      auto eight = [&](int c) {   // channels c .. c + 7
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 x = *reinterpret_cast<const float4*>(&lo[c + i][0]), y = *reinterpret_cast<const float4*>(&lo[c + i][4]);
+          const float l[TOK] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) acc[j][t] = fmaf(l[t], w[j][R_ ? c + i : i], acc[j][t]);
+        }
+      };
+      if (R_) {
+#pragma unroll
+        for (int c = 0; c < R_; c += 8) eight(c);
+      } else {
+        for (int c = 0; c < R; c += 8) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            float t[8];
+            Vec<T, 8>::load(W + (size_t)(n + j) * R + c, t);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[j][i] = t[i];
+          }
+          eight(c);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) {
+        if (r0 + t >= (size_t)p.rows) break;
+        T xr[2], yr[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          xr[j] = from_f<T>(acc[j][t]);
+          float y = -softplusf(-to_f(xr[j])) * inv;
+          if (p.has_clamp_min && y < p.clamp_min) y = p.clamp_min;
+          yr[j] = from_f<T>(y);
+        }
+        const size_t o = (r0 + t) * p.N + n;
+        struct __align__(2 * sizeof(T)) Two { T a, b; };
+        if (p.x) *reinterpret_cast<Two*>(reinterpret_cast<T*>(p.x) + o) = Two{xr[0], xr[1]};
+        *reinterpret_cast<Two*>(reinterpret_cast<T*>(p.y) + o) = Two{yr[0], yr[1]};
+      }
+    }
+    __syncthreads();
+  }
+}
+
+int lowrank_gate_fwd(const tops_lowrank_gate_params& p, cudaStream_t st) {
+  if (p.rows < 1 || p.R < 8 || p.R > 64 || p.R % 8 != 0 || p.N < 8 || p.N % 8 != 0 || p.low_pitch < p.R || !(p.normalizer != 0.f))
+    return TOPS_E_BAD_SHAPE;
+  if (!aligned16(p.W) || !aligned16(p.x) || !aligned16(p.y)) return TOPS_E_ALIGN;
+  const size_t need = ((size_t)p.rows + 7) / 8;
+  const dim3 grid((unsigned)(need < 148 * 4 ? need : 148 * 4), (p.N + 511) / 512);
+  KernelScope ks("lowrank_gate_fwd", st);
+  int rc = dispatch(p.dtype, [&](auto* t) {
+    using T = std::remove_pointer_t<decltype(t)>;
+    if (p.R == 16) k_lowrank_gate<T, 16><<<grid, 256, 0, st>>>(p);
+    else k_lowrank_gate<T, 0><<<grid, 256, 0, st>>>(p);
+    return TOPS_OK;
+  });
+  return rc ? rc : post_launch();
+}
+
 int norm_check(const tops_norm_params& p) {
+  if ((p.gate_pitch || p.dgate_pitch) && (p.heads < 1 || p.rows > 0xffffffffll || p.gate_pitch % 8 || p.dgate_pitch % 8))
+    return TOPS_E_BAD_SHAPE;
   if (p.rows < 1 || p.D < 4 || p.D > 1024 || p.D % 4 != 0) return TOPS_E_BAD_SHAPE;
   if (!p.x || !p.y) return TOPS_E_NULL;
   if (!aligned16(p.x) || !aligned16(p.y) || !aligned16(p.gate) || !aligned16(p.weight) || !aligned16(p.dy) ||
@@ -779,8 +906,8 @@ int rmsnorm_gated_fwd(const tops_norm_params& p, cudaStream_t st) {
     return dispatch_row(rs, [&](auto vw, auto nv, auto lg) {
       constexpr int VW = decltype(vw)::value, NV = decltype(nv)::value, LG = decltype(lg)::value;
       k_rmsnorm_gated_fwd<T, VW, NV, LG><<<row_blocks(p.rows, rs.lg, rows_in_flight2<NV>()), 256, 0, st>>>(
-          reinterpret_cast<const T*>(p.x), reinterpret_cast<const T*>(p.gate), p.weight, reinterpret_cast<T*>(p.y),
-          (size_t)p.rows, p.D, p.eps);
+          reinterpret_cast<const T*>(p.x), reinterpret_cast<const T*>(p.gate), NormWeight{p.weight, p.weight_dtype},
+          reinterpret_cast<T*>(p.y), (size_t)p.rows, p.D, p.eps, RowPitch{p.gate_pitch, p.heads});
       return TOPS_OK;
     });
   });
@@ -805,8 +932,9 @@ int rmsnorm_gated_bwd(const tops_norm_params& p, void* ws, cudaStream_t st) {
       return dispatch_row(rs, [&](auto vw, auto nv, auto lg) {
         constexpr int VW = decltype(vw)::value, NV = decltype(nv)::value, LG = decltype(lg)::value;
         k_rmsnorm_gated_bwd<T, VW, NV, LG><<<blocks, 256, smem, st>>>(
-            reinterpret_cast<const T*>(p.x), reinterpret_cast<const T*>(p.gate), p.weight, reinterpret_cast<const T*>(p.dy),
-            reinterpret_cast<T*>(p.dx), reinterpret_cast<T*>(p.dgate), part, (size_t)p.rows, p.D, p.eps);
+            reinterpret_cast<const T*>(p.x), reinterpret_cast<const T*>(p.gate), NormWeight{p.weight, p.weight_dtype},
+            reinterpret_cast<const T*>(p.dy), reinterpret_cast<T*>(p.dx), reinterpret_cast<T*>(p.dgate), part, (size_t)p.rows,
+            p.D, p.eps, RowPitch{p.gate_pitch, p.heads}, RowPitch{p.dgate_pitch, p.heads});
         return TOPS_OK;
       });
     });

@@ -8,6 +8,7 @@
 namespace tops {
 namespace elementwise {
 int gate_check(const tops_gate_act_params& p);
+int lowrank_gate_fwd(const tops_lowrank_gate_params& p, cudaStream_t st);
 int gate_fwd(const tops_gate_act_params& p, cudaStream_t st);
 size_t gate_bwd_workspace_bytes(const tops_gate_act_bwd_params& p);
 int gate_bwd(const tops_gate_act_bwd_params& p, void* ws, cudaStream_t st);

@@ -1208,6 +1208,7 @@ struct BwdParams {
   // writes fp32 partial sums, every launch but the first adds the partial sums of the one before.
   int vs;
   const float *add_dq, *add_dk, *add_dg;   // null: nothing to add
+  long long dqk_pitch, dv_pitch;           // GEN: elements between tokens of dq and dk, and of dv
 };
 
 // Warp roles: warps 0-15 gate q and k of the next chunk and write the gradients of a chunk out of
@@ -1318,7 +1319,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     const int q4 = warp & 3, seg = warp >> 2, col = q4 * 32 + lane;
     const uint32_t lane_base = q4 * 32;
     const ColAddr ca = col_prep(64, col);
-    const size_t ostride = (size_t)p.H * K, vstride = (size_t)p.H * V;
+    const size_t ostride = (size_t)p.H * K, vstride = GEN ? (size_t)p.dv_pitch : ostride;
     const bool has_k = !GEN || col < K, has_v = !GEN || yc + col < V;
     TG* const dq_out = reinterpret_cast<TG*>(p.dq);
     TG* const dk_out = reinterpret_cast<TG*>(p.dk);
@@ -1426,7 +1427,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       const uint8_t* qt = qs + sl * TILE64;
       const uint8_t* kt = ks + sl * TILE64;
       const size_t obase = ((size_t)(row + seg * SEG) * p.H + h) * K + col;
-      const size_t vbase = ((size_t)(row + seg * SEG) * p.H + h) * V + yc + col;
+      size_t vbase = obase;
+      if (GEN) vbase = (size_t)(row + seg * SEG) * vstride + (size_t)h * V + yc + col;
       const size_t obase4 = obase - (lane & 3) + (size_t)(lane & 3) * ostride;   // channel group, own time row
       float dgl[SEG];
       float run = 0.f, tail = 0.f;
@@ -1457,9 +1459,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
             if (seg * SEG + t < len) {
               if (has_v) st_out(p.dv, vbase + t * vstride, dv[u]);
               if (has_k) {
-                const size_t o = obase + t * ostride;
-                st_out(dq_out, o, p.add_dq ? fmaf(e, dqs, p.add_dq[o]) : e * dqs);
-                st_out(dk_out, o, p.add_dk ? fmaf(r, dks, p.add_dk[o]) : r * dks);
+                float gq = e * dqs, gk = r * dks;
+                if (p.add_dq) {
+                  gq += p.add_dq[obase + t * ostride];
+                  gk += p.add_dk[obase + t * ostride];
+                }
+                const size_t o = (size_t)(row + seg * SEG + t) * p.dqk_pitch + (size_t)h * K + col;
+                st_out(dq_out, o, gq);
+                st_out(dk_out, o, gk);
               }
             }
           } else {
@@ -1746,8 +1753,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   if (tid == 0 && abort_flag && nit > 0) {
     int h, row, hrow;
     chunk_rows(0, h, row, hrow);
-    poison(reinterpret_cast<TG*>(p.dq) + ((size_t)row * p.H + h) * K);
-    poison(p.dv + ((size_t)row * p.H + h) * V + yc);
+    poison(reinterpret_cast<TG*>(p.dq) + (GEN ? (size_t)row * p.dqk_pitch : (size_t)row * p.H * K) + (size_t)h * K);
+    poison(p.dv + (GEN ? (size_t)row * p.dv_pitch : (size_t)row * p.H * V) + (size_t)h * V + yc);
   }
 }
 
@@ -2145,13 +2152,15 @@ struct GenSegs {
 };
 bool scalar_kind(int kind) { return kind != TOPS_GATE_PER_CHANNEL; }
 
+// pitch: of x and y where they are q, k or v (x_pitch 0 and y_pitch 0: contiguous)
+struct XYPitch { int64_t x = 0, y = 0; };
 int run_scan_gen(bool bwd, bool sum, const tops_chunk_problem& pb, const GenPlan& g, const void* x, const void* gate, const void* y,
-                 const float* s0, const float* s0_seg, void* states, float* s_final, float* gsum, cudaStream_t st) {
+                 XYPitch pitch, const float* s0, const float* s0_seg, void* states, float* s_final, float* gsum, cudaStream_t st) {
   ScanParams sp;
   const int BT = pb.B * pb.T;
   const bool scalar = scalar_kind(pb.gate_kind);
   int rc;
-  if ((rc = act_map(&sp.mx, x, BT, pb.H, pb.K)) || (rc = act_map(&sp.my, y, BT, pb.H, pb.V))) return rc;
+  if ((rc = act_map(&sp.mx, x, BT, pb.H, pb.K, pitch.x)) || (rc = act_map(&sp.my, y, BT, pb.H, pb.V, pitch.y))) return rc;
   if (!scalar && (rc = act_map(&sp.mg, gate, BT, pb.H, pb.K))) return rc;
   sp.gscalar = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(gate) : nullptr;
   sp.gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(gate) : nullptr;
@@ -2176,9 +2185,9 @@ int run_scan_gen(bool bwd, bool sum, const tops_chunk_problem& pb, const GenPlan
 
 // summary pass + join for the sequences that are cut into runs
 int gen_starts(bool bwd, const tops_chunk_problem& pb, const GenPlan& g, const void* x, const void* gate, const void* y,
-               const float* first, float* last, const GenSegs& sc, cudaStream_t st) {
+               XYPitch pitch, const float* first, float* last, const GenSegs& sc, cudaStream_t st) {
   if (!g.cut) return TOPS_OK;
-  int rc = run_scan_gen(bwd, true, pb, g, x, gate, y, nullptr, nullptr, nullptr, sc.ends, sc.gsum, st);
+  int rc = run_scan_gen(bwd, true, pb, g, x, gate, y, pitch, nullptr, nullptr, nullptr, sc.ends, sc.gsum, st);
   if (rc) return rc;
   KernelScope ks("sm100_join_segments", st);
   const int slices = cdiv(pb.K * pb.V, 1024);
@@ -2227,6 +2236,7 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
   if (!aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || (pb.gate_kind != TOPS_GATE_GAMMA && !aligned16(p.g)) ||
       !aligned16(p.o) || !aligned16(p.h0) || !aligned16(p.ht) || !aligned16(p.saved_out) || !aligned16(ws))
     return TOPS_E_ALIGN;
+  if (p.pitch % 8 != 0) return TOPS_E_ALIGN;
   GenPlan g(pb);
   char* wsp = reinterpret_cast<char*>(ws);
   int rc = g.upload(pb, wsp, st);
@@ -2236,15 +2246,16 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
   void* h = p.saved_out;
   if (!h && !fused) { h = wsp; wsp += g.state_bytes(); }
   const GenSegs sc(wsp, g);
-  if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, p.h0, p.ht, sc, st))) return rc;
+  const XYPitch kv{p.pitch, p.pitch};
+  if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, kv, p.h0, p.ht, sc, st))) return rc;
   const int BT = pb.B * pb.T;
   const __nv_bfloat16* gs = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(p.g) : nullptr;
   const float* gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(p.g) : nullptr;
   const size_t state_rows = (size_t)g.total_chunks * g.HV * D;
   if (fused) {
     FusedParams up;
-    if ((rc = act_map(&up.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&up.mk, p.k, BT, pb.H, pb.K)) ||
-        (rc = act_map(&up.mv, p.v, BT, pb.H, pb.V)))
+    if ((rc = act_map(&up.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&up.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
+        (rc = act_map(&up.mv, p.v, BT, pb.H, pb.V, p.pitch)))
       return rc;
     if (!scalar && (rc = act_map(&up.mg, p.g, BT, pb.H, pb.K))) return rc;
     up.gscalar = gs; up.gamma = gamma; up.states = nullptr;
@@ -2260,10 +2271,10 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
     else k_fwd_fused<false, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
     return post_launch();
   }
-  if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, p.h0, sc.starts, h, p.ht, nullptr, st))) return rc;
+  if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, kv, p.h0, sc.starts, h, p.ht, nullptr, st))) return rc;
   FwdOParams fp;
-  if ((rc = act_map(&fp.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&fp.mk, p.k, BT, pb.H, pb.K)) ||
-      (rc = act_map(&fp.mv, p.v, BT, pb.H, pb.V)) || (rc = state_map(&fp.mh, h, state_rows)))
+  if ((rc = act_map(&fp.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&fp.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
+      (rc = act_map(&fp.mv, p.v, BT, pb.H, pb.V, p.pitch)) || (rc = state_map(&fp.mh, h, state_rows)))
     return rc;
   if (!scalar && (rc = act_map(&fp.mg, p.g, BT, pb.H, pb.K))) return rc;
   fp.gscalar = gs; fp.gamma = gamma; fp.geo = g.geo;
@@ -2297,6 +2308,7 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
       !aligned16(p.do_) || !aligned16(p.h0) || !aligned16(p.dht) || !aligned16(p.dh0) || !aligned16(p.dq) || !aligned16(p.dk) ||
       !aligned16(p.dv) || !aligned16(p.dg) || !aligned16(p.h_saved) || !aligned16(ws))
     return TOPS_E_ALIGN;
+  if (p.pitch % 8 != 0 || p.grad_pitch % 8 != 0) return TOPS_E_ALIGN;
   GenPlan g(pb);
   char* wsp = reinterpret_cast<char*>(ws);
   int rc = g.upload(pb, wsp, st);
@@ -2309,18 +2321,20 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
   const GenSegs sc(wsp, g); wsp += g.seg_bytes();
   float* part = reinterpret_cast<float*>(wsp);
   if (!h) {
-    if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, p.h0, nullptr, sc, st))) return rc;
-    if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, p.h0, sc.starts, hw, nullptr, nullptr, st))) return rc;
+    const XYPitch kv{p.pitch, p.pitch};
+    if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, kv, p.h0, nullptr, sc, st))) return rc;
+    if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, kv, p.h0, sc.starts, hw, nullptr, nullptr, st))) return rc;
     h = hw;
   }
-  if ((rc = gen_starts(true, pb, g, p.q, p.g, p.do_, p.dht, p.dh0, sc, st))) return rc;
-  if ((rc = run_scan_gen(true, false, pb, g, p.q, p.g, p.do_, p.dht, sc.starts, dh, p.dh0, nullptr, st))) return rc;
+  const XYPitch qdo{p.pitch, 0};
+  if ((rc = gen_starts(true, pb, g, p.q, p.g, p.do_, qdo, p.dht, p.dh0, sc, st))) return rc;
+  if ((rc = run_scan_gen(true, false, pb, g, p.q, p.g, p.do_, qdo, p.dht, sc.starts, dh, p.dh0, nullptr, st))) return rc;
   BwdParams bp;
   const int BT = pb.B * pb.T;
   const size_t rows = (size_t)g.total_chunks * g.HV * D;
   const bool scalar = scalar_kind(pb.gate_kind);
-  if ((rc = act_map(&bp.mq, p.q, BT, pb.H, pb.K)) || (rc = act_map(&bp.mk, p.k, BT, pb.H, pb.K)) ||
-      (rc = act_map(&bp.mv, p.v, BT, pb.H, pb.V)) || (rc = act_map(&bp.mdo, p.do_, BT, pb.H, pb.V)) ||
+  if ((rc = act_map(&bp.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&bp.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
+      (rc = act_map(&bp.mv, p.v, BT, pb.H, pb.V, p.pitch)) || (rc = act_map(&bp.mdo, p.do_, BT, pb.H, pb.V)) ||
       (rc = state_map(&bp.mh, h, rows)) || (rc = state_map(&bp.mdh, dh, rows)))
     return rc;
   if (!scalar && (rc = act_map(&bp.mg, p.g, BT, pb.H, pb.K))) return rc;
@@ -2334,6 +2348,8 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
   for (int vs = 0; vs < g.geo.VS; ++vs) {
     const bool last = vs == g.geo.VS - 1;
     bp.vs = vs;
+    bp.dqk_pitch = last && p.grad_pitch ? p.grad_pitch : (long long)pb.H * pb.K;
+    bp.dv_pitch = p.grad_pitch ? p.grad_pitch : (long long)pb.H * pb.V;
     bp.dq = last ? p.dq : pdq; bp.dk = last ? p.dk : pdk; bp.dg = last ? p.dg : pdg;
     bp.add_dq = vs ? pdq : nullptr; bp.add_dk = vs ? pdk : nullptr; bp.add_dg = vs ? pdg : nullptr;
     if (scalar) rc = (!last || p.grad_dtype == TOPS_F32) ? launch_bwd_main<float, float, true, true>(bp, st)

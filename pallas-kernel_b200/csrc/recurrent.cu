@@ -57,14 +57,16 @@ __global__ void __launch_bounds__(FW_THREADS) k_rec_fwd(tops_recurrent_fwd_param
   for (int step = 0; step < len; ++step) {
     const int t = a.reverse ? sr.eos - 1 - step : sr.bos + step;
     const size_t tok = ((size_t)sr.b * a.T + t) * a.H + h;
+    const size_t row = (size_t)sr.b * a.T + t;
+    const size_t qk = a.pitch ? row * a.pitch + (size_t)h * K : tok * K, vo = a.pitch ? row * a.pitch + (size_t)h * V : tok * V;
     for (int i = tid; i < K; i += FW_THREADS) {
-      qs[i] = load_any(a.q, a.dtype, tok * K + i) * a.scale;
-      ks[i] = load_any(a.k, a.dtype, tok * K + i);
+      qs[i] = load_any(a.q, a.dtype, qk + i) * a.scale;
+      ks[i] = load_any(a.k, a.dtype, qk + i);
       eks[i] = a.gk ? expf(load_any(a.gk, a.gate_dtype, tok * K + i)) : 1.f;
     }
     if (tid < FW_BV) {
       bool ok = v0 + tid < V;
-      vs[tid] = ok ? load_any(a.v, a.dtype, tok * V + v0 + tid) : 0.f;
+      vs[tid] = ok ? load_any(a.v, a.dtype, vo + v0 + tid) : 0.f;
       evs[tid] = (ok && a.gv) ? expf(load_any(a.gv, a.gate_dtype, tok * V + v0 + tid)) : 1.f;
     }
     __syncthreads();

@@ -34,18 +34,20 @@ inline EncodeFn encode_fn() {
 struct MapKey {
   int dev, kind;
   const void* ptr;
-  uint64_t a, b;
-  bool operator==(const MapKey& o) const { return dev == o.dev && kind == o.kind && ptr == o.ptr && a == o.a && b == o.b; }
+  uint64_t a, b, c;
+  bool operator==(const MapKey& o) const {
+    return dev == o.dev && kind == o.kind && ptr == o.ptr && a == o.a && b == o.b && c == o.c;
+  }
 };
 struct MapSlot { MapKey key; CUtensorMap map; bool used; };
 constexpr int kMapSlots = 64;
 inline std::mutex g_map_mu;
 inline MapSlot g_maps[kMapSlots];
 template <class Encode>
-inline int cached_map(CUtensorMap* m, int kind, const void* ptr, uint64_t a, uint64_t b, Encode encode) {
+inline int cached_map(CUtensorMap* m, int kind, const void* ptr, uint64_t a, uint64_t b, uint64_t c, Encode encode) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return TOPS_E_CUDA; }
-  const MapKey key{dev, kind, ptr, a, b};
+  const MapKey key{dev, kind, ptr, a, b, c};
   const size_t slot = (reinterpret_cast<uintptr_t>(ptr) >> 8) * 0x9E3779B97F4A7C15ull >> 58;   // 6 bits
   std::lock_guard<std::mutex> lk(g_map_mu);
   MapSlot& s = g_maps[(slot + (size_t)kind) % kMapSlots];
@@ -68,11 +70,12 @@ inline int cached_map(CUtensorMap* m, int kind, const void* ptr, uint64_t a, uin
 }
 
 // [B*T, H, W] bf16 activations (W a multiple of 8): box = 64 channels x 1 head x 64 tokens; what a box covers
-// beyond the tensor is filled with zeros
-inline int act_map(CUtensorMap* m, const void* ptr, int BT, int H, int W = kHeadDim) {
-  return cached_map(m, 0, ptr, (uint64_t)BT, (uint64_t)H | ((uint64_t)W << 32), [&](CUtensorMap* out) {
+// beyond the tensor is filled with zeros.  `pitch`: elements between tokens (0: H * W)
+inline int act_map(CUtensorMap* m, const void* ptr, int BT, int H, int W = kHeadDim, int64_t pitch = 0) {
+  if (!pitch) pitch = (int64_t)H * W;
+  return cached_map(m, 0, ptr, (uint64_t)BT, (uint64_t)H | ((uint64_t)W << 32), (uint64_t)pitch, [&](CUtensorMap* out) {
     cuuint64_t dims[3] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)BT};
-    cuuint64_t strides[2] = {(cuuint64_t)W * 2, (cuuint64_t)H * W * 2};
+    cuuint64_t strides[2] = {(cuuint64_t)W * 2, (cuuint64_t)pitch * 2};
     cuuint32_t box[3] = {64, 1, 64};
     cuuint32_t es[3] = {1, 1, 1};
     return encode_fn()(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es,
@@ -82,7 +85,7 @@ inline int act_map(CUtensorMap* m, const void* ptr, int BT, int H, int W = kHead
 }
 // [B*T, H, 64] bf16 per-chunk matrices (row i of a chunk at token i): box = 64 columns x 1 head x 64 tokens
 inline int mat_map(CUtensorMap* m, const void* ptr, int BT, int H) {
-  return cached_map(m, 2, ptr, (uint64_t)BT, (uint64_t)H, [&](CUtensorMap* out) {
+  return cached_map(m, 2, ptr, (uint64_t)BT, (uint64_t)H, 0, [&](CUtensorMap* out) {
     cuuint64_t dims[3] = {64, (cuuint64_t)H, (cuuint64_t)BT};
     cuuint64_t strides[2] = {64 * 2, (cuuint64_t)H * 64 * 2};
     cuuint32_t box[3] = {64, 1, 64};
@@ -94,7 +97,7 @@ inline int mat_map(CUtensorMap* m, const void* ptr, int BT, int H) {
 }
 // [rows, 128] bf16 chunk states: box = 64 columns x 128 rows
 inline int state_map(CUtensorMap* m, const void* ptr, size_t rows) {
-  return cached_map(m, 1, ptr, (uint64_t)rows, 0, [&](CUtensorMap* out) {
+  return cached_map(m, 1, ptr, (uint64_t)rows, 0, 0, [&](CUtensorMap* out) {
     cuuint64_t dims[2] = {(cuuint64_t)kHeadDim, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)kHeadDim * 2};
     cuuint32_t box[2] = {64, 128};

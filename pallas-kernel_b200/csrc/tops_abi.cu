@@ -14,6 +14,7 @@
 #include "kda.cuh"
 #include "kda_sm100.cuh"
 #include "recurrent.cuh"
+#include "skinny.cuh"
 
 namespace tops {
 static std::atomic<int64_t> g_launches{0};
@@ -131,12 +132,16 @@ Family family(const tops_chunk_problem& pb, bool plain_only = false) {
   return sm100::supported(pb) ? FAMILY_PLAIN : FAMILY_GENERIC;
 }
 // optional outputs only the generic kernels write; segment summaries only the plain form takes
+// (q, k, v inside a wider matrix: only the general form follows their pitch)
 Family family(const tops_chunk_fwd_params& p) {
   if (p.g_cumsum_out || p.A_out || p.h_out) return FAMILY_GENERIC;
+  if (p.pitch) return p.pb.impl == TOPS_IMPL_AUTO && sm100::supported_gen(p.pb) ? FAMILY_GENERAL : FAMILY_GENERIC;
   return family(p.pb, p.segments != nullptr);
 }
 Family family(const tops_chunk_bwd_params& p) {
   if (!sm100::bwd_dtypes_ok(p)) return FAMILY_GENERIC;
+  if (p.pitch || p.grad_pitch)
+    return p.pb.impl == TOPS_IMPL_AUTO && sm100::supported_gen(p.pb) ? FAMILY_GENERAL : FAMILY_GENERIC;
   return family(p.pb, p.rev_segments != nullptr);
 }
 
@@ -309,6 +314,7 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
   const Family f = family(*p);
   if (f == FAMILY_PLAIN) return sm100::chunk_fwd(*p, workspace, workspace_bytes, st);
   if (f == FAMILY_GENERAL) return sm100::gen_chunk_fwd(*p, workspace, st);
+  if (p->pitch) return TOPS_E_UNSUPPORTED;
 
   Problem pb;
   float* gcum = nullptr;
@@ -420,6 +426,7 @@ extern "C" int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* wor
   const Family f = family(*p);
   if (f == FAMILY_PLAIN) return sm100::chunk_bwd(*p, workspace, workspace_bytes, st);
   if (f == FAMILY_GENERAL) return sm100::gen_chunk_bwd(*p, workspace, st);
+  if (p->pitch || p->grad_pitch) return TOPS_E_UNSUPPORTED;
   if (p->dg_dtype != TOPS_F32) return TOPS_E_UNSUPPORTED;   // the generic kernels write fp32 dg per gate element
 
   Problem pb;
@@ -535,6 +542,17 @@ extern "C" int tops_b200_gate_act_fwd(const tops_gate_act_params* p, void* strea
   if (!valid_dtype(p->dtype) || !valid_dtype(p->out_dtype)) return TOPS_E_BAD_DTYPE;
   int rc = elementwise::gate_check(*p);
   return rc ? rc : elementwise::gate_fwd(*p, (cudaStream_t)stream);
+}
+
+extern "C" int tops_b200_lowrank_gate_fwd(const tops_lowrank_gate_params* p, void* stream) {
+  if (!p || !p->low || !p->W || !p->bias || !p->y) return TOPS_E_NULL;
+  if (!valid_dtype(p->dtype)) return TOPS_E_BAD_DTYPE;
+  return elementwise::lowrank_gate_fwd(*p, (cudaStream_t)stream);
+}
+
+extern "C" int tops_b200_skinny_linear(const tops_skinny_linear_params* p, void* stream) {
+  if (!p || !p->x) return TOPS_E_NULL;
+  return skinny::linear(*p, (cudaStream_t)stream);
 }
 
 extern "C" size_t tops_b200_gate_act_bwd_workspace_bytes(const tops_gate_act_bwd_params* p) {

@@ -29,7 +29,7 @@ GATE_NONE, GATE_PER_CHANNEL, GATE_SCALAR, GATE_GAMMA = 0, 1, 2, 3
 IMPL_AUTO, IMPL_GENERIC, IMPL_SM100 = 0, 1, 2
 
 _DT = {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}
-_i32, _f32, _vp, _sz = C.c_int32, C.c_float, C.c_void_p, C.c_size_t
+_i32, _i64, _f32, _vp, _sz = C.c_int32, C.c_int64, C.c_float, C.c_void_p, C.c_size_t
 
 
 def dtype_code(dt: torch.dtype) -> int:
@@ -60,20 +60,20 @@ class BwdDhParams(C.Structure):
 
 class ChunkFwdParams(C.Structure):
     _fields_ = [("pb", ChunkProblem), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("h0", _vp), ("o", _vp),
-                ("ht", _vp), ("g_cumsum_out", _vp), ("A_out", _vp), ("h_out", _vp), ("saved_out", _vp), ("segments", _vp)]
+                ("ht", _vp), ("g_cumsum_out", _vp), ("A_out", _vp), ("h_out", _vp), ("saved_out", _vp), ("segments", _vp), ("pitch", _i64)]
 
 
 class ChunkBwdParams(C.Structure):
     _fields_ = [("pb", ChunkProblem), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("h0", _vp), ("do_", _vp),
                 ("dht", _vp), ("dq", _vp), ("dk", _vp), ("grad_dtype", _i32), ("dv", _vp), ("dg", _vp),
-                ("dh0", _vp), ("h_saved", _vp), ("dg_dtype", _i32), ("rev_segments", _vp)]
+                ("dh0", _vp), ("h_saved", _vp), ("dg_dtype", _i32), ("rev_segments", _vp), ("pitch", _i64), ("grad_pitch", _i64)]
 
 
 class RecurrentFwdParams(C.Structure):
     _fields_ = [("B", _i32), ("T", _i32), ("H", _i32), ("K", _i32), ("V", _i32), ("dtype", _i32),
                 ("gate_dtype", _i32), ("o_dtype", _i32), ("reverse", _i32), ("scale", _f32), ("q", _vp),
                 ("k", _vp), ("v", _vp), ("gk", _vp), ("gv", _vp), ("state_in", _vp), ("state_out", _vp),
-                ("o", _vp), ("cu_seqlens", _vp), ("N", _i32)]
+                ("o", _vp), ("cu_seqlens", _vp), ("N", _i32), ("pitch", _i64)]
 
 
 class RecurrentBwdParams(C.Structure):
@@ -104,7 +104,6 @@ class ChunkKdaFwdParams(C.Structure):
                 ("saved_vnew", _vp), ("saved_T", _vp), ("saved_R", _vp)]
 
 
-_i64 = C.c_int64
 GATE_ACT_KDA, GATE_ACT_KDA_LOWER_BOUND, GATE_ACT_LOG_SIGMOID = 0, 1, 2
 
 
@@ -120,7 +119,8 @@ class GateActBwdParams(C.Structure):
 
 class NormParams(C.Structure):
     _fields_ = [("rows", _i64), ("D", _i32), ("dtype", _i32), ("eps", _f32), ("x", _vp), ("gate", _vp), ("weight", _vp),
-                ("y", _vp), ("rstd", _vp), ("dy", _vp), ("dx", _vp), ("dgate", _vp), ("dweight", _vp)]
+                ("y", _vp), ("rstd", _vp), ("dy", _vp), ("dx", _vp), ("dgate", _vp), ("dweight", _vp),
+                ("gate_pitch", _i64), ("dgate_pitch", _i64), ("heads", _i32), ("weight_dtype", _i32)]
 
 
 class ChunkKdaBwdParams(C.Structure):

@@ -6,7 +6,7 @@ optional causal depthwise short convolutions (`tops/modules/convolution.py`), th
 `log_sigmoid(gk) / gate_logit_normalizer` (`gla_gate`), `fused_recurrent_gla` for sequences of at most
 64 tokens and the configured mode otherwise (chunk_size 16 as upstream), the fused RMS-norm + swish gate
 on the output (`FusedRMSNormGated`) or the plain RMS norm followed by the gate activation, and the output
-projection.  The linear projections and the short convolution are torch's own (they are outside the path
+projection.  The layer its constructor's defaults make runs as one call of the torch extension (`_forward_fused`).  The linear projections and the short convolution are torch's own (they are outside the path
 this package replaces); everything between them runs on this package's kernels.
 """
 from __future__ import annotations
@@ -15,6 +15,7 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
+from ._lib import ops_ext as X
 from .ops.gate import gla_gate
 from .ops.gla import chunk_gla, fused_chunk_gla, fused_recurrent_gla
 from .ops.norm import FusedRMSNormGated
@@ -127,11 +128,56 @@ class GatedLinearAttention(nn.Module):
         x = x.reshape(*x.shape[:-1], -1, head_dim)
         return x if groups == 1 else x.repeat_interleave(groups, dim=-2)
 
+    def _plain(self):
+        """The projections are ordinary bf16 linears nobody watches: they may be computed without calling the modules."""
+        lin = (self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.gk_proj[0], self.gk_proj[1], self.o_proj)
+        for m in (*lin, self.gk_proj, self.g_norm_swish_gate):
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks):
+                return False
+        return all(type(m) is nn.Linear and m.weight.dtype == torch.bfloat16 and m.weight.is_contiguous()
+                   and (m.bias is None) == (m is not self.gk_proj[1]) for m in lin)
+
+    def _forward_fused(self, x, past_key_values, use_cache, cu_seqlens):
+        """The whole layer in one call of the torch extension, for the layer its constructor's defaults make: all
+        heads of their own, fused norm + gate, no convolution, no feature map, chunked mode (or up to 64 tokens without
+        gradients).  None where it does not apply."""
+        if not (self.use_output_gate and self.fuse_norm_and_gate) or self.use_short_conv or self.feature_map_fn is not None \
+                or self.num_kv_groups != 1 or torch.is_autocast_enabled():
+            return None
+        q_len = x.shape[1]
+        recurrent = q_len <= 64 or self.mode == "fused_recurrent"
+        if not X.gla_layer_takes(x, self.key_dim, self.value_dim, self.gk_proj[0].weight.shape[0], self.num_heads, recurrent):
+            return None
+        if (torch._C._get_tracing_state() is not None or torch.nn.modules.module._has_any_global_hook() or not self._plain()):
+            return None
+        last = None
+        if past_key_values is not None and self.layer_idx is not None and len(past_key_values) > self.layer_idx:
+            last = past_key_values[self.layer_idx]
+        state = last["recurrent_state"] if last is not None else None
+        cu = [] if cu_seqlens is None else [int(c) for c in cu_seqlens]
+        if cu:
+            assert x.shape[0] == 1, f"B must be 1 for varlen, got {x.shape[0]}"
+            assert cu[0] == 0 and cu[-1] == q_len and all(b > a for a, b in zip(cu[:-1], cu[1:])), "cu_seqlens must span [0, T]"
+        if state is not None:
+            want = (len(cu) - 1 if cu else x.shape[0], self.num_heads, self.head_k_dim, self.head_v_dim)
+            assert state.shape == want, f"recurrent state shape {tuple(state.shape)} != expected {want}"
+        norm = self.g_norm_swish_gate
+        o, state = X.gla_layer(x, self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.g_proj.weight,
+                               self.gk_proj[0].weight, self.gk_proj[1].weight, self.gk_proj[1].bias, norm.weight, self.o_proj.weight,
+                               self.num_heads, norm.eps, float(self.gate_logit_normalizer), self.clamp_min, state, bool(use_cache),
+                               cu, recurrent)
+        if past_key_values is not None:
+            past_key_values.update(recurrent_state=state, conv_state=None, layer_idx=self.layer_idx, offset=q_len)
+        return o
+
     def forward(self, hidden_states, attention_mask=None, past_key_values=None, use_cache=False,
                 output_attentions=False, **kwargs):
         if attention_mask is not None:
             assert attention_mask.ndim == 2, "Expected attention_mask as a 0-1 matrix with shape [batch_size, seq_len]."
         q_len = hidden_states.shape[1]
+        fused = self._forward_fused(hidden_states, past_key_values, use_cache, kwargs.get("cu_seqlens"))
+        if fused is not None:
+            return fused, None, past_key_values
         mode = "fused_recurrent" if q_len <= 64 else self.mode
         last_state = None
         if past_key_values is not None and self.layer_idx is not None and len(past_key_values) > self.layer_idx:

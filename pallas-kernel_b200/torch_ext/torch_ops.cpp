@@ -7,148 +7,15 @@
 //
 // Python keeps the argument checks that name shapes (AssertionError) and the reference's signatures; what arrives here
 // has consistent shapes.  Tensors are made contiguous here.
-#include <torch/extension.h>
+#include "common.h"
 
-#include <ATen/cuda/EmptyTensor.h>
-#include <c10/cuda/CUDAGuard.h>
-#include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/utils.h>
-#include <torch/csrc/autograd/saved_variable.h>
-
-#include <optional>
-#include <vector>
-
-#include "tops_b200.h"
-
-namespace py = pybind11;
-using at::Tensor;
-using torch::autograd::Node;
-using torch::autograd::SavedVariable;
-using torch::autograd::variable_list;
-using OptTensor = std::optional<Tensor>;
+using namespace tops_torch;
 
 namespace {
-
-PyObject* g_error_class = nullptr;   // tops_b200.TopsError
-bool g_check_device = false;         // read the device error word after every backward
-
-void raise_tops(const std::string& text) {
-  if (g_error_class && PyGILState_Check()) {
-    PyErr_SetString(g_error_class, text.c_str());
-    throw py::error_already_set();
-  }
-  TORCH_CHECK(false, text);
-}
-void check(int rc, const char* what) {
-  if (rc == 0) return;
-  std::string text = std::string(what) + ": " + tops_b200_strerror(rc) + " (code " + std::to_string(rc) + ")";
-  if (rc == TOPS_E_CUDA) {
-    char buf[256] = "";
-    tops_b200_last_cuda_error(buf, sizeof buf);
-    text += std::string(" [") + buf + "]";
-  }
-  raise_tops(text);
-}
-void check_device_word(const char* what) {
-  if (!g_check_device) return;
-  int code = 0;
-  check(tops_b200_device_error(&code), "device_error");
-  if (code == 0) return;
-  tops_b200_device_error_reset();
-  raise_tops(std::string(what) + ": a kernel gave up on a bounded device-side wait (code " + std::to_string(code) +
-             "); its outputs are invalid");
-}
-
-int code_of(at::ScalarType t) {
-  if (t == at::kFloat) return TOPS_F32;
-  if (t == at::kBFloat16) return TOPS_BF16;
-  if (t == at::kHalf) return TOPS_F16;
-  if (PyGILState_Check()) {
-    PyErr_SetString(PyExc_AssertionError, "unsupported dtype (fp32, bf16, fp16 only)");
-    throw py::error_already_set();
-  }
-  TORCH_CHECK(false, "unsupported dtype (fp32, bf16, fp16 only)");
-}
-int code_of(const Tensor& t) { return code_of(t.scalar_type()); }
-
-// every tensor of a call lives on the first one's GPU
-struct Call {
-  c10::Device dev;
-  c10::cuda::CUDAGuard guard;
-  explicit Call(const Tensor& t) : dev(t.device()), guard(need_cuda(t)) {}
-  static c10::Device need_cuda(const Tensor& t) {
-    if (!t.is_cuda()) {
-      if (PyGILState_Check()) {
-        PyErr_SetString(PyExc_AssertionError, "tops_b200 ops take CUDA tensors; there is no CPU path");
-        throw py::error_already_set();
-      }
-      TORCH_CHECK(false, "tops_b200 ops take CUDA tensors; there is no CPU path");
-    }
-    return t.device();
-  }
-  void* stream() const { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
-  Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const { return Tensor(at::detail::empty_cuda(sizes, t, dev, std::nullopt)); }
-  Tensor empty_as(const Tensor& t) const { return empty(t.sizes(), t.scalar_type()); }
-  Tensor bytes(size_t n) const { return empty({(int64_t)(n < 256 ? 256 : n)}, at::kByte); }
-  Tensor in(const Tensor& t) const {   // contiguous, on this GPU
-    if (!t.defined()) return t;
-    need_cuda(t);
-    return t.is_contiguous() ? t : t.contiguous();
-  }
-  Tensor in(const OptTensor& t) const { return t.has_value() ? in(*t) : Tensor(); }
-  Tensor in_as(const Tensor& t, at::ScalarType type) const { return t.defined() ? in(t.scalar_type() == type ? t : t.to(type)) : t; }
-};
-template <class T = void> T* ptr(const Tensor& t) { return t.defined() ? reinterpret_cast<T*>(t.data_ptr()) : nullptr; }
-Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
-
-template <class... Ts> bool wants_grad(const Ts&... ts) {
-  return at::GradMode::is_enabled() && ((ts.defined() && ts.requires_grad()) || ...);
-}
-
-// A node whose saved tensors are given back after use.
-struct OpNode : public Node {
-  std::vector<SavedVariable> saved;
-  bool released = false;
-  void keep(std::initializer_list<Tensor> ts) {
-    saved.reserve(ts.size());
-    for (const Tensor& t : ts) saved.emplace_back(t, false);
-  }
-  variable_list unpack() {
-    TORCH_CHECK(!released, "Trying to backward through the graph a second time (or directly access saved tensors after they "
-                           "have already been freed): specify retain_graph=True");
-    variable_list r;
-    r.reserve(saved.size());
-    for (auto& s : saved) r.push_back(s.unpack());
-    return r;
-  }
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    saved.clear();
-    released = true;
-  }
-};
-template <class N, class... Ts> std::shared_ptr<N> make_node(const Ts&... inputs) {
-  auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
-  node->set_next_edges(torch::autograd::collect_next_edges(inputs...));
-  return node;
-}
-void attach(const Tensor& out, const std::shared_ptr<Node>& node) {
-  if (out.defined()) torch::autograd::set_history(out, node);
-}
-Tensor cotangent(const Tensor& g, const Tensor& like_sizes_of, at::ScalarType type, const Call& c) {
-  if (!g.defined()) return at::zeros(like_sizes_of.sizes(), at::TensorOptions().dtype(type).device(c.dev));
-  return c.in_as(g, type);
-}
 
 // ---------------------------------------------------------------------------------------------------
 // chunked GLA and simple_gla
 // ---------------------------------------------------------------------------------------------------
-struct ChunkShape {
-  int kind = 0, chunk = 64, N = 0;
-  double scale = 1.0;
-  std::vector<int32_t> cu;
-};
 tops_chunk_problem chunk_problem(const ChunkShape& s, const Tensor& q, const Tensor& v, const Tensor& gate) {
   tops_chunk_problem pb{};
   pb.B = (int)q.size(0); pb.T = (int)q.size(1); pb.H = (int)q.size(2); pb.K = (int)q.size(3); pb.V = (int)v.size(3);
@@ -627,4 +494,6 @@ PYBIND11_MODULE(_torch_ops, m) {
   m.def("gate", &gate);
   m.def("l2norm", &l2norm);
   m.def("rmsnorm_gated", &rmsnorm_gated);
+  m.def("gla_layer", &gla_layer);
+  m.def("gla_layer_takes", &gla_layer_takes);
 }

@@ -1,0 +1,107 @@
+"""`GatedLinearAttention` as one call (bf16) against the same weights run module by module in fp32, and the few-row
+projection kernel against torch, at the sizes where they switch form."""
+import copy
+
+import pytest
+import torch
+
+from tests.util import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(hidden, heads, **kw):
+    from tops_b200.layers import GatedLinearAttention
+    torch.manual_seed(3)
+    return GatedLinearAttention(hidden_size=hidden, num_heads=heads, layer_idx=0, **kw).cuda().to(torch.bfloat16)
+
+
+def _labels(fn):
+    import ctypes
+
+    from tops_b200 import _lib as L
+    L.lib.tops_b200_profile_enable(1)
+    out = fn()
+    torch.cuda.synchronize()
+    L.lib.tops_b200_profile_enable(0)
+    buf = ctypes.create_string_buffer(4096)
+    L.lib.tops_b200_profile_read(buf, len(buf))
+    return out, [ln.split()[0] for ln in buf.value.decode().splitlines()]
+
+
+@pytest.mark.parametrize("B,T,hidden,heads,cu", [(2, 65, 512, 4, None), (1, 200, 1024, 4, [0, 70, 71, 200]), (2, 128, 256, 2, None)])
+def test_training_step(B, T, hidden, heads, cu):
+    layer = _layer(hidden, heads)
+    ref = copy.deepcopy(layer).float()
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(B, T, hidden, generator=gen, device="cuda").to(torch.bfloat16)
+    do = torch.randn(B, T, hidden, generator=gen, device="cuda").to(torch.bfloat16)
+
+    def run(m, dt):
+        leaf = x.to(dt).requires_grad_()
+        o = m(leaf, cu_seqlens=cu)[0]
+        return [o, *torch.autograd.grad(o, [leaf, *m.parameters()], do.to(dt))]
+    got, labels = _labels(lambda: run(layer, torch.bfloat16))
+    assert "lowrank_gate_fwd" in labels
+    names = ["o", "x", *(n for n, _ in layer.named_parameters())]
+    for n, a, b in zip(names, got, run(ref, torch.float32)):
+        assert a.dtype == torch.bfloat16 and a.shape == b.shape
+        # dq and dk (and so dx) of a sequence's first token are what is left of do . o / |o|^2 after the norm's
+        # projection: rounding noise of do, amplified; everything else keeps the bf16 bar
+        bar = 0.2 if n in ("x", "q_proj.weight", "k_proj.weight") else 2e-2
+        assert rel_l2(a, b) <= bar, (n, rel_l2(a, b))
+
+
+@pytest.mark.parametrize("T1", [1, 3, 64, 65, 130])
+@pytest.mark.parametrize("B,hidden,heads", [(1, 1024, 4), (9, 512, 4)])
+def test_prompt_then_tokens(B, hidden, heads, T1):
+    from tops_b200.layers import Cache
+    layer = _layer(hidden, heads, clamp_min=-0.2)
+    ref = copy.deepcopy(layer).float()
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    xs = [torch.randn(B, T, hidden, generator=gen, device="cuda").to(torch.bfloat16) for T in (T1, 1, 2)]
+    with torch.no_grad():
+        caches = Cache(), Cache()
+        for x in xs:
+            (o, _, _), labels = _labels(lambda: layer(x, past_key_values=caches[0], use_cache=True))
+            assert ("lowrank_gate_fwd" in labels) == (x.shape[1] > 64 or B * x.shape[1] <= 64)
+            want = ref(x.float(), past_key_values=caches[1], use_cache=True)[0]
+            assert rel_l2(o, want) <= 2e-2
+            assert rel_l2(caches[0][0]["recurrent_state"], caches[1][0]["recurrent_state"]) <= 2e-2
+
+
+def test_watched_or_replaced_projections_are_called():
+    layer = _layer(512, 4)
+    x = torch.randn(1, 70, 512, device="cuda", dtype=torch.bfloat16)
+    seen = []
+    handle = layer.o_proj.register_forward_hook(lambda *a: seen.append(1))
+    layer(x)
+    handle.remove()
+    layer.v_proj = torch.nn.Sequential(layer.v_proj)   # no longer a plain linear
+    _, labels = _labels(lambda: layer(x))
+    assert seen and "lowrank_gate_fwd" not in labels
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16, 31, 33, 64])
+@pytest.mark.parametrize("K,Ns", [(32, (8,)), (96, (17, 16, 1)), (2048, (512, 40))])
+def test_skinny_linear(rows, K, Ns):
+    import ctypes as C
+
+    from tops_b200 import _lib as L
+    gen = torch.Generator(device="cuda").manual_seed(rows * K)
+    x = torch.randn(rows, K, generator=gen, device="cuda").to(torch.bfloat16)
+    Ws = [torch.randn(n, K, generator=gen, device="cuda").to(torch.bfloat16) for n in Ns]
+    ys = [torch.full((rows, n + 3), 7.0, device="cuda", dtype=torch.bfloat16) for n in Ns]
+
+    class Params(C.Structure):
+        _fields_ = [("rows", C.c_int32), ("K", C.c_int32), ("count", C.c_int32), ("x_pitch", C.c_int64), ("x", C.c_void_p),
+                    ("W", C.c_void_p * 6), ("y", C.c_void_p * 6), ("N", C.c_int32 * 6), ("y_pitch", C.c_int64 * 6)]
+    p = Params(rows, K, len(Ns), K, x.data_ptr())
+    for i, (W, y, n) in enumerate(zip(Ws, ys, Ns)):
+        p.W[i], p.y[i], p.N[i], p.y_pitch[i] = W.data_ptr(), y.data_ptr(), n, n + 3
+    L.check(L.lib.tops_b200_skinny_linear(C.byref(p), C.c_void_p(L.stream_ptr(x.device))), "skinny_linear")
+    for W, y, n in zip(Ws, ys, Ns):
+        want = x.double() @ W.double().t()
+        # fp32 sums of K products, one rounding to bf16 (2^-9 of the value)
+        bar = want.abs() * 2 ** -8 + (x.double().abs() @ W.double().abs().t()) * K * 2 ** -24
+        assert ((y[:, :n].double() - want).abs() <= bar).all() and (y[:, n:] == 7).all()
