@@ -357,11 +357,11 @@ int tops_b200_kda_fwd(const tops_kda_fwd_params* p, void* stream);
  *   Aqk_out, Akk_out  fp32 `[B,T,H,64]`: row i of its chunk at token i —
  *                     tril(scale q k^T exp(G_i - G_j)) and (I + stril(beta k k^T exp(G_i - G_j)))^-1,
  *                     the matrices `chunk_kda_fwd` returns;
- *   saved_h     bf16 `[B,NT,H,K,V]`  chunk-start states times exp(mid) per key channel,
- *   saved_vnew  bf16 `[B,T,H,V]`     the delta-corrected values v' = u - w h,
- *   saved_R     bf16 `[B,T,H,V]`     beta (v - k exp(G) h), the right-hand side of the solve (v' = Akk R),
- *   saved_T     bf16 `[B,T,H,64]`    the inverse above in bf16:
- *               residuals `tops_b200_chunk_kda_bwd` takes back (opaque to callers).
+ *   saved       what `tops_b200_chunk_kda_bwd` takes back, tops_b200_chunk_kda_saved_bytes of it (opaque: the chunks'
+ *               gated operands, Aqk, Akk and w = Akk diag(beta) k exp(G) as the scans read them, the chunk-start
+ *               states and the delta-corrected values v' = u - w h).
+ * Without `saved` the call needs tops_b200_chunk_kda_fwd_workspace_bytes of scratch in `workspace`; a NULL workspace is
+ * taken from the stream's memory pool for the length of the call.
  * ------------------------------------------------------------------------ */
 typedef struct {
   int32_t B, T, H, K, V, chunk;
@@ -372,9 +372,13 @@ typedef struct {
   void* o;         /* [B,T,H,V] */
   float* ht;       /* [B,H,K,V] or NULL */
   float *Aqk_out, *Akk_out;
-  void *saved_h, *saved_vnew, *saved_T, *saved_R;
+  void* saved;
+  void* workspace;
+  size_t workspace_bytes;
 } tops_chunk_kda_fwd_params;
 int tops_b200_chunk_kda_supported(const tops_chunk_kda_fwd_params* p);
+size_t tops_b200_chunk_kda_saved_bytes(const tops_chunk_kda_fwd_params* p);
+size_t tops_b200_chunk_kda_fwd_workspace_bytes(const tops_chunk_kda_fwd_params* p);
 int tops_b200_chunk_kda_fwd(const tops_chunk_kda_fwd_params* p, void* stream);
 
 /* ------------------------------------------------------------------------ *
@@ -386,11 +390,11 @@ int tops_b200_chunk_kda_fwd(const tops_chunk_kda_fwd_params* p, void* stream);
  * the WY backward), the gradients of the two per-chunk matrices (dAqk of `chunk_kda_bwd_dAv`, the
  * inverse's gradient of `prepare_wy_repr_bwd` `tops/cpu/ops/kda/wy_fast.py:96-224`), and the chunk
  * outputs (`chunk_kda_bwd_wy_dqkg_fused` + `chunk_kda_bwd_intra` + the reverse cumsum of dg).
- * `saved_*` are the residuals the forward wrote.  dq, dk, dg `[B,T,H,K]` and dbeta `[B,T,H]` in
+ * `saved` is what the forward wrote.  dq, dk, dg `[B,T,H,K]` and dbeta `[B,T,H]` in
  * `grad_dtype` (TOPS_F32 as the reference's orchestrator returns them, or TOPS_BF16); dv bf16;
  * dg is with respect to the natural-log gate; dh0 fp32 (NULL to skip).
  * State gradient only: with dq = dk = dg = dbeta = NULL the call runs the reverse scan alone and
- * writes dh0 (and dv).  The state gradient entering a span of tokens depends on the one leaving it
+ * writes dh0 (dv is left alone).  The state gradient entering a span of tokens depends on the one leaving it
  * linearly, dh_in = M^T dh_out + D; a call with dht = NULL gives D, the summary a rank needs when one
  * sequence is sharded over time (no counterpart in the reference, which has no multi-device path).
  * ------------------------------------------------------------------------ */
@@ -401,7 +405,7 @@ typedef struct {
   const void *q, *k, *v, *g, *beta;
   const void* do_;
   const float* dht; /* [B,H,K,V] or NULL */
-  const void *saved_h, *saved_vnew, *saved_T, *saved_R;
+  const void* saved;
   void *dq, *dk, *dg, *dbeta; /* all four, or all NULL (state gradient only) */
   int32_t grad_dtype;
   void* dv;

@@ -8,9 +8,14 @@
 //     q~ = q exp(E) scale      k^ = k exp(E)      k~ = k exp(-E)
 //     Aqk = tril(q~ k~^T)                                  (the scale rides on q~)
 //     L   = stril(diag(beta) k^ k~^T)        T = (I + L)^-1          (unit lower triangular, 64 x 64)
-//     v'  = T (beta (v - k^ h'))                            (= u - w h of the reference, u = T beta v, w = T beta k exp(G))
+//     T'  = T diag(beta)        w = T' k^
+//     v'  = T' v - w h'
 //     o   = q~ h' + Aqk v'
 //     h  <- h exp(G_n) + exp(G_n - mid) (k~^T v')
+// Everything down to w is a chunk's own business: k_kda_prep computes it for all chunks at once.  What is left to walk
+// from chunk to chunk (k_kda_scan_fwd) is two dependent products, w h' and k~^T v'; the reverse scan of the state
+// gradient (k_kda_scan_bwd) has the same shape, k~ dh^ and w^T dv', and reads the same tiles.  The rest of the backward
+// is chunk-parallel again (k_kda_bwd_intra, k_kda_bwd_out).
 // The cumulative gates are a tensor-core product of the gate tile with a constant 0 / +-1/2 / 1 pattern
 // (sm100_tiles.cuh), every contraction is a tcgen05.mma on bf16 tiles in shared memory with fp32
 // accumulators in tensor memory, the running state is fp32 in registers, and the 64 x 64 triangular
@@ -24,34 +29,12 @@ namespace tops {
 namespace sm100 {
 namespace {
 
-struct KdaFwdParams {
-  CUtensorMap mq, mk, mg, mv;
-  CUtensorMap mst;              // the states tensor as [B*NT*H*128, 128] (TMA stores); unused when states == nullptr
-  const __nv_bfloat16* beta;    // [B,T,H]
-  const float* s0;              // [B,H,K,V] or null (zero)
-  float* s_final;               // [B,H,K,V] or null
-  __nv_bfloat16* o;             // [B,T,H,V]
-  __nv_bfloat16* states;        // h' [B,NT,H,K,V] or null
-  __nv_bfloat16* vnew;          // v' [B,T,H,V] or null
-  __nv_bfloat16* rsave;         // R = beta (v - k^ h') [B,T,H,V] or null
-  __nv_bfloat16* t_saved;       // T  [B,T,H,64] bf16 or null
-  float* Aqk_out;               // [B,T,H,64] fp32 or null
-  float* Akk_out;               // [B,T,H,64] fp32 or null
-  int T, H, NT;
-  float scale;
-};
-
-struct KdaFwdShared {
-  uint64_t fullqkg[2], fullv, ebar, abar, pbar, vbar, sbar, obar;
-  uint32_t tmem_slot;
-  int abort_flag;
-  float a[D], g0[D];        // G_n - mid and G_0 per channel of the current chunk
-  float beta[2][C];
-};
-
-constexpr uint32_t KDA_STAGE = 3 * TILE64;   // q, k, g
-constexpr size_t KDA_FWD_SMEM = 2 * KDA_STAGE + 3 * TILE64 + TILE128 + 2 * SLAB64 + 2 * SLAB64 + sizeof(KdaFwdShared);
-constexpr int KDA_THREADS = NTHREADS + 32;
+// What k_kda_prep leaves of a chunk of one head, in the order and the (swizzled) form the scans' shared memory wants it,
+// so that one untiled bulk copy brings it in: T' | k~ | -w | q~ | Aqk | (G_n, mid) per channel | T.
+constexpr uint32_t PREP_TB = 0, PREP_K = SLAB64, PREP_W = PREP_K + TILE64, PREP_Q = PREP_W + TILE64, PREP_A = PREP_Q + TILE64,
+                   PREP_F = PREP_A + SLAB64, PREP_T = PREP_F + D * 8, PREP_BYTES = PREP_T + SLAB64;
+constexpr uint32_t PREP_FWD = PREP_T;            // the forward scan reads all but T
+constexpr uint32_t PREP_BWD = PREP_T - PREP_K;   // the reverse scan k~ .. (G_n, mid)
 
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory"); }
 
@@ -112,732 +95,679 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ Lm, 
   compute_sync();
 }
 
-// One block per (batch, head): 16 compute warps (state in registers: thread (q4, lane, seg) owns state row
-// k = 32 q4 + lane, columns 32 seg .. + 31) and a driver warp whose first thread issues every product and
-// copy.  Four block-wide barriers per chunk separate the dependent steps:
-//   B1  q~, k^, k~ are in shared memory                 -> Aqk, L products
-//   B2  h' is staged, L (fp32) and Aqk (bf16) are out   -> k^ h', q~ h' products (and the h' store)
-//       meanwhile the compute warps invert I + L
-//   B3  T (bf16) and R = beta (v - k^ h') are out        -> v' = T R
-//   B4  v' is in shared memory                           -> k~^T v', o += Aqk v'; exponents of the next chunk
-__global__ void __launch_bounds__(KDA_THREADS, 1) k_kda_fwd(const __grid_constant__ KdaFwdParams p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* in = smem;                       // 2 stages x (q, k, g); the g tile later holds L in fp32
-  uint8_t* vs = in + 2 * KDA_STAGE;         // v
-  uint8_t* khs = vs + TILE64;               // k^
-  uint8_t* rt = khs + TILE64;               // T in fp32 during the inversion, then R, then v'
-  uint8_t* hst = rt + TILE64;               // h' (128 x 128)
-  uint8_t* tt = hst + TILE128;              // T bf16 (64 x 64); scratch of the inversion before that
-  uint8_t* at = tt + SLAB64;                // Aqk bf16 (64 x 64)
-  uint8_t* mt = at + SLAB64;                // TRI_MID pattern, rows repeated to 128
-  KdaFwdShared& sh = *reinterpret_cast<KdaFwdShared*>(mt + 2 * SLAB64);
-  volatile int* abort_flag = &sh.abort_flag;
+// ===========================================================================
+// Chunk-parallel part of the forward
+// ===========================================================================
+struct KdaPrepParams {
+  CUtensorMap mq, mk, mg;
+  const __nv_bfloat16* beta;    // [B,T,H]
+  uint8_t* prep;                // [B*NT*H] x PREP_BYTES
+  float* Aqk_out;               // [B,T,H,64] fp32 or null
+  float* Akk_out;               // [B,T,H,64] fp32 or null
+  int T, H, NT, total;          // total = B * H * NT chunks
+  float scale;
+};
+struct KdaPrepShared {
+  uint64_t bar_load, bar_e, bar_a, bar_w;
+  uint32_t tmem_slot;
+  float a[D], g0[D];      // G_n - mid and G_0 per channel
+  alignas(16) float2 f[D];   // (G_n, mid): the source of a bulk copy
+  float beta[C];
+};
+constexpr size_t KDA_PREP_SMEM = 4 * TILE64 + 3 * SLAB64 + 2 * SLAB64 + sizeof(KdaPrepShared) + 1024;
+
+// Persistent, two blocks per SM (104 KB of shared memory, 256 tensor-memory columns each): a chunk is a chain of short
+// dependent steps (exponents, gating, two products, the inversion, w), and the other block's chunk fills the waits.
+__global__ void __launch_bounds__(NTHREADS, 2) k_kda_prep(const __grid_constant__ KdaPrepParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  uint8_t* qs = smem;                 // q -> q~ in place; then T in fp32 during the inversion
+  uint8_t* ks = qs + TILE64;          // k -> k~ in place
+  uint8_t* gs = ks + TILE64;          // g; then L in fp32
+  uint8_t* khs = gs + TILE64;         // k^; then -w
+  uint8_t* tb = khs + TILE64;         // T' (bf16); scratch of the inversion before that
+  uint8_t* ts = tb + SLAB64;          // T (bf16)
+  uint8_t* at = ts + SLAB64;          // Aqk (bf16)
+  uint8_t* mt = at + SLAB64;          // TRI_MID pattern, rows repeated to 128
+  KdaPrepShared& sh = *reinterpret_cast<KdaPrepShared*>(mt + 2 * SLAB64);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool driver = warp == 16;
-  const int q4 = warp & 3, seg = (warp >> 2) & 3, col = q4 * 32 + lane;
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const int NT = p.NT;
-  constexpr uint32_t cE = 0, cD = 128, cO = 256, cA = 384, cK = 448;   // cE later holds k^ h' and then v'
-  if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
-    if (tid == 0) fail(12);
-    return;
-  }
-  auto issue_qkg = [&](int pp) {
-    uint8_t* qs = in + (pp & 1) * KDA_STAGE;
-    uint8_t *ks = qs + TILE64, *gs = ks + TILE64;
-    uint64_t* bar = &sh.fullqkg[pp & 1];
-    const int row = b * p.T + pp * C;
-    mbar_expect_tx(bar, KDA_STAGE);
-    tma_load_3d(gs, &p.mg, bar, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, bar, 64, h, row);
-    tma_load_3d(qs, &p.mq, bar, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, bar, 64, h, row);
-    tma_load_3d(ks, &p.mk, bar, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, bar, 64, h, row);
-  };
-  auto issue_v = [&](int pp) {
-    const int row = b * p.T + pp * C;
-    mbar_expect_tx(&sh.fullv, TILE64);
-    tma_load_3d(vs, &p.mv, &sh.fullv, 0, h, row); tma_load_3d(vs + SLAB64, &p.mv, &sh.fullv, 64, h, row);
-  };
-  auto load_beta = [&](int pp) {   // threads 0..63
-    sh.beta[pp & 1][tid] = __bfloat162float(p.beta[((size_t)b * p.T + pp * C + tid) * p.H + h]);
-  };
+  const int q4 = warp & 3, seg = warp >> 2;
+  constexpr uint32_t cE = 0, cA = 128, cK = 192;   // cE later holds w
   if (tid == 0) {
-    mbar_init(&sh.fullqkg[0], 1); mbar_init(&sh.fullqkg[1], 1); mbar_init(&sh.fullv, 1);
-    mbar_init(&sh.ebar, 1); mbar_init(&sh.abar, 1); mbar_init(&sh.pbar, 1); mbar_init(&sh.vbar, 1);
-    mbar_init(&sh.sbar, 1); mbar_init(&sh.obar, 1);
+    mbar_init(&sh.bar_load, 1); mbar_init(&sh.bar_e, 1); mbar_init(&sh.bar_a, 1); mbar_init(&sh.bar_w, 1);
     fence_barrier_init();
-    tma_prefetch_desc(&p.mq); tma_prefetch_desc(&p.mk); tma_prefetch_desc(&p.mg); tma_prefetch_desc(&p.mv);
-    if (p.states) tma_prefetch_desc(&p.mst);
-    sh.abort_flag = 0;
-    issue_qkg(0);
-    issue_v(0);
-    if (NT > 1) issue_qkg(1);
+    tma_prefetch_desc(&p.mq); tma_prefetch_desc(&p.mk); tma_prefetch_desc(&p.mg);
   }
   __syncwarp();
-  if (warp == 0) { tmem_alloc(&sh.tmem_slot, 512); tmem_relinquish(); }
-  if (tid < C) load_beta(0);
+  if (warp == 0) { tmem_alloc(&sh.tmem_slot, 256); tmem_relinquish(); }
   build_tri_tile(mt, 128, TRI_MID);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm = sh.tmem_slot;
-  const uint32_t lane_base = q4 * 32;
-
-  if (driver) {
-    // ------------------------------------------------------------------ products and copies
-    auto issue_exponents = [&](int pp) {
-      if (!mbar_wait(&sh.fullqkg[pp & 1], (pp >> 1) & 1)) { *abort_flag = 1; fail(3); }
+  const uint32_t tm = sh.tmem_slot, lane_base = q4 * 32;
+  const int ri = 16 * q4 + lane;   // row of an M = 64 accumulator held by lanes 0..15 of each quarter
+  const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), kha = smem_u32(khs), ga = smem_u32(gs), ma = smem_u32(mt), tba = smem_u32(tb);
+  bool ok = true;
+  int it = 0;
+  for (int cid = blockIdx.x; cid < p.total; cid += gridDim.x, ++it) {
+    const uint32_t ph = it & 1;
+    const int h = cid % p.H, row = (cid / p.H) * C;   // chunks are numbered (batch, chunk, head): token row = 64 x (batch, chunk)
+    uint8_t* out = p.prep + (size_t)cid * PREP_BYTES;
+    if (tid == 0) {
+      tma_store_wait_read();   // the previous chunk's tiles have been read
+      mbar_expect_tx(&sh.bar_load, 3 * TILE64);
+      tma_load_3d(gs, &p.mg, &sh.bar_load, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, &sh.bar_load, 64, h, row);
+      tma_load_3d(qs, &p.mq, &sh.bar_load, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, &sh.bar_load, 64, h, row);
+      tma_load_3d(ks, &p.mk, &sh.bar_load, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, &sh.bar_load, 64, h, row);
+    }
+    if (tid < C) sh.beta[tid] = __bfloat162float(p.beta[(size_t)(row + tid) * p.H + h]);
+    ok = __syncthreads_and(mbar_wait(&sh.bar_load, ph));
+    if (!ok) { fail(3); break; }
+    if (tid == 0) {
       tc_fence_after();
-      const uint32_t ga = smem_u32(in + (pp & 1) * KDA_STAGE + 2 * TILE64), ma = smem_u32(mt);
 #pragma unroll
       for (int j0 = 0; j0 < C; j0 += 16)   // E = G - mid: [time (repeated to 128 lanes)][channel]
         umma_bf16(tm + cE, desc_kmajor(ma, 128, 0, j0), desc_mnmajor(ga, 64, j0, 0), umma_idesc(128, 128, 0, 1), j0 > 0);
-      umma_commit(&sh.ebar);
-    };
-    if (lane == 0) issue_exponents(0);
-    __syncwarp();
-    for (int pp = 0; pp < NT; ++pp) {
-      const uint32_t ph = pp & 1;
-      uint8_t* qs = in + (pp & 1) * KDA_STAGE;
-      uint8_t* ks = qs + TILE64;
-      const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), kha = smem_u32(khs), ha = smem_u32(hst), ra = smem_u32(rt),
-                     ta = smem_u32(tt), aa = smem_u32(at);
-      // the state store of the previous chunk has read its staging tile, which the compute warps refill
-      // after the next barrier
-      if (lane == 0) tma_store_wait_read();
-      if (__syncthreads_or(*abort_flag)) break;   // B1
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // Aqk = q~ k~^T
-          umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // k^ k~^T
-          umma_bf16(tm + cK, desc_kmajor(kha, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-        umma_commit(&sh.abar);
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B2
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // P = k^ h'
-          umma_bf16(tm + cE, desc_kmajor(kha, 64, 0, k0), desc_mnmajor(ha, 128, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
-        umma_commit(&sh.pbar);
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // o = q~ h'
-          umma_bf16(tm + cO, desc_kmajor(qa, 64, 0, k0), desc_mnmajor(ha, 128, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
-        if (p.states) {
-          const int hrow = ((b * NT + pp) * p.H + h) * D;
-          tma_store_2d(&p.mst, hst, 0, hrow);
-          tma_store_2d(&p.mst, hst + TILE128 / 2, 64, hrow);
-          tma_store_commit();
-        }
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B3
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // v' = T R
-          umma_bf16(tm + cE, desc_kmajor(ta, 64, 0, k0), desc_mnmajor(ra, 64, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
-        umma_commit(&sh.vbar);
-        if (pp + 1 < NT) issue_v(pp + 1);    // R has been formed: the v tile is free
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B4
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_j k~[j][k] v'[j][v]
-          umma_bf16(tm + cD, desc_mnmajor(ka, 64, k0, 0), desc_mnmajor(ra, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
-        umma_commit(&sh.sbar);
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // o += Aqk v'
-          umma_bf16(tm + cO, desc_kmajor(aa, 64, 0, k0), desc_mnmajor(ra, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
-        umma_commit(&sh.obar);
-        if (pp + 1 < NT) issue_exponents(pp + 1);   // (v' has left tensor memory before B4)
-        if (pp + 2 < NT) {                          // every tile of this stage is dead once these products are complete
-          if (!mbar_wait(&sh.obar, ph)) { *abort_flag = 1; fail(5); }
-          issue_qkg(pp + 2);
-        }
-      }
-      __syncwarp();
+      umma_commit(&sh.bar_e);
     }
-    if (lane == 0) tma_store_wait_all();
-  } else {
-    // ------------------------------------------------------------------ state in registers
+    __syncwarp();
+    ok = __syncthreads_and(mbar_wait(&sh.bar_e, ph));
+    if (!ok) { fail(9); break; }
+    tc_fence_after();
+    {   // gate q and k: thread (q4, lane, seg) owns time row (32 q4 + lane) mod 64 and 16 channels
+      const int i = (q4 * 32 + lane) & 63;
+      const int cg = (q4 >> 1) * 4 + seg;
+      float em[16];
+      tmem_ld16(tmem_addr(tm, lane_base, cE + cg * 16), em);
+      const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
+      if (i == 63) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t) sh.a[cg * 16 + t] = em[t];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
+        if (i == 0) {   // G_0 = g_0
+          const uint4 graw = *reinterpret_cast<const uint4*>(gs + off);
+          const __nv_bfloat162* pg = reinterpret_cast<const __nv_bfloat162*>(&graw);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 x = __bfloat1622float2(pg[t]);
+            sh.g0[cg * 16 + 8 * u + 2 * t] = x.x;
+            sh.g0[cg * 16 + 8 * u + 2 * t + 1] = x.y;
+          }
+        }
+        float f[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) f[t] = fast_exp(-em[8 * u + t]);
+        const uint4 kraw = *reinterpret_cast<const uint4*>(ks + off);
+        *reinterpret_cast<uint4*>(ks + off) = scale8(kraw, f);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) f[t] = fast_exp(em[8 * u + t]);
+        *reinterpret_cast<uint4*>(khs + off) = scale8(kraw, f);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) f[t] *= p.scale;
+        *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), f);
+      }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid < D) sh.f[tid] = make_float2(2.f * sh.a[tid] + sh.g0[tid], sh.a[tid] + sh.g0[tid]);
+    if (tid == 0) {
+      tc_fence_after();
+#pragma unroll
+      for (int k0 = 0; k0 < D; k0 += 16)   // k^ k~^T
+        umma_bf16(tm + cK, desc_kmajor(kha, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+#pragma unroll
+      for (int k0 = 0; k0 < D; k0 += 16)   // Aqk = q~ k~^T
+        umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+      umma_commit(&sh.bar_a);
+      bulk_store(out + PREP_K, ks, TILE64);
+      bulk_store(out + PREP_Q, qs, TILE64);
+      tma_store_commit();
+    }
+    __syncwarp();
+    ok = __syncthreads_and(mbar_wait(&sh.bar_a, ph));
+    if (!ok) { fail(4); break; }
+    tc_fence_after();
+    float* Lm = reinterpret_cast<float*>(gs);
+    float* Tm = reinterpret_cast<float*>(qs);
+    {   // L = stril(beta k^ k~^T) in fp32 for the inversion; Aqk -> bf16
+      float a[16];
+      tmem_ld16(tmem_addr(tm, lane_base, cK + seg * 16), a);
+      if (lane < 16) {
+        const float bi = sh.beta[ri];
+#pragma unroll
+        for (int t = 0; t < 16; t += 4) {
+          const int j = seg * 16 + t;
+          *reinterpret_cast<float4*>(Lm + ri * C + j) =
+              make_float4(j < ri ? bi * a[t] : 0.f, j + 1 < ri ? bi * a[t + 1] : 0.f, j + 2 < ri ? bi * a[t + 2] : 0.f,
+                          j + 3 < ri ? bi * a[t + 3] : 0.f);
+        }
+      }
+      tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
+      if (lane < 16) {
+        store_tril16(at, ri, seg * 16, a, 1.f);
+        if (p.Aqk_out) {
+          float* dst = p.Aqk_out + ((size_t)(row + ri) * p.H + h) * C + seg * 16;
+#pragma unroll
+          for (int t = 0; t < 16; t += 4) {
+            const int j = seg * 16 + t;
+            *reinterpret_cast<float4*>(dst + t) = make_float4(j <= ri ? a[t] : 0.f, j + 1 <= ri ? a[t + 1] : 0.f,
+                                                              j + 2 <= ri ? a[t + 2] : 0.f, j + 3 <= ri ? a[t + 3] : 0.f);
+          }
+        }
+      }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    if (tid == 0) tma_store_wait_read();   // q~ has left: its tile holds T from here on
+    __syncthreads();
+    invert_unit_lower(Lm, Tm, reinterpret_cast<float*>(tb), tid);
+    {
+      const int i = tid >> 3, j0 = (tid & 7) * 8;
+      const float4 x = *reinterpret_cast<const float4*>(Tm + i * C + j0);
+      const float4 y = *reinterpret_cast<const float4*>(Tm + i * C + j0 + 4);
+      const float* bj = sh.beta + j0;
+      *reinterpret_cast<uint4*>(ts + slab_off(i, j0)) =
+          make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
+      *reinterpret_cast<uint4*>(tb + slab_off(i, j0)) =
+          make_uint4(pack_bf16(x.x * bj[0], x.y * bj[1]), pack_bf16(x.z * bj[2], x.w * bj[3]), pack_bf16(y.x * bj[4], y.y * bj[5]),
+                     pack_bf16(y.z * bj[6], y.w * bj[7]));
+      if (p.Akk_out) {
+        float* dst = p.Akk_out + ((size_t)(row + i) * p.H + h) * C + j0;
+        *reinterpret_cast<float4*>(dst) = x;
+        *reinterpret_cast<float4*>(dst + 4) = y;
+      }
+    }
+    fence_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+#pragma unroll
+      for (int k0 = 0; k0 < C; k0 += 16)   // w[i][k] = sum_j T'[i][j] k^[j][k]
+        umma_bf16(tm + cE, desc_kmajor(tba, 64, 0, k0), desc_mnmajor(kha, 64, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
+      umma_commit(&sh.bar_w);
+      bulk_store(out + PREP_TB, tb, SLAB64);
+      bulk_store(out + PREP_A, at, SLAB64);
+      bulk_store(out + PREP_F, sh.f, D * 8);
+      bulk_store(out + PREP_T, ts, SLAB64);
+      tma_store_commit();
+    }
+    __syncwarp();
+    ok = __syncthreads_and(mbar_wait(&sh.bar_w, ph));
+    if (!ok) { fail(5); break; }
+    tc_fence_after();
+    {
+      float x[32];
+      tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), x);
+      if (lane < 16) {
+#pragma unroll
+        for (int t = 0; t < 32; t += 8)
+          *reinterpret_cast<uint4*>(khs + tile_off(64, ri, seg * 32 + t)) =
+              make_uint4(pack_bf16(-x[t], -x[t + 1]), pack_bf16(-x[t + 2], -x[t + 3]), pack_bf16(-x[t + 4], -x[t + 5]),
+                         pack_bf16(-x[t + 6], -x[t + 7]));
+      }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      bulk_store(out + PREP_W, khs, TILE64);
+      tma_store_commit();
+    }
+  }
+  if (tid == 0) tma_store_wait_all();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tm, 256);
+  if (tid == 0 && !ok) poison(reinterpret_cast<__nv_bfloat16*>(p.prep + (size_t)blockIdx.x * PREP_BYTES + PREP_W));
+}
+
+// ===========================================================================
+// Forward scan and outputs
+// ===========================================================================
+// One block per (batch, head) walks its chunks.  The chain from one state to the next is
+//     h' staged -> v' += (-w) h' -> v' to bf16 -> k~^T v' -> state update -> h' staged
+// (T' v is in the accumulator before h' is there); the outputs q~ h' + Aqk v' run beside it and are written by warps of
+// their own.  The roles meet only through mbarriers:
+//   warps 0-15   state in registers: thread (q4, lane, seg) owns state row k = 32 q4 + lane, columns 32 seg .. + 31;
+//                stage h', pack v', update the state
+//   warps 16-19  write the outputs of a chunk
+//   warp 20      one thread issues every product and the stores of h' and v' for a backward pass
+//   warp 21      one thread issues the loads, two chunks ahead
+// A form with everything of a chunk in one chain (four dependent product rounds and the inversion) took 10.4 us a
+// chunk; this one FWD_US.
+struct KdaScanFwdParams {
+  CUtensorMap mv, mvn, mst;     // v; v' [B*T,H,128] and h' [B*NT*H*128, 128] (TMA stores, only when kept)
+  const uint8_t* prep;
+  const float* s0;              // [B,H,K,V] or null (zero)
+  float* s_final;               // [B,H,K,V] or null
+  __nv_bfloat16* o;             // [B,T,H,V]
+  int keep;                     // store h' and v'
+  int T, H, NT;
+};
+struct KdaScanFwdShared {
+  uint64_t full[2], hready, vbar, vready, sbar, obar[2], ofree[2];
+  uint32_t tmem_slot;
+  volatile int abort_flag;
+};
+constexpr int KDA_SF_THREADS = NTHREADS + 192;
+constexpr uint32_t KDA_SF_STAGE = PREP_FWD + TILE64;   // + v
+constexpr size_t KDA_SF_SMEM = 2 * KDA_SF_STAGE + TILE128 + TILE64 + sizeof(KdaScanFwdShared);
+
+// bounded wait that also gives up when another role has failed
+__device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  fail(code);
+  return false;
+}
+
+__global__ void __launch_bounds__(KDA_SF_THREADS, 1) k_kda_scan_fwd(const __grid_constant__ KdaScanFwdParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* hst = smem + 2 * KDA_SF_STAGE;   // h' (128 x 128)
+  uint8_t* vts = hst + TILE128;             // v' (64 x 128)
+  KdaScanFwdShared& sh = *reinterpret_cast<KdaScanFwdShared*>(vts + TILE64);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x % p.H, b = blockIdx.x / p.H, NT = p.NT;
+  constexpr uint32_t cV = 0, cD = 128, cO = 256;   // cO: two accumulators
+  if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
+    if (tid == 0) fail(12);
+    return;
+  }
+  auto stage = [&](int c) { return smem + (c & 1) * KDA_SF_STAGE; };
+  auto slot = [&](int c) { return (size_t)(b * NT + c) * p.H + h; };
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return role_wait(bar, parity, &sh.abort_flag, code); };
+  if (tid == 0) {
+    mbar_init(&sh.full[0], 1); mbar_init(&sh.full[1], 1); mbar_init(&sh.hready, NTHREADS); mbar_init(&sh.vready, NTHREADS);
+    mbar_init(&sh.vbar, 1); mbar_init(&sh.sbar, 1); mbar_init(&sh.obar[0], 1); mbar_init(&sh.obar[1], 1);
+    mbar_init(&sh.ofree[0], 128); mbar_init(&sh.ofree[1], 128);
+    fence_barrier_init();
+    sh.abort_flag = 0;
+  }
+  __syncwarp();
+  if (warp == 0) { tmem_alloc(&sh.tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tm = sh.tmem_slot;
+
+  if (warp < 16) {
+    // ------------------------------------------------------------------ state
+    const int q4 = warp & 3, seg = warp >> 2, col = q4 * 32 + lane, ri = 16 * q4 + lane;
+    const uint32_t lane_base = q4 * 32;
     float S[32];
     {
-      const float* src = p.s0 ? p.s0 + ((size_t)bh * D + col) * D + seg * 32 : nullptr;
+      const float* src = p.s0 ? p.s0 + ((size_t)blockIdx.x * D + col) * D + seg * 32 : nullptr;
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
         float4 x = src ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
         S[j] = x.x; S[j + 1] = x.y; S[j + 2] = x.z; S[j + 3] = x.w;
       }
     }
-    float* Lm = nullptr;
-    float* Tm = reinterpret_cast<float*>(rt);
-    float* Ws = reinterpret_cast<float*>(tt);
-    const int ri = 16 * q4 + lane;   // row of an M = 64 accumulator held by lanes 0..15 of each quarter
-    for (int pp = 0; pp < NT; ++pp) {
-      const uint32_t ph = pp & 1;
-      uint8_t* qs = in + (pp & 1) * KDA_STAGE;
-      uint8_t *ks = qs + TILE64, *gs = ks + TILE64;
-      Lm = reinterpret_cast<float*>(gs);
-      const int row0 = b * p.T + pp * C;
-      // ---- gate q and k: thread (q4, lane, seg) owns time row (32 q4 + lane) mod 64 and 16 channels
-      if (!mbar_wait(&sh.fullqkg[pp & 1], (pp >> 1) & 1) || !mbar_wait(&sh.ebar, ph)) { *abort_flag = 1; fail(9); }
-      tc_fence_after();
-      {
-        const int i = (q4 * 32 + lane) & 63;
-        const int cg = (q4 >> 1) * 4 + seg;
-        float em[16];
-        tmem_ld16(tmem_addr(tm, lane_base, cE + cg * 16), em);
-        const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
-        if (i == 63) {
+    auto factors = [&](int c) { return reinterpret_cast<const float2*>(stage(c) + PREP_F)[col]; };   // (G_n, mid)
+    bool ok = wait(&sh.full[0], 0, 3);
+    float2 f = ok ? factors(0) : make_float2(0.f, 0.f);
+    for (int c = 0; ok && c < NT; ++c) {
+      const float hscale = fast_exp(f.y), decay = fast_exp(f.x), c2 = fast_exp(f.x - f.y);
 #pragma unroll
-          for (int t = 0; t < 16; ++t) sh.a[cg * 16 + t] = em[t];
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-          float f[8], fs[8], r[8];
-#pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            f[t] = fast_exp(em[8 * u + t]);
-            fs[t] = f[t] * p.scale;
-            r[t] = fast_exp(-em[8 * u + t]);
-          }
-          const uint4 kraw = *reinterpret_cast<const uint4*>(ks + off);
-          if (i == 0) {   // G_0 = g_0
-            const uint4 graw = *reinterpret_cast<const uint4*>(gs + off);
-            const __nv_bfloat162* pg = reinterpret_cast<const __nv_bfloat162*>(&graw);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float2 x = __bfloat1622float2(pg[t]);
-              sh.g0[cg * 16 + 8 * u + 2 * t] = x.x;
-              sh.g0[cg * 16 + 8 * u + 2 * t + 1] = x.y;
-            }
-          }
-          *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), fs);
-          *reinterpret_cast<uint4*>(khs + off) = scale8(kraw, f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8(kraw, r);
-        }
-      }
+      for (int j = 0; j < 32; j += 8)
+        *reinterpret_cast<uint4*>(hst + tile_off(128, col, seg * 32 + j)) =
+            make_uint4(pack_bf16(S[j] * hscale, S[j + 1] * hscale), pack_bf16(S[j + 2] * hscale, S[j + 3] * hscale),
+                       pack_bf16(S[j + 4] * hscale, S[j + 5] * hscale), pack_bf16(S[j + 6] * hscale, S[j + 7] * hscale));
       fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B1
-      // ---- per-channel factors of this thread's state row; stage h' = h exp(mid)
-      const float av = sh.a[col], g0v = sh.g0[col];
-      const float decay = fast_exp(2.f * av + g0v);   // exp(G_n)
-      const float c2 = fast_exp(av);                  // exp(G_n - mid)
-      {
-        const float hscale = fast_exp(av + g0v);      // exp(mid)
-#pragma unroll
-        for (int j = 0; j < 32; j += 8)
-          *reinterpret_cast<uint4*>(hst + tile_off(128, col, seg * 32 + j)) =
-              make_uint4(pack_bf16(S[j] * hscale, S[j + 1] * hscale), pack_bf16(S[j + 2] * hscale, S[j + 3] * hscale),
-                         pack_bf16(S[j + 4] * hscale, S[j + 5] * hscale), pack_bf16(S[j + 6] * hscale, S[j + 7] * hscale));
-      }
-      // ---- L = stril(beta k^ k~^T) in fp32 for the inversion; Aqk -> bf16 operand
-      if (!mbar_wait(&sh.abar, ph)) { *abort_flag = 1; fail(4); }
+      mbar_arrive(&sh.hready);
+      if (!(ok = wait(&sh.vbar, c & 1, 7))) break;
       tc_fence_after();
       {
-        float a[16];
-        tmem_ld16(tmem_addr(tm, lane_base, cK + seg * 16), a);
+        float x[32];
+        tmem_ld32(tmem_addr(tm, lane_base, cV + seg * 32), x);
         if (lane < 16) {
-          const float bi = sh.beta[ph][ri];
-#pragma unroll
-          for (int t = 0; t < 16; t += 4) {
-            const int j = seg * 16 + t;
-            *reinterpret_cast<float4*>(Lm + ri * C + j) =
-                make_float4(j < ri ? bi * a[t] : 0.f, j + 1 < ri ? bi * a[t + 1] : 0.f, j + 2 < ri ? bi * a[t + 2] : 0.f,
-                            j + 3 < ri ? bi * a[t + 3] : 0.f);
-          }
-        }
-        tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
-        if (lane < 16) {
-          store_tril16(at, ri, seg * 16, a, 1.f);
-          if (p.Aqk_out) {
-            float* dst = p.Aqk_out + ((size_t)(row0 + ri) * p.H + h) * C + seg * 16;
-#pragma unroll
-            for (int t = 0; t < 16; t += 4) {
-              const int j = seg * 16 + t;
-              *reinterpret_cast<float4*>(dst + t) = make_float4(j <= ri ? a[t] : 0.f, j + 1 <= ri ? a[t + 1] : 0.f,
-                                                                j + 2 <= ri ? a[t + 2] : 0.f, j + 3 <= ri ? a[t + 3] : 0.f);
-            }
-          }
-        }
-      }
-      fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B2
-      // ---- T = (I + L)^-1 while the tensor core forms k^ h' and q~ h'
-      invert_unit_lower(Lm, Tm, Ws, tid);
-      {
-        const int i = tid >> 3, j0 = (tid & 7) * 8;
-        const float4 x = *reinterpret_cast<const float4*>(Tm + i * C + j0);
-        const float4 y = *reinterpret_cast<const float4*>(Tm + i * C + j0 + 4);
-        const uint4 packed = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
-        *reinterpret_cast<uint4*>(tt + slab_off(i, j0)) = packed;
-        const size_t orow = ((size_t)(row0 + i) * p.H + h) * C + j0;
-        if (p.t_saved) *reinterpret_cast<uint4*>(p.t_saved + orow) = packed;
-        if (p.Akk_out) {
-          *reinterpret_cast<float4*>(p.Akk_out + orow) = x;
-          *reinterpret_cast<float4*>(p.Akk_out + orow + 4) = y;
-        }
-      }
-      compute_sync();   // T (fp32) has been read: its place is free for R
-      // ---- R = beta (v - k^ h')
-      if (!mbar_wait(&sh.fullv, ph) || !mbar_wait(&sh.pbar, ph)) { *abort_flag = 1; fail(6); }
-      tc_fence_after();
-      {
-        float pv[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), pv);
-        if (lane < 16) {
-          const float bi = sh.beta[ph][ri];
-          __nv_bfloat16* rdst = p.rsave ? p.rsave + ((size_t)(row0 + ri) * p.H + h) * D + seg * 32 : nullptr;
-#pragma unroll
-          for (int t = 0; t < 32; t += 8) {
-            const uint32_t off = tile_off(64, ri, seg * 32 + t);
-            const uint4 vraw = *reinterpret_cast<const uint4*>(vs + off);
-            const __nv_bfloat162* pvv = reinterpret_cast<const __nv_bfloat162*>(&vraw);
-            uint32_t w[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float2 x = __bfloat1622float2(pvv[u]);
-              w[u] = pack_bf16(bi * (x.x - pv[t + 2 * u]), bi * (x.y - pv[t + 2 * u + 1]));
-            }
-            *reinterpret_cast<uint4*>(rt + off) = make_uint4(w[0], w[1], w[2], w[3]);
-            if (rdst) *reinterpret_cast<uint4*>(rdst + t) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-        }
-      }
-      fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B3
-      // ---- v' -> bf16 operand (in the place of R) and, for a backward pass, to global memory
-      if (!mbar_wait(&sh.vbar, ph)) { *abort_flag = 1; fail(7); }
-      tc_fence_after();
-      {
-        float nv[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), nv);
-        if (lane < 16) {
-          __nv_bfloat16* dst = p.vnew ? p.vnew + ((size_t)(row0 + ri) * p.H + h) * D + seg * 32 : nullptr;
-#pragma unroll
-          for (int t = 0; t < 32; t += 8) {
-            const uint4 packed = make_uint4(pack_bf16(nv[t], nv[t + 1]), pack_bf16(nv[t + 2], nv[t + 3]),
-                                            pack_bf16(nv[t + 4], nv[t + 5]), pack_bf16(nv[t + 6], nv[t + 7]));
-            *reinterpret_cast<uint4*>(rt + tile_off(64, ri, seg * 32 + t)) = packed;
-            if (dst) *reinterpret_cast<uint4*>(dst + t) = packed;
-          }
-        }
-      }
-      if (tid < C && pp + 1 < NT) load_beta(pp + 1);
-      fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B4
-      // ---- state update, outputs
-      if (!mbar_wait(&sh.sbar, ph)) { *abort_flag = 1; fail(2); }
-      tc_fence_after();
-      {
-        float d[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cD + seg * 32), d);
-#pragma unroll
-        for (int t = 0; t < 32; ++t) S[t] = fmaf(S[t], decay, c2 * d[t]);
-      }
-      if (!mbar_wait(&sh.obar, ph)) { *abort_flag = 1; fail(5); }
-      tc_fence_after();
-      {
-        float a[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cO + seg * 32), a);
-        if (lane < 16) {
-          __nv_bfloat16* dst = p.o + ((size_t)(row0 + ri) * p.H + h) * D + seg * 32;
 #pragma unroll
           for (int t = 0; t < 32; t += 8)
-            __stcs(reinterpret_cast<uint4*>(dst + t), make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]),
-                                                                   pack_bf16(a[t + 4], a[t + 5]), pack_bf16(a[t + 6], a[t + 7])));
+            *reinterpret_cast<uint4*>(vts + tile_off(64, ri, seg * 32 + t)) =
+                make_uint4(pack_bf16(x[t], x[t + 1]), pack_bf16(x[t + 2], x[t + 3]), pack_bf16(x[t + 4], x[t + 5]),
+                           pack_bf16(x[t + 6], x[t + 7]));
         }
       }
+      fence_async_smem();
+      tc_fence_before();
+      mbar_arrive(&sh.vready);
+      if (c + 1 < NT) {   // the next chunk's factors, while its product runs
+        if (!(ok = wait(&sh.full[(c + 1) & 1], ((c + 1) >> 1) & 1, 3))) break;
+        f = factors(c + 1);
+      }
+      if (!(ok = wait(&sh.sbar, c & 1, 2))) break;
+      tc_fence_after();
+      float d[32];
+      tmem_ld32(tmem_addr(tm, lane_base, cD + seg * 32), d);
+#pragma unroll
+      for (int t = 0; t < 32; ++t) S[t] = fmaf(S[t], decay, c2 * d[t]);
       tc_fence_before();
     }
-    if (!*abort_flag && p.s_final) {
-      float* dst = p.s_final + ((size_t)bh * D + col) * D + seg * 32;
+    if (ok && p.s_final) {
+      float* dst = p.s_final + ((size_t)blockIdx.x * D + col) * D + seg * 32;
 #pragma unroll
       for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
     }
+  } else if (warp < 20) {
+    // ------------------------------------------------------------------ outputs
+    const int g4 = warp & 3;
+    for (int c = 0; c < NT; ++c) {
+      if (!wait(&sh.obar[c & 1], (c >> 1) & 1, 5)) break;
+      tc_fence_after();
+      __nv_bfloat16* dst = p.o + ((size_t)(b * p.T + c * C + 16 * g4 + lane) * p.H + h) * D;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        float a[32];
+        tmem_ld32(tmem_addr(tm, g4 * 32, cO + (c & 1) * 128 + s * 32), a);
+        if (lane < 16) {
+#pragma unroll
+          for (int t = 0; t < 32; t += 8)
+            __stcs(reinterpret_cast<uint4*>(dst + s * 32 + t),
+                   make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]), pack_bf16(a[t + 4], a[t + 5]),
+                              pack_bf16(a[t + 6], a[t + 7])));
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&sh.ofree[c & 1]);
+    }
+  } else if (warp == 20) {
+    // ------------------------------------------------------------------ products, stores of h' and v'
+    if (lane == 0) {
+      const uint32_t ha = smem_u32(hst), va = smem_u32(vts);
+      auto issue_tv = [&](int c) {   // v' = T' v (to which -w h' is added)
+        const uint32_t tba = smem_u32(stage(c) + PREP_TB), vraw = smem_u32(stage(c) + PREP_FWD);
+        tc_fence_after();
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)
+          umma_bf16(tm + cV, desc_kmajor(tba, 64, 0, k0), desc_mnmajor(vraw, 64, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
+      };
+      bool ok = wait(&sh.full[0], 0, 3);
+      if (ok) issue_tv(0);
+      for (int c = 0; ok && c < NT; ++c) {
+        const uint32_t ka = smem_u32(stage(c) + PREP_K), wa = smem_u32(stage(c) + PREP_W), qa = smem_u32(stage(c) + PREP_Q),
+                       aa = smem_u32(stage(c) + PREP_A);
+        if (!wait(&sh.hready, c & 1, 8)) break;
+        tc_fence_after();
+        if (p.keep) tma_store_wait_read();   // v' of the chunk before has been read (its tile is refilled after vbar)
+#pragma unroll
+        for (int k0 = 0; k0 < D; k0 += 16)   // v' += (-w) h'
+          umma_bf16(tm + cV, desc_kmajor(wa, 64, 0, k0), desc_mnmajor(ha, 128, k0, 0), umma_idesc(64, 128, 0, 1), 1);
+        umma_commit(&sh.vbar);
+        if (c >= 2 && !wait(&sh.ofree[c & 1], ((c - 2) >> 1) & 1, 10)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k0 = 0; k0 < D; k0 += 16)   // o = q~ h'
+          umma_bf16(tm + cO + (c & 1) * 128, desc_kmajor(qa, 64, 0, k0), desc_mnmajor(ha, 128, k0, 0), umma_idesc(64, 128, 0, 1), k0 > 0);
+        if (p.keep) {
+          const int hrow = (int)slot(c) * D;
+          tma_store_2d(&p.mst, hst, 0, hrow);
+          tma_store_2d(&p.mst, hst + TILE128 / 2, 64, hrow);
+          tma_store_commit();
+        }
+        if (!wait(&sh.vready, c & 1, 11)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_j k~[j][k] v'[j][v]
+          umma_bf16(tm + cD, desc_mnmajor(ka, 64, k0, 0), desc_mnmajor(va, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
+        if (p.keep) {
+          const int row = b * p.T + c * C;
+          tma_store_3d(&p.mvn, vts, 0, h, row);
+          tma_store_3d(&p.mvn, vts + SLAB64, 64, h, row);
+          tma_store_commit();
+          tma_store_wait_read1();   // h' has been read: the state warps refill its tile after sbar
+        }
+        umma_commit(&sh.sbar);
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)   // o += Aqk v'
+          umma_bf16(tm + cO + (c & 1) * 128, desc_kmajor(aa, 64, 0, k0), desc_mnmajor(va, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
+        umma_commit(&sh.obar[c & 1]);        // and the stage is free
+        if (c + 1 < NT) {
+          if (!wait(&sh.full[(c + 1) & 1], ((c + 1) >> 1) & 1, 3)) break;
+          issue_tv(c + 1);                   // (v' has left tensor memory)
+        }
+      }
+      tma_store_wait_all();
+    }
+  } else {
+    // ------------------------------------------------------------------ loads
+    if (lane == 0) {
+      for (int c = 0; c < NT; ++c) {
+        if (c >= 2 && !wait(&sh.obar[c & 1], ((c - 2) >> 1) & 1, 5)) break;
+        uint64_t* bar = &sh.full[c & 1];
+        uint8_t* dst = stage(c);
+        const int row = b * p.T + c * C;
+        mbar_expect_tx(bar, KDA_SF_STAGE);
+        bulk_load(dst, p.prep + slot(c) * PREP_BYTES, PREP_FWD, bar);
+        tma_load_3d(dst + PREP_FWD, &p.mv, bar, 0, h, row);
+        tma_load_3d(dst + PREP_FWD + SLAB64, &p.mv, bar, 64, h, row);
+      }
+    }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && sh.abort_flag) {
     poison(p.o + ((size_t)b * p.T * p.H + h) * D);
-    if (p.s_final) poison(p.s_final + (size_t)bh * D * D);
+    if (p.s_final) poison(p.s_final + (size_t)blockIdx.x * D * D);
   }
 }
 
 // ===========================================================================
 // Backward, part A: the reverse scan of the state gradient
 // ===========================================================================
-// dh is the gradient with respect to the state a chunk hands on (h_next); per chunk, right to left,
-// with dh^ = exp(G_n - mid) dh (per key channel) and k^b = beta k^ (rows scaled by beta):
+// dh is the gradient with respect to the state a chunk hands on (h_next); per chunk, right to left, with
+// dh^ = exp(G_n - mid) dh (per key channel):
 //     dv'  = Aqk^T do + k~ dh^                         gradient of the delta-corrected values
-//     dR   = T^T dv'                                    gradient of the right-hand side of the solve
-//     dv   = beta dR                                    (output)        dbeta1 = sum_v dR v
-//     D    = q~^T do - k^b^T dR                         gradient with respect to h' = h exp(mid)
+//     D    = q~^T do - w^T dv'                         gradient with respect to h' = h exp(mid)
 //     dh  <- dh exp(G_n) + exp(mid) D
-// dh^ (bf16, [B,NT,H,K,V]), dv' and -dR (bf16, [B,T,H,V]) are kept for the chunk-parallel kernels that
-// finish dq, dk, dg and dbeta.  One block per (batch, head), dh in registers like the forward state.
-struct KdaScanParams {
-  CUtensorMap mq, mk, mg, mdo, mt;   // mt: T as [B*T, H, 64]
-  CUtensorMap mst;                   // dh^ states as [B*NT*H*128, 128] (TMA stores)
-  const __nv_bfloat16* beta;         // [B,T,H]
-  const __nv_bfloat16* v;            // [B,T,H,V]
+// Aqk^T do and q~^T do are in their accumulators before the chunk's dh^ is there, so the chain is two products as in
+// the forward scan: dh^ staged -> k~ dh^ -> dv' to bf16 -> w^T dv' -> update.  dh^ (bf16, [B,NT,H,K,V]) and dv' (bf16,
+// [B,T,H,V]) are kept for the chunk-parallel kernels.  Roles as above, without the output warps.
+struct KdaScanBwdParams {
+  CUtensorMap mdo, mdvn, mst;        // do; dv' and dh^ (TMA stores)
+  const uint8_t* prep;
   const float* dht;                  // [B,H,K,V] or null (zero)
   float* dh0;                        // [B,H,K,V] or null
-  __nv_bfloat16* dv;                 // [B,T,H,V] output
-  __nv_bfloat16* dvn;                // dv'  [B,T,H,V] scratch
-  __nv_bfloat16* ndr;                // -dR  [B,T,H,V] scratch
-  float* dbeta1;                     // [B,T,H] scratch: sum_v dR v
+  __nv_bfloat16* dvn;                // dv' (for the poison of a failed block)
   int T, H, NT;
-  float scale;
 };
-struct KdaScanShared {
-  uint64_t fullqkt[2], fullg, fulldo, ebar, abar, vbar, rbar, sbar;
+struct KdaScanBwdShared {
+  uint64_t full[2], free[2], hready, vbar, vready, sbar;
   uint32_t tmem_slot;
-  int abort_flag;
-  float a[D], g0[D];
-  float beta[2][C];
-  float db[C];
+  volatile int abort_flag;
 };
-constexpr uint32_t KDA_SCAN_STAGE = 2 * TILE64 + SLAB64;   // q, k, T
-constexpr size_t KDA_SCAN_SMEM = 2 * KDA_SCAN_STAGE + 5 * TILE64 + TILE128 + SLAB64 + 2 * SLAB64 + sizeof(KdaScanShared);
+constexpr int KDA_SB_THREADS = NTHREADS + 64;
+constexpr uint32_t KDA_SB_STAGE = PREP_BWD + TILE64;   // + do
+constexpr size_t KDA_SB_SMEM = 2 * KDA_SB_STAGE + TILE128 + TILE64 + sizeof(KdaScanBwdShared);
 
-__global__ void __launch_bounds__(KDA_THREADS, 1) k_kda_bwd_scan(const __grid_constant__ KdaScanParams p) {
+__global__ void __launch_bounds__(KDA_SB_THREADS, 1) k_kda_scan_bwd(const __grid_constant__ KdaScanBwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* in = smem;                        // 2 stages x (q, k, T)
-  uint8_t* gs = in + 2 * KDA_SCAN_STAGE;     // g
-  uint8_t* dos = gs + TILE64;                // do
-  uint8_t* khs = dos + TILE64;               // beta k^
-  uint8_t* dvs = khs + TILE64;               // dv'
-  uint8_t* nrs = dvs + TILE64;               // -dR
-  uint8_t* dhst = nrs + TILE64;              // dh^ (128 x 128)
-  uint8_t* at = dhst + TILE128;              // Aqk bf16 (64 x 64)
-  uint8_t* mt = at + SLAB64;                 // TRI_MID pattern, rows repeated to 128
-  KdaScanShared& sh = *reinterpret_cast<KdaScanShared*>(mt + 2 * SLAB64);
-  volatile int* abort_flag = &sh.abort_flag;
+  uint8_t* dhst = smem + 2 * KDA_SB_STAGE;   // dh^ (128 x 128)
+  uint8_t* dvs = dhst + TILE128;             // dv' (64 x 128)
+  KdaScanBwdShared& sh = *reinterpret_cast<KdaScanBwdShared*>(dvs + TILE64);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool driver = warp == 16;
-  const int q4 = warp & 3, seg = (warp >> 2) & 3, col = q4 * 32 + lane;
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const int NT = p.NT;
-  constexpr uint32_t cE = 0, cD = 128, cA = 256;   // cE later holds dv' and then dR
+  const int h = blockIdx.x % p.H, b = blockIdx.x / p.H, NT = p.NT;
+  constexpr uint32_t cV = 0, cD = 128;   // cD: two accumulators
   if ((smem_u32(smem) & 1023u) != 0) {
     if (tid == 0) fail(12);
     return;
   }
-  auto chunk_of = [&](int pp) { return NT - 1 - pp; };
-  auto issue_qkt = [&](int pp) {
-    uint8_t* qs = in + (pp & 1) * KDA_SCAN_STAGE;
-    uint8_t *ks = qs + TILE64, *ts = ks + TILE64;
-    uint64_t* bar = &sh.fullqkt[pp & 1];
-    const int row = b * p.T + chunk_of(pp) * C;
-    mbar_expect_tx(bar, KDA_SCAN_STAGE);
-    tma_load_3d(qs, &p.mq, bar, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, bar, 64, h, row);
-    tma_load_3d(ks, &p.mk, bar, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, bar, 64, h, row);
-    tma_load_3d(ts, &p.mt, bar, 0, h, row);
-  };
-  auto issue_g = [&](int pp) {
-    const int row = b * p.T + chunk_of(pp) * C;
-    mbar_expect_tx(&sh.fullg, TILE64);
-    tma_load_3d(gs, &p.mg, &sh.fullg, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, &sh.fullg, 64, h, row);
-  };
-  auto issue_do = [&](int pp) {
-    const int row = b * p.T + chunk_of(pp) * C;
-    mbar_expect_tx(&sh.fulldo, TILE64);
-    tma_load_3d(dos, &p.mdo, &sh.fulldo, 0, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &sh.fulldo, 64, h, row);
-  };
-  auto load_beta = [&](int pp) {   // threads 0..63
-    sh.beta[pp & 1][tid] = __bfloat162float(p.beta[((size_t)b * p.T + chunk_of(pp) * C + tid) * p.H + h]);
-  };
+  // (the stage holds the chunk's tiles from PREP_K on)
+  auto stage = [&](int c) { return smem + (c & 1) * KDA_SB_STAGE; };
+  auto chunk_of = [&](int c) { return NT - 1 - c; };
+  auto slot = [&](int c) { return (size_t)(b * NT + chunk_of(c)) * p.H + h; };
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return role_wait(bar, parity, &sh.abort_flag, code); };
   if (tid == 0) {
-    mbar_init(&sh.fullqkt[0], 1); mbar_init(&sh.fullqkt[1], 1); mbar_init(&sh.fullg, 1); mbar_init(&sh.fulldo, 1);
-    mbar_init(&sh.ebar, 1); mbar_init(&sh.abar, 1); mbar_init(&sh.vbar, 1); mbar_init(&sh.rbar, 1); mbar_init(&sh.sbar, 1);
+    mbar_init(&sh.full[0], 1); mbar_init(&sh.full[1], 1); mbar_init(&sh.free[0], 1); mbar_init(&sh.free[1], 1);
+    mbar_init(&sh.hready, NTHREADS); mbar_init(&sh.vready, NTHREADS); mbar_init(&sh.vbar, 1); mbar_init(&sh.sbar, 1);
     fence_barrier_init();
-    tma_prefetch_desc(&p.mq); tma_prefetch_desc(&p.mk); tma_prefetch_desc(&p.mg); tma_prefetch_desc(&p.mdo);
-    tma_prefetch_desc(&p.mt); tma_prefetch_desc(&p.mst);
     sh.abort_flag = 0;
-    issue_qkt(0);
-    issue_g(0);
-    issue_do(0);
-    if (NT > 1) issue_qkt(1);
   }
   __syncwarp();
   if (warp == 0) { tmem_alloc(&sh.tmem_slot, 512); tmem_relinquish(); }
-  if (tid < C) { load_beta(0); sh.db[tid] = 0.f; }
-  build_tri_tile(mt, 128, TRI_MID);
-  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sh.tmem_slot;
-  const uint32_t lane_base = q4 * 32;
 
-  if (driver) {
-    auto issue_exponents = [&](int pp) {
-      if (!mbar_wait(&sh.fullg, pp & 1)) { *abort_flag = 1; fail(3); }
-      tc_fence_after();
-      const uint32_t ga = smem_u32(gs), ma = smem_u32(mt);
-#pragma unroll
-      for (int j0 = 0; j0 < C; j0 += 16)   // E = G - mid: [time (repeated to 128 lanes)][channel]
-        umma_bf16(tm + cE, desc_kmajor(ma, 128, 0, j0), desc_mnmajor(ga, 64, j0, 0), umma_idesc(128, 128, 0, 1), j0 > 0);
-      umma_commit(&sh.ebar);
-    };
-    if (lane == 0) issue_exponents(0);
-    __syncwarp();
-    for (int pp = 0; pp < NT; ++pp) {
-      const uint32_t ph = pp & 1;
-      uint8_t* qs = in + (pp & 1) * KDA_SCAN_STAGE;
-      uint8_t *ks = qs + TILE64, *ts = ks + TILE64;
-      const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), ta = smem_u32(ts), kha = smem_u32(khs), doa = smem_u32(dos),
-                     dva = smem_u32(dvs), nra = smem_u32(nrs), dha = smem_u32(dhst), aa = smem_u32(at);
-      if (lane == 0) tma_store_wait_read();       // the dh^ store of the previous chunk has read its tile
-      if (__syncthreads_or(*abort_flag)) break;   // B1: q~, beta k^, k~ are in shared memory
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // Aqk = q~ k~^T
-          umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-        umma_commit(&sh.abar);
-        if (pp + 1 < NT) issue_g(pp + 1);    // the exponent product of this chunk is complete
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B2: dh^ is staged, Aqk (bf16) is out
-      if (lane == 0) {
-        if (!mbar_wait(&sh.fulldo, ph)) { *abort_flag = 1; fail(6); }
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // dv'[j][v] = sum_i Aqk[i][j] do[i][v]
-          umma_bf16(tm + cE, desc_mnmajor(aa, 64, k0, 0), desc_mnmajor(doa, 64, k0, 0), umma_idesc(64, 128, 1, 1), k0 > 0);
-#pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // dv' += k~ dh^
-          umma_bf16(tm + cE, desc_kmajor(ka, 64, 0, k0), desc_mnmajor(dha, 128, k0, 0), umma_idesc(64, 128, 0, 1), 1);
-        umma_commit(&sh.vbar);
-        const int hrow = ((b * NT + chunk_of(pp)) * p.H + h) * D;
-        tma_store_2d(&p.mst, dhst, 0, hrow);
-        tma_store_2d(&p.mst, dhst + TILE128 / 2, 64, hrow);
-        tma_store_commit();
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B3: dv' (bf16) is in shared memory
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // dR[j][v] = sum_i T[i][j] dv'[i][v]
-          umma_bf16(tm + cE, desc_mnmajor(ta, 64, k0, 0), desc_mnmajor(dva, 64, k0, 0), umma_idesc(64, 128, 1, 1), k0 > 0);
-        umma_commit(&sh.rbar);
-      }
-      if (__syncthreads_or(*abort_flag)) break;   // B4: -dR (bf16) is in shared memory
-      if (lane == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_i q~[i][k] do[i][v]
-          umma_bf16(tm + cD, desc_mnmajor(qa, 64, k0, 0), desc_mnmajor(doa, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
-#pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16)   // D += (beta k^)^T (-dR)
-          umma_bf16(tm + cD, desc_mnmajor(kha, 64, k0, 0), desc_mnmajor(nra, 64, k0, 0), umma_idesc(128, 128, 1, 1), 1);
-        umma_commit(&sh.sbar);
-        if (pp + 1 < NT) issue_exponents(pp + 1);   // (dR has left tensor memory before B4)
-        if (pp + 1 < NT) {
-          if (!mbar_wait(&sh.sbar, ph)) { *abort_flag = 1; fail(2); }
-          issue_do(pp + 1);                  // do, q~, k~, T of this chunk are dead
-          if (pp + 2 < NT) issue_qkt(pp + 2);
-        }
-      }
-      __syncwarp();
-    }
-    if (lane == 0) tma_store_wait_all();
-  } else {
+  if (warp < 16) {
+    const int q4 = warp & 3, seg = warp >> 2, col = q4 * 32 + lane, ri = 16 * q4 + lane;
+    const uint32_t lane_base = q4 * 32;
     float S[32];   // dh: row k = col, columns 32 seg .. + 31
     {
-      const float* src = p.dht ? p.dht + ((size_t)bh * D + col) * D + seg * 32 : nullptr;
+      const float* src = p.dht ? p.dht + ((size_t)blockIdx.x * D + col) * D + seg * 32 : nullptr;
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
         float4 x = src ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
         S[j] = x.x; S[j + 1] = x.y; S[j + 2] = x.z; S[j + 3] = x.w;
       }
     }
-    const int ri = 16 * q4 + lane;
-    for (int pp = 0; pp < NT; ++pp) {
-      const uint32_t ph = pp & 1;
-      uint8_t* qs = in + (pp & 1) * KDA_SCAN_STAGE;
-      uint8_t* ks = qs + TILE64;
-      const int row0 = b * p.T + chunk_of(pp) * C;
-      // this thread's 32 values of v (rows of M = 64 accumulators sit in lanes 0..15), for dbeta1
-      uint4 vreg[4];
-      if (lane < 16) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.v + ((size_t)(row0 + ri) * p.H + h) * D + seg * 32);
+    auto factors = [&](int c) { return reinterpret_cast<const float2*>(stage(c) + PREP_F - PREP_K)[col]; };   // (G_n, mid)
+    bool ok = wait(&sh.full[0], 0, 3);
+    float2 f = ok ? factors(0) : make_float2(0.f, 0.f);
+    for (int c = 0; ok && c < NT; ++c) {
+      const float cmid = fast_exp(f.y), decay = fast_exp(f.x), c2 = fast_exp(f.x - f.y);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) vreg[t] = __ldg(src + t);
-      }
-      // ---- gate q and k
-      if (!mbar_wait(&sh.fullqkt[pp & 1], (pp >> 1) & 1) || !mbar_wait(&sh.ebar, ph)) { *abort_flag = 1; fail(9); }
-      tc_fence_after();
-      {
-        const int i = (q4 * 32 + lane) & 63;
-        const int cg = (q4 >> 1) * 4 + seg;
-        float em[16];
-        tmem_ld16(tmem_addr(tm, lane_base, cE + cg * 16), em);
-        const uint32_t rowoff = (uint32_t)(cg >> 2) * SLAB64 + (uint32_t)i * 128u;
-        const float bi = sh.beta[ph][i];
-        if (i == 63) {
-#pragma unroll
-          for (int t = 0; t < 16; ++t) sh.a[cg * 16 + t] = em[t];
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-          float fb[8], fs[8], r[8];
-#pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float f = fast_exp(em[8 * u + t]);
-            fb[t] = f * bi;
-            fs[t] = f * p.scale;
-            r[t] = fast_exp(-em[8 * u + t]);
-          }
-          const uint4 kraw = *reinterpret_cast<const uint4*>(ks + off);
-          if (i == 0) {   // G_0 = g_0
-            const uint4 graw = *reinterpret_cast<const uint4*>(gs + off);
-            const __nv_bfloat162* pg = reinterpret_cast<const __nv_bfloat162*>(&graw);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float2 x = __bfloat1622float2(pg[t]);
-              sh.g0[cg * 16 + 8 * u + 2 * t] = x.x;
-              sh.g0[cg * 16 + 8 * u + 2 * t + 1] = x.y;
-            }
-          }
-          *reinterpret_cast<uint4*>(qs + off) = scale8(*reinterpret_cast<const uint4*>(qs + off), fs);
-          *reinterpret_cast<uint4*>(khs + off) = scale8(kraw, fb);
-          *reinterpret_cast<uint4*>(ks + off) = scale8(kraw, r);
-        }
-      }
+      for (int j = 0; j < 32; j += 8)
+        *reinterpret_cast<uint4*>(dhst + tile_off(128, col, seg * 32 + j)) =
+            make_uint4(pack_bf16(S[j] * c2, S[j + 1] * c2), pack_bf16(S[j + 2] * c2, S[j + 3] * c2),
+                       pack_bf16(S[j + 4] * c2, S[j + 5] * c2), pack_bf16(S[j + 6] * c2, S[j + 7] * c2));
       fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B1
-      // (beta of the next chunk: loaded here, stored to shared memory three barriers later)
-      __nv_bfloat16 beta_in = __float2bfloat16(0.f);
-      if (tid < C && pp + 1 < NT) beta_in = p.beta[((size_t)b * p.T + chunk_of(pp + 1) * C + tid) * p.H + h];
-      const float av = sh.a[col], g0v = sh.g0[col];
-      const float decay = fast_exp(2.f * av + g0v);   // exp(G_n)
-      const float cmid = fast_exp(av + g0v);          // exp(mid)
-      {
-        const float c2 = fast_exp(av);                // exp(G_n - mid)
-#pragma unroll
-        for (int j = 0; j < 32; j += 8)
-          *reinterpret_cast<uint4*>(dhst + tile_off(128, col, seg * 32 + j)) =
-              make_uint4(pack_bf16(S[j] * c2, S[j + 1] * c2), pack_bf16(S[j + 2] * c2, S[j + 3] * c2),
-                         pack_bf16(S[j + 4] * c2, S[j + 5] * c2), pack_bf16(S[j + 6] * c2, S[j + 7] * c2));
-      }
-      if (!mbar_wait(&sh.abar, ph)) { *abort_flag = 1; fail(4); }
-      tc_fence_after();
-      {
-        float a[16];
-        tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
-        if (lane < 16) store_tril16(at, ri, seg * 16, a, 1.f);
-      }
-      fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B2
-      // ---- dv' -> bf16 operand and scratch
-      if (!mbar_wait(&sh.vbar, ph)) { *abort_flag = 1; fail(7); }
+      mbar_arrive(&sh.hready);
+      if (!(ok = wait(&sh.vbar, c & 1, 7))) break;
       tc_fence_after();
       {
         float x[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), x);
+        tmem_ld32(tmem_addr(tm, lane_base, cV + seg * 32), x);
         if (lane < 16) {
-          __nv_bfloat16* dst = p.dvn + ((size_t)(row0 + ri) * p.H + h) * D + seg * 32;
 #pragma unroll
-          for (int t = 0; t < 32; t += 8) {
-            const uint4 packed = make_uint4(pack_bf16(x[t], x[t + 1]), pack_bf16(x[t + 2], x[t + 3]),
-                                            pack_bf16(x[t + 4], x[t + 5]), pack_bf16(x[t + 6], x[t + 7]));
-            *reinterpret_cast<uint4*>(dvs + tile_off(64, ri, seg * 32 + t)) = packed;
-            *reinterpret_cast<uint4*>(dst + t) = packed;
-          }
+          for (int t = 0; t < 32; t += 8)
+            *reinterpret_cast<uint4*>(dvs + tile_off(64, ri, seg * 32 + t)) =
+                make_uint4(pack_bf16(x[t], x[t + 1]), pack_bf16(x[t + 2], x[t + 3]), pack_bf16(x[t + 4], x[t + 5]),
+                           pack_bf16(x[t + 6], x[t + 7]));
         }
       }
       fence_async_smem();
       tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B3
-      // ---- dR: dv = beta dR (output), -dR (operand and scratch), dbeta1 = sum_v dR v
-      if (!mbar_wait(&sh.rbar, ph)) { *abort_flag = 1; fail(8); }
+      mbar_arrive(&sh.vready);
+      if (c + 1 < NT) {
+        if (!(ok = wait(&sh.full[(c + 1) & 1], ((c + 1) >> 1) & 1, 3))) break;
+        f = factors(c + 1);
+      }
+      if (!(ok = wait(&sh.sbar, c & 1, 2))) break;
       tc_fence_after();
-      {
-        float x[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), x);
-        if (lane < 16) {
-          const float bi = sh.beta[ph][ri];
-          const size_t g0i = ((size_t)(row0 + ri) * p.H + h) * D + seg * 32;
-          float dot = 0.f;
+      float d[32];
+      tmem_ld32(tmem_addr(tm, lane_base, cD + (c & 1) * 128 + seg * 32), d);
 #pragma unroll
-          for (int t = 0; t < 32; t += 8) {
-            const __nv_bfloat162* pv = reinterpret_cast<const __nv_bfloat162*>(&vreg[t >> 3]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float2 vv = __bfloat1622float2(pv[u]);
-              dot = fmaf(x[t + 2 * u], vv.x, dot);
-              dot = fmaf(x[t + 2 * u + 1], vv.y, dot);
-            }
-            const uint4 neg = make_uint4(pack_bf16(-x[t], -x[t + 1]), pack_bf16(-x[t + 2], -x[t + 3]),
-                                         pack_bf16(-x[t + 4], -x[t + 5]), pack_bf16(-x[t + 6], -x[t + 7]));
-            *reinterpret_cast<uint4*>(nrs + tile_off(64, ri, seg * 32 + t)) = neg;
-            *reinterpret_cast<uint4*>(p.ndr + g0i + t) = neg;
-            __stcs(reinterpret_cast<uint4*>(p.dv + g0i + t),
-                   make_uint4(pack_bf16(bi * x[t], bi * x[t + 1]), pack_bf16(bi * x[t + 2], bi * x[t + 3]),
-                              pack_bf16(bi * x[t + 4], bi * x[t + 5]), pack_bf16(bi * x[t + 6], bi * x[t + 7])));
-          }
-          atomicAdd(&sh.db[ri], dot);
-        }
-      }
-      if (tid < C && pp + 1 < NT) sh.beta[(pp + 1) & 1][tid] = __bfloat162float(beta_in);
-      fence_async_smem();
-      tc_fence_before();
-      if (__syncthreads_or(*abort_flag)) break;   // B4
-      if (tid < C) {
-        p.dbeta1[((size_t)row0 + tid) * p.H + h] = sh.db[tid];
-        sh.db[tid] = 0.f;
-      }
-      // ---- dh <- dh exp(G_n) + exp(mid) D
-      if (!mbar_wait(&sh.sbar, ph)) { *abort_flag = 1; fail(2); }
-      tc_fence_after();
-      {
-        float d[32];
-        tmem_ld32(tmem_addr(tm, lane_base, cD + seg * 32), d);
-#pragma unroll
-        for (int t = 0; t < 32; ++t) S[t] = fmaf(S[t], decay, cmid * d[t]);
-      }
+      for (int t = 0; t < 32; ++t) S[t] = fmaf(S[t], decay, cmid * d[t]);
       tc_fence_before();
     }
-    if (!*abort_flag && p.dh0) {
-      float* dst = p.dh0 + ((size_t)bh * D + col) * D + seg * 32;
+    if (ok && p.dh0) {
+      float* dst = p.dh0 + ((size_t)blockIdx.x * D + col) * D + seg * 32;
 #pragma unroll
       for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
     }
+  } else if (warp == 16) {
+    // ------------------------------------------------------------------ products, stores of dh^ and dv'
+    if (lane == 0) {
+      const uint32_t dha = smem_u32(dhst), dva = smem_u32(dvs);
+      auto issue_do = [&](int c) {
+        const uint32_t qa = smem_u32(stage(c) + PREP_Q - PREP_K), aa = smem_u32(stage(c) + PREP_A - PREP_K),
+                       doa = smem_u32(stage(c) + PREP_BWD);
+        tc_fence_after();
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)   // dv'[j][v] = sum_i Aqk[i][j] do[i][v]
+          umma_bf16(tm + cV, desc_mnmajor(aa, 64, k0, 0), desc_mnmajor(doa, 64, k0, 0), umma_idesc(64, 128, 1, 1), k0 > 0);
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_i q~[i][k] do[i][v]
+          umma_bf16(tm + cD + (c & 1) * 128, desc_mnmajor(qa, 64, k0, 0), desc_mnmajor(doa, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
+      };
+      bool ok = wait(&sh.full[0], 0, 3);
+      if (ok) issue_do(0);
+      for (int c = 0; ok && c < NT; ++c) {
+        const uint32_t ka = smem_u32(stage(c)), wa = smem_u32(stage(c) + PREP_W - PREP_K);
+        if (!wait(&sh.hready, c & 1, 8)) break;
+        tc_fence_after();
+        tma_store_wait_read();   // dv' of the chunk before has been read
+#pragma unroll
+        for (int k0 = 0; k0 < D; k0 += 16)   // dv' += k~ dh^
+          umma_bf16(tm + cV, desc_kmajor(ka, 64, 0, k0), desc_mnmajor(dha, 128, k0, 0), umma_idesc(64, 128, 0, 1), 1);
+        umma_commit(&sh.vbar);
+        {
+          const int hrow = (int)slot(c) * D;
+          tma_store_2d(&p.mst, dhst, 0, hrow);
+          tma_store_2d(&p.mst, dhst + TILE128 / 2, 64, hrow);
+          tma_store_commit();
+        }
+        if (!wait(&sh.vready, c & 1, 11)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k0 = 0; k0 < C; k0 += 16)   // D += (-w)^T dv'
+          umma_bf16(tm + cD + (c & 1) * 128, desc_mnmajor(wa, 64, k0, 0), desc_mnmajor(dva, 64, k0, 0), umma_idesc(128, 128, 1, 1), 1);
+        const int row = b * p.T + chunk_of(c) * C;
+        tma_store_3d(&p.mdvn, dvs, 0, h, row);
+        tma_store_3d(&p.mdvn, dvs + SLAB64, 64, h, row);
+        tma_store_commit();
+        tma_store_wait_read1();   // dh^ has been read: its tile is refilled after sbar
+        umma_commit(&sh.sbar);
+        umma_commit(&sh.free[c & 1]);
+        if (c + 1 < NT) {
+          if (!wait(&sh.full[(c + 1) & 1], ((c + 1) >> 1) & 1, 3)) break;
+          issue_do(c + 1);        // (dv' has left tensor memory)
+        }
+      }
+      tma_store_wait_all();
+    }
+  } else {
+    // ------------------------------------------------------------------ loads
+    if (lane == 0) {
+      for (int c = 0; c < NT; ++c) {
+        if (c >= 2 && !wait(&sh.free[c & 1], ((c - 2) >> 1) & 1, 5)) break;
+        uint64_t* bar = &sh.full[c & 1];
+        uint8_t* dst = stage(c);
+        const int row = b * p.T + chunk_of(c) * C;
+        mbar_expect_tx(bar, KDA_SB_STAGE);
+        bulk_load(dst, p.prep + slot(c) * PREP_BYTES + PREP_K, PREP_BWD, bar);
+        tma_load_3d(dst + PREP_BWD, &p.mdo, bar, 0, h, row);
+        tma_load_3d(dst + PREP_BWD + SLAB64, &p.mdo, bar, 64, h, row);
+      }
+    }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && sh.abort_flag) {
-    poison(p.dv + ((size_t)b * p.T * p.H + h) * D);
-    if (p.dh0) poison(p.dh0 + (size_t)bh * D * D);
+    poison(p.dvn + ((size_t)b * p.T * p.H + h) * D);
+    if (p.dh0) poison(p.dh0 + (size_t)blockIdx.x * D * D);
   }
 }
 
 // ===========================================================================
-// Backward, part B1: gradients of the two per-chunk matrices (one block per chunk and head)
+// Backward, part B1: gradients of the two per-chunk matrices and of the solve's right-hand side (one block per chunk
+// and head)
 // ===========================================================================
-//     dS = tril(do v'^T)                 gradient of q~ k~^T (the scale rides on q~)
-//     dL = -stril(T^T stril(dv' R^T) T^T)    gradient of L = stril(beta k^ k~^T) through T = (I + L)^-1
-// Both leave as bf16 [B,T,H,64] (row i of a chunk at token i).
+//     dR = T^T dv'                 gradient of R in v' = T R, R = beta (v - k^ h')
+//     dv = beta dR (output)        dbeta1 = sum_v dR v        (the h' part of dbeta comes with dk^b below)
+//     dS = tril(do v'^T)           gradient of q~ k~^T (the scale rides on q~)
+//     dL = -stril(dR v'^T)         gradient of L = stril(beta k^ k~^T) through T = (I + L)^-1: dT = dv' R^T and
+//                                  dL = -T^T dT T^T = -(T^T dv') (T R)^T
+// -dR (bf16 [B,T,H,V]), dS and dL (bf16 [B,T,H,64], row i of a chunk at token i) are scratch for part B2.
 struct KdaIntraParams {
-  CUtensorMap mdo, mvn, mdvn, mr, mt;
-  __nv_bfloat16* dS;
-  __nv_bfloat16* dL;
+  CUtensorMap mdo, mvn, mdvn, mv;
+  const uint8_t* prep;
+  const __nv_bfloat16* beta;
+  __nv_bfloat16 *dS, *dL, *ndr, *dv;
+  float* dbeta1;
   int T, H, NT;
 };
 
@@ -847,29 +777,31 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_kda_bwd_intra(const __grid_cons
   uint8_t* dos = smem;                 // do
   uint8_t* vns = dos + TILE64;         // v'
   uint8_t* dvs = vns + TILE64;         // dv'
-  uint8_t* rs = dvs + TILE64;          // R
-  uint8_t* ts = rs + TILE64;           // T (64 x 64)
-  uint8_t* dts = ts + SLAB64;          // stril(dT) bf16
-  uint8_t* wsm = dts + SLAB64;         // T^T dT bf16
-  __shared__ uint64_t bar_load, bar_1, bar_2, bar_3;
+  uint8_t* vs = dvs + TILE64;          // v
+  uint8_t* nrs = vs + TILE64;          // -dR
+  uint8_t* ts = nrs + TILE64;          // T (64 x 64)
+  __shared__ uint64_t bar_r, bar_s, bar_1, bar_2;
   __shared__ uint32_t tmem_slot;
+  __shared__ float db_s[C];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, seg = warp >> 2;
   const int h = blockIdx.x, ci = blockIdx.y, b = blockIdx.z;
   const int row = b * p.T + ci * C;
-  constexpr uint32_t cS = 0, cT = 64, cW = 128, cL = 192;
+  constexpr uint32_t cS = 0, cL = 64, cR = 128;
   if (tid == 0) {
-    mbar_init(&bar_load, 1); mbar_init(&bar_1, 1); mbar_init(&bar_2, 1); mbar_init(&bar_3, 1);
+    mbar_init(&bar_r, 1); mbar_init(&bar_s, 1); mbar_init(&bar_1, 1); mbar_init(&bar_2, 1);
     fence_barrier_init();
-    mbar_expect_tx(&bar_load, 4 * TILE64 + SLAB64);
-    tma_load_3d(dos, &p.mdo, &bar_load, 0, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &bar_load, 64, h, row);
-    tma_load_3d(vns, &p.mvn, &bar_load, 0, h, row); tma_load_3d(vns + SLAB64, &p.mvn, &bar_load, 64, h, row);
-    tma_load_3d(dvs, &p.mdvn, &bar_load, 0, h, row); tma_load_3d(dvs + SLAB64, &p.mdvn, &bar_load, 64, h, row);
-    tma_load_3d(rs, &p.mr, &bar_load, 0, h, row); tma_load_3d(rs + SLAB64, &p.mr, &bar_load, 64, h, row);
-    tma_load_3d(ts, &p.mt, &bar_load, 0, h, row);
+    mbar_expect_tx(&bar_r, 2 * TILE64 + SLAB64);   // what the longer chain needs first
+    tma_load_3d(dvs, &p.mdvn, &bar_r, 0, h, row); tma_load_3d(dvs + SLAB64, &p.mdvn, &bar_r, 64, h, row);
+    bulk_load(ts, p.prep + ((size_t)(b * p.NT + ci) * p.H + h) * PREP_BYTES + PREP_T, SLAB64, &bar_r);
+    tma_load_3d(vs, &p.mv, &bar_r, 0, h, row); tma_load_3d(vs + SLAB64, &p.mv, &bar_r, 64, h, row);
+    mbar_expect_tx(&bar_s, 2 * TILE64);
+    tma_load_3d(vns, &p.mvn, &bar_s, 0, h, row); tma_load_3d(vns + SLAB64, &p.mvn, &bar_s, 64, h, row);
+    tma_load_3d(dos, &p.mdo, &bar_s, 0, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &bar_s, 64, h, row);
   }
   __syncwarp();
   if (warp == 0) { tmem_alloc(&tmem_slot, 256); tmem_relinquish(); }
+  if (tid < C) db_s[tid] = 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -877,101 +809,93 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_kda_bwd_intra(const __grid_cons
   const uint32_t lane_base = q4 * 32;
   const int ri = 16 * q4 + lane;   // rows of an M = 64 accumulator sit in lanes 0..15 of each quarter
   const size_t orow = ((size_t)(row + ri) * p.H + h) * C + seg * 16;
-  bool ok = __syncthreads_and(mbar_wait(&bar_load, 0));
+  const float bi = lane < 16 ? __bfloat162float(p.beta[(size_t)(row + ri) * p.H + h]) : 0.f;
+  bool ok = __syncthreads_and(mbar_wait(&bar_r, 0) && mbar_wait(&bar_s, 0));
   if (!ok) fail(3);
   if (ok && tid == 0) {
     tc_fence_after();
-    const uint32_t doa = smem_u32(dos), vna = smem_u32(vns), dva = smem_u32(dvs), ra = smem_u32(rs);
+    const uint32_t doa = smem_u32(dos), vna = smem_u32(vns), dva = smem_u32(dvs), ta = smem_u32(ts);
+#pragma unroll
+    for (int k0 = 0; k0 < C; k0 += 16)   // dR[j][v] = sum_i T[i][j] dv'[i][v]
+      umma_bf16(tm + cR, desc_mnmajor(ta, 64, k0, 0), desc_mnmajor(dva, 64, k0, 0), umma_idesc(64, 128, 1, 1), k0 > 0);
+    umma_commit(&bar_1);
 #pragma unroll
     for (int k0 = 0; k0 < D; k0 += 16)   // dS[i][j] = do v'^T
       umma_bf16(tm + cS, desc_kmajor(doa, 64, 0, k0), desc_kmajor(vna, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-#pragma unroll
-    for (int k0 = 0; k0 < D; k0 += 16)   // dT[i][j] = dv' R^T
-      umma_bf16(tm + cT, desc_kmajor(dva, 64, 0, k0), desc_kmajor(ra, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-    umma_commit(&bar_1);
   }
   __syncwarp();
   if (ok) { ok = __syncthreads_and(mbar_wait(&bar_1, 0)); if (!ok) fail(4); }
   if (ok) {
     tc_fence_after();
-    float a[16];
-    tmem_ld16(tmem_addr(tm, lane_base, cS + seg * 16), a);
+    float x[32];
+    tmem_ld32(tmem_addr(tm, lane_base, cR + seg * 32), x);
     if (lane < 16) {
-      uint32_t w[8];
+      const size_t g0i = ((size_t)(row + ri) * p.H + h) * D + seg * 32;
+      float dot = 0.f;
+#pragma unroll
+      for (int t = 0; t < 32; t += 8) {
+        const uint32_t off = tile_off(64, ri, seg * 32 + t);
+        const uint4 vraw = *reinterpret_cast<const uint4*>(vs + off);
+        const __nv_bfloat162* pv = reinterpret_cast<const __nv_bfloat162*>(&vraw);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float2 vv = __bfloat1622float2(pv[u]);
+          dot = fmaf(x[t + 2 * u], vv.x, dot);
+          dot = fmaf(x[t + 2 * u + 1], vv.y, dot);
+        }
+        const uint4 neg = make_uint4(pack_bf16(-x[t], -x[t + 1]), pack_bf16(-x[t + 2], -x[t + 3]),
+                                     pack_bf16(-x[t + 4], -x[t + 5]), pack_bf16(-x[t + 6], -x[t + 7]));
+        *reinterpret_cast<uint4*>(nrs + off) = neg;
+        *reinterpret_cast<uint4*>(p.ndr + g0i + t) = neg;
+        __stcs(reinterpret_cast<uint4*>(p.dv + g0i + t),
+               make_uint4(pack_bf16(bi * x[t], bi * x[t + 1]), pack_bf16(bi * x[t + 2], bi * x[t + 3]),
+                          pack_bf16(bi * x[t + 4], bi * x[t + 5]), pack_bf16(bi * x[t + 6], bi * x[t + 7])));
+      }
+      atomicAdd(&db_s[ri], dot);
+    }
+    fence_async_smem();
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (ok && tid == 0) {
+    tc_fence_after();
+    const uint32_t nra = smem_u32(nrs), vna = smem_u32(vns);
+#pragma unroll
+    for (int k0 = 0; k0 < D; k0 += 16)   // dL[i][j] = -dR v'^T
+      umma_bf16(tm + cL, desc_kmajor(nra, 64, 0, k0), desc_kmajor(vna, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+    umma_commit(&bar_2);
+  }
+  if (ok && tid < C) p.dbeta1[(size_t)(row + tid) * p.H + h] = db_s[tid];
+  __syncwarp();
+  if (ok) { ok = __syncthreads_and(mbar_wait(&bar_2, 0)); if (!ok) fail(6); }
+  if (ok) {
+    tc_fence_after();
+    float a[16], l[16];
+    tmem_ld16(tmem_addr(tm, lane_base, cS + seg * 16), a);
+    tmem_ld16(tmem_addr(tm, lane_base, cL + seg * 16), l);
+    if (lane < 16) {
+      uint32_t w[8], x[8];
 #pragma unroll
       for (int t = 0; t < 16; t += 2) {
         const int j = seg * 16 + t;
         w[t >> 1] = pack_bf16(j <= ri ? a[t] : 0.f, j + 1 <= ri ? a[t + 1] : 0.f);
+        x[t >> 1] = pack_bf16(j < ri ? l[t] : 0.f, j + 1 < ri ? l[t + 1] : 0.f);
       }
       *reinterpret_cast<uint4*>(p.dS + orow) = make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4*>(p.dS + orow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-    }
-    tmem_ld16(tmem_addr(tm, lane_base, cT + seg * 16), a);
-    if (lane < 16) {
-#pragma unroll
-      for (int t = 0; t < 16; ++t) a[t] = (seg * 16 + t < ri) ? a[t] : 0.f;   // strictly below the diagonal
-      store_tril16(dts, ri, seg * 16, a, 1.f);
-    }
-    fence_async_smem();
-    tc_fence_before();
-  }
-  __syncthreads();
-  if (ok && tid == 0) {
-    tc_fence_after();
-    const uint32_t ta = smem_u32(ts), dta = smem_u32(dts);
-#pragma unroll
-    for (int k0 = 0; k0 < C; k0 += 16)   // W[a][j] = sum_i T[i][a] dT[i][j]
-      umma_bf16(tm + cW, desc_mnmajor(ta, 64, k0, 0), desc_mnmajor(dta, 64, k0, 0), umma_idesc(64, 64, 1, 1), k0 > 0);
-    umma_commit(&bar_2);
-  }
-  __syncwarp();
-  if (ok) { ok = __syncthreads_and(mbar_wait(&bar_2, 0)); if (!ok) fail(5); }
-  if (ok) {
-    tc_fence_after();
-    float a[16];
-    tmem_ld16(tmem_addr(tm, lane_base, cW + seg * 16), a);
-    if (lane < 16) {
-#pragma unroll
-      for (int c8 = 0; c8 < 16; c8 += 8)
-        *reinterpret_cast<uint4*>(wsm + slab_off(ri, seg * 16 + c8)) =
-            make_uint4(pack_bf16(a[c8], a[c8 + 1]), pack_bf16(a[c8 + 2], a[c8 + 3]), pack_bf16(a[c8 + 4], a[c8 + 5]),
-                       pack_bf16(a[c8 + 6], a[c8 + 7]));
-    }
-    fence_async_smem();
-    tc_fence_before();
-  }
-  __syncthreads();
-  if (ok && tid == 0) {
-    tc_fence_after();
-    const uint32_t ta = smem_u32(ts), wa = smem_u32(wsm);
-#pragma unroll
-    for (int k0 = 0; k0 < C; k0 += 16)   // X[a][c] = sum_j W[a][j] T[c][j]
-      umma_bf16(tm + cL, desc_kmajor(wa, 64, 0, k0), desc_kmajor(ta, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-    umma_commit(&bar_3);
-  }
-  __syncwarp();
-  if (ok) { ok = __syncthreads_and(mbar_wait(&bar_3, 0)); if (!ok) fail(6); }
-  if (ok) {
-    tc_fence_after();
-    float a[16];
-    tmem_ld16(tmem_addr(tm, lane_base, cL + seg * 16), a);
-    if (lane < 16) {
-      uint32_t w[8];
-#pragma unroll
-      for (int t = 0; t < 16; t += 2) {
-        const int j = seg * 16 + t;
-        w[t >> 1] = pack_bf16(j < ri ? -a[t] : 0.f, j + 1 < ri ? -a[t + 1] : 0.f);
-      }
-      *reinterpret_cast<uint4*>(p.dL + orow) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(p.dL + orow + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+      *reinterpret_cast<uint4*>(p.dL + orow) = make_uint4(x[0], x[1], x[2], x[3]);
+      *reinterpret_cast<uint4*>(p.dL + orow + 8) = make_uint4(x[4], x[5], x[6], x[7]);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
-  if (tid == 0 && !ok) poison(p.dL + ((size_t)row * p.H + h) * C);
+  if (tid == 0 && !ok) {
+    poison(p.dL + ((size_t)row * p.H + h) * C);
+    poison(p.dv + ((size_t)row * p.H + h) * D);
+  }
 }
-constexpr size_t KDA_INTRA_SMEM = 4 * TILE64 + 3 * SLAB64 + 1024;
+constexpr size_t KDA_INTRA_SMEM = 5 * TILE64 + SLAB64 + 1024;
 
 // ===========================================================================
 // Backward, part B2: dq, dk, dg, dbeta of a chunk (one block per chunk and head)
@@ -1270,46 +1194,72 @@ bool kda_supported(const tops_chunk_kda_fwd_params& p) {
   if (p.dtype != TOPS_BF16 || p.gate_dtype != TOPS_BF16) return false;
   if (p.K != D || p.V != D || p.chunk != C || p.T % C != 0) return false;
   if (!(p.scale > 0.f) || !(p.scale < 1e30f)) return false;
-  if ((size_t)p.B * p.T >= (1u << 31)) return false;
+  if ((size_t)p.B * p.T >= (1u << 31) || (size_t)p.B * p.T * p.H * 2 >= (1u << 31)) return false;   // (32-bit state rows)
   return device_is_sm100() && encode_fn() != nullptr;
 }
 
+// saved for a backward pass: [prep] [h'] [v']; without one only [prep] is needed, as scratch
+static size_t prep_bytes(int B, int T, int H) { return align_up((size_t)B * (T / C) * H * PREP_BYTES); }
+static size_t chunk_state_bytes(int B, int T, int H) { return align_up((size_t)B * (T / C) * H * D * D * 2); }
+static size_t activation_bytes(int B, int T, int H) { return align_up((size_t)B * T * H * D * 2); }
+size_t kda_chunk_saved_bytes(const tops_chunk_kda_fwd_params& p) {
+  return prep_bytes(p.B, p.T, p.H) + chunk_state_bytes(p.B, p.T, p.H) + activation_bytes(p.B, p.T, p.H);
+}
+size_t kda_chunk_fwd_workspace_bytes(const tops_chunk_kda_fwd_params& p) { return p.saved ? 0 : prep_bytes(p.B, p.T, p.H); }
+
 int kda_chunk_fwd(const tops_chunk_kda_fwd_params& p, cudaStream_t st) {
   if (!aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !aligned16(p.g) || !aligned16(p.o) || !aligned16(p.h0) ||
-      !aligned16(p.ht) || !aligned16(p.saved_h) || !aligned16(p.saved_vnew) || !aligned16(p.saved_T) || !aligned16(p.saved_R) ||
-      !aligned16(p.Aqk_out) || !aligned16(p.Akk_out))
+      !aligned16(p.ht) || !aligned16(p.saved) || !aligned16(p.workspace) || !aligned16(p.Aqk_out) || !aligned16(p.Akk_out))
     return TOPS_E_ALIGN;
-  KdaFwdParams kp;
   const int BT = p.B * p.T, NT = p.T / C;
   int rc;
-  if ((rc = act_map(&kp.mq, p.q, BT, p.H)) || (rc = act_map(&kp.mk, p.k, BT, p.H)) ||
-      (rc = act_map(&kp.mg, p.g, BT, p.H)) || (rc = act_map(&kp.mv, p.v, BT, p.H)))
-    return rc;
-  kp.states = reinterpret_cast<__nv_bfloat16*>(p.saved_h);
-  if (p.saved_h && (rc = state_map(&kp.mst, p.saved_h, (size_t)p.B * NT * p.H * D))) return rc;
-  kp.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);
-  kp.s0 = p.h0; kp.s_final = p.ht; kp.o = reinterpret_cast<__nv_bfloat16*>(p.o);
-  kp.vnew = reinterpret_cast<__nv_bfloat16*>(p.saved_vnew);
-  kp.rsave = reinterpret_cast<__nv_bfloat16*>(p.saved_R);
-  kp.t_saved = reinterpret_cast<__nv_bfloat16*>(p.saved_T);
-  kp.Aqk_out = p.Aqk_out; kp.Akk_out = p.Akk_out;
-  kp.T = p.T; kp.H = p.H; kp.NT = NT; kp.scale = p.scale;
-  if ((rc = opt_in_smem(k_kda_fwd, KDA_FWD_SMEM))) return rc;
-  KernelScope ks("sm100_kda_fwd", st);
-  k_kda_fwd<<<p.B * p.H, KDA_THREADS, KDA_FWD_SMEM, st>>>(kp);
-  return post_launch();
+  // a caller that passes no scratch gets it from the stream's memory pool for the length of the call
+  void* own = nullptr;
+  uint8_t* prep = reinterpret_cast<uint8_t*>(p.saved ? p.saved : p.workspace);
+  if (!p.saved && p.workspace_bytes < kda_chunk_fwd_workspace_bytes(p)) {
+    if (p.workspace) return TOPS_E_WORKSPACE;
+    TOPS_CUDA_OK(cudaMallocAsync(&own, kda_chunk_fwd_workspace_bytes(p), st));
+    prep = reinterpret_cast<uint8_t*>(own);
+  }
+  auto run = [&]() -> int {
+    {
+      KdaPrepParams pp;
+      if ((rc = act_map(&pp.mq, p.q, BT, p.H)) || (rc = act_map(&pp.mk, p.k, BT, p.H)) || (rc = act_map(&pp.mg, p.g, BT, p.H))) return rc;
+      pp.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);
+      pp.prep = prep; pp.Aqk_out = p.Aqk_out; pp.Akk_out = p.Akk_out;
+      pp.T = p.T; pp.H = p.H; pp.NT = NT; pp.total = p.B * NT * p.H; pp.scale = p.scale;
+      if ((rc = opt_in_smem(k_kda_prep, KDA_PREP_SMEM))) return rc;
+      const int grid = pp.total < 2 * sm_count() ? pp.total : 2 * sm_count();
+      KernelScope ks("sm100_kda_prep", st);
+      k_kda_prep<<<grid, NTHREADS, KDA_PREP_SMEM, st>>>(pp);
+      if ((rc = post_launch())) return rc;
+    }
+    KdaScanFwdParams sp;
+    if ((rc = act_map(&sp.mv, p.v, BT, p.H))) return rc;
+    sp.keep = p.saved != nullptr;
+    if (p.saved) {
+      uint8_t* h = prep + prep_bytes(p.B, p.T, p.H);
+      if ((rc = state_map(&sp.mst, h, (size_t)p.B * NT * p.H * D)) || (rc = act_map(&sp.mvn, h + chunk_state_bytes(p.B, p.T, p.H), BT, p.H)))
+        return rc;
+    }
+    sp.prep = prep; sp.s0 = p.h0; sp.s_final = p.ht; sp.o = reinterpret_cast<__nv_bfloat16*>(p.o);
+    sp.T = p.T; sp.H = p.H; sp.NT = NT;
+    if ((rc = opt_in_smem(k_kda_scan_fwd, KDA_SF_SMEM))) return rc;
+    KernelScope ks("sm100_kda_scan_fwd", st);
+    k_kda_scan_fwd<<<p.B * p.H, KDA_SF_THREADS, KDA_SF_SMEM, st>>>(sp);
+    return post_launch();
+  };
+  rc = run();
+  if (own && cudaFreeAsync(own, st) != cudaSuccess && rc == TOPS_OK) rc = TOPS_E_CUDA;
+  return rc;
 }
 
-static size_t kda_state_bytes(const tops_chunk_kda_bwd_params& p) {
-  return align_up((size_t)p.B * (p.T / C) * p.H * D * D * 2);
-}
-static size_t kda_act_bytes(const tops_chunk_kda_bwd_params& p) { return align_up((size_t)p.B * p.T * p.H * D * 2); }
 static size_t kda_mat_bytes(const tops_chunk_kda_bwd_params& p) { return align_up((size_t)p.B * p.T * p.H * C * 2); }
 static size_t kda_beta_bytes(const tops_chunk_kda_bwd_params& p) { return align_up((size_t)p.B * p.T * p.H * 4); }
 
 size_t kda_chunk_bwd_workspace_bytes(const tops_chunk_kda_bwd_params& p) {
   // [dh^] [dv'] [-dR] [dS] [dL] [dbeta1]
-  return kda_state_bytes(p) + 2 * kda_act_bytes(p) + 2 * kda_mat_bytes(p) + kda_beta_bytes(p) + 256;
+  return chunk_state_bytes(p.B, p.T, p.H) + 2 * activation_bytes(p.B, p.T, p.H) + 2 * kda_mat_bytes(p) + kda_beta_bytes(p) + 256;
 }
 
 bool kda_bwd_supported(const tops_chunk_kda_bwd_params& p) {
@@ -1320,45 +1270,42 @@ bool kda_bwd_supported(const tops_chunk_kda_bwd_params& p) {
 }
 
 int kda_chunk_bwd(const tops_chunk_kda_bwd_params& p, void* ws, cudaStream_t st) {
-  const void* ptrs[] = {p.q, p.k, p.v, p.g, p.do_, p.dht, p.saved_h, p.saved_vnew, p.saved_T, p.saved_R,
-                        p.dq, p.dk, p.dv, p.dg, p.dh0, ws};
+  const void* ptrs[] = {p.q, p.k, p.v, p.g, p.do_, p.dht, p.saved, p.dq, p.dk, p.dv, p.dg, p.dh0, ws};
   for (const void* x : ptrs)
     if (!aligned16(x)) return TOPS_E_ALIGN;
   const int BT = p.B * p.T, NT = p.T / C;
   const size_t rows = (size_t)p.B * NT * p.H * D;
+  const uint8_t* prep = reinterpret_cast<const uint8_t*>(p.saved);
+  const uint8_t* hsaved = prep + prep_bytes(p.B, p.T, p.H);
+  const uint8_t* vnsaved = hsaved + chunk_state_bytes(p.B, p.T, p.H);
   char* w = reinterpret_cast<char*>(ws);
-  __nv_bfloat16* dh = reinterpret_cast<__nv_bfloat16*>(w); w += kda_state_bytes(p);
-  __nv_bfloat16* dvn = reinterpret_cast<__nv_bfloat16*>(w); w += kda_act_bytes(p);
-  __nv_bfloat16* ndr = reinterpret_cast<__nv_bfloat16*>(w); w += kda_act_bytes(p);
+  __nv_bfloat16* dh = reinterpret_cast<__nv_bfloat16*>(w); w += chunk_state_bytes(p.B, p.T, p.H);
+  __nv_bfloat16* dvn = reinterpret_cast<__nv_bfloat16*>(w); w += activation_bytes(p.B, p.T, p.H);
+  __nv_bfloat16* ndr = reinterpret_cast<__nv_bfloat16*>(w); w += activation_bytes(p.B, p.T, p.H);
   __nv_bfloat16* dS = reinterpret_cast<__nv_bfloat16*>(w); w += kda_mat_bytes(p);
   __nv_bfloat16* dL = reinterpret_cast<__nv_bfloat16*>(w); w += kda_mat_bytes(p);
   float* dbeta1 = reinterpret_cast<float*>(w);
   int rc;
   {
-    KdaScanParams sp;
-    if ((rc = act_map(&sp.mq, p.q, BT, p.H)) || (rc = act_map(&sp.mk, p.k, BT, p.H)) ||
-        (rc = act_map(&sp.mg, p.g, BT, p.H)) || (rc = act_map(&sp.mdo, p.do_, BT, p.H)) ||
-        (rc = mat_map(&sp.mt, p.saved_T, BT, p.H)) || (rc = state_map(&sp.mst, dh, rows)))
-      return rc;
-    sp.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);
-    sp.v = reinterpret_cast<const __nv_bfloat16*>(p.v);
-    sp.dht = p.dht; sp.dh0 = p.dh0; sp.dv = reinterpret_cast<__nv_bfloat16*>(p.dv);
-    sp.dvn = dvn; sp.ndr = ndr; sp.dbeta1 = dbeta1;
-    sp.T = p.T; sp.H = p.H; sp.NT = NT; sp.scale = p.scale;
-    if ((rc = opt_in_smem(k_kda_bwd_scan, KDA_SCAN_SMEM))) return rc;
+    KdaScanBwdParams sp;
+    if ((rc = act_map(&sp.mdo, p.do_, BT, p.H)) || (rc = act_map(&sp.mdvn, dvn, BT, p.H)) || (rc = state_map(&sp.mst, dh, rows))) return rc;
+    sp.prep = prep; sp.dht = p.dht; sp.dh0 = p.dh0; sp.dvn = dvn;
+    sp.T = p.T; sp.H = p.H; sp.NT = NT;
+    if ((rc = opt_in_smem(k_kda_scan_bwd, KDA_SB_SMEM))) return rc;
     KernelScope ks("sm100_kda_bwd_scan", st);
-    k_kda_bwd_scan<<<p.B * p.H, KDA_THREADS, KDA_SCAN_SMEM, st>>>(sp);
+    k_kda_scan_bwd<<<p.B * p.H, KDA_SB_THREADS, KDA_SB_SMEM, st>>>(sp);
     if ((rc = post_launch())) return rc;
   }
   const bool state_gradient_only = !p.dq && !p.dk && !p.dg && !p.dbeta;
   if (state_gradient_only) return TOPS_OK;
   {
     KdaIntraParams ip;
-    if ((rc = act_map(&ip.mdo, p.do_, BT, p.H)) || (rc = act_map(&ip.mvn, p.saved_vnew, BT, p.H)) ||
-        (rc = act_map(&ip.mdvn, dvn, BT, p.H)) || (rc = act_map(&ip.mr, p.saved_R, BT, p.H)) ||
-        (rc = mat_map(&ip.mt, p.saved_T, BT, p.H)))
+    if ((rc = act_map(&ip.mdo, p.do_, BT, p.H)) || (rc = act_map(&ip.mvn, vnsaved, BT, p.H)) ||
+        (rc = act_map(&ip.mdvn, dvn, BT, p.H)) || (rc = act_map(&ip.mv, p.v, BT, p.H)))
       return rc;
-    ip.dS = dS; ip.dL = dL; ip.T = p.T; ip.H = p.H; ip.NT = NT;
+    ip.prep = prep; ip.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);
+    ip.dS = dS; ip.dL = dL; ip.ndr = ndr; ip.dv = reinterpret_cast<__nv_bfloat16*>(p.dv); ip.dbeta1 = dbeta1;
+    ip.T = p.T; ip.H = p.H; ip.NT = NT;
     if ((rc = opt_in_smem(k_kda_bwd_intra, KDA_INTRA_SMEM))) return rc;
     KernelScope ks("sm100_kda_bwd_intra", st);
     k_kda_bwd_intra<<<dim3(p.H, NT, p.B), NTHREADS, KDA_INTRA_SMEM, st>>>(ip);
@@ -1368,8 +1315,8 @@ int kda_chunk_bwd(const tops_chunk_kda_bwd_params& p, void* ws, cudaStream_t st)
     KdaBwdOutParams op;
     if ((rc = act_map(&op.mq, p.q, BT, p.H)) || (rc = act_map(&op.mk, p.k, BT, p.H)) ||
         (rc = act_map(&op.mg, p.g, BT, p.H)) || (rc = act_map(&op.mdo, p.do_, BT, p.H)) ||
-        (rc = act_map(&op.mvn, p.saved_vnew, BT, p.H)) || (rc = act_map(&op.mndr, ndr, BT, p.H)) ||
-        (rc = state_map(&op.mh, p.saved_h, rows)) || (rc = state_map(&op.mdh, dh, rows)) ||
+        (rc = act_map(&op.mvn, vnsaved, BT, p.H)) || (rc = act_map(&op.mndr, ndr, BT, p.H)) ||
+        (rc = state_map(&op.mh, hsaved, rows)) || (rc = state_map(&op.mdh, dh, rows)) ||
         (rc = mat_map(&op.mdS, dS, BT, p.H)) || (rc = mat_map(&op.mdL, dL, BT, p.H)))
       return rc;
     op.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);

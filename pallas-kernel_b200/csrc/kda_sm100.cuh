@@ -8,6 +8,8 @@ namespace sm100 {
 // chunk 64, whole chunks, dense batch).
 bool kda_supported(const tops_chunk_kda_fwd_params& p);
 int kda_chunk_fwd(const tops_chunk_kda_fwd_params& p, cudaStream_t st);
+size_t kda_chunk_saved_bytes(const tops_chunk_kda_fwd_params& p);
+size_t kda_chunk_fwd_workspace_bytes(const tops_chunk_kda_fwd_params& p);
 bool kda_bwd_supported(const tops_chunk_kda_bwd_params& p);
 size_t kda_chunk_bwd_workspace_bytes(const tops_chunk_kda_bwd_params& p);
 int kda_chunk_bwd(const tops_chunk_kda_bwd_params& p, void* ws, cudaStream_t st);

@@ -493,6 +493,14 @@ extern "C" int tops_b200_chunk_kda_supported(const tops_chunk_kda_fwd_params* p)
   return sm100::kda_supported(*p) ? 1 : 0;
 }
 
+extern "C" size_t tops_b200_chunk_kda_saved_bytes(const tops_chunk_kda_fwd_params* p) {
+  return tops_b200_chunk_kda_supported(p) ? sm100::kda_chunk_saved_bytes(*p) : 0;
+}
+
+extern "C" size_t tops_b200_chunk_kda_fwd_workspace_bytes(const tops_chunk_kda_fwd_params* p) {
+  return tops_b200_chunk_kda_supported(p) ? sm100::kda_chunk_fwd_workspace_bytes(*p) : 0;
+}
+
 extern "C" int tops_b200_chunk_kda_fwd(const tops_chunk_kda_fwd_params* p, void* stream) {
   if (!p || !p->q || !p->k || !p->v || !p->g || !p->beta || !p->o) return TOPS_E_NULL;
   if (p->B < 1 || p->T < 1 || p->H < 1 || p->K < 1 || p->V < 1) return TOPS_E_BAD_SHAPE;
@@ -508,9 +516,7 @@ extern "C" size_t tops_b200_chunk_kda_bwd_workspace_bytes(const tops_chunk_kda_b
 
 extern "C" int tops_b200_chunk_kda_bwd(const tops_chunk_kda_bwd_params* p, void* workspace, size_t workspace_bytes,
                                        void* stream) {
-  if (!p || !p->q || !p->k || !p->v || !p->g || !p->beta || !p->do_ || !p->saved_h || !p->saved_vnew || !p->saved_T ||
-      !p->saved_R || !p->dv)
-    return TOPS_E_NULL;
+  if (!p || !p->q || !p->k || !p->v || !p->g || !p->beta || !p->do_ || !p->saved || !p->dv) return TOPS_E_NULL;
   {   // dq, dk, dg, dbeta: all four, or none (state gradient only, which must then be asked for)
     const int given = !!p->dq + !!p->dk + !!p->dg + !!p->dbeta;
     if ((given != 0 && given != 4) || (given == 0 && !p->dh0)) return TOPS_E_NULL;

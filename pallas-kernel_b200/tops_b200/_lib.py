@@ -100,8 +100,8 @@ class KdaBwdParams(C.Structure):
 class ChunkKdaFwdParams(C.Structure):
     _fields_ = [("B", _i32), ("T", _i32), ("H", _i32), ("K", _i32), ("V", _i32), ("chunk", _i32), ("dtype", _i32),
                 ("gate_dtype", _i32), ("scale", _f32), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("beta", _vp),
-                ("h0", _vp), ("o", _vp), ("ht", _vp), ("Aqk_out", _vp), ("Akk_out", _vp), ("saved_h", _vp),
-                ("saved_vnew", _vp), ("saved_T", _vp), ("saved_R", _vp)]
+                ("h0", _vp), ("o", _vp), ("ht", _vp), ("Aqk_out", _vp), ("Akk_out", _vp), ("saved", _vp),
+                ("workspace", _vp), ("workspace_bytes", _sz)]
 
 
 GATE_ACT_KDA, GATE_ACT_KDA_LOWER_BOUND, GATE_ACT_LOG_SIGMOID = 0, 1, 2
@@ -126,7 +126,7 @@ class NormParams(C.Structure):
 class ChunkKdaBwdParams(C.Structure):
     _fields_ = [("B", _i32), ("T", _i32), ("H", _i32), ("K", _i32), ("V", _i32), ("chunk", _i32), ("dtype", _i32),
                 ("gate_dtype", _i32), ("scale", _f32), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("beta", _vp),
-                ("do_", _vp), ("dht", _vp), ("saved_h", _vp), ("saved_vnew", _vp), ("saved_T", _vp), ("saved_R", _vp),
+                ("do_", _vp), ("dht", _vp), ("saved", _vp),
                 ("dq", _vp), ("dk", _vp), ("dg", _vp), ("dbeta", _vp), ("grad_dtype", _i32), ("dv", _vp), ("dh0", _vp)]
 
 
@@ -175,6 +175,9 @@ for _name, _ptype, _ws in [
     _f.argtypes = [C.POINTER(_ptype), _vp, _sz, _vp] if _ws else [C.POINTER(_ptype), _vp]
 lib.tops_b200_chunk_kda_supported.restype = C.c_int
 lib.tops_b200_chunk_kda_supported.argtypes = [C.POINTER(ChunkKdaFwdParams)]
+for _name in ("tops_b200_chunk_kda_saved_bytes", "tops_b200_chunk_kda_fwd_workspace_bytes"):
+    getattr(lib, _name).restype = _sz
+    getattr(lib, _name).argtypes = [C.POINTER(ChunkKdaFwdParams)]
 lib.tops_b200_chunk_kda_fwd.restype = C.c_int
 lib.tops_b200_chunk_kda_fwd.argtypes = [C.POINTER(ChunkKdaFwdParams), _vp]
 for _name, _ptype, _ws in [

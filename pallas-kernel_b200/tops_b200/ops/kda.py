@@ -105,7 +105,7 @@ def chunk_kernels_take(q, k, v, g, beta, chunk_size=64):
 @L.on_tensor_device
 def _chunk_fwd_call(q, k, v, g, beta, scale, initial_state, output_final_state, chunk_size, want_A, want_saved):
     """One call of tops_b200_chunk_kda_fwd.  Returns (o, ht, Aqk, Akk, saved) with Aqk / Akk fp32
-    `[B,T,H,C]` when `want_A`, and saved = (h', v', T, R) residuals for the backward when `want_saved`."""
+    `[B,T,H,C]` when `want_A`, and saved the opaque residuals for the backward when `want_saved`."""
     B, T, H, K, V = _check(q, k, v, g, beta, initial_state)
     dev = q.device
     q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
@@ -115,17 +115,16 @@ def _chunk_fwd_call(q, k, v, g, beta, scale, initial_state, output_final_state, 
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
     Aqk = torch.empty(B, T, H, chunk_size, dtype=torch.float32, device=dev) if want_A else None
     Akk = torch.empty(B, T, H, chunk_size, dtype=torch.float32, device=dev) if want_A else None
-    saved = None
-    if want_saved:
-        saved = (torch.empty(B, T // chunk_size, H, K, V, dtype=q.dtype, device=dev),
-                 torch.empty(B, T, H, V, dtype=q.dtype, device=dev),
-                 torch.empty(B, T, H, chunk_size, dtype=q.dtype, device=dev),
-                 torch.empty(B, T, H, V, dtype=q.dtype, device=dev))
+    saved = ws = None
     p = _chunk_params(q, k, v, g, beta_c, scale, chunk_size)
     p.q, p.k, p.v, p.g, p.beta, p.h0 = L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta_c), L.ptr(h0)
     p.o, p.ht, p.Aqk_out, p.Akk_out = L.ptr(o), L.ptr(ht), L.ptr(Aqk), L.ptr(Akk)
-    if saved is not None:
-        p.saved_h, p.saved_vnew, p.saved_T, p.saved_R = (L.ptr(t) for t in saved)
+    if want_saved:
+        saved = L.workspace(L.lib.tops_b200_chunk_kda_saved_bytes(C.byref(p)), dev)
+        p.saved = L.ptr(saved)
+    else:
+        ws = L.workspace(L.lib.tops_b200_chunk_kda_fwd_workspace_bytes(C.byref(p)), dev)
+        p.workspace, p.workspace_bytes = L.ptr(ws), ws.numel()
     L.check(L.lib.tops_b200_chunk_kda_fwd(C.byref(p), L.stream_ptr(dev)), "chunk_kda_fwd")
     return o, ht, Aqk, Akk, saved
 
@@ -171,7 +170,7 @@ def _chunk_bwd_call(q, k, v, g, beta, do, scale, dht, saved, want_dh0, grad_dtyp
     p.dtype, p.gate_dtype, p.scale = L.dtype_code(q.dtype), L.dtype_code(g.dtype), float(scale)
     p.q, p.k, p.v, p.g, p.beta, p.do_, p.dht = (L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta_c), L.ptr(do),
                                                 L.ptr(dhtc))
-    p.saved_h, p.saved_vnew, p.saved_T, p.saved_R = (L.ptr(t) for t in saved)
+    p.saved = L.ptr(saved)
     p.dq, p.dk, p.dg, p.dbeta, p.dv, p.dh0 = L.ptr(dq), L.ptr(dk), L.ptr(dg), L.ptr(dbeta), L.ptr(dv), L.ptr(dh0)
     p.grad_dtype = L.dtype_code(grad_dtype)
     ws = L.workspace(L.lib.tops_b200_chunk_kda_bwd_workspace_bytes(C.byref(p)), dev)
@@ -197,7 +196,7 @@ def _chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved):
     p.dtype, p.gate_dtype, p.scale = L.dtype_code(q.dtype), L.dtype_code(g.dtype), float(scale)
     p.q, p.k, p.v, p.g, p.beta, p.do_, p.dht = (L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta_c), L.ptr(do),
                                                 L.ptr(dhtc))
-    p.saved_h, p.saved_vnew, p.saved_T, p.saved_R = (L.ptr(t) for t in saved)
+    p.saved = L.ptr(saved)
     p.dv, p.dh0 = L.ptr(dv), L.ptr(dh0)
     p.grad_dtype = L.F32
     ws = L.workspace(L.lib.tops_b200_chunk_kda_bwd_workspace_bytes(C.byref(p)), dev)

@@ -242,7 +242,7 @@ struct KdaNode : public OpNode {
       p.B = (int)q.size(0); p.T = (int)q.size(1); p.H = (int)q.size(2); p.K = (int)q.size(3); p.V = (int)v.size(3); p.chunk = 64;
       p.dtype = code_of(q); p.gate_dtype = code_of(g); p.scale = (float)scale;
       p.q = ptr(qc); p.k = ptr(kc); p.v = ptr(vc); p.g = ptr(gc); p.beta = ptr(bc); p.do_ = ptr(doc); p.dht = ptr<float>(dht);
-      p.saved_h = ptr(t[6]); p.saved_vnew = ptr(t[7]); p.saved_T = ptr(t[8]); p.saved_R = ptr(t[9]);
+      p.saved = ptr(t[6]);
       p.dq = ptr(dq); p.dk = ptr(dk); p.dg = ptr(dg); p.dbeta = ptr(db); p.dv = ptr(dv); p.dh0 = ptr<float>(dh0);
       p.grad_dtype = code_of(type);
       Tensor ws = c.bytes(tops_b200_chunk_kda_bwd_workspace_bytes(&p));
@@ -286,20 +286,20 @@ std::tuple<Tensor, OptTensor> kda(const Tensor& q, const Tensor& k, const Tensor
   Tensor qc = c.in(q), kc = c.in(k), vc = c.in(v), gc = c.in(g), bc = c.in_as(beta, type), h0c = c.in_as(h0, at::kFloat);
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3);
   const bool grad = wants_grad(q, k, v, g, beta, h0);
-  Tensor ht, o, sh, sv, st, sr;
+  Tensor ht, o, saved, ws;
   if (want_ht) ht = c.empty({B, H, K, V}, at::kFloat);
   tops_chunk_kda_fwd_params p = kda_chunk_params(q, v, g, scale);
   chunked = chunked && tops_b200_chunk_kda_supported(&p) != 0;
   if (chunked) {
     o = c.empty({B, T, H, V}, type);
     if (grad) {
-      sh = c.empty({B, T / 64, H, K, V}, type);
-      sv = c.empty({B, T, H, V}, type);
-      st = c.empty({B, T, H, 64}, type);
-      sr = c.empty({B, T, H, V}, type);
+      saved = c.bytes(tops_b200_chunk_kda_saved_bytes(&p));
+    } else {
+      ws = c.bytes(tops_b200_chunk_kda_fwd_workspace_bytes(&p));
+      p.workspace = ptr(ws); p.workspace_bytes = (size_t)ws.numel();
     }
     p.q = ptr(qc); p.k = ptr(kc); p.v = ptr(vc); p.g = ptr(gc); p.beta = ptr(bc); p.h0 = ptr<float>(h0c); p.o = ptr(o);
-    p.ht = ptr<float>(ht); p.saved_h = ptr(sh); p.saved_vnew = ptr(sv); p.saved_T = ptr(st); p.saved_R = ptr(sr);
+    p.ht = ptr<float>(ht); p.saved = ptr(saved);
     check(tops_b200_chunk_kda_fwd(&p, c.stream()), "chunk_kda_fwd");
   } else {
     o = kda_run(c, qc, kc, vc, gc, bc, scale, ptr<float>(h0c), ptr<float>(ht));
@@ -307,7 +307,7 @@ std::tuple<Tensor, OptTensor> kda(const Tensor& q, const Tensor& k, const Tensor
   if (grad) {
     auto node = make_node<KdaNode>(q, k, v, g, beta, h0);
     node->scale = scale; node->chunked = chunked;
-    node->keep({q, k, v, g, beta, h0, sh, sv, st, sr});
+    node->keep({q, k, v, g, beta, h0, saved});
     attach(o, node);
     attach(ht, node);
   }
