@@ -635,12 +635,10 @@ struct FwdOParams {
   __nv_bfloat16* o;
   int T, H, NT;
   float scale;
-  const float* gamma;             // constant gates [H] (SCALAR GEN kernel)
-  Geo geo;                        // GEN kernel
 };
 
 // SCALAR: no gate tile and no exponent product; every warp cumulates the chunk's 64 gates in registers.
-template <bool SCALAR, bool GEN>
+template <bool SCALAR>
 __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ FwdOParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -650,20 +648,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   uint8_t* vt = gs + TILE64;
   uint8_t* hs = vt + TILE64;          // h_c exp(mid) scale, 128 x 128 (scaled by the scan kernel)
   uint8_t* mt = hs + TILE128;         // TRI_MID pattern, 64 x 64
-  float* diag = reinterpret_cast<float*>(gs + SLAB64);   // GEN: partial q_i . k_i [4][64] (the gates are consumed by then)
   __shared__ uint64_t bar_load, bar_e, bar_a, bar_o;
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, seg = warp >> 2;
   // heads vary fastest over the blocks in flight: together they read whole token rows of the
   // [B,T,H,D] activations (all heads of a time step are contiguous in memory)
-  // (grid: heads x value slices, chunks of a sequence, sequences; packed: heads x value slices, all chunks, 1)
-  const int VS = GEN ? p.geo.VS : 1, V = GEN ? p.geo.V : D;
-  const int h = GEN ? blockIdx.x / VS : blockIdx.x, vs = GEN ? blockIdx.x % VS : 0, ci = blockIdx.y, b = blockIdx.z;
-  const int slot = b * p.NT + ci;
-  int row = b * p.T + ci * C, end = (b + 1) * p.T;
-  if (GEN && p.geo.chunks) { const ChunkEntry e = p.geo.chunks[slot]; row = e.row; end = e.end; }
-  const int len = GEN ? min(C, end - row) : C;
+  const int h = blockIdx.x, ci = blockIdx.y, b = blockIdx.z;
+  const int row = b * p.T + ci * C;
   constexpr uint32_t cO = 0, cE = 0, cA = 128;   // E is consumed before O is produced
 
   if (tid == 0) {
@@ -673,19 +665,17 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     if (!SCALAR) { tma_load_3d(gs, &p.mg, &bar_load, 0, h, row); tma_load_3d(gs + SLAB64, &p.mg, &bar_load, 64, h, row); }
     tma_load_3d(qs, &p.mq, &bar_load, 0, h, row); tma_load_3d(qs + SLAB64, &p.mq, &bar_load, 64, h, row);
     tma_load_3d(ks, &p.mk, &bar_load, 0, h, row); tma_load_3d(ks + SLAB64, &p.mk, &bar_load, 64, h, row);
-    tma_load_3d(vt, &p.mv, &bar_load, vs * D, h, row); tma_load_3d(vt + SLAB64, &p.mv, &bar_load, vs * D + 64, h, row);
-    const int hrow = ((slot * p.H + h) * VS + vs) * D;
+    tma_load_3d(vt, &p.mv, &bar_load, 0, h, row); tma_load_3d(vt + SLAB64, &p.mv, &bar_load, 64, h, row);
+    const int hrow = ((b * p.NT + ci) * p.H + h) * D;
     tma_load_2d(hs, &p.mh, &bar_load, 0, hrow); tma_load_2d(hs + TILE128 / 2, &p.mh, &bar_load, 64, hrow);
   }
   __syncwarp();
   if (warp == 0) { tmem_alloc(&tmem_slot, 256); tmem_relinquish(); }
   __nv_bfloat16 greg_lo = __float2bfloat16(0.f), greg_hi = greg_lo;   // SCALAR: the gates of time steps lane and lane + 32
   if (SCALAR) {   // (one chunk per block: the loads have the whole tile fetch to land)
-    if (!GEN || p.gscalar) {
-      const __nv_bfloat16* src = p.gscalar + (size_t)(row + lane) * p.H + h;
-      if (!GEN || lane < len) greg_lo = src[0];
-      if (!GEN || lane + 32 < len) greg_hi = src[(size_t)32 * p.H];
-    }
+    const __nv_bfloat16* src = p.gscalar + (size_t)(row + lane) * p.H + h;
+    greg_lo = src[0];
+    greg_hi = src[(size_t)32 * p.H];
   } else {
     build_tri_tile(mt, 64, TRI_MID);
   }
@@ -697,14 +687,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   const uint32_t lane_base = q4 * 32;
   bool ok = __syncthreads_and(mbar_wait(&bar_load, 0));
   if (!ok) fail(3);
-  if (GEN && len < C) {   // (uniform over the block)
-    if (!SCALAR) zero_rows(gs, len, tid, NTHREADS);
-    zero_rows(vt, len, tid, NTHREADS);
-    zero_rows(qs, len, tid, NTHREADS);
-    zero_rows(ks, len, tid, NTHREADS);
-    fence_async_smem();
-    __syncthreads();
-  }
   if (!SCALAR && ok && tid == 0) {
     tc_fence_after();
     const uint32_t ga = smem_u32(gs), ma = smem_u32(mt);
@@ -721,27 +703,19 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   if (SCALAR && ok) {
     // thread (q4, lane < 16, seg) gates 32 channels of time row 16 q4 + lane, whose cumulative gate sits in
     // lane (16 q4 + lane) mod 32 of the warp
-    float g_lo = __bfloat162float(greg_lo), g_hi = __bfloat162float(greg_hi);
-    if (GEN && p.gamma) {
-      g_lo = lane < len ? p.gamma[h] : 0.f;
-      g_hi = lane + 32 < len ? p.gamma[h] : 0.f;
-    }
-    const WarpGates w = warp_cumulate(g_lo, g_hi, lane);
+    const WarpGates w = warp_cumulate(__bfloat162float(greg_lo), __bfloat162float(greg_hi), lane);
     const int i = 16 * q4 + (lane & 15);
     const float E = __shfl_sync(0xffffffffu, (q4 >> 1) ? w.hi : w.lo, i & 31) - w.mid();
     const float f = fast_exp(E), r = fast_exp(-E);
     if (lane < 16) {
-      float dot = 0.f;
       const uint32_t rowoff = (uint32_t)(seg >> 1) * SLAB64 + (uint32_t)i * 128u;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t off = rowoff + (((uint32_t)((seg & 1) * 4 + u) ^ (uint32_t)i) & 7u) * 16u;
         const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-        if (GEN) dot = dot8(qr, kr, dot);
         *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
         *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
       }
-      if (GEN) diag[seg * C + i] = dot;
     }
     fence_async_smem();
     tc_fence_before();
@@ -752,7 +726,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     tmem_ld32(tmem_addr(tm, lane_base, cE + seg * 32), e);
     if (lane < 16) {   // rows of an M = 64 accumulator sit in lanes 0..15 of each 32-lane quarter
       const int i = 16 * q4 + lane;
-      float dot = 0.f;
       const uint32_t rowoff = (uint32_t)(seg >> 1) * SLAB64 + (uint32_t)i * 128u;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -761,11 +734,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
 #pragma unroll
         for (int t = 0; t < 8; ++t) { f[t] = fast_exp(e[8 * u + t]); r[t] = fast_exp(-e[8 * u + t]); }
         const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-        if (GEN) dot = dot8(qr, kr, dot);
         *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
         *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
       }
-      if (GEN) diag[seg * C + i] = dot;
     }
     fence_async_smem();
     tc_fence_before();
@@ -792,7 +763,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
     const int i = 16 * q4 + lane;
     float a[16];
     tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
-    if (GEN && lane < 16 && seg == q4) set_diagonal(a, diag, 4, i, lane);
     if (lane < 16) store_tril16(gs, i, seg * 16, a, p.scale);
     fence_async_smem();
     tc_fence_before();
@@ -814,21 +784,20 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_fwd_o(const __grid_constant__ F
   if (ok) {
     tc_fence_after();
     const int i = 16 * q4 + lane;
-    const int vc = vs * D + seg * 32;
-    __nv_bfloat16* dst = p.o + ((size_t)(row + i) * p.H + h) * V + vc;
+    __nv_bfloat16* dst = p.o + ((size_t)(row + i) * p.H + h) * D + seg * 32;
     float a[32];
     tmem_ld32(tmem_addr(tm, lane_base, cO + seg * 32), a);
-    if (lane < 16 && (!GEN || i < len)) {
+    if (lane < 16) {
 #pragma unroll
       for (int t = 0; t < 32; t += 8)
-        if (!GEN || vc + t < V) *reinterpret_cast<uint4*>(dst + t) = make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]),
+        *reinterpret_cast<uint4*>(dst + t) = make_uint4(pack_bf16(a[t], a[t + 1]), pack_bf16(a[t + 2], a[t + 3]),
                                                         pack_bf16(a[t + 4], a[t + 5]), pack_bf16(a[t + 6], a[t + 7]));
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
-  if (tid == 0 && !ok) poison(p.o + ((size_t)row * p.H + h) * V + vs * D);
+  if (tid == 0 && !ok) poison(p.o + ((size_t)row * p.H + h) * D);
 }
 
 // ===========================================================================
@@ -875,6 +844,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* in = smem;                         // 2 stages x (q, k, g, v)
   uint8_t* hst = in + 2 * FUSED_STAGE;        // 2 x (128 x 128) bf16: h' of the current chunk
+  uint8_t* qlo = hst + TILE128;               // GEN: one h' tile; what bf16 leaves of q~ (then of A) and of k~
+  uint8_t* klo = qlo + TILE64;
   uint8_t* mt = hst + 2 * TILE128;            // TRI_MID pattern, rows repeated to 128
   uint8_t* wt = mt + 2 * SLAB64;              // 16 x 64 pattern for G_n and G_n - mid
   uint8_t* ost = wt + 2048;                   // 64 x 128 bf16: the outputs of a chunk, row-major, before they leave
@@ -979,7 +950,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       const uint32_t ph = pp & 1;
       uint8_t* qs = in + (pp & 1) * FUSED_STAGE;
       uint8_t *ks = qs + TILE64, *gs = ks + TILE64, *vs = gs + TILE64;
-      uint8_t* ht = hst + (pp & 1) * TILE128;
+      uint8_t* ht = GEN ? hst : hst + (pp & 1) * TILE128;
       // the state store of chunk pp-1 has read its staging tile, which the compute warps refill after
       // the next barrier (with the state of chunk pp+1)
       if (lane == 0) tma_store_wait_read();
@@ -991,10 +962,25 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // A = q~ k~^T
           umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+        if (GEN) {
+          const uint32_t qla = smem_u32(qlo), kla = smem_u32(klo);
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(kla, 64, 0, k0), umma_idesc(64, 64, 0, 0), 1);
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cA, desc_kmajor(qla, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), 1);
+        }
         umma_commit(&sh.abar);
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_j k~[j][k] v[j][v]
           umma_bf16(tm + cD, desc_mnmajor(ka, 64, k0, 0), desc_mnmajor(va, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
+        if (GEN) {
+          const uint32_t kla = smem_u32(klo);
+#pragma unroll
+          for (int k0 = 0; k0 < C; k0 += 16)
+            umma_bf16(tm + cD, desc_mnmajor(kla, 64, k0, 0), desc_mnmajor(va, 64, k0, 0), umma_idesc(128, 128, 1, 1), 1);
+        }
         umma_commit(&sh.sbar);
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // o = q~ h'
@@ -1004,6 +990,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
           tma_store_2d(&p.mst, ht, 0, hrow);
           tma_store_2d(&p.mst, ht + TILE128 / 2, 64, hrow);
           tma_store_commit();
+          if (GEN) tma_store_wait_read();   // (the one h' tile is refilled after B2)
         }
       }
       // B2: tril(A) scale is in shared memory (in the gate tile of this stage)
@@ -1014,6 +1001,12 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 16)   // o += tril(A) scale v
           umma_bf16(tm + cO, desc_kmajor(pa, 64, 0, k0), desc_mnmajor(va, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
+        if (GEN) {
+          const uint32_t pla = smem_u32(qlo);
+#pragma unroll
+          for (int k0 = 0; k0 < C; k0 += 16)
+            umma_bf16(tm + cO, desc_kmajor(pla, 64, 0, k0), desc_mnmajor(va, 64, k0, 0), umma_idesc(64, 128, 0, 1), 1);
+        }
         umma_commit(&sh.obar);
       }
       // exponents of the next chunk (E and W of this one were read before B1)
@@ -1050,7 +1043,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       const uint32_t ph = pp & 1;
       uint8_t* qs = in + (pp & 1) * FUSED_STAGE;
       uint8_t *ks = qs + TILE64, *gs = ks + TILE64;
-      uint8_t* ht = hst + (pp & 1) * TILE128;
+      uint8_t* ht = GEN ? hst : hst + (pp & 1) * TILE128;
       float* diag = reinterpret_cast<float*>(gs + SLAB64);   // GEN: partial q_i . k_i [8][64], in the consumed gate tile
       if (!mbar_wait(&sh.fullin[pp & 1], (pp >> 1) & 1) || (!SCALAR && !mbar_wait(&sh.ebar, ph))) { *abort_flag = 1; fail(9); }
       tc_fence_after();
@@ -1095,6 +1088,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
           *reinterpret_cast<uint4*>(qs + off) = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(ks + off) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(qlo + off) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(klo + off) = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(gs + TILE64 + off) = make_uint4(0u, 0u, 0u, 0u);   // v
         }
       } else if (SCALAR) {
@@ -1108,9 +1103,17 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         for (int u = 0; u < 2; ++u) {
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
           const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-          if (GEN) dot = dot8(qr, kr, dot);
-          *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
+          if constexpr (GEN) {
+            uint4 l;
+            dot = dot8(qr, kr, dot);
+            *reinterpret_cast<uint4*>(qs + off) = scale8_by_split(qr, f, l);
+            *reinterpret_cast<uint4*>(qlo + off) = l;
+            *reinterpret_cast<uint4*>(ks + off) = scale8_by_split(kr, r, l);
+            *reinterpret_cast<uint4*>(klo + off) = l;
+          } else {
+            *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
+            *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
+          }
         }
         if (GEN) diag[cg * C + i] = dot;
       } else {
@@ -1128,9 +1131,17 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
             r[t] = fast_exp(-em[8 * u + t]);
           }
           const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-          if (GEN) dot = dot8(qr, kr, dot);
-          *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
-          *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
+          if constexpr (GEN) {
+            uint4 l;
+            dot = dot8(qr, kr, dot);
+            *reinterpret_cast<uint4*>(qs + off) = scale8_split(qr, f, l);
+            *reinterpret_cast<uint4*>(qlo + off) = l;
+            *reinterpret_cast<uint4*>(ks + off) = scale8_split(kr, r, l);
+            *reinterpret_cast<uint4*>(klo + off) = l;
+          } else {
+            *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
+            *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
+          }
         }
         if (GEN) diag[cg * C + i] = dot;
       }
@@ -1147,7 +1158,10 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         float a[16];
         tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
         if (GEN && lane < 16 && seg == q4) set_diagonal(a, diag, 8, i, lane);
-        if (lane < 16) store_tril16(gs, i, seg * 16, a, p.scale);
+        if (lane < 16) {
+          if (GEN) store_tril16_split(gs, qlo, i, seg * 16, a, p.scale);   // (q~'s lower half has been read)
+          else store_tril16(gs, i, seg * 16, a, p.scale);
+        }
       }
       fence_async_smem();
       tc_fence_before();
@@ -1230,9 +1244,9 @@ template <typename TG, typename TD, bool SCALAR, bool GEN>
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_constant__ BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint8_t* qs = smem;                 // 2 x: q -> q exp(G - mid) in place
-  uint8_t* ks = qs + 2 * TILE64;      // 2 x: k -> k exp(mid - G) in place
-  uint8_t* gs = ks + 2 * TILE64;      // g
+  uint8_t* qs = smem;                 // 2 x: q -> q exp(G - mid) in place (GEN: one, and what bf16 leaves of it)
+  uint8_t* ks = qs + 2 * TILE64;      // 2 x: k -> k exp(mid - G) in place (GEN: likewise)
+  uint8_t* gs = ks + 2 * TILE64;      // g (GEN: then what bf16 leaves of tril(A) scale and tril(dA) scale)
   uint8_t* vs = gs + TILE64;
   uint8_t* dos = vs + TILE64;
   uint8_t* hs = dos + TILE64;         // h_c exp(mid) scale, 128 x 128
@@ -1249,11 +1263,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   __shared__ float tails[2][4][D];    // per-segment sum_i dk_inter k
   __shared__ float hdh_s[2][D];       // sum_v h' dh'
   __shared__ float dgk_s[2][C];       // SCALAR: dg of a chunk summed over the channels
-  __shared__ float diag[2][GEN ? 8 * C : 1];   // GEN: partial q_i . k_i [8][64] of a chunk
+  __shared__ float diag[1][GEN ? 8 * C : 1];   // GEN: partial q_i . k_i [8][64] of a chunk
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // tensor-memory columns: the exponent tile E_mid is consumed by the gating before A and dA take its place
-  constexpr uint32_t cEm = 0, cA = 0, cdA = 64, cET = 128, cdq = 256, cdk1 = 320, cdk2 = 384, cdv = 448;
+  constexpr uint32_t cEm = 0, cA = 0, cET = 128, cdq = 256, cdk1 = 320, cdk2 = 384, cdv = 448;
+  constexpr uint32_t cdA = GEN ? cdk1 : 64;
   const int nit = (p.total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
   const int K = GEN ? p.geo.K : D, V = GEN ? p.geo.V : D;
@@ -1299,7 +1314,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     mbar_init(&full_qk[0], 1); mbar_init(&full_qk[1], 1); mbar_init(&full_hdo, 1);
     mbar_init(&full_dhv, 1); mbar_init(&bar_gate, 1); mbar_init(&bar_A, 1); mbar_init(&bar_r1, 1); mbar_init(&bar_r2, 1);
     mbar_init(&bar_main, 1);
-    mbar_init(&gated, BWD_EPI_THREADS); mbar_init(&conv_done, BWD_GATE_THREADS);
+    mbar_init(&gated, BWD_EPI_THREADS); mbar_init(&conv_done, GEN ? BWD_EPI_THREADS : BWD_GATE_THREADS);
     mbar_init(&hdh_done[0], BWD_GATE_THREADS); mbar_init(&hdh_done[1], BWD_GATE_THREADS);
     mbar_init(&e_done[0], BWD_EPI_THREADS); mbar_init(&e_done[1], BWD_EPI_THREADS);
     fence_barrier_init();
@@ -1345,9 +1360,35 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       if (!GEN || lane + 32 < glen) greg_hi = src[(size_t)32 * p.H];
     };
     if (SCALAR && nit > 0) load_gates(0);
+    auto store_gated = [&](uint32_t off, bool mine, uint4 qh, uint4 ql, uint4 kh, uint4 kl) {   // GEN
+      const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(qs + off) = mine ? qh : none;
+      *reinterpret_cast<uint4*>(qs + TILE64 + off) = mine ? ql : none;
+      *reinterpret_cast<uint4*>(ks + off) = mine ? kh : none;
+      *reinterpret_cast<uint4*>(ks + TILE64 + off) = mine ? kl : none;
+    };
+    // GEN: A and dA -> masked hi + lo operands, 16 columns of both per thread (rows of an M = 64 accumulator sit in
+    // lanes 0..15 of each quarter)
+    auto convert = [&](int it) -> bool {
+      if (!__all_sync(0xffffffffu, wait(&bar_A, it & 1, 7))) return false;
+      tc_fence_after();
+      const int ri = 16 * q4 + lane;
+      float a[16], da[16];
+      tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
+      tmem_ld16(tmem_addr(tm, lane_base, cdA + seg * 16), da);
+      if (lane < 16) {
+        if (seg == q4) set_diagonal(a, diag[0], 8, ri, lane);
+        store_tril16_split(Ps, gs, ri, seg * 16, a, p.scale);
+        store_tril16_split(dAs, gs + SLAB64, ri, seg * 16, da, p.scale);
+      }
+      fence_async_smem();
+      tc_fence_before();
+      mbar_arrive(&conv_done);
+      return true;
+    };
     auto gate_chunk = [&](int it) -> bool {
-      const int sl = it & 1;
-      bool landed = (SCALAR || wait(&bar_gate, it & 1, 9)) && wait(&full_qk[sl], (it >> 1) & 1, 6);
+      const int sl = GEN ? 0 : it & 1;
+      bool landed = (SCALAR || wait(&bar_gate, it & 1, 9)) && wait(&full_qk[sl], GEN ? it & 1 : (it >> 1) & 1, 6);
       if (SCALAR) landed = __all_sync(0xffffffffu, landed);   // (shuffles follow: the whole warp takes one path)
       if (!landed) return false;
       tc_fence_after();
@@ -1377,11 +1418,17 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         for (int u = 0; u < 2; ++u) {
           const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
           const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-          if (GEN) dot = dot8(qr, kr, dot);
-          *reinterpret_cast<uint4*>(qs + off) = mine ? scale8_by(qr, f) : make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(ks + off) = mine ? scale8_by(kr, r) : make_uint4(0u, 0u, 0u, 0u);
+          if constexpr (GEN) {
+            uint4 ql, kl;
+            dot = dot8(qr, kr, dot);
+            const uint4 qh = scale8_by_split(qr, f, ql), kh = scale8_by_split(kr, r, kl);
+            store_gated(off, mine, qh, ql, kh, kl);
+          } else {
+            *reinterpret_cast<uint4*>(qs + off) = scale8_by(qr, f);
+            *reinterpret_cast<uint4*>(ks + off) = scale8_by(kr, r);
+          }
         }
-        if (GEN) diag[sl][cg * C + i] = mine ? dot : 0.f;
+        if (GEN) diag[0][cg * C + i] = mine ? dot : 0.f;
         fence_async_smem();
         tc_fence_before();
         mbar_arrive(&gated);
@@ -1400,32 +1447,44 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           r[t] = fast_exp(-em[8 * u + t]);
         }
         const uint4 qr = *reinterpret_cast<const uint4*>(qs + off), kr = *reinterpret_cast<const uint4*>(ks + off);
-        if (GEN) dot = dot8(qr, kr, dot);
-        *reinterpret_cast<uint4*>(qs + off) = mine ? scale8(qr, f) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(ks + off) = mine ? scale8(kr, r) : make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (GEN) {
+          uint4 ql, kl;
+          dot = dot8(qr, kr, dot);
+          const uint4 qh = scale8_split(qr, f, ql), kh = scale8_split(kr, r, kl);
+          store_gated(off, mine, qh, ql, kh, kl);
+        } else {
+          *reinterpret_cast<uint4*>(qs + off) = scale8(qr, f);
+          *reinterpret_cast<uint4*>(ks + off) = scale8(kr, r);
+        }
       }
-      if (GEN) diag[sl][cg * C + i] = mine ? dot : 0.f;
+      if (GEN) diag[0][cg * C + i] = mine ? dot : 0.f;
       fence_async_smem();
       tc_fence_before();
       mbar_arrive(&gated);
       return true;
     };
-    bool live = nit > 0 && gate_chunk(0);
-    if (SCALAR && nit > 1) load_gates(1);
+    bool live = nit > 0 && (GEN || gate_chunk(0));
+    if (SCALAR && !GEN && nit > 1) load_gates(1);
     for (int it = 0; live && it < nit; ++it) {
       const int sl = it & 1;
       int h, row, hrow;
       const int len = chunk_rows(it, h, row, hrow);
+      if (GEN && !gate_chunk(it)) break;
       const float fw = fw_next, rw = rw_next;   // (SCALAR) of this chunk
-      // the next chunk's gating runs while the tensor core works on this chunk's gradient products
-      if (it + 1 < nit && !gate_chunk(it + 1)) break;
-      if (SCALAR && it + 2 < nit) load_gates(it + 2);   // fetched where the thread waits anyway
+      if constexpr (GEN) {
+        if (SCALAR && it + 1 < nit) load_gates(it + 1);
+        if (!convert(it)) break;
+      } else {
+        // the next chunk's gating runs while the tensor core works on this chunk's gradient products
+        if (it + 1 < nit && !gate_chunk(it + 1)) break;
+        if (SCALAR && it + 2 < nit) load_gates(it + 2);   // fetched where the thread waits anyway
+      }
       bool done = wait(&bar_main, it & 1, 8) && wait(&hdh_done[sl], (it >> 1) & 1, 11);
       if (SCALAR) done = __all_sync(0xffffffffu, done);   // (shuffles follow: the whole warp takes one path)
       if (!done) break;
       tc_fence_after();
-      const uint8_t* qt = qs + sl * TILE64;
-      const uint8_t* kt = ks + sl * TILE64;
+      const uint8_t* qt = qs + (GEN ? 0 : sl) * TILE64;
+      const uint8_t* kt = ks + (GEN ? 0 : sl) * TILE64;
       const size_t obase = ((size_t)(row + seg * SEG) * p.H + h) * K + col;
       size_t vbase = obase;
       if (GEN) vbase = (size_t)(row + seg * SEG) * vstride + (size_t)h * V + yc + col;
@@ -1445,7 +1504,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         for (int u = 7; u >= 0; --u) {
           const int t = blk * 8 + u;
           const uint32_t off = ca.at(seg * SEG + t);
-          const float qv = ld_bf16(qt, off), kv = ld_bf16(kt, off);   // q~, k~
+          float qv = ld_bf16(qt, off), kv = ld_bf16(kt, off);   // q~, k~
+          if (GEN) {
+            qv += ld_bf16(qt + TILE64, off);
+            kv += ld_bf16(kt + TILE64, off);
+          }
           // exp(G - mid), exp(mid - G) of time step 16 seg + t
           const float e = SCALAR ? __shfl_sync(0xffffffffu, fw, (seg * SEG + t) & 31) : fast_exp(et[u]);
           const float r = SCALAR ? __shfl_sync(0xffffffffu, rw, (seg * SEG + t) & 31) : fast_exp(-et[u]);
@@ -1527,22 +1590,23 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
     const int g4 = warp & 3;
     const uint32_t lane_base = g4 * 32;
     for (int it = 0; it < nit; ++it) {
-      // rows of the M = 64 accumulators sit in lanes 0..15 of each quarter
-      if (!wait(&bar_A, it & 1, 7)) break;
-      tc_fence_after();
-      const int ri = 16 * g4 + lane;
+      if constexpr (!GEN) {
+        // rows of the M = 64 accumulators sit in lanes 0..15 of each quarter
+        if (!wait(&bar_A, it & 1, 7)) break;
+        tc_fence_after();
+        const int ri = 16 * g4 + lane;
 #pragma unroll
-      for (int sg = 0; sg < 4; ++sg) {
-        float a[16];
-        tmem_ld16(tmem_addr(tm, lane_base, cA + sg * 16), a);
-        if (GEN && lane < 16 && sg == g4) set_diagonal(a, diag[it & 1], 8, ri, lane);
-        if (lane < 16) store_tril16(Ps, ri, sg * 16, a, p.scale);
-        tmem_ld16(tmem_addr(tm, lane_base, cdA + sg * 16), a);
-        if (lane < 16) store_tril16(dAs, ri, sg * 16, a, p.scale);
+        for (int sg = 0; sg < 4; ++sg) {
+          float a[16];
+          tmem_ld16(tmem_addr(tm, lane_base, cA + sg * 16), a);
+          if (lane < 16) store_tril16(Ps, ri, sg * 16, a, p.scale);
+          tmem_ld16(tmem_addr(tm, lane_base, cdA + sg * 16), a);
+          if (lane < 16) store_tril16(dAs, ri, sg * 16, a, p.scale);
+        }
+        fence_async_smem();
+        tc_fence_before();
+        mbar_arrive(&conv_done);
       }
-      fence_async_smem();
-      tc_fence_before();
-      mbar_arrive(&conv_done);
       // sum_v h'[k][v] dh'[k][v] for k = this thread, while the gradient products read the same tiles
       if (!wait(&full_hdo, it & 1, 6) || !wait(&full_dhv, it & 1, 6)) break;
       {
@@ -1596,17 +1660,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         umma_commit(&bar_gate);
       };
       auto issue_A = [&](int it) {
-        if (GEN && lane != 0) return;
         const uint32_t qta = smem_u32(qs + (it & 1) * TILE64), kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // A[i][j] = q~ k~^T
           umma_bf16(tm + cA, desc_kmajor(qta, 64, 0, k0), desc_kmajor(kta, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
       };
       auto issue_dA = [&](int it) {
-        if (GEN) {
-          zero_foreign(it, vs, dos);
-          if (lane != 0) return;
-        }
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // dA[i][j] = do v^T
           umma_bf16(tm + cdA, desc_kmajor(doa, 64, 0, k0), desc_kmajor(va, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
@@ -1616,7 +1675,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       // the chunk's tiles have landed, while the conversion warps still work on A and dA; after it dh'
       // and v are dead and the next chunk's are fetched.  The second group needs the converted operands.
       auto issue_inter = [&](int it) {
-        if (GEN && lane != 0) return;
         const uint32_t kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < D; k0 += 16)   // dq_inter^T[k][i] = h' do^T
@@ -1630,7 +1688,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         umma_commit(&bar_r2);
       };
       auto issue_intra = [&](int it) {
-        if (GEN && lane != 0) return;
         const uint32_t qta = smem_u32(qs + (it & 1) * TILE64), kta = smem_u32(ks + (it & 1) * TILE64);
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 16)   // dv^T[v][j] += sum_i do[i][v] A[i][j]
@@ -1649,39 +1706,111 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
         const bool r = wait(bar, parity, code);
         return GEN ? (bool)__all_sync(0xffffffffu, r) : r;
       };
-      bool ok = SCALAR || waitw(&full_g, 0, 6);
-      if (ok) {
-        tc_fence_after();
-        if (!SCALAR) issue_gate(0);
-        ok = waitw(&gated, 0, 12);
-      }
-      if (ok) {
-        tc_fence_after();
-        issue_A(0);
-        ok = waitw(&full_hdo, 0, 6) && waitw(&full_dhv, 0, 6);
-      }
-      if (ok) issue_dA(0);
-      for (int it = 0; ok && it < nit; ++it) {
-        // A and dA of this chunk are issued; the previous chunk has left tensor memory
-        if (it >= 1 && !waitw(&e_done[(it - 1) & 1], ((it - 1) >> 1) & 1, 14)) break;
-        tc_fence_after();
-        issue_inter(it);
-        if (!waitw(&conv_done, it & 1, 13)) break;   // A and dA of this chunk are in shared memory
-        tc_fence_after();
-        const bool more = it + 1 < nit;
-        if (more && !SCALAR) {   // the next chunk's exponents take the place of A and dA in tensor memory
-          if (!waitw(&full_g, (it + 1) & 1, 6)) break;
-          issue_gate(it + 1);
-        }
-        issue_intra(it);
-        if (more) {
-          if (!waitw(&gated, (it + 1) & 1, 12)) break;
+      if constexpr (GEN) {
+        // q~, k~, A and dA are hi + lo: the products of two of them are hi hi + hi lo + lo hi.
+        auto issue_before_gating = [&]() {   // dA, dq_inter, dk_inter: everything without q~ or k~
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cdA, desc_kmajor(doa, 64, 0, k0), desc_kmajor(va, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cdq, desc_kmajor(ha, 128, 0, k0), desc_kmajor(doa, 64, 0, k0), umma_idesc(128, 64, 0, 0), k0 > 0);
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cdk2, desc_kmajor(dha, 128, 0, k0), desc_kmajor(va, 64, 0, k0), umma_idesc(128, 64, 0, 0), k0 > 0);
+        };
+        const uint32_t qta = smem_u32(qs), kta = smem_u32(ks), qla = qta + TILE64, kla = kta + TILE64;
+        const uint32_t pla = ga, dala = ga + SLAB64;
+        auto mul_A = [&](uint32_t x, uint32_t y, uint32_t acc) {
+#pragma unroll
+          for (int k0 = 0; k0 < D; k0 += 16)
+            umma_bf16(tm + cA, desc_kmajor(x, 64, 0, k0), desc_kmajor(y, 64, 0, k0), umma_idesc(64, 64, 0, 0), acc | (k0 > 0));
+        };
+        auto mul_dv = [&](uint32_t a) {    // dv^T[v][j] += sum_i do[i][v] A[i][j]
+#pragma unroll
+          for (int k0 = 0; k0 < C; k0 += 16)
+            umma_bf16(tm + cdv, desc_mnmajor(doa, 64, k0, 0), desc_mnmajor(a, 64, k0, 0), umma_idesc(128, 64, 1, 1), 1);
+        };
+        auto mul_dq = [&](uint32_t k, uint32_t da) {   // dq^T[k][i] += sum_j k~[j][k] dA[i][j]
+#pragma unroll
+          for (int k0 = 0; k0 < C; k0 += 16)
+            umma_bf16(tm + cdq, desc_mnmajor(k, 64, k0, 0), desc_kmajor(da, 64, 0, k0), umma_idesc(128, 64, 1, 0), 1);
+        };
+        auto mul_dk = [&](uint32_t q, uint32_t da, uint32_t acc) {   // dk_intra^T[k][j] = sum_i q~[i][k] dA[i][j]
+#pragma unroll
+          for (int k0 = 0; k0 < C; k0 += 16)
+            umma_bf16(tm + cdk1, desc_mnmajor(q, 64, k0, 0), desc_mnmajor(da, 64, k0, 0), umma_idesc(128, 64, 1, 1), acc | (k0 > 0));
+        };
+        for (int it = 0; it < nit; ++it) {
+          if (!SCALAR) {
+            if (!waitw(&full_g, it & 1, 6)) break;
+            tc_fence_after();
+            issue_gate(it);
+            __syncwarp();
+          }
+          // the tiles have landed, the previous chunk has left tensor memory
+          if (!waitw(&full_hdo, it & 1, 6) || !waitw(&full_dhv, it & 1, 6)) break;
+          zero_foreign(it, vs, dos);
+          if (it >= 1 && !waitw(&e_done[(it - 1) & 1], ((it - 1) >> 1) & 1, 14)) break;
           tc_fence_after();
-          issue_A(it + 1);
-          if (!waitw(&full_hdo, (it + 1) & 1, 6) || !waitw(&full_dhv, (it + 1) & 1, 6)) break;
-          issue_dA(it + 1);
+          if (lane == 0) issue_before_gating();
+          __syncwarp();
+          if (!waitw(&gated, it & 1, 12)) break;
+          tc_fence_after();
+          if (lane == 0) {
+            mul_A(qta, kta, 0); mul_A(qta, kla, 1); mul_A(qla, kta, 1);
+            umma_commit(&bar_A);
+#pragma unroll
+            for (int k0 = 0; k0 < D; k0 += 16)   // dv^T[v][j] = dh'^T k~^T
+              umma_bf16(tm + cdv, desc_mnmajor(dha, 128, k0, 0), desc_kmajor(kta, 64, 0, k0), umma_idesc(128, 64, 1, 0), k0 > 0);
+            umma_commit(&bar_r2);   // dh' and v are dead
+          }
+          __syncwarp();
+          if (!waitw(&conv_done, it & 1, 13)) break;
+          tc_fence_after();
+          if (lane == 0) {
+            mul_dv(pa); mul_dv(pla);
+            umma_commit(&bar_r1);   // h' and do are dead
+            mul_dq(kta, daa); mul_dq(kta, dala); mul_dq(kla, daa);
+            mul_dk(qta, daa, 0); mul_dk(qta, dala, 1); mul_dk(qla, daa, 1);
+            umma_commit(&bar_main);
+          }
+          __syncwarp();
         }
-        if (GEN) __syncwarp();
+      } else {
+        bool ok = SCALAR || waitw(&full_g, 0, 6);
+        if (ok) {
+          tc_fence_after();
+          if (!SCALAR) issue_gate(0);
+          ok = waitw(&gated, 0, 12);
+        }
+        if (ok) {
+          tc_fence_after();
+          issue_A(0);
+          ok = waitw(&full_hdo, 0, 6) && waitw(&full_dhv, 0, 6);
+        }
+        if (ok) issue_dA(0);
+        for (int it = 0; ok && it < nit; ++it) {
+          // A and dA of this chunk are issued; the previous chunk has left tensor memory
+          if (it >= 1 && !waitw(&e_done[(it - 1) & 1], ((it - 1) >> 1) & 1, 14)) break;
+          tc_fence_after();
+          issue_inter(it);
+          if (!waitw(&conv_done, it & 1, 13)) break;   // A and dA of this chunk are in shared memory
+          tc_fence_after();
+          const bool more = it + 1 < nit;
+          if (more && !SCALAR) {   // the next chunk's exponents take the place of A and dA in tensor memory
+            if (!waitw(&full_g, (it + 1) & 1, 6)) break;
+            issue_gate(it + 1);
+          }
+          issue_intra(it);
+          if (more) {
+            if (!waitw(&gated, (it + 1) & 1, 12)) break;
+            tc_fence_after();
+            issue_A(it + 1);
+            if (!waitw(&full_hdo, (it + 1) & 1, 6) || !waitw(&full_dhv, (it + 1) & 1, 6)) break;
+            issue_dA(it + 1);
+          }
+        }
       }
     }
   } else {
@@ -1696,9 +1825,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       auto load_qk = [&](int it) {
         int h, row, hrow;
         chunk_rows(it, h, row, hrow);
-        uint64_t* bar = &full_qk[it & 1];
-        uint8_t* qd = qs + (it & 1) * TILE64;
-        uint8_t* kd = ks + (it & 1) * TILE64;
+        const int sl = GEN ? 0 : it & 1;
+        uint64_t* bar = &full_qk[sl];
+        uint8_t* qd = qs + sl * TILE64;
+        uint8_t* kd = ks + sl * TILE64;
         mbar_expect_tx(bar, 2 * TILE64);
         tma_load_3d(qd, &p.mq, bar, 0, h, row); tma_load_3d(qd + SLAB64, &p.mq, bar, 64, h, row);
         tma_load_3d(kd, &p.mk, bar, 0, h, row); tma_load_3d(kd + SLAB64, &p.mk, bar, 64, h, row);
@@ -1722,7 +1852,25 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       load_hdo(0);
       load_dhv(0);
       bool ok = true;
-      if (nit > 1) {
+      if (GEN) {   // one slot of q and k: refilled when the write-out has read them (from L2, fetched ahead)
+        for (int it = 0; it + 1 < nit; ++it) {
+          int h, row, hrow;
+          chunk_rows(it + 1, h, row, hrow);
+          tma_prefetch_l2_3d(&p.mq, 0, h, row); tma_prefetch_l2_3d(&p.mq, 64, h, row);
+          tma_prefetch_l2_3d(&p.mk, 0, h, row); tma_prefetch_l2_3d(&p.mk, 64, h, row);
+          if (!wait(&bar_r2, it & 1, 8) || !wait(&hdh_done[it & 1], (it >> 1) & 1, 11)) break;
+          load_dhv(it + 1);
+          if (!wait(&bar_r1, it & 1, 8)) break;
+          load_hdo(it + 1);
+          if (!SCALAR) {   // (the gate tile held the lower halves of A and dA)
+            if (!wait(&bar_main, it & 1, 8)) break;
+            load_g(it + 1);
+          }
+          if (!wait(&e_done[it & 1], (it >> 1) & 1, 14)) break;
+          load_qk(it + 1);
+        }
+        ok = false;   // (the loop below is the plain form's)
+      } else if (nit > 1) {
         load_qk(1);
         if (!SCALAR) {
           ok = wait(&bar_gate, 0, 9);   // the exponent products of chunk 0 have read its gates
@@ -1925,10 +2073,10 @@ int chunk_fwd(const tops_chunk_fwd_params& p, void* ws, size_t, cudaStream_t st)
   if (!scalar && (rc = act_map(&fp.mg, p.g, BT, pb.H))) return rc;
   fp.gscalar = reinterpret_cast<const __nv_bfloat16*>(p.g);
   fp.o = reinterpret_cast<__nv_bfloat16*>(p.o); fp.T = pb.T; fp.H = pb.H; fp.NT = NT; fp.scale = pb.scale;
-  if ((rc = opt_in_smem(k_fwd_o<true, false>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false, false>, FWD_O_SMEM))) return rc;
+  if ((rc = opt_in_smem(k_fwd_o<true>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false>, FWD_O_SMEM))) return rc;
   KernelScope ks("sm100_fwd_o", st);
-  if (scalar) k_fwd_o<true, false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
-  else k_fwd_o<false, false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
+  if (scalar) k_fwd_o<true><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
+  else k_fwd_o<false><<<dim3(pb.H, NT, pb.B), NTHREADS, FWD_O_SMEM, st>>>(fp);
   return post_launch();
 }
 
@@ -2088,8 +2236,6 @@ struct GenPlan {
   int run_len(int n) const { return cdiv(nch[n], cdiv(nch[n], cps)); }
   int count(int n) const { return cdiv(nch[n], run_len(n)); }
   int blocks() const { return runs * HV; }
-  // (the chunk-parallel output kernel numbers chunks in a 16-bit grid dimension)
-  bool fused() const { return blocks() >= kFusedMinBlocks || total_chunks > 65535; }
   size_t words() const { return nch.empty() ? 0 : 3 * (size_t)N + (size_t)align_up(N + 1, 4) + (3 * (size_t)N % 4 ? 4 - 3 * (size_t)N % 4 : 0) + 8 * (size_t)runs; }
   size_t table_bytes() const { return nch.empty() ? 0 : align_up(words() * 4) + align_up((size_t)total_chunks * sizeof(ChunkEntry)); }
   size_t state_bytes() const { return align_up((size_t)total_chunks * HV * D * D * 2); }
@@ -2227,7 +2373,7 @@ size_t gen_saved_bytes(const tops_chunk_problem& pb) { return GenPlan(pb).state_
 
 size_t gen_fwd_workspace_bytes(const tops_chunk_fwd_params& p) {
   const GenPlan g(p.pb);
-  return g.table_bytes() + (p.saved_out || g.fused() ? 0 : g.state_bytes()) + g.seg_bytes() + 256;
+  return g.table_bytes() + g.seg_bytes() + 256;
 }
 
 int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
@@ -2242,9 +2388,7 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
   int rc = g.upload(pb, wsp, st);
   if (rc) return rc;
   wsp += g.table_bytes();
-  const bool fused = g.fused();
   void* h = p.saved_out;
-  if (!h && !fused) { h = wsp; wsp += g.state_bytes(); }
   const GenSegs sc(wsp, g);
   const XYPitch kv{p.pitch, p.pitch};
   if ((rc = gen_starts(false, pb, g, p.k, p.g, p.v, kv, p.h0, p.ht, sc, st))) return rc;
@@ -2252,40 +2396,22 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
   const __nv_bfloat16* gs = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(p.g) : nullptr;
   const float* gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(p.g) : nullptr;
   const size_t state_rows = (size_t)g.total_chunks * g.HV * D;
-  if (fused) {
-    FusedParams up;
-    if ((rc = act_map(&up.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&up.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
-        (rc = act_map(&up.mv, p.v, BT, pb.H, pb.V, p.pitch)))
-      return rc;
-    if (!scalar && (rc = act_map(&up.mg, p.g, BT, pb.H, pb.K))) return rc;
-    up.gscalar = gs; up.gamma = gamma; up.states = nullptr;
-    if (h) {
-      if ((rc = state_map(&up.mst, h, state_rows))) return rc;
-      up.states = reinterpret_cast<__nv_bfloat16*>(h);
-    }
-    up.s0 = p.h0; up.s0_seg = sc.starts; up.s_final = p.ht; up.o = reinterpret_cast<__nv_bfloat16*>(p.o);
-    up.T = pb.T; up.H = pb.H; up.NT = 0; up.nseg = 1; up.scale = pb.scale; up.geo = g.geo;
-    if ((rc = opt_in_smem(k_fwd_fused<true, true>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false, true>, FUSED_SMEM))) return rc;
-    KernelScope ks("sm100_fwd_fused", st);
-    if (scalar) k_fwd_fused<true, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
-    else k_fwd_fused<false, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
-    return post_launch();
-  }
-  if ((rc = run_scan_gen(false, false, pb, g, p.k, p.g, p.v, kv, p.h0, sc.starts, h, p.ht, nullptr, st))) return rc;
-  FwdOParams fp;
-  if ((rc = act_map(&fp.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&fp.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
-      (rc = act_map(&fp.mv, p.v, BT, pb.H, pb.V, p.pitch)) || (rc = state_map(&fp.mh, h, state_rows)))
+  FusedParams up;
+  if ((rc = act_map(&up.mq, p.q, BT, pb.H, pb.K, p.pitch)) || (rc = act_map(&up.mk, p.k, BT, pb.H, pb.K, p.pitch)) ||
+      (rc = act_map(&up.mv, p.v, BT, pb.H, pb.V, p.pitch)))
     return rc;
-  if (!scalar && (rc = act_map(&fp.mg, p.g, BT, pb.H, pb.K))) return rc;
-  fp.gscalar = gs; fp.gamma = gamma; fp.geo = g.geo;
-  fp.o = reinterpret_cast<__nv_bfloat16*>(p.o); fp.T = pb.T; fp.H = pb.H; fp.scale = pb.scale;
-  const bool packed = !g.nch.empty();
-  fp.NT = packed ? g.total_chunks : g.geo.NTseq;
-  if ((rc = opt_in_smem(k_fwd_o<true, true>, FWD_O_SMEM)) || (rc = opt_in_smem(k_fwd_o<false, true>, FWD_O_SMEM))) return rc;
-  const dim3 grid(g.HV, fp.NT, packed ? 1 : pb.B);
-  KernelScope ks("sm100_fwd_o", st);
-  if (scalar) k_fwd_o<true, true><<<grid, NTHREADS, FWD_O_SMEM, st>>>(fp);
-  else k_fwd_o<false, true><<<grid, NTHREADS, FWD_O_SMEM, st>>>(fp);
+  if (!scalar && (rc = act_map(&up.mg, p.g, BT, pb.H, pb.K))) return rc;
+  up.gscalar = gs; up.gamma = gamma; up.states = nullptr;
+  if (h) {
+    if ((rc = state_map(&up.mst, h, state_rows))) return rc;
+    up.states = reinterpret_cast<__nv_bfloat16*>(h);
+  }
+  up.s0 = p.h0; up.s0_seg = sc.starts; up.s_final = p.ht; up.o = reinterpret_cast<__nv_bfloat16*>(p.o);
+  up.T = pb.T; up.H = pb.H; up.NT = 0; up.nseg = 1; up.scale = pb.scale; up.geo = g.geo;
+  if ((rc = opt_in_smem(k_fwd_fused<true, true>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false, true>, FUSED_SMEM))) return rc;
+  KernelScope ks("sm100_fwd_fused", st);
+  if (scalar) k_fwd_fused<true, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
+  else k_fwd_fused<false, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
   return post_launch();
 }
 

@@ -167,6 +167,36 @@ __device__ __forceinline__ uint4 scale8(uint4 x, const float* f) {
   return y;
 }
 
+// What rounding to bf16 leaves of 8 products, rounded to bf16 in its turn: the two together keep 16 bits.
+// x: what is left of; returns hi, sets lo.
+__device__ __forceinline__ uint4 split8(const float (&x)[8], uint4& lo) {
+  uint4 hi;
+  uint32_t *ph = reinterpret_cast<uint32_t*>(&hi), *pl = reinterpret_cast<uint32_t*>(&lo);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    ph[t] = pack_bf16(x[2 * t], x[2 * t + 1]);
+    // (what overflowed to infinity leaves nothing: inf - inf would be a NaN)
+    const float a = __uint_as_float(ph[t] << 16), b = __uint_as_float(ph[t] & 0xffff0000u);
+    pl[t] = pack_bf16(fabsf(a) <= 3.4e38f ? x[2 * t] - a : 0.f, fabsf(b) <= 3.4e38f ? x[2 * t + 1] - b : 0.f);
+  }
+  return hi;
+}
+__device__ __forceinline__ uint4 scale8_split(uint4 x, const float* f, uint4& lo) {
+  const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&x);
+  float y[8];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float2 v = __bfloat1622float2(px[t]);
+    y[2 * t] = v.x * f[2 * t];
+    y[2 * t + 1] = v.y * f[2 * t + 1];
+  }
+  return split8(y, lo);
+}
+__device__ __forceinline__ uint4 scale8_by_split(uint4 x, float f, uint4& lo) {
+  const float fs[8] = {f, f, f, f, f, f, f, f};
+  return scale8_split(x, fs, lo);
+}
+
 // masked, scaled bf16 copy of 16 columns [16 seg, 16 seg + 16) of row i of a
 // 64 x 64 fp32 accumulator into a K-major 64 x 64 tile
 __device__ __forceinline__ void store_tril16(uint8_t* dst, int i, int j0, const float (&a)[16], float scale) {
@@ -179,6 +209,19 @@ __device__ __forceinline__ void store_tril16(uint8_t* dst, int i, int j0, const 
       w[t >> 1] = pack_bf16(j <= i ? a[c8 + t] * scale : 0.f, j + 1 <= i ? a[c8 + t + 1] * scale : 0.f);
     }
     *reinterpret_cast<uint4*>(dst + slab_off(i, j0 + c8)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// the same as hi + lo in two tiles
+__device__ __forceinline__ void store_tril16_split(uint8_t* hi, uint8_t* lo, int i, int j0, const float (&a)[16], float scale) {
+#pragma unroll
+  for (int c8 = 0; c8 < 16; c8 += 8) {
+    float x[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) x[t] = j0 + c8 + t <= i ? a[c8 + t] * scale : 0.f;
+    uint4 l;
+    *reinterpret_cast<uint4*>(hi + slab_off(i, j0 + c8)) = split8(x, l);
+    *reinterpret_cast<uint4*>(lo + slab_off(i, j0 + c8)) = l;
   }
 }
 
