@@ -248,8 +248,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   float* const racc = &sh.e0[0][0];
   float racc_s = 0.f;
   // x / y stages: three; a summary pass, which is bound by how many bytes it keeps in flight, has two more in the
-  // state staging tiles it does not use
-  constexpr int NXY = SUM ? 5 : 3;
+  // state staging tiles it does not use (GEN: one more, and two tiles for what bf16 leaves of the gated x: its sums end
+  // up in the caller's fp32 state)
+  constexpr bool SPLIT = SUM && GEN;
+  constexpr int NXY = SPLIT ? 4 : SUM ? 5 : 3;
+  auto x_low = [&](int pp) { return hst + TILE128 + (pp & 1) * TILE64; };   // (read by the product of chunk pp, gone before gating pp + 2)
   auto x_stage = [&](int pp) { const int st = pp % NXY; return st < 3 ? xs + st * TILE64 : hst + (st - 3) * 2 * TILE64; };
   auto y_stage = [&](int pp) { const int st = pp % NXY; return st < 3 ? ys + st * TILE64 : hst + (st - 3) * 2 * TILE64 + TILE64; };
   auto xy_bar = [&](int pp) { return &sh.fullxy[pp % NXY]; };
@@ -345,6 +348,12 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
     for (int k0 = 0; k0 < C; k0 += 16)   // (SUM: every chunk accumulates into the first tile)
       umma_bf16(tm + cS + (SUM ? 0 : (pp & 1) * 128), desc_mnmajor(xa, 64, k0, 0), desc_mnmajor(ya, 64, k0, 0),
                 umma_idesc(128, 128, 1, 1), k0 > 0 || (SUM && pp > 0));
+    if (SPLIT) {
+      const uint32_t xla = smem_u32(x_low(pp));
+#pragma unroll
+      for (int k0 = 0; k0 < C; k0 += 16)
+        umma_bf16(tm + cS, desc_mnmajor(xla, 64, k0, 0), desc_mnmajor(ya, 64, k0, 0), umma_idesc(128, 128, 1, 1), 1);
+    }
     umma_commit(&sh.sbar[pp & 1]);
   };
   // gate x of chunk pp in place and publish G_n (and G_n - G_0, or G_0) of its channels
@@ -384,8 +393,15 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-        *reinterpret_cast<uint4*>(xt + off) =
-            mine ? scale8_by(*reinterpret_cast<const uint4*>(xt + off), f) : make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (SPLIT) {
+          uint4 l;
+          const uint4 hi = scale8_by_split(*reinterpret_cast<const uint4*>(xt + off), f, l);
+          *reinterpret_cast<uint4*>(xt + off) = mine ? hi : make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(x_low(pp) + off) = mine ? l : make_uint4(0u, 0u, 0u, 0u);
+        } else {
+          *reinterpret_cast<uint4*>(xt + off) =
+              mine ? scale8_by(*reinterpret_cast<const uint4*>(xt + off), f) : make_uint4(0u, 0u, 0u, 0u);
+        }
       }
       fence_async_smem();
       tc_fence_before();
@@ -420,8 +436,15 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t off = rowoff + (((uint32_t)((cg & 3) * 2 + u) ^ (uint32_t)i) & 7u) * 16u;
-      *reinterpret_cast<uint4*>(xt + off) =
-          mine ? scale8(*reinterpret_cast<const uint4*>(xt + off), e + 8 * u) : make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (SPLIT) {
+        uint4 l;
+        const uint4 hi = scale8_split(*reinterpret_cast<const uint4*>(xt + off), e + 8 * u, l);
+        *reinterpret_cast<uint4*>(xt + off) = mine ? hi : make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(x_low(pp) + off) = mine ? l : make_uint4(0u, 0u, 0u, 0u);
+      } else {
+        *reinterpret_cast<uint4*>(xt + off) =
+            mine ? scale8(*reinterpret_cast<const uint4*>(xt + off), e + 8 * u) : make_uint4(0u, 0u, 0u, 0u);
+      }
     }
     fence_async_smem();
     tc_fence_before();
