@@ -38,13 +38,44 @@ constexpr uint32_t PREP_BWD = PREP_T - PREP_K;   // the reverse scan k~ .. (G_n,
 
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory"); }
 
+// sum_k a[k] b[S k] over N entries of a row (read 16 bytes at a time) and a column
+template <int N, int S>
+__device__ __forceinline__ float dot_row_col(const float* __restrict__ a, const float* __restrict__ b) {
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < N; k += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k);
+    s = fmaf(x.x, b[k * S], s);
+    s = fmaf(x.y, b[(k + 1) * S], s);
+    s = fmaf(x.z, b[(k + 2) * S], s);
+    s = fmaf(x.w, b[(k + 3) * S], s);
+  }
+  return s;
+}
+// the same for the rows a and a + step of 32 entries, which share the column: 6 shared-memory loads for 8 multiply-adds
+// where one row at a time takes 16 (two resident blocks saturate the load path: k_kda_prep 808 -> 770 us at B = 4,
+// T = 8192, H = 32)
+__device__ __forceinline__ float2 dot_rows_col32(const float* __restrict__ a, int step, const float* __restrict__ b, int bstride) {
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(a + step + k);
+    const float b0 = b[k * bstride], b1 = b[(k + 1) * bstride], b2 = b[(k + 2) * bstride], b3 = b[(k + 3) * bstride];
+    s.x = fmaf(x.x, b0, s.x); s.y = fmaf(y.x, b0, s.y);
+    s.x = fmaf(x.y, b1, s.x); s.y = fmaf(y.y, b1, s.y);
+    s.x = fmaf(x.z, b2, s.x); s.y = fmaf(y.z, b2, s.y);
+    s.x = fmaf(x.w, b3, s.x); s.y = fmaf(y.w, b3, s.y);
+  }
+  return s;
+}
+
 // T = (I + L)^-1 for a strictly lower triangular 64 x 64 L, fp32, row-major with row stride 64, by the
 // 512 compute threads.  W: 1024 floats of scratch.
 __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ Lm, float* __restrict__ Tm,
                                                   float* __restrict__ W, int tid) {
-  for (int idx = tid; idx < C * C; idx += NTHREADS) {
-    const int i = idx >> 6, j = idx & 63;
-    if ((j >> 4) > (i >> 4)) Tm[idx] = 0.f;
+  for (int idx = tid; idx < C * C / 4; idx += NTHREADS) {
+    const int i = idx >> 4, j = (idx & 15) * 4;
+    if ((j >> 4) > (i >> 4)) *reinterpret_cast<float4*>(Tm + i * C + j) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (tid < 64) {   // 16 x 16 diagonal blocks: column c of block b by forward substitution
     const int b = tid >> 4, c = tid & 15;
@@ -54,7 +85,13 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ Lm, 
     for (int i = 0; i < 16; ++i) {
       float s = i == c ? 1.f : 0.f;
 #pragma unroll
-      for (int j = 0; j < i; ++j) s = fmaf(-Lb[i * C + j], x[j], s);
+      for (int j0 = 0; j0 < i; j0 += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(Lb + i * C + j0);
+        s = fmaf(-l.x, x[j0], s);
+        if (j0 + 1 < i) s = fmaf(-l.y, x[j0 + 1], s);
+        if (j0 + 2 < i) s = fmaf(-l.z, x[j0 + 2], s);
+        if (j0 + 3 < i) s = fmaf(-l.w, x[j0 + 3], s);
+      }
       x[i] = s;
     }
 #pragma unroll
@@ -63,34 +100,20 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ Lm, 
   compute_sync();
   {   // 32 x 32 diagonal blocks: T_10 = -T_11 (L_10 T_00), T_32 = -T_33 (L_32 T_22)
     const int p = tid >> 8, i = (tid >> 4) & 15, j = tid & 15, o = 32 * p;
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) s = fmaf(Lm[(o + 16 + i) * C + o + k], Tm[(o + k) * C + o + j], s);
-    W[tid] = s;
+    W[tid] = dot_row_col<16, C>(Lm + (o + 16 + i) * C + o, Tm + o * C + o + j);
     compute_sync();
-    s = 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) s = fmaf(Tm[(o + 16 + i) * C + o + 16 + k], W[p * 256 + k * 16 + j], s);
-    Tm[(o + 16 + i) * C + o + j] = -s;
+    Tm[(o + 16 + i) * C + o + j] = -dot_row_col<16, 16>(Tm + (o + 16 + i) * C + o + 16, W + p * 256 + j);
   }
   compute_sync();
-  // the 32 x 32 block below the diagonal: T_lo = -T_hh (L_lo T_00')
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int idx = tid + NTHREADS * u, i = idx >> 5, j = idx & 31;
-    float s = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) s = fmaf(Lm[(32 + i) * C + k], Tm[k * C + j], s);
-    W[idx] = s;
-  }
-  compute_sync();
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int idx = tid + NTHREADS * u, i = idx >> 5, j = idx & 31;
-    float s = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) s = fmaf(Tm[(32 + i) * C + 32 + k], W[k * 32 + j], s);
-    Tm[(32 + i) * C + j] = -s;
+  {   // the 32 x 32 block below the diagonal: T_lo = -T_hh (L_lo T_00')
+    const int i = tid >> 5, j = tid & 31;   // rows i and i + 16
+    const float2 s = dot_rows_col32(Lm + (32 + i) * C, 16 * C, Tm + j, C);
+    W[i * 32 + j] = s.x;
+    W[(16 + i) * 32 + j] = s.y;
+    compute_sync();
+    const float2 t = dot_rows_col32(Tm + (32 + i) * C + 32, 16 * C, W + j, 32);
+    Tm[(32 + i) * C + j] = -t.x;
+    Tm[(48 + i) * C + j] = -t.y;
   }
   compute_sync();
 }
@@ -154,6 +177,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_kda_prep(const __grid_constant_
     const uint32_t ph = it & 1;
     const int h = cid % p.H, row = (cid / p.H) * C;   // chunks are numbered (batch, chunk, head): token row = 64 x (batch, chunk)
     uint8_t* out = p.prep + (size_t)cid * PREP_BYTES;
+    if (tid == 32 && cid + gridDim.x < p.total) {   // the tiles of this block's next chunk, on their way to L2
+      const int nc = cid + gridDim.x, nh = nc % p.H, nrow = (nc / p.H) * C;
+      tma_prefetch_l2_3d(&p.mg, 0, nh, nrow); tma_prefetch_l2_3d(&p.mg, 64, nh, nrow);
+      tma_prefetch_l2_3d(&p.mq, 0, nh, nrow); tma_prefetch_l2_3d(&p.mq, 64, nh, nrow);
+      tma_prefetch_l2_3d(&p.mk, 0, nh, nrow); tma_prefetch_l2_3d(&p.mk, 64, nh, nrow);
+    }
     if (tid == 0) {
       tma_store_wait_read();   // the previous chunk's tiles have been read
       mbar_expect_tx(&sh.bar_load, 3 * TILE64);
@@ -339,7 +368,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_kda_prep(const __grid_constant_
 //   warp 20      one thread issues every product and the stores of h' and v' for a backward pass
 //   warp 21      one thread issues the loads, two chunks ahead
 // A form with everything of a chunk in one chain (four dependent product rounds and the inversion) took 10.4 us a
-// chunk; this one FWD_US.
+// chunk; this one takes 3.3.
 struct KdaScanFwdParams {
   CUtensorMap mv, mvn, mst;     // v; v' [B*T,H,128] and h' [B*NT*H*128, 128] (TMA stores, only when kept)
   const uint8_t* prep;

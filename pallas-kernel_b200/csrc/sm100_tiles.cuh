@@ -20,9 +20,9 @@ constexpr uint32_t SLAB64 = 64 * 128;        // bytes of a 64-row slab
 constexpr uint32_t TILE64 = 2 * SLAB64;      // 64 x 128 bf16 tile
 constexpr uint32_t TILE128 = 2 * 128 * 128;  // 128 x 128 bf16 tile
 
-__device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
-  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
-}
+// (an offset from p, not a cast through an integer: the compiler has to see that the result is shared memory, or every
+// access to the tiles becomes a generic one)
+__device__ __forceinline__ uint8_t* align1024(uint8_t* p) { return p + ((1024u - (smem_u32(p) & 1023u)) & 1023u); }
 __device__ __forceinline__ float ld_bf16(const uint8_t* tile, uint32_t off) {
   return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + off));
 }
