@@ -960,13 +960,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_kda_bwd_out(const __grid_consta
   uint8_t* ks = qs + TILE64;           // k -> k~ in place
   uint8_t* gs = ks + TILE64;           // g
   uint8_t* khs = gs + TILE64;          // beta k^
-  uint8_t* dos = khs + TILE64;         // do
-  uint8_t* vns = dos + TILE64;         // v'
-  uint8_t* nrs = vns + TILE64;         // -dR
-  uint8_t* hs = nrs + TILE64;          // h' (128 x 128)
+  uint8_t* drs = khs + TILE64;         // do and -dR as one tile of 128 rows: they meet the same h'
+  uint8_t* vns = drs + 2 * TILE64;     // v'
+  uint8_t* hs = vns + TILE64;          // h' (128 x 128)
   uint8_t* dhs = hs + TILE128;         // dh^ (128 x 128)
-  uint8_t* dSs = dhs + TILE128;        // dS (64 x 64)
-  uint8_t* dLs = dSs + SLAB64;         // dL (64 x 64)
+  uint8_t* dSs = dhs + TILE128;        // dS (64 x 64) and below it dL: a slab of 128 rows that meets the same k~
+  uint8_t* dLs = dSs + SLAB64;
   uint8_t* mtm = dLs + SLAB64;         // TRI_MID pattern, rows repeated to 128
   // every barrier completes once per chunk (parity it & 1)
   __shared__ uint64_t bar_g, bar_qk, bar_rest, bar_e, bar_main;
@@ -975,7 +974,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_kda_bwd_out(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, seg = warp >> 2, col = q4 * 32 + lane;
   const int nit = (p.total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  constexpr uint32_t cE = 0, cET = 128, cdq = 192, cdki = 256, cdkr = 320, cdkb = 384;
+  constexpr uint32_t cE = 0, cET = 128, cdq = 192, cdkb = 256, cdki = 320, cdkr = 384;   // dq~ and dk^b side by side
   auto chunk_rows = [&](int it, int& h, int& row, int& hrow) {
     const int cid = blockIdx.x + it * gridDim.x;
     const int ci = (cid / p.H) % p.NT, b = cid / (p.H * p.NT);
@@ -1006,9 +1005,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_kda_bwd_out(const __grid_consta
     int h, row, hrow;
     chunk_rows(it, h, row, hrow);
     mbar_expect_tx(&bar_rest, 3 * TILE64 + 2 * TILE128 + 2 * SLAB64);
-    tma_load_3d(dos, &p.mdo, &bar_rest, 0, h, row); tma_load_3d(dos + SLAB64, &p.mdo, &bar_rest, 64, h, row);
+    tma_load_3d(drs, &p.mdo, &bar_rest, 0, h, row); tma_load_3d(drs + 2 * SLAB64, &p.mdo, &bar_rest, 64, h, row);
     tma_load_3d(vns, &p.mvn, &bar_rest, 0, h, row); tma_load_3d(vns + SLAB64, &p.mvn, &bar_rest, 64, h, row);
-    tma_load_3d(nrs, &p.mndr, &bar_rest, 0, h, row); tma_load_3d(nrs + SLAB64, &p.mndr, &bar_rest, 64, h, row);
+    tma_load_3d(drs + SLAB64, &p.mndr, &bar_rest, 0, h, row); tma_load_3d(drs + 3 * SLAB64, &p.mndr, &bar_rest, 64, h, row);
     tma_load_2d(hs, &p.mh, &bar_rest, 0, hrow); tma_load_2d(hs + TILE128 / 2, &p.mh, &bar_rest, 64, hrow);
     tma_load_2d(dhs, &p.mdh, &bar_rest, 0, hrow); tma_load_2d(dhs + TILE128 / 2, &p.mdh, &bar_rest, 64, hrow);
     tma_load_3d(dSs, &p.mdS, &bar_rest, 0, h, row);
@@ -1101,14 +1100,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_kda_bwd_out(const __grid_consta
     if (!ok) { fail(6); break; }
     if (tid == 0) {
       tc_fence_after();
-      const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), kha = smem_u32(khs), doa = smem_u32(dos), vna = smem_u32(vns),
-                     nra = smem_u32(nrs), ha = smem_u32(hs), dha = smem_u32(dhs), dSa = smem_u32(dSs), dLa = smem_u32(dLs);
+      const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), kha = smem_u32(khs), dra = smem_u32(drs), vna = smem_u32(vns),
+                     ha = smem_u32(hs), dha = smem_u32(dhs), dSa = smem_u32(dSs), dLa = smem_u32(dLs);
 #pragma unroll
-      for (int k0 = 0; k0 < D; k0 += 16)   // dq~^T[k][i] = h' do^T
-        umma_bf16(tm + cdq, desc_kmajor(ha, 128, 0, k0), desc_kmajor(doa, 64, 0, k0), umma_idesc(128, 64, 0, 0), k0 > 0);
+      for (int k0 = 0; k0 < D; k0 += 16)   // dq~^T[k][i] = h' do^T;  dk^b^T[k][j] = h' (-dR)^T
+        umma_bf16(tm + cdq, desc_kmajor(ha, 128, 0, k0), desc_kmajor(dra, 128, 0, k0), umma_idesc(128, 128, 0, 0), k0 > 0);
 #pragma unroll
-      for (int k0 = 0; k0 < C; k0 += 16)   // dq~^T[k][i] += sum_j k~[j][k] dS[i][j]
-        umma_bf16(tm + cdq, desc_mnmajor(ka, 64, k0, 0), desc_kmajor(dSa, 64, 0, k0), umma_idesc(128, 64, 1, 0), 1);
+      for (int k0 = 0; k0 < C; k0 += 16)   // dq~^T[k][i] += sum_j k~[j][k] dS[i][j];  dk^b^T[k][j] += sum_i k~[i][k] dL[j][i]
+        umma_bf16(tm + cdq, desc_mnmajor(ka, 64, k0, 0), desc_kmajor(dSa, 128, 0, k0), umma_idesc(128, 128, 1, 0), 1);
 #pragma unroll
       for (int k0 = 0; k0 < D; k0 += 16)   // dk~_inter^T[k][j] = dh^ v'^T
         umma_bf16(tm + cdki, desc_kmajor(dha, 128, 0, k0), desc_kmajor(vna, 64, 0, k0), umma_idesc(128, 64, 0, 0), k0 > 0);
@@ -1118,12 +1117,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_kda_bwd_out(const __grid_consta
 #pragma unroll
       for (int k0 = 0; k0 < C; k0 += 16)   // dk~_rest^T[k][j] += sum_i (beta k^)[i][k] dL[i][j]
         umma_bf16(tm + cdkr, desc_mnmajor(kha, 64, k0, 0), desc_mnmajor(dLa, 64, k0, 0), umma_idesc(128, 64, 1, 1), 1);
-#pragma unroll
-      for (int k0 = 0; k0 < D; k0 += 16)   // dk^b^T[k][j] = h' (-dR)^T
-        umma_bf16(tm + cdkb, desc_kmajor(ha, 128, 0, k0), desc_kmajor(nra, 64, 0, k0), umma_idesc(128, 64, 0, 0), k0 > 0);
-#pragma unroll
-      for (int k0 = 0; k0 < C; k0 += 16)   // dk^b^T[k][j] += sum_i k~[i][k] dL[j][i]
-        umma_bf16(tm + cdkb, desc_mnmajor(ka, 64, k0, 0), desc_kmajor(dLa, 64, 0, k0), umma_idesc(128, 64, 1, 0), 1);
       umma_commit(&bar_main);
     }
     __syncwarp();
