@@ -177,10 +177,11 @@ typedef struct {
   float* A_out;
   void* h_out;
   /* Optional scratch kept for the backward call of the same problem:
-   * tops_b200_chunk_saved_bytes of it.  Its content is private to the
-   * kernel family that ran (the tcgen05 kernels store pre-scaled bf16 states);
-   * hand it to tops_b200_chunk_gla_bwd as `h_saved` only when
-   * tops_b200_chunk_selected_impl reports TOPS_IMPL_SM100 for the problem. */
+   * tops_b200_chunk_saved_bytes of it, 16-byte aligned.  Its content is private to the
+   * kernel family that ran (the tcgen05 kernels store pre-scaled bf16 states, the
+   * CUDA-core kernels fp32 states and cumulated gates); hand it to
+   * tops_b200_chunk_gla_bwd of the same problem as `h_saved`.  Ignored where
+   * tops_b200_chunk_saved_bytes is 0. */
   void* saved_out;
   /* Optional (tcgen05 path, few (batch, head) pairs): the workspace a `tops_b200_chunk_state_exchange_pack`
    * call (reverse = 0) on this same problem left behind.  It holds the time segments' summaries, so the
@@ -259,7 +260,7 @@ typedef struct {
   void* dg;
   float* dh0; /* NULL unless h0 given and wanted */
   /* Optional: the `saved_out` scratch written by the forward call on the same
-   * inputs (tcgen05 path only).  When given the backward skips recomputing the
+   * inputs.  When given the backward skips recomputing the
    * chunk-start states; NULL recomputes (the reference always recomputes,
    * `tops/cpu/ops/gla/chunk.py:551-561`). */
   const void* h_saved;

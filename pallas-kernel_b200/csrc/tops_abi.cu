@@ -179,8 +179,29 @@ extern "C" int tops_b200_chunk_selected_impl(const tops_chunk_problem* pb) {
   return family(*pb) == FAMILY_GENERIC ? TOPS_IMPL_GENERIC : TOPS_IMPL_SM100;
 }
 
+// What the CUDA-core forward keeps for its backward: the chunk-start states and the cumulated gates, which the backward
+// would compute again bit for bit (fp32 only: it wants fp32 states, the forward of the other types rounds them).  Not
+// where the states take more room than q, k, v and g together (K V / C > 2 (K + V)): held from a forward to its backward
+// they would then more than double what a training step holds.  K = V = 64, chunk 16 is on the line.
+// fp32 forward + backward at B = 2, T = 2048, H = 4, K = V = 64: 241 -> 197 us.
+struct GenericSaved {
+  float *h, *gcum;
+  size_t bytes;
+};
+static GenericSaved generic_saved(const tops_chunk_problem& pb, const void* base) {
+  GenericSaved r{};
+  if (pb.dtype != TOPS_F32 || (size_t)pb.K * pb.V > 2 * (size_t)pb.chunk * (pb.K + pb.V)) return r;
+  Carver cv(const_cast<void*>(base));
+  r.h = cv.take<float>(state_elems(pb));
+  const size_t ge = gate_elems(pb);
+  if (ge) r.gcum = cv.take<float>(ge);
+  r.bytes = cv.off;
+  return r;
+}
+
 extern "C" size_t tops_b200_chunk_saved_bytes(const tops_chunk_problem* pb) {
-  if (!pb || check_problem(*pb) || family(*pb) == FAMILY_GENERIC) return 0;
+  if (!pb || check_problem(*pb)) return 0;
+  if (family(*pb) == FAMILY_GENERIC) return generic_saved(*pb, nullptr).bytes;
   return sm100::gen_saved_bytes(*pb);   // (the two forms keep the same tiles)
 }
 
@@ -282,10 +303,12 @@ static size_t fwd_layout(const tops_chunk_fwd_params* p, void* ws, cudaStream_t 
   int rc = make_problem(p->pb, cv, st, pb, launch);
   if (rc_out) *rc_out = rc;
   size_t ge = gate_elems(p->pb);
-  float* g = (p->g_cumsum_out || ge == 0) ? p->g_cumsum_out : cv.take<float>(ge);
-  if (p->g_cumsum_out == nullptr && ge != 0 && ws == nullptr) g = nullptr;
-  char* hh = p->h_out ? reinterpret_cast<char*>(p->h_out)
-                      : reinterpret_cast<char*>(cv.take<char>(state_elems(p->pb) * dtype_size(p->pb.dtype)));
+  const GenericSaved kept = p->saved_out ? generic_saved(p->pb, p->saved_out) : GenericSaved{};
+  float* own_g = p->g_cumsum_out ? p->g_cumsum_out : kept.gcum;
+  float* g = (own_g || ge == 0) ? own_g : cv.take<float>(ge);
+  if (own_g == nullptr && ge != 0 && ws == nullptr) g = nullptr;
+  char* own_h = reinterpret_cast<char*>(p->h_out ? p->h_out : kept.h);
+  char* hh = own_h ? own_h : cv.take<char>(state_elems(p->pb) * dtype_size(p->pb.dtype));
   float* sc = cv.take<float>(generic::scan_scratch_floats(*pb, p->pb.dtype == TOPS_F32));
   if (gcum) *gcum = g;
   if (h) *h = hh;
@@ -330,6 +353,13 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
     pb.gcum = reinterpret_cast<const float*>(p->g);
   }
   if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, h, p->pb.dtype == TOPS_F32, p->ht, scratch, st))) return rc;
+  if (p->saved_out) {   // (a caller that asked for them as outputs too gets both)
+    const GenericSaved kept = generic_saved(p->pb, p->saved_out);
+    if (kept.h && h != kept.h)
+      TOPS_CUDA_OK(cudaMemcpyAsync(kept.h, h, state_elems(p->pb) * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (kept.gcum && gcum != kept.gcum)
+      TOPS_CUDA_OK(cudaMemcpyAsync(kept.gcum, gcum, gate_elems(p->pb) * sizeof(float), cudaMemcpyDeviceToDevice, st));
+  }
   int round_A = p->pb.gate_kind == TOPS_GATE_PER_CHANNEL || p->pb.gate_kind == TOPS_GATE_NONE;
   return generic::launch_fwd_o(pb, p->q, p->k, p->v, h, 0, p->o, p->A_out, round_A, st);
 }
@@ -380,6 +410,7 @@ struct BwdLayout {
   size_t dg_stride;
   int tilesK;
   float* scratch;
+  bool kept;        // gcum and h are the forward's
 };
 
 static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t st, bool launch, Problem* pb,
@@ -389,9 +420,11 @@ static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t 
   if (rc_out) *rc_out = rc;
   BwdLayout l{};
   size_t ge = gate_elems(p->pb);
-  l.gcum = ge ? cv.take<float>(ge) : nullptr;
   size_t se = state_elems(p->pb);
-  l.h = cv.take<float>(se);
+  const GenericSaved kept = p->h_saved ? generic_saved(p->pb, p->h_saved) : GenericSaved{};
+  l.kept = kept.h != nullptr;
+  l.gcum = l.kept ? kept.gcum : ge ? cv.take<float>(ge) : nullptr;
+  l.h = l.kept ? kept.h : cv.take<float>(se);
   l.dh = cv.take<float>(se);
   size_t ae = (size_t)pb->total_chunks * p->pb.H * p->pb.chunk * p->pb.chunk;
   l.A = cv.take<float>(ae);
@@ -436,12 +469,12 @@ extern "C" int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* wor
   const int kind = p->pb.gate_kind;
   if (kind == TOPS_GATE_PER_CHANNEL || kind == TOPS_GATE_SCALAR) {
     int D = kind == TOPS_GATE_PER_CHANNEL ? p->pb.K : 1;
-    if ((rc = generic::launch_cumsum(pb.m, pb.H, D, p->pb.gate_dtype, 0, p->g, L.gcum, pb.total_chunks, st))) return rc;
+    if (!L.kept && (rc = generic::launch_cumsum(pb.m, pb.H, D, p->pb.gate_dtype, 0, p->g, L.gcum, pb.total_chunks, st))) return rc;
     pb.gcum = L.gcum;
   } else if (kind == TOPS_GATE_GAMMA) {
     pb.gcum = reinterpret_cast<const float*>(p->g);
   }
-  if ((rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, L.h, 1, nullptr, L.scratch, st))) return rc;
+  if (!L.kept && (rc = generic::launch_scan(pb, false, p->k, p->v, p->h0, L.h, 1, nullptr, L.scratch, st))) return rc;
   if ((rc = generic::launch_scan(pb, true, p->q, p->do_, p->dht, L.dh, 1, p->dh0, L.scratch, st))) return rc;
   BwdBuffers b{};
   b.q = p->q; b.k = p->k; b.v = p->v; b.do_ = p->do_; b.A = L.A; b.dA = L.dA; b.h = L.h; b.dh = L.dh;

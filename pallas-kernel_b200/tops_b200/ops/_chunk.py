@@ -116,7 +116,8 @@ def chunk_bwd_call(q, k, v, gate, gate_kind, scale, h0, do, dht, chunk, grad_dty
     p.dg_dtype = L.dtype_code(dg_dtype)
     if h_saved is not None:
         assert h_saved.dtype == q.dtype
-        p.h_saved = L.ptr(h_saved)
+        if fast:   # (chunk_fwd_call returns none of the other family's)
+            p.h_saved = L.ptr(h_saved)
     if rev_segments is not None and fast:
         p.rev_segments = L.ptr(rev_segments)
     ws = L.workspace(L.lib.tops_b200_chunk_bwd_workspace_bytes(C.byref(p)), dev)
