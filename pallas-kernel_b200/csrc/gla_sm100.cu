@@ -23,8 +23,8 @@
 //   k_fwd_fused    the forward scan and the outputs in one pass, state kept on chip
 //   k_bwd_main     dA, dv, dq, dk, dg of one chunk from q, k, v, g, do, h'_c, dh'_c
 //   k_join_segments  chains the time segments a sequence is cut into when there are few sequences
-// A forward is k_fwd_fused when there are enough (batch, head, segment) blocks to fill the GPU,
-// else k_scan<false> + k_fwd_o; a backward is k_scan<true> + k_bwd_main (and k_scan<false> first
+// A forward is k_fwd_fused when there are enough (batch, head, segment) blocks to fill the GPU (always in the general
+// form), else k_scan<false> + k_fwd_o; a backward is k_scan<true> + k_bwd_main (and k_scan<false> first
 // when the caller did not keep the forward's states).
 // G is the chunk-local cumulative gate and q~ = q exp(G - mid),
 // k~ = k exp(mid - G), mid = (G_0 + G_n) / 2 per channel.  The cumulative
@@ -67,6 +67,13 @@ namespace {
 //     while they are gated (the products of the gated bf16 operands lose about 2^-9 |q| |k|, which is all there is of a
 //     diagonal entry where q_i and k_i are nearly orthogonal; the output of a sequence's first token is that entry
 //     times v, and an output norm divides by it).
+//   * q~, k~, A and dA are two bf16 halves each (hi + lo, 16 bits) and a product of two of them is hi hi + hi lo + lo hi,
+//     as is the gated x of a summary scan: the CUDA-core kernels these calls ran on before keep A and dA in fp32, and
+//     with single halves o was 3.23e-3 from the fp64 result where it had been 2.82e-3 (now 1.87e-3; dq 2.87e-3, 2.28e-3,
+//     1.77e-3).  The second halves take the room of the second h' tile (forward) and of the second q, k slot and the
+//     consumed gate tile (backward), so a chunk is gated after the one before has been written out: 16384 tokens in 13
+//     documents, H = 16, forward 125 -> 181 us, chunk gradients 314 -> 350 us.  Not where K = V = 128 and all chunks are
+//     whole: those calls have had single halves all along.
 //   * channels beyond K or V are zero-filled by TMA; the state tiles in scratch are always 128 x 128.
 //   * V > 128 runs as VS slices of 128 value channels that share q, k and g.
 //   * packed batches find their segments and chunks in tables that k_plan writes.
@@ -2187,8 +2194,10 @@ namespace {
 
 // Time (us) of a pass over runs of chunks, one block per SM: a block costs `fixed` (its first loads, tensor memory, the
 // states in and out) plus `per` a chunk; when there are more blocks than SMs they follow one another, longest first,
-// and the last ones to finish leave some imbalance.  Measured: fused forward 28 us for runs of 6 chunks, 212 us for 64;
-// summary scan 18 us for 6, 1.1 us a chunk.
+// and the last ones to finish leave some imbalance.  The constants are those of operands in single halves (fused forward
+// 28 us for runs of 6 chunks, 212 us for 64; summary scan 18 us for 6, 1.1 us a chunk).  With two halves they are 11 + 4.7
+// a chunk and 8.5 + 1.75, but all passes grew alike: plans made with those, and with the scan's own in the backward, were
+// no faster (13 documents, H = 16: scans and fused forward 357 -> 364 us; 30 documents, H = 4: forward 84 -> 89 us).
 struct RunCost { long long chunks = 0; int blocks = 0, longest = 0; };
 double pass_time(const RunCost& r, int sms, double fixed, double per) {
   if (!r.blocks) return 0.0;
