@@ -180,8 +180,10 @@ typedef struct {
    * tops_b200_chunk_saved_bytes of it, 16-byte aligned.  Its content is private to the
    * kernel family that ran (the tcgen05 kernels store pre-scaled bf16 states, the
    * CUDA-core kernels fp32 states and cumulated gates); hand it to
-   * tops_b200_chunk_gla_bwd of the same problem as `h_saved`.  Ignored where
-   * tops_b200_chunk_saved_bytes is 0. */
+   * tops_b200_chunk_gla_bwd of the same problem as `h_saved`, with the same size in `saved_bytes`.
+   * Ignored (nothing is kept, the backward computes it again) where tops_b200_chunk_saved_bytes is 0 and where
+   * `saved_bytes` is less than it.  A `saved_bytes` of 0 states no size: it is taken to be B*NT*H*K*V bf16, and the
+   * scratch is used only where that is what is needed (K = V = 128, T a multiple of the chunk, dense). */
   void* saved_out;
   /* Optional (tcgen05 path, few (batch, head) pairs): the workspace a `tops_b200_chunk_state_exchange_pack`
    * call (reverse = 0) on this same problem left behind.  It holds the time segments' summaries, so the
@@ -191,6 +193,7 @@ typedef struct {
    * output of one projection); 0: contiguous tensors.  tcgen05 kernels only (TOPS_E_UNSUPPORTED otherwise); a multiple
    * of 8, every pointer 16-byte aligned. */
   int64_t pitch;
+  size_t saved_bytes; /* behind saved_out */
 } tops_chunk_fwd_params;
 /* Which kernel family TOPS_IMPL_AUTO resolves to for this problem on the current device. */
 int tops_b200_chunk_selected_impl(const tops_chunk_problem* pb);
@@ -270,6 +273,7 @@ typedef struct {
   void* rev_segments;
   int64_t pitch;      /* of q, k, v: see tops_chunk_fwd_params */
   int64_t grad_pitch; /* the same for dq, dk and dv */
+  size_t saved_bytes; /* behind h_saved: see saved_out of tops_chunk_fwd_params */
 } tops_chunk_bwd_params;
 size_t tops_b200_chunk_bwd_workspace_bytes(const tops_chunk_bwd_params* p);
 int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* workspace, size_t workspace_bytes,

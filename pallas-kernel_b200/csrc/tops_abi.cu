@@ -205,6 +205,22 @@ extern "C" size_t tops_b200_chunk_saved_bytes(const tops_chunk_problem* pb) {
   return sm100::gen_saved_bytes(*pb);   // (the two forms keep the same tiles)
 }
 
+// Whether the scratch kept for a backward can be used: it holds what the problem's kernels store.  (No size stated: a
+// caller that knows of the plain tcgen05 form only, whose tiles are what B*NT*H*K*V elements hold.)
+static bool saved_fits(const tops_chunk_problem& pb, size_t bytes) {
+  if (!bytes) return pb.impl != TOPS_IMPL_GENERIC && sm100::supported(pb);
+  const size_t need = tops_b200_chunk_saved_bytes(&pb);
+  return need && bytes >= need;
+}
+static tops_chunk_fwd_params usable(tops_chunk_fwd_params p) {
+  if (p.saved_out && !saved_fits(p.pb, p.saved_bytes)) p.saved_out = nullptr;
+  return p;
+}
+static tops_chunk_bwd_params usable(tops_chunk_bwd_params p) {
+  if (p.h_saved && !saved_fits(p.pb, p.saved_bytes)) p.h_saved = nullptr;
+  return p;
+}
+
 extern "C" int tops_b200_device_error(int* out) {
   if (!out) return TOPS_E_NULL;
   int a = 0, b = 0;
@@ -318,6 +334,8 @@ static size_t fwd_layout(const tops_chunk_fwd_params* p, void* ws, cudaStream_t 
 
 extern "C" size_t tops_b200_chunk_fwd_workspace_bytes(const tops_chunk_fwd_params* p) {
   if (!p || check_problem(p->pb)) return 0;
+  const tops_chunk_fwd_params checked = usable(*p);
+  p = &checked;
   const Family f = family(*p);
   if (f == FAMILY_PLAIN) return sm100::fwd_workspace_bytes(*p);
   if (f == FAMILY_GENERAL) return sm100::gen_fwd_workspace_bytes(*p);
@@ -330,6 +348,8 @@ extern "C" int tops_b200_chunk_gla_fwd(const tops_chunk_fwd_params* p, void* wor
   if (!p || !p->q || !p->k || !p->v || !p->o) return TOPS_E_NULL;
   int rc = check_problem(p->pb);
   if (rc) return rc;
+  const tops_chunk_fwd_params checked = usable(*p);
+  p = &checked;
   if (p->pb.gate_kind != TOPS_GATE_NONE && !p->g) return TOPS_E_NULL;
   if (p->pb.impl == TOPS_IMPL_SM100 && !sm100::supported(p->pb)) return TOPS_E_UNSUPPORTED;
   if (!workspace || workspace_bytes < tops_b200_chunk_fwd_workspace_bytes(p)) return TOPS_E_WORKSPACE;
@@ -439,6 +459,8 @@ static size_t bwd_layout(const tops_chunk_bwd_params* p, void* ws, cudaStream_t 
 
 extern "C" size_t tops_b200_chunk_bwd_workspace_bytes(const tops_chunk_bwd_params* p) {
   if (!p || check_problem(p->pb)) return 0;
+  const tops_chunk_bwd_params checked = usable(*p);
+  p = &checked;
   const Family f = family(*p);
   if (f == FAMILY_PLAIN) return sm100::bwd_workspace_bytes(*p);
   if (f == FAMILY_GENERAL) return sm100::gen_bwd_workspace_bytes(*p);
@@ -451,6 +473,8 @@ extern "C" int tops_b200_chunk_gla_bwd(const tops_chunk_bwd_params* p, void* wor
   if (!p || !p->q || !p->k || !p->v || !p->do_ || !p->dq || !p->dk || !p->dv) return TOPS_E_NULL;
   int rc = check_problem(p->pb);
   if (rc) return rc;
+  const tops_chunk_bwd_params checked = usable(*p);
+  p = &checked;
   if (p->pb.gate_kind != TOPS_GATE_NONE && !p->g) return TOPS_E_NULL;
   if (!valid_dtype(p->grad_dtype)) return TOPS_E_BAD_DTYPE;
   if (p->pb.impl == TOPS_IMPL_SM100 && !sm100::supported(p->pb)) return TOPS_E_UNSUPPORTED;

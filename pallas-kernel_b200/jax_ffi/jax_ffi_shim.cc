@@ -44,7 +44,7 @@ tops_chunk_problem problem(const ffi::AnyBuffer& q, const ffi::AnyBuffer& v, con
 }
 
 // chunk_gla / chunk_simple_gla forward: (q, k, v, g, h0) -> (o, ht, saved)
-// `saved` is the residual the backward takes back ([B,NT,H,K,V] in q's dtype).
+// `saved` is the residual the backward takes back: bytes, at least tops_b200_chunk_saved_bytes of them.
 ffi::Error ChunkFwd(cudaStream_t stream, ffi::ScratchAllocator scratch, ffi::AnyBuffer q, ffi::AnyBuffer k,
                     ffi::AnyBuffer v, ffi::AnyBuffer g, ffi::AnyBuffer h0, ffi::Result<ffi::AnyBuffer> o,
                     ffi::Result<ffi::AnyBuffer> ht, ffi::Result<ffi::AnyBuffer> saved, float scale, int32_t chunk) {
@@ -54,7 +54,9 @@ ffi::Error ChunkFwd(cudaStream_t stream, ffi::ScratchAllocator scratch, ffi::Any
   p.h0 = reinterpret_cast<const float*>(h0.untyped_data());
   p.o = o->untyped_data();
   p.ht = reinterpret_cast<float*>(ht->untyped_data());
-  if (tops_b200_chunk_selected_impl(&p.pb) == TOPS_IMPL_SM100) p.saved_out = saved->untyped_data();
+  p.saved_bytes = saved->size_bytes();
+  if (p.saved_bytes < tops_b200_chunk_saved_bytes(&p.pb)) return ffi::Error::InvalidArgument("tops_b200: residual buffer too small");
+  if (p.saved_bytes) p.saved_out = saved->untyped_data();
   const size_t n = tops_b200_chunk_fwd_workspace_bytes(&p);
   auto ws = scratch.Allocate(n);
   if (!ws.has_value()) return ffi::Error::Internal("tops_b200: no scratch memory");
@@ -78,7 +80,9 @@ ffi::Error ChunkBwd(cudaStream_t stream, ffi::ScratchAllocator scratch, ffi::Any
   p.dh0 = reinterpret_cast<float*>(dh0->untyped_data());
   p.grad_dtype = dtype_code(dq->element_type());
   p.dg_dtype = dtype_code(dg->element_type());
-  if (tops_b200_chunk_selected_impl(&p.pb) == TOPS_IMPL_SM100) p.h_saved = saved.untyped_data();
+  p.saved_bytes = saved.size_bytes();
+  if (p.saved_bytes < tops_b200_chunk_saved_bytes(&p.pb)) return ffi::Error::InvalidArgument("tops_b200: residual buffer too small");
+  if (p.saved_bytes) p.h_saved = saved.untyped_data();
   const size_t n = tops_b200_chunk_bwd_workspace_bytes(&p);
   auto ws = scratch.Allocate(n);
   if (!ws.has_value()) return ffi::Error::Internal("tops_b200: no scratch memory");

@@ -60,13 +60,15 @@ class BwdDhParams(C.Structure):
 
 class ChunkFwdParams(C.Structure):
     _fields_ = [("pb", ChunkProblem), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("h0", _vp), ("o", _vp),
-                ("ht", _vp), ("g_cumsum_out", _vp), ("A_out", _vp), ("h_out", _vp), ("saved_out", _vp), ("segments", _vp), ("pitch", _i64)]
+                ("ht", _vp), ("g_cumsum_out", _vp), ("A_out", _vp), ("h_out", _vp), ("saved_out", _vp), ("segments", _vp), ("pitch", _i64),
+                ("saved_bytes", _sz)]
 
 
 class ChunkBwdParams(C.Structure):
     _fields_ = [("pb", ChunkProblem), ("q", _vp), ("k", _vp), ("v", _vp), ("g", _vp), ("h0", _vp), ("do_", _vp),
                 ("dht", _vp), ("dq", _vp), ("dk", _vp), ("grad_dtype", _i32), ("dv", _vp), ("dg", _vp),
-                ("dh0", _vp), ("h_saved", _vp), ("dg_dtype", _i32), ("rev_segments", _vp), ("pitch", _i64), ("grad_pitch", _i64)]
+                ("dh0", _vp), ("h_saved", _vp), ("dg_dtype", _i32), ("rev_segments", _vp), ("pitch", _i64), ("grad_pitch", _i64),
+                ("saved_bytes", _sz)]
 
 
 class RecurrentFwdParams(C.Structure):

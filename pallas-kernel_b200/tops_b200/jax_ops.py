@@ -20,17 +20,34 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _PATH = os.path.join(_HERE, "libtops_b200_jax.so")
 if not os.path.exists(_PATH):
     raise ImportError(f"{_PATH} is missing: build it with `python pallas-kernel_b200/build.py --jax`")
-ctypes.CDLL(os.path.join(_HERE, "libtops_b200.so"), mode=ctypes.RTLD_GLOBAL)
+_lib = ctypes.CDLL(os.path.join(_HERE, "libtops_b200.so"), mode=ctypes.RTLD_GLOBAL)
+_lib.tops_b200_chunk_saved_bytes.restype = ctypes.c_size_t
 _shim = ctypes.CDLL(_PATH)
 for _name in ("tops_b200_ffi_chunk_fwd", "tops_b200_ffi_chunk_bwd", "tops_b200_ffi_recurrent_step"):
     jax.ffi.register_ffi_target(_name, jax.ffi.pycapsule(getattr(_shim, _name)), platform="CUDA")
+
+
+class _ChunkProblem(ctypes.Structure):   # tops_chunk_problem of include/tops_b200.h
+    _fields_ = [(n, ctypes.c_int32) for n in ("B", "T", "H", "K", "V", "chunk", "dtype", "gate_dtype", "gate_kind", "impl")] \
+        + [("scale", ctypes.c_float), ("cu_seqlens", ctypes.c_void_p), ("cu_seqlens_host", ctypes.c_void_p), ("N", ctypes.c_int32)]
+
+
+_CODES = {"float32": 0, "bfloat16": 1, "float16": 2}   # TOPS_F32, TOPS_BF16, TOPS_F16
+
+
+def _saved_bytes(q, v, g, scale, chunk):
+    """What the kernels that serve this problem keep for its backward."""
+    B, T, H, K = q.shape
+    pb = _ChunkProblem(B, T, H, K, v.shape[-1], chunk, _CODES[jnp.dtype(q.dtype).name], _CODES[jnp.dtype(g.dtype).name],
+                       1 if len(g.shape) == 4 else 2, 0, scale)   # TOPS_GATE_PER_CHANNEL / TOPS_GATE_SCALAR, TOPS_IMPL_AUTO
+    return int(_lib.tops_b200_chunk_saved_bytes(ctypes.byref(pb)))
 
 
 def _chunk_fwd(q, k, v, g, h0, scale, chunk):
     B, T, H, K = q.shape
     V = v.shape[-1]
     out = (jax.ShapeDtypeStruct(v.shape, v.dtype), jax.ShapeDtypeStruct((B, H, K, V), jnp.float32),
-           jax.ShapeDtypeStruct((B, -(-T // chunk), H, K, V), q.dtype))
+           jax.ShapeDtypeStruct((_saved_bytes(q, v, g, scale, chunk),), jnp.uint8))
     return jax.ffi.ffi_call("tops_b200_ffi_chunk_fwd", out)(q, k, v, g, h0, scale=np.float32(scale), chunk=np.int32(chunk))
 
 

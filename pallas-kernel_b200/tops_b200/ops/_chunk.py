@@ -54,7 +54,7 @@ def chunk_fwd_call(q, k, v, gate, gate_kind, scale, h0, want_ht, chunk, cu_seqle
     fast = not extra and L.lib.tops_b200_chunk_selected_impl(C.byref(p.pb)) == L.IMPL_SM100
     if fast and want_saved:
         hs = torch.empty(L.lib.tops_b200_chunk_saved_bytes(C.byref(p.pb)) // 2, dtype=k.dtype, device=dev)
-        p.saved_out = L.ptr(hs)
+        p.saved_out, p.saved_bytes = L.ptr(hs), hs.numel() * hs.element_size()
     if fast and segments is not None:
         p.segments = L.ptr(segments)
     if cu_seqlens is not None and not fast:
@@ -117,7 +117,7 @@ def chunk_bwd_call(q, k, v, gate, gate_kind, scale, h0, do, dht, chunk, grad_dty
     if h_saved is not None:
         assert h_saved.dtype == q.dtype
         if fast:   # (chunk_fwd_call returns none of the other family's)
-            p.h_saved = L.ptr(h_saved)
+            p.h_saved, p.saved_bytes = L.ptr(h_saved), h_saved.numel() * h_saved.element_size()
     if rev_segments is not None and fast:
         p.rev_segments = L.ptr(rev_segments)
     ws = L.workspace(L.lib.tops_b200_chunk_bwd_workspace_bytes(C.byref(p)), dev)

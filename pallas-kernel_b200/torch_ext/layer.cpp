@@ -89,7 +89,7 @@ struct LayerNode : public OpNode {
       if (h0.defined()) dh0 = c.empty(h0.sizes(), at::kFloat);
       p.q = ptr(q); p.k = ptr(k); p.v = ptr(v); p.g = ptr(gk); p.h0 = ptr<float>(h0c); p.do_ = ptr(d_o); p.dht = ptr<float>(dht);
       p.dq = at_col(dY, 0); p.dk = at_col(dY, d.K); p.dv = at_col(dY, 2 * d.K); p.dg = ptr(dgk); p.dh0 = ptr<float>(dh0);
-      p.grad_dtype = p.dg_dtype = TOPS_BF16; p.h_saved = ptr(hs); p.grad_pitch = cols;
+      p.grad_dtype = p.dg_dtype = TOPS_BF16; p.h_saved = ptr(hs); p.saved_bytes = hs.nbytes(); p.grad_pitch = cols;
       Tensor ws = c.bytes(tops_b200_chunk_bwd_workspace_bytes(&p));
       check(tops_b200_chunk_gla_bwd(&p, ws.data_ptr(), (size_t)ws.numel(), c.stream()), "chunk_gla_bwd");
       check_device_word("layer backward");
@@ -238,6 +238,7 @@ std::tuple<Tensor, OptTensor> gla_layer(const Tensor& x_, const Tensor& Wq, cons
     p.q = ptr(q); p.k = ptr(k); p.v = ptr(v); p.g = ptr(gk); p.h0 = ptr<float>(h0c); p.o = ptr(o); p.ht = ptr<float>(ht);
     hs = c.empty({(int64_t)(tops_b200_chunk_saved_bytes(&p.pb) / 2)}, at::kBFloat16);
     p.saved_out = ptr(hs);
+    p.saved_bytes = hs.nbytes();
     Tensor ws = c.bytes(tops_b200_chunk_fwd_workspace_bytes(&p));
     check(tops_b200_chunk_gla_fwd(&p, ws.data_ptr(), (size_t)ws.numel(), c.stream()), "chunk_gla_fwd");
     on = c.empty({d.n, d.V}, at::kBFloat16);

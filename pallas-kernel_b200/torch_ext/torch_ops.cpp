@@ -63,6 +63,7 @@ struct ChunkNode : public OpNode {
     p.q = ptr(qc); p.k = ptr(kc); p.v = ptr(vc); p.g = ptr(gc); p.h0 = ptr<float>(h0c); p.do_ = ptr(doc); p.dht = ptr<float>(dht);
     p.dq = ptr(dq); p.dk = ptr(dk); p.dv = ptr(dv); p.dg = ptr(dg); p.dh0 = ptr<float>(dh0);
     p.grad_dtype = code_of(grad_type); p.dg_dtype = code_of(dg_type); p.h_saved = ptr(hs);
+    p.saved_bytes = hs.defined() ? hs.nbytes() : 0;
     const size_t need = tops_b200_chunk_bwd_workspace_bytes(&p);
     Tensor ws = c.bytes(need);
     check(tops_b200_chunk_gla_bwd(&p, ws.data_ptr(), (size_t)ws.numel(), c.stream()), "chunk_gla_bwd");
@@ -98,6 +99,7 @@ std::tuple<Tensor, OptTensor> chunk(const Tensor& q, const Tensor& k, const Tens
     if (n) {
       hs = c.empty({(int64_t)(n / 2)}, at::kBFloat16);
       p.saved_out = ptr(hs);
+      p.saved_bytes = hs.nbytes();
     }
   }
   if (!s.cu.empty() && tops_b200_chunk_selected_impl(&p.pb) != TOPS_IMPL_SM100) cu_dev = device_boundaries(s, p.pb, c);
