@@ -144,11 +144,15 @@ class GatedLinearAttention(nn.Module):
         if not (self.use_output_gate and self.fuse_norm_and_gate) or self.use_short_conv or self.feature_map_fn is not None \
                 or self.num_kv_groups != 1 or torch.is_autocast_enabled():
             return None
+        if (torch._C._get_tracing_state() is not None or torch.nn.modules.module._has_any_global_hook() or not self._plain()):
+            return None
         q_len = x.shape[1]
         recurrent = q_len <= 64 or self.mode == "fused_recurrent"
-        if not X.gla_layer_takes(x, self.key_dim, self.value_dim, self.gk_proj[0].weight.shape[0], self.num_heads, recurrent):
-            return None
-        if (torch._C._get_tracing_state() is not None or torch.nn.modules.module._has_any_global_hook() or not self._plain()):
+        norm = self.g_norm_swish_gate
+        low, gk = self.gk_proj
+        weights = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.g_proj.weight, low.weight, gk.weight, gk.bias,
+                   norm.weight, self.o_proj.weight)
+        if not X.gla_layer_takes(x, *weights, self.num_heads, recurrent):
             return None
         last = None
         if past_key_values is not None and self.layer_idx is not None and len(past_key_values) > self.layer_idx:
@@ -161,11 +165,8 @@ class GatedLinearAttention(nn.Module):
         if state is not None:
             want = (len(cu) - 1 if cu else x.shape[0], self.num_heads, self.head_k_dim, self.head_v_dim)
             assert state.shape == want, f"recurrent state shape {tuple(state.shape)} != expected {want}"
-        norm = self.g_norm_swish_gate
-        o, state = X.gla_layer(x, self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.g_proj.weight,
-                               self.gk_proj[0].weight, self.gk_proj[1].weight, self.gk_proj[1].bias, norm.weight, self.o_proj.weight,
-                               self.num_heads, norm.eps, float(self.gate_logit_normalizer), self.clamp_min, state, bool(use_cache),
-                               cu, recurrent)
+        o, state = X.gla_layer(x, *weights, self.num_heads, norm.eps, float(self.gate_logit_normalizer), self.clamp_min, state,
+                               bool(use_cache), cu, recurrent)
         if past_key_values is not None:
             past_key_values.update(recurrent_state=state, conv_state=None, layer_idx=self.layer_idx, offset=q_len)
         return o

@@ -30,6 +30,7 @@ def rmsnorm_gated(x, g, weight=None, eps=1e-5):
     """x * rsqrt(mean(x^2, -1) + eps) * weight * silu(g) in x's dtype (fp32 arithmetic)."""
     _check(x)
     assert g.shape == x.shape, f"g shape {tuple(g.shape)} != x shape {tuple(x.shape)}"
+    assert weight is None or weight.numel() == x.shape[-1], f"weight shape {tuple(weight.shape)} != ({x.shape[-1]},)"
     return X.rmsnorm_gated(x, g, weight, float(eps))
 
 

@@ -146,6 +146,7 @@ std::tuple<Tensor, OptTensor> gla_layer(const Tensor& x, const Tensor& Wq, const
                                         const Tensor& Wlow, const Tensor& Wgk, const Tensor& bgk, const OptTensor& norm_weight,
                                         const Tensor& Wo, int heads, double eps, double normalizer, std::optional<double> clamp,
                                         const OptTensor& state, bool want_state, std::vector<int32_t> cu, bool recurrent);
-bool gla_layer_takes(const Tensor& x, int64_t key_dim, int64_t value_dim, int64_t rank, int heads, bool recurrent);
+bool gla_layer_takes(const Tensor& x, const Tensor& Wq, const Tensor& Wk, const Tensor& Wv, const Tensor& Wg, const Tensor& Wlow,
+                     const Tensor& Wgk, const Tensor& bgk, const OptTensor& norm_weight, const Tensor& Wo, int heads, bool recurrent);
 
 }  // namespace tops_torch

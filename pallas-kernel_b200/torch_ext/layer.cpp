@@ -191,9 +191,25 @@ std::tuple<Tensor, OptTensor> prompt(const Call& c, const Dims& d, const Law& l,
 
 }  // namespace
 
-// bf16 on the GPU at sizes every kernel of the path takes
-bool gla_layer_takes(const Tensor& x, int64_t key_dim, int64_t value_dim, int64_t rank, int heads, bool recurrent) {
+// bf16 on the GPU at sizes every kernel of the path takes, and weights that fit the input and one another: nothing below
+// checks a shape, the few-row kernel reads hid columns of every row whatever a weight holds.  (What does not fit goes
+// through the modules, which refuse it by name.)
+bool gla_layer_takes(const Tensor& x, const Tensor& Wq, const Tensor& Wk, const Tensor& Wv, const Tensor& Wg, const Tensor& Wlow,
+                     const Tensor& Wgk, const Tensor& bgk, const OptTensor& nw, const Tensor& Wo, int heads, bool recurrent) {
   if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 3) return false;
+  const int64_t hid = x.size(2), key_dim = Wq.size(0), value_dim = Wv.size(0), rank = Wlow.size(0);
+  auto like = [&](const Tensor& w, at::IntArrayRef sizes) {
+    return w.scalar_type() == at::kBFloat16 && w.device() == x.device() && w.sizes() == sizes && w.is_contiguous() &&
+           (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0;
+  };
+  if (!like(Wq, {key_dim, hid}) || !like(Wk, {key_dim, hid}) || !like(Wv, {value_dim, hid}) || !like(Wg, {value_dim, hid}) ||
+      !like(Wlow, {rank, hid}) || !like(Wgk, {key_dim, rank}) || !like(bgk, {key_dim}) || !like(Wo, {hid, value_dim}))
+    return false;
+  if (key_dim % heads != 0 || value_dim % heads != 0) return false;
+  if (nw.has_value() && (nw->device() != x.device() || nw->dim() != 1 || nw->size(0) != value_dim / heads || !nw->is_contiguous() ||
+                         (reinterpret_cast<uintptr_t>(nw->data_ptr()) & 15) != 0 ||
+                         (nw->scalar_type() != at::kFloat && nw->scalar_type() != at::kBFloat16 && nw->scalar_type() != at::kHalf)))
+    return false;
   const int64_t K = key_dim / heads, V = value_dim / heads, n = x.size(0) * x.size(1);
   if (n < 1 || x.size(2) % 32 != 0 || key_dim % 8 != 0 || value_dim % 32 != 0 || rank < 8 || rank > 64 || rank % 8 != 0) return false;
   if (V % 4 != 0 || V > 1024) return false;

@@ -105,3 +105,36 @@ def test_skinny_linear(rows, K, Ns):
         # fp32 sums of K products, one rounding to bf16 (2^-9 of the value)
         bar = want.abs() * 2 ** -8 + (x.double().abs() @ W.double().abs().t()) * K * 2 ** -24
         assert ((y[:, :n].double() - want).abs() <= bar).all() and (y[:, n:] == 7).all()
+
+
+@pytest.mark.parametrize("T", [1, 70])
+@pytest.mark.parametrize("change", ["wide", "narrow", "bias", "o_proj", "k_proj", "norm"])
+def test_what_does_not_fit_is_refused(T, change):
+    """Inputs and weights whose shapes or types do not belong together go through the modules, which refuse them."""
+    from torch import nn
+    layer = _layer(512, 4)
+    hid = {"wide": 544, "narrow": 480}.get(change, 512)
+    new = lambda i, o, **kw: nn.Linear(i, o, bias=False, device="cuda", dtype=torch.bfloat16, **kw)
+    if change == "bias":
+        layer.gk_proj[1].bias.data = layer.gk_proj[1].bias.data.float()
+    elif change == "o_proj":
+        layer.o_proj = new(544, 512)
+    elif change == "k_proj":
+        layer.k_proj = new(512, 288)
+    elif change == "norm":
+        layer.g_norm_swish_gate.weight.data = torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(2, T, hid, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad(), pytest.raises((RuntimeError, AssertionError)):
+        layer(x)
+
+
+@pytest.mark.parametrize("T", [1, 70])
+def test_an_output_of_another_width(T):
+    """An output projection that widens is not the layer the one call is made for; the modules take it."""
+    layer = _layer(512, 4)
+    layer.o_proj = torch.nn.Linear(512, 96, bias=False, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(2, T, 512, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        (o, _, _), labels = _labels(lambda: layer(x))
+        want = copy.deepcopy(layer).float()(x.float())[0]
+    assert o.shape == (2, T, 96) and "lowrank_gate_fwd" not in labels and rel_l2(o, want) <= 2e-2
