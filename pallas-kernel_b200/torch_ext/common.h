@@ -66,7 +66,7 @@ inline int code_of(at::ScalarType t) {
 }
 inline int code_of(const Tensor& t) { return code_of(t.scalar_type()); }
 
-// every tensor of a call lives on the first one's GPU
+// a call runs on the first tensor's GPU; every other tensor is checked to be on a GPU
 struct Call {
   c10::Device dev;
   c10::cuda::CUDAGuard guard;
@@ -85,7 +85,12 @@ struct Call {
   Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const { return Tensor(at::detail::empty_cuda(sizes, t, dev, std::nullopt)); }
   Tensor empty_as(const Tensor& t) const { return empty(t.sizes(), t.scalar_type()); }
   Tensor bytes(size_t n) const { return empty({(int64_t)(n < 256 ? 256 : n)}, at::kByte); }
-  Tensor in(const Tensor& t) const {   // contiguous, on this GPU
+  // a tensor that is updated where it lies (fp32 and contiguous by the caller's checks)
+  float* state(const Tensor& t) const {
+    need_cuda(t);
+    return t.data_ptr<float>();
+  }
+  Tensor in(const Tensor& t) const {   // contiguous, on a GPU
     if (!t.defined()) return t;
     need_cuda(t);
     return t.is_contiguous() ? t : t.contiguous();

@@ -206,7 +206,7 @@ Tensor recurrent_decode(const Tensor& q, const Tensor& k, const Tensor& v, const
   Tensor qc = c.in(q), kc = c.in(k), vc = c.in(v), gk = c.in(gk_), gv = c.in(gv_);
   Tensor o = c.empty({q.size(0), q.size(1), q.size(2), v.size(3)}, q.scalar_type());
   tops_recurrent_fwd_params p = rec_fwd_params(qc, kc, vc, gk, gv, scale, false, q.scalar_type());
-  p.state_in = ptr<float>(state); p.state_out = ptr<float>(state); p.o = ptr(o); p.N = p.B;
+  p.state_in = p.state_out = c.state(state); p.o = ptr(o); p.N = p.B;
   check(tops_b200_fused_recurrent_gla_fwd(&p, c.stream()), "fused_recurrent_gla_fwd");
   return o;
 }
@@ -319,7 +319,7 @@ std::tuple<Tensor, OptTensor> kda(const Tensor& q, const Tensor& k, const Tensor
 Tensor kda_decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double scale,
                   const Tensor& state) {
   Call c(q);
-  return kda_run(c, c.in(q), c.in(k), c.in(v), c.in(g), c.in_as(beta, q.scalar_type()), scale, ptr<float>(state), ptr<float>(state));
+  return kda_run(c, c.in(q), c.in(k), c.in(v), c.in(g), c.in_as(beta, q.scalar_type()), scale, c.state(state), c.state(state));
 }
 
 // ---------------------------------------------------------------------------------------------------
