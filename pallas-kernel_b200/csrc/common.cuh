@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "tops_b200.h"
 
 namespace tops {
@@ -40,6 +42,7 @@ inline int post_launch(const char* where = "kernel launch") {
   return TOPS_E_CUDA;
 }
 
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 inline size_t dtype_size(int dt) { return dt == TOPS_F32 ? 4 : 2; }

@@ -671,8 +671,6 @@ unsigned norm_bwd_blocks(size_t rows, int lg) {
   return n < 148 * 4 ? n : 148 * 4;
 }
 
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
 }  // namespace
 
 int gate_check(const tops_gate_act_params& p) {

@@ -485,14 +485,13 @@ constexpr size_t BW_SMEM = sizeof(TokenTile) + (SEGMENT * 32 + 2 * 2 * 4 * 128 +
 //     p = k^T S',   r = q^T S',   e = beta (v - p),   o = scale (r + (q . k) e),   S = S' + k (x) e
 // both reductions over the keys come from one pass over the registers, so a token costs one exchange through shared
 // memory.  B = 16, H = 32, K = V = 128, one token: 73.6 -> 18.2 us (3.7 TB/s; B = 128: 93.6 us, 5.8 TB/s).
-template <int RK>
+template <int RK, bool VEC>   // VEC: the state's rows go as float4
 __global__ void __launch_bounds__(FW_THREADS) k_kda_step(tops_kda_fwd_params a) {
   __shared__ float qs[16 * RK], ks[16 * RK], egs[16 * RK];
   __shared__ float red_p[4][FW_BV], red_r[4][FW_BV], red_qk[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, vq = tid & 7, kr = tid >> 3;
   const int b = blockIdx.y / a.H, h = blockIdx.y % a.H;
   const int K = a.K, V = a.V, v0 = blockIdx.x * FW_BV, col = v0 + 4 * vq;
-  const bool vec = (V % 4) == 0;
   const size_t sbase = (size_t)blockIdx.y * K * (size_t)V;
   float S[RK][4];
 #pragma unroll
@@ -501,10 +500,10 @@ __global__ void __launch_bounds__(FW_THREADS) k_kda_step(tops_kda_fwd_params a) 
 #pragma unroll
     for (int c = 0; c < 4; ++c) S[r][c] = 0.f;
     if (a.h0 && k < K) {
-      if (vec && col < V) {
+      if (VEC && col < V) {
         const float4 x = __ldcs(reinterpret_cast<const float4*>(a.h0 + sbase + (size_t)k * V + col));
         S[r][0] = x.x; S[r][1] = x.y; S[r][2] = x.z; S[r][3] = x.w;
-      } else {
+      } else if (!VEC) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (col + c < V) S[r][c] = a.h0[sbase + (size_t)k * V + col + c];
@@ -581,9 +580,9 @@ __global__ void __launch_bounds__(FW_THREADS) k_kda_step(tops_kda_fwd_params a) 
     for (int r = 0; r < RK; ++r) {
       const int k = kr + 16 * r;
       if (k >= K) continue;
-      if (vec && col < V) {
+      if (VEC && col < V) {
         __stcs(reinterpret_cast<float4*>(a.ht + sbase + (size_t)k * V + col), make_float4(S[r][0], S[r][1], S[r][2], S[r][3]));
-      } else {
+      } else if (!VEC) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (col + c < V) a.ht[sbase + (size_t)k * V + col + c] = S[r][c];
@@ -599,9 +598,15 @@ static int launch_fwd(const tops_kda_fwd_params& p, float* seg_states, cudaStrea
   dim3 grid(cdiv(p.V, FW_BV), p.B * p.H);
   if (!seg_states && p.T <= kStepTokens && p.K <= 256) {
     KernelScope ks("kda_step", st);
-    if (p.K <= 64) k_kda_step<4><<<grid, FW_THREADS, 0, st>>>(p);
-    else if (p.K <= 128) k_kda_step<8><<<grid, FW_THREADS, 0, st>>>(p);
-    else k_kda_step<16><<<grid, FW_THREADS, 0, st>>>(p);
+    // (a state may be a view into a larger cache, on any 4-byte boundary)
+    auto launch = [&](auto rows) {
+      constexpr int RK = decltype(rows)::value;
+      if (p.V % 4 == 0 && aligned16(p.h0) && aligned16(p.ht)) k_kda_step<RK, true><<<grid, FW_THREADS, 0, st>>>(p);
+      else k_kda_step<RK, false><<<grid, FW_THREADS, 0, st>>>(p);
+    };
+    if (p.K <= 64) launch(std::integral_constant<int, 4>());
+    else if (p.K <= 128) launch(std::integral_constant<int, 8>());
+    else launch(std::integral_constant<int, 16>());
     return post_launch();
   }
   KernelScope ks("kda_recurrent_fwd", st);

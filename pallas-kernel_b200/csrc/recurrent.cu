@@ -20,7 +20,7 @@ __device__ __forceinline__ SeqRange seq_range(const int32_t* cu, int n, int T) {
 constexpr int FW_THREADS = 128;
 constexpr int FW_BV = 32;
 
-template <int RK>
+template <int RK, bool VEC>   // VEC: the state's rows go as float4
 __global__ void __launch_bounds__(FW_THREADS) k_rec_fwd(tops_recurrent_fwd_params a, long long qk_pitch, long long v_pitch) {
   __shared__ float qs[16 * RK], ks[16 * RK], eks[16 * RK];
   __shared__ float vs[FW_BV], evs[FW_BV];
@@ -30,7 +30,6 @@ __global__ void __launch_bounds__(FW_THREADS) k_rec_fwd(tops_recurrent_fwd_param
   const int v0 = blockIdx.x * FW_BV;
   const int K = a.K, V = a.V;
   const SeqRange sr = seq_range(a.cu_seqlens, n, a.T);
-  const bool vec = (V % 4) == 0;
   const size_t sbase = ((size_t)n * a.H + h) * K * (size_t)V;
   const int col = v0 + 4 * vq;
 
@@ -41,11 +40,11 @@ __global__ void __launch_bounds__(FW_THREADS) k_rec_fwd(tops_recurrent_fwd_param
 #pragma unroll
     for (int c = 0; c < 4; ++c) S[r][c] = 0.f;
     if (a.state_in && k < K) {
-      if (vec && col < V) {
+      if (VEC && col < V) {
         // the state is touched once per call: streaming loads and stores keep it from displacing the rest of L2
         float4 x = __ldcs(reinterpret_cast<const float4*>(a.state_in + sbase + (size_t)k * V + col));
         S[r][0] = x.x; S[r][1] = x.y; S[r][2] = x.z; S[r][3] = x.w;
-      } else {
+      } else if (!VEC) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (col + c < V) S[r][c] = a.state_in[sbase + (size_t)k * V + col + c];
@@ -103,10 +102,10 @@ __global__ void __launch_bounds__(FW_THREADS) k_rec_fwd(tops_recurrent_fwd_param
     for (int r = 0; r < RK; ++r) {
       int k = kr + 16 * r;
       if (k >= K) continue;
-      if (vec && col < V) {
+      if (VEC && col < V) {
         __stcs(reinterpret_cast<float4*>(a.state_out + sbase + (size_t)k * V + col),
                make_float4(S[r][0], S[r][1], S[r][2], S[r][3]));
-      } else {
+      } else if (!VEC) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (col + c < V) a.state_out[sbase + (size_t)k * V + col + c] = S[r][c];
@@ -121,9 +120,15 @@ int fwd(const tops_recurrent_fwd_params& p, cudaStream_t st) {
   KernelScope ks("recurrent_fwd", st);
   // (contiguous tensors have a pitch too: choosing in the kernel cost 0.4 us of the 94 us of a step at B = 128, H = 32)
   const long long qkp = p.pitch ? p.pitch : (long long)p.H * p.K, vp = p.pitch ? p.pitch : (long long)p.H * p.V;
-  if (p.K <= 64) k_rec_fwd<4><<<grid, FW_THREADS, 0, st>>>(p, qkp, vp);
-  else if (p.K <= 128) k_rec_fwd<8><<<grid, FW_THREADS, 0, st>>>(p, qkp, vp);
-  else if (p.K <= 256) k_rec_fwd<16><<<grid, FW_THREADS, 0, st>>>(p, qkp, vp);
+  // (a state may be a view into a larger cache, on any 4-byte boundary)
+  auto launch = [&](auto rows) {
+    constexpr int RK = decltype(rows)::value;
+    if (p.V % 4 == 0 && aligned16(p.state_in) && aligned16(p.state_out)) k_rec_fwd<RK, true><<<grid, FW_THREADS, 0, st>>>(p, qkp, vp);
+    else k_rec_fwd<RK, false><<<grid, FW_THREADS, 0, st>>>(p, qkp, vp);
+  };
+  if (p.K <= 64) launch(std::integral_constant<int, 4>());
+  else if (p.K <= 128) launch(std::integral_constant<int, 8>());
+  else if (p.K <= 256) launch(std::integral_constant<int, 16>());
   else return TOPS_E_BAD_SHAPE;
   return post_launch();
 }

@@ -152,6 +152,5 @@ inline int opt_in_smem(F f, size_t bytes) {
   return TOPS_E_CUDA;
 }
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 }  // namespace sm100
 }  // namespace tops
