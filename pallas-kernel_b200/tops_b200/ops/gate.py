@@ -33,6 +33,7 @@ def _fill(p, g, H, K, kind, A_log, dt_bias, lower_bound, normalizer, clamp_min, 
 def _check_gate(g):
     assert g.ndim >= 2, f"g must have at least 2 dims, got shape {tuple(g.shape)}"
     assert g.shape[-1] % 4 == 0, "K must be a multiple of 4"
+    assert g.shape[-1] > 0 and g.shape[-2] > 0, f"g has no heads or channels: {tuple(g.shape)}"
 
 
 def _check_params(A_log, dt_bias, H, K):

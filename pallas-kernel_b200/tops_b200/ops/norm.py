@@ -17,7 +17,7 @@ from .._lib import ops_ext as X
 
 def _check(x):
     D = x.shape[-1]
-    assert D % 4 == 0 and D <= 1024, f"last dimension must be a multiple of 4 and <= 1024, got {D}"
+    assert D % 4 == 0 and 0 < D <= 1024, f"last dimension must be a multiple of 4 and <= 1024, got {D}"
 
 
 def l2norm(x, eps=1e-6):

@@ -50,3 +50,15 @@ def test_gate_kernels(dtype, lower_bound, rows, H, K):
         got = _grads(lambda a: gla_gate(a, 16.0, None), (g.cuda(),), dy.cuda())
         for a, b in zip(got, want):
             assert_close("gla_gate", a.float().cpu(), b.float(), dtype)
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 0), (0, 3, 64), (2, 0, 64)])
+def test_tensors_without_elements_are_refused(shape):
+    """Rows of no channels, no rows, no heads: an error that can be caught, in whatever layer finds it."""
+    from tops_b200._lib import TopsError
+    from tops_b200.ops.gate import gla_gate, kda_gate_fwd
+    from tops_b200.ops.norm import l2norm, rmsnorm_gated
+    x = torch.empty(shape, device="cuda", dtype=torch.bfloat16)
+    for call in (lambda: l2norm(x), lambda: rmsnorm_gated(x, x), lambda: gla_gate(x), lambda: kda_gate_fwd(x, torch.zeros(3, device="cuda"))):
+        with pytest.raises((AssertionError, TopsError)):
+            call()
