@@ -74,6 +74,7 @@ namespace {
 //     consumed gate tile (backward), so a chunk is gated after the one before has been written out: 16384 tokens in 13
 //     documents, H = 16, forward 125 -> 181 us, chunk gradients 314 -> 350 us.  Not where K = V = 128 and all chunks are
 //     whole: those calls have had single halves all along.
+//   * the gated operands stay in range whatever the gates: see kSpan below.
 //   * channels beyond K or V are zero-filled by TMA; the state tiles in scratch are always 128 x 128.
 //   * V > 128 runs as VS slices of 128 value channels that share q, k and g.
 //   * packed batches find their segments and chunks in tables that k_plan writes.
@@ -158,6 +159,130 @@ __device__ __forceinline__ void store_state32(float* base, const float (&S)[32],
       *reinterpret_cast<float4*>(base + (size_t)row * V + c0 + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
 }
 
+// ---------------------------------------------------------------------------
+// Strong gates (general form)
+// ---------------------------------------------------------------------------
+// exp(G - mid) and exp(mid - G) leave fp32 once a channel's gates sum to some -176 over a chunk (-2.8 a token); every
+// result is finite all the same.  So the per-channel references of the stored tiles are kept within kSpan of zero,
+//     h' = h exp(ref) scale,  dh' = dh exp(refd),   ref = clamp(mid), refd = clamp(G_n - mid)
+// (the clamps are continuous: two kernels that see a mid on either side of the limit still agree), and a chunk in which
+// a clamp takes effect, a "wide" one, is gated as
+//     q~ = q exp(G - ref),  k~ = k exp(G_n - G - refd)
+// whose exponents are at most kSpan for gates that do not grow.  These k~ and q~ no longer make the intra-chunk matrix:
+// a wide chunk's A, dq_intra and dk_intra are summed pair by pair on the CUDA cores, with exp(G_i - G_j) as a product of
+// the gates between.  All of it starts from the caller's q, k and gates (in L2).  kSpan = 64 leaves operands of any
+// magnitude that fits bf16 activations a factor of 1e10 before fp32 ends.
+// Kept out of the narrow chunks' way: a forward block that meets a wide chunk walks its run once more (fused_walk), the
+// backward does the wide ones in a launch of their own (launch_bwd_main); where there are none that costs the forward 1 %
+// and the backward about 5 us.  With every chunk wide: 13 documents in T = 16384, H = 16 forward + backward 0.74 -> 12.9 ms
+// (16.8 on the CUDA-core kernels at chunk 16, which hold gates down to -11.8 a token), prompt of T = 3001 67 -> 600 us (1637).
+constexpr float kSpan = 64.f;
+// The backward takes a chunk as wide too when a channel's gates fall below -2 a token: the shares of the pairs (i, i) in
+// q dq - k dk cancel, and what the products leave of them (2^-17) is no longer small beside dg, which is e^g of them.
+__device__ __forceinline__ bool wide_span(float mid, float half, int len) {   // half: G_n - mid
+  return fabsf(mid) > kSpan || fabsf(half) > kSpan || fabsf(mid + half) > 2.f * len;
+}
+__device__ __forceinline__ float clamp_span(float x) { return fminf(fmaxf(x, -kSpan), kSpan); }
+// a chunk of one head as it lies in the caller's tensors
+struct RawChunk {
+  const __nv_bfloat16 *q, *k;   // first token, first channel
+  const __nv_bfloat16* g;       // the same; scalar gates: the first token's; null: gconst at every token
+  long long pitch, gstep;       // elements between tokens
+  float gconst;
+  int K, len;
+};
+template <bool SCALAR>
+__device__ __forceinline__ float raw_gate(const RawChunk& r, int i, int c) {
+  if (SCALAR) return r.g ? __bfloat162float(r.g[i * r.gstep]) : r.gconst;
+  return __bfloat162float(r.g[i * r.gstep + c]);
+}
+// tril(A) scale of a wide chunk as hi + lo tiles: 16 warps, warp w columns w, w + 16, w + 32, w + 48, a lane four channels
+template <bool SCALAR>
+__device__ __forceinline__ void wide_matrix(const RawChunk r, uint8_t* hi, uint8_t* lo, float scale, int warp, int lane) {
+  const int c0 = 4 * lane;
+  const bool on = c0 < r.K;   // (K is a multiple of 8)
+  float k[4][4], w[4][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int j = warp + 16 * m;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      k[m][c] = on && j < r.len ? __bfloat162float(r.k[j * r.pitch + c0 + c]) * scale : 0.f;
+      w[m][c] = 1.f;
+    }
+  }
+#pragma unroll 1
+  for (int i = 0; i < C; ++i) {
+    const bool in = on && i < r.len;
+    float q[4], eg[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      q[c] = in ? __bfloat162float(r.q[i * r.pitch + c0 + c]) : 0.f;
+      eg[c] = in ? fast_exp(raw_gate<SCALAR>(r, i, c0 + c)) : 1.f;
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int j = warp + 16 * m;
+      float a = 0.f;
+      if (i > j) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[m][c] *= eg[c];
+      }
+      if (i >= j) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a = fmaf(q[c] * k[m][c], w[m][c], a);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == m) {
+        const __nv_bfloat16 top = __float2bfloat16_rn(a);
+        const float f = __bfloat162float(top);
+        *reinterpret_cast<__nv_bfloat16*>(hi + slab_off(i, j)) = top;
+        *reinterpret_cast<__nv_bfloat16*>(lo + slab_off(i, j)) = __float2bfloat16_rn(fabsf(f) <= 3.4e38f ? a - f : 0.f);
+      }
+    }
+  }
+}
+// summed gates of channel c: before token i0, and of the whole chunk; the first token's
+struct WideSums { float before, total, first; };
+template <bool SCALAR>
+__device__ __forceinline__ WideSums wide_sums(const RawChunk& r, int c, int i0) {
+  WideSums s{0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int i = 0; i < r.len; ++i) {
+    if (i == i0) s.before = s.total;
+    s.total += raw_gate<SCALAR>(r, i, c);
+    if (i == 0) s.first = s.total;
+  }
+  return s;
+}
+// gates a wide chunk again: thread (channel, 16 time steps).  q~ only where a product needs it (qs null: not).
+template <bool SCALAR>
+__device__ __forceinline__ void wide_operands(const RawChunk r, uint8_t* qs, uint8_t* ks, uint8_t* klo, int col, int seg) {
+  const ColAddr ca = col_prep(64, col);
+  if (col >= r.K) {   // channels that do not exist: a scalar gate's infinity times their zeros is no zero
+    for (int i = seg * SEG; i < seg * SEG + SEG; ++i) {
+      *reinterpret_cast<unsigned short*>(ks + ca.at(i)) = *reinterpret_cast<unsigned short*>(klo + ca.at(i)) = 0;
+      if (qs) *reinterpret_cast<unsigned short*>(qs + ca.at(i)) = 0;
+    }
+    return;
+  }
+  const WideSums s = wide_sums<SCALAR>(r, col, seg * SEG);
+  const float mid = 0.5f * (s.first + s.total), ref = clamp_span(mid), refd = clamp_span(s.total - mid);
+  float G = s.before;
+#pragma unroll 1
+  for (int t = 0; t < SEG; ++t) {
+    const int i = seg * SEG + t;
+    if (i >= r.len) break;
+    G += raw_gate<SCALAR>(r, i, col);
+    const float k = __bfloat162float(r.k[i * r.pitch + col]) * fast_exp(s.total - G - refd);
+    const __nv_bfloat16 kh = __float2bfloat16_rn(k);
+    *reinterpret_cast<__nv_bfloat16*>(ks + ca.at(i)) = kh;
+    *reinterpret_cast<__nv_bfloat16*>(klo + ca.at(i)) = __float2bfloat16_rn(k - __bfloat162float(kh));
+    if (qs) *reinterpret_cast<__nv_bfloat16*>(qs + ca.at(i)) = __float2bfloat16_rn(__bfloat162float(r.q[i * r.pitch + col]) * fast_exp(G - ref));
+  }
+}
+
 // ===========================================================================
 // State scans
 // ===========================================================================
@@ -175,6 +300,7 @@ struct ScanParams {
   const __nv_bfloat16* gscalar;   // scalar gates [B,T,H] (SCALAR kernels; mg is unused then)
   const float* gamma;      // constant gates [H] (SCALAR GEN kernels; gscalar is null then; both null: no gate)
   Geo geo;                 // GEN kernels
+  uint8_t* wide;           // GEN reverse scan: [chunk][H][4], one byte per quarter of the channels: the chunk is wide
   int skip_xy;             // test hook: the x/y tile load of this chunk is never issued (-1: none), so that the
                            // bounded wait for it runs out and the kernel leaves through its error path
 };
@@ -461,6 +587,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) k_scan(const __grid_constant_
   auto gn_of = [&](int pp) { return SCALAR ? gn_next : sh.gn[pp & 1][col]; };   // (SCALAR: of the chunk gated last)
   auto state_scale = [&](int pp) {
     const float gnv = gn_of(pp), e0 = SCALAR ? e0_next : sh.e0[pp & 1][col];
+    if (GEN && BWD && !SUM && seg == 0 && bp.vs == 0) {
+      const unsigned any = __ballot_sync(0xffffffffu, wide_span(0.5f * (gnv + e0), 0.5f * (gnv - e0), chunk_len(pp)));
+      if (lane == 0) p.wide[((size_t)(bp.slot + chunk_of(pp)) * p.H + h) * 4 + q4] = any != 0;
+    }
+    if (GEN) return BWD ? fast_exp(clamp_span(0.5f * (gnv - e0))) : fast_exp(clamp_span(gnv - 0.5f * e0)) * p.scale;
     return BWD ? fast_exp(0.5f * (gnv - e0)) : fast_exp(gnv - 0.5f * e0) * p.scale;
   };
 
@@ -858,20 +989,24 @@ struct FusedParams {
   float scale;
   const float* gamma;      // constant gates [H] (SCALAR GEN kernel)
   Geo geo;                 // GEN kernel
+  const __nv_bfloat16 *q, *k, *g;   // GEN: what the tensor maps fetch, for wide chunks
+  long long qk_pitch;               // GEN: elements between tokens of q and k
 };
 struct FusedShared {
   uint64_t fullin[2], ebar, abar, sbar, obar;
   uint32_t tmem_slot;
   int abort_flag;
+  int wide_at[2];   // WIDE: the last wide chunk of either parity
 };
 constexpr uint32_t FUSED_STAGE = 4 * TILE64;   // q, k, g, v
 constexpr size_t FUSED_SMEM = 2 * FUSED_STAGE + 2 * TILE128 + 2 * SLAB64 + 2048 + TILE64 + sizeof(FusedShared);
 
 // SCALAR: no gate tile is fetched and no exponent product issued; every compute warp cumulates the chunk's 64
 // gates in registers (warp_cumulate), which gives its threads E of their time row, G_n and mid directly.
-template <bool SCALAR, bool GEN>
-__global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_constant__ FusedParams p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
+// WIDE: the walk over the run once more, where it has wide chunks (see kSpan): the tiles go by clamped references, and a
+// wide chunk's tril(A) and gated operands are formed by the CUDA cores.  Returns whether the run has to be walked again.
+template <bool SCALAR, bool GEN, bool WIDE>
+__device__ __forceinline__ bool fused_walk(const FusedParams& p, uint8_t* smem) {
   uint8_t* in = smem;                         // 2 stages x (q, k, g, v)
   uint8_t* hst = in + 2 * FUSED_STAGE;        // 2 x (128 x 128) bf16: h' of the current chunk
   uint8_t* qlo = hst + TILE128;               // GEN: one h' tile; what bf16 leaves of q~ (then of A) and of k~
@@ -899,10 +1034,6 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
                                                        : (p.s0 ? p.s0 + bp.seqh * K * V : nullptr);
   auto chunk_len = [&](int pp) { return GEN ? min(C, bp.end - (bp.row + pp * C)) : C; };
   constexpr uint32_t cE = 0, cD = 128, cO = 256, cA = 384, cW = 448;
-  if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
-    if (tid == 0) fail(12);
-    return;
-  }
   auto issue_load = [&](int pp) {
     uint8_t* qs = in + (pp & 1) * FUSED_STAGE;
     uint8_t *ks = qs + TILE64, *gs = ks + TILE64, *vs = gs + TILE64;
@@ -915,17 +1046,20 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
     tma_load_3d(vs, &p.mv, bar, yc, h, row); tma_load_3d(vs + SLAB64, &p.mv, bar, yc + 64, h, row);
   };
   if (tid == 0) {
+    if (WIDE)
+      for (uint64_t* bar : {&sh.fullin[0], &sh.fullin[1], &sh.ebar, &sh.abar, &sh.sbar, &sh.obar}) mbar_inval(bar);
     mbar_init(&sh.fullin[0], 1); mbar_init(&sh.fullin[1], 1);
     mbar_init(&sh.ebar, 1); mbar_init(&sh.abar, 1); mbar_init(&sh.sbar, 1); mbar_init(&sh.obar, 1);
     fence_barrier_init();
     tma_prefetch_desc(&p.mq); tma_prefetch_desc(&p.mk); tma_prefetch_desc(&p.mv);
     if (!SCALAR) tma_prefetch_desc(&p.mg);
     sh.abort_flag = 0;
+    if (WIDE) sh.wide_at[0] = sh.wide_at[1] = -1;
     issue_load(0);
     if (NT > 1) issue_load(1);
   }
   __syncwarp();
-  if (warp == 0) { tmem_alloc(&sh.tmem_slot, 512); tmem_relinquish(); }
+  if (!WIDE && warp == 0) { tmem_alloc(&sh.tmem_slot, 512); tmem_relinquish(); }
   // SCALAR: the gates of time steps lane and lane + 32 of the next chunk, in registers, loaded right after the
   // first barrier of the chunk before: a chunk is long enough here for the load to land before the loop's back
   // edge (where a register with a load in flight stalls the warp; the state scans, whose chunks are short, use
@@ -950,6 +1084,9 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
   tc_fence_after();
   const uint32_t tm = sh.tmem_slot;
   const uint32_t lane_base = q4 * 32;
+  bool wide_any = false;   // GEN: this thread has seen a wide chunk
+  // (known after B1)
+  auto wide_chunk = [&](int pp) { return WIDE && *reinterpret_cast<volatile int*>(&sh.wide_at[pp & 1]) == pp; };
 
   if (driver) {
     // ------------------------------------------------------------------ products and copies
@@ -986,13 +1123,17 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       if (lane == 0) tma_store_wait_read();
       // B1: q~, k~ and h' of chunk pp are in shared memory, E and W have been read
       if (__syncthreads_or(*abort_flag)) break;
+      const bool wide = wide_chunk(pp);
+      if (wide && __syncthreads_or(*abort_flag)) break;   // q~, k~ once more, tril(A) scale
       if (lane == 0) {
         tc_fence_after();
         const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), va = smem_u32(vs), ha = smem_u32(ht);
+        if (!wide) {
 #pragma unroll
-        for (int k0 = 0; k0 < D; k0 += 16)   // A = q~ k~^T
-          umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
-        if (GEN) {
+          for (int k0 = 0; k0 < D; k0 += 16)   // A = q~ k~^T
+            umma_bf16(tm + cA, desc_kmajor(qa, 64, 0, k0), desc_kmajor(ka, 64, 0, k0), umma_idesc(64, 64, 0, 0), k0 > 0);
+        }
+        if (GEN && !wide) {
           const uint32_t qla = smem_u32(qlo), kla = smem_u32(klo);
 #pragma unroll
           for (int k0 = 0; k0 < D; k0 += 16)
@@ -1090,6 +1231,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
       // per-channel factors of this thread's state row
       float decay, c2;
       float em[16];
+      bool wide_here = false;
       {
         float w[8];
         if (SCALAR) {
@@ -1101,8 +1243,16 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
           tmem_ld16(tmem_addr(tm, lane_base, cE + ((q4 >> 1) * 4 + seg) * 16), em);
         }
         decay = fast_exp(w[0]);                    // exp(G_n)
+        float mid = w[0] - w[1];
+        if (GEN) wide_here = fabsf(mid) > kSpan || fabsf(w[1]) > kSpan;
+        if (WIDE) {
+          mid = clamp_span(mid);
+          w[1] = clamp_span(w[1]);
+        } else {
+          wide_any |= wide_here;
+        }
         c2 = fast_exp(w[1]);                       // exp(G_n - mid)
-        const float hscale = fast_exp(w[0] - w[1]) * p.scale;   // exp(mid) scale
+        const float hscale = fast_exp(mid) * p.scale;   // exp(mid) scale
 #pragma unroll
         for (int j = 0; j < 32; j += 8)
           *reinterpret_cast<uint4*>(ht + tile_off(128, col, seg * 32 + j)) =
@@ -1175,15 +1325,27 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
         }
         if (GEN) diag[cg * C + i] = dot;
       }
+      if (WIDE && wide_here) sh.wide_at[ph] = pp;
       fence_async_smem();
       tc_fence_before();
       if (__syncthreads_or(*abort_flag)) { ok = false; break; }   // B1
       if (pp > 0) copy_out(pp - 1);   // staged before the barrier; the products of this chunk run meanwhile
       if (SCALAR && pp + 1 < NT) load_gates(pp + 1);
       // tril(A) scale -> bf16 operand in the (dead) gate tile
-      if (!mbar_wait(&sh.abar, ph)) { *abort_flag = 1; fail(4); }
-      tc_fence_after();
-      {
+      if (wide_chunk(pp)) {
+        if constexpr (WIDE) {
+          const size_t row = (size_t)bp.row + pp * C;
+          RawChunk raw{p.q + row * p.qk_pitch + (size_t)h * K, p.k + row * p.qk_pitch + (size_t)h * K, nullptr, p.qk_pitch, 0, gconst, K, len};
+          if (!SCALAR) { raw.g = p.g + (row * p.H + h) * K; raw.gstep = (long long)p.H * K; }
+          else if (p.gscalar) { raw.g = p.gscalar + row * p.H + h; raw.gstep = p.H; }
+          wide_operands<SCALAR>(raw, qs, ks, klo, col, seg);
+          wide_matrix<SCALAR>(raw, gs, qlo, p.scale, warp, lane);
+        }
+        fence_async_smem();
+        if (__syncthreads_or(*abort_flag)) { ok = false; break; }
+      } else {
+        if (!mbar_wait(&sh.abar, ph)) { *abort_flag = 1; fail(4); }
+        tc_fence_after();
         const int i = 16 * q4 + lane;   // rows of an M = 64 accumulator sit in lanes 0..15 of each quarter
         float a[16];
         tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
@@ -1226,12 +1388,30 @@ __global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_consta
     if (ok && p.s_final && bp.cnt == 1) store_state32(p.s_final + bp.seqh * K * V, S, col, yc + seg * 32, K, V);
   }
   tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tm, 512);
+  const bool again = __syncthreads_or(wide_any) != 0;
   if (tid == 0 && sh.abort_flag) {
     poison(p.o + ((size_t)bp.row * p.H + h) * V + yc);
     if (p.s_final && bp.cnt == 1) poison(p.s_final + bp.seqh * K * V + yc);
   }
+  return again && !sh.abort_flag;
+}
+// (a function of its own, so that the walk above has its registers to itself: with wide chunks taken care of inside it the
+// kernel took 193 us where it takes 184, T = 16384 in 13 documents, H = 16)
+template <bool SCALAR>
+__device__ __noinline__ void fused_walk_wide(const FusedParams& p, uint8_t* smem) { fused_walk<SCALAR, true, true>(p, smem); }
+
+template <bool SCALAR, bool GEN>
+__global__ void __launch_bounds__(FUSED_THREADS) k_fwd_fused(const __grid_constant__ FusedParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if ((smem_u32(smem) & 1023u) != 0) {   // uniform over the block
+    if (threadIdx.x == 0) fail(12);
+    return;
+  }
+  const bool again = fused_walk<SCALAR, GEN, false>(p, smem);
+  if constexpr (GEN) {
+    if (again) fused_walk_wide<SCALAR>(p, smem);   // (o, states and final state are written once more)
+  }
+  if (threadIdx.x < 32) tmem_dealloc(reinterpret_cast<FusedShared*>(smem + FUSED_SMEM - sizeof(FusedShared))->tmem_slot, 512);
 }
 
 // ===========================================================================
@@ -1253,7 +1433,96 @@ struct BwdParams {
   int vs;
   const float *add_dq, *add_dk, *add_dg;   // null: nothing to add
   long long dqk_pitch, dv_pitch;           // GEN: elements between tokens of dq and dk, and of dv
+  const __nv_bfloat16 *q, *k, *g;          // WIDE: what the tensor maps fetch
+  long long qk_pitch;                      // WIDE: elements between tokens of q and k
+  const int* wide;                         // WIDE: [chunk][H], not zero for the chunks to do
 };
+// chunks a block of a WIDE launch looks through at most
+constexpr int kWideList = 512;
+
+// The gradients of a wide chunk (see kSpan) for one channel and 16 time steps: what narrow chunks read from the products of
+// q~, k~ and dA is summed here over the pairs of the chunk, from the caller's q, k and gates and the dA tiles (hi + lo).
+// Leaves at scratch[time][channel] the 16 time steps' share of dg: the sum of q dq - k dk_intra from that step on and of
+// k dk_inter before it.  (Narrow chunks add k dk_inter of all steps and take away that of the later ones; where the gates
+// are strong both are larger than dg by more than fp32 holds.)
+// run, tail: the two sums over all 16 steps; h_scale: exp(G_n - ref - refd), which sum_v h' dh' lacks
+struct WideResult { float run, tail, h_scale; };
+struct WideChannel {
+  const float *add_dq, *add_dk;   // partial sums at the chunk's first token and this channel, or null
+  void *dq, *dk;                  // outputs, likewise
+  __nv_bfloat16* dv;              // null: no such value channel
+  long long add_step, dqk_step, dv_step;
+};
+template <typename TG, bool SCALAR>
+__device__ __noinline__ WideResult wide_gradients(const RawChunk r, const WideChannel out, uint32_t acc_dq, uint32_t acc_dk, uint32_t acc_dv,
+                                                  const uint8_t* dA_hi, const uint8_t* dA_lo, float* scratch, int col, int seg) {
+  const bool on = col < r.K;
+  WideResult res{0.f, 0.f, 0.f};
+  WideSums s{0.f, 0.f, 0.f};
+  if (on) s = wide_sums<SCALAR>(r, col, seg * SEG);
+  const float mid = 0.5f * (s.first + s.total), ref = clamp_span(mid), refd = clamp_span(s.total - mid);
+  res.h_scale = fast_exp(s.total - ref - refd);
+  float kdk[SEG];   // k dk_inter
+#pragma unroll
+  for (int t = 0; t < SEG; ++t) kdk[t] = 0.f;
+  auto dA = [&](int i, int j) { return ld_bf16(dA_hi, slab_off(i, j)) + ld_bf16(dA_lo, slab_off(i, j)); };
+  float G = s.before;   // of time step seg * SEG + 15
+  if (on)
+    for (int i = seg * SEG; i < seg * SEG + SEG && i < r.len; ++i) G += raw_gate<SCALAR>(r, i, col);
+#pragma unroll
+  for (int blk = 1; blk >= 0; --blk) {
+    float dq[8], dk[8], dv[8];   // inter-chunk: with respect to q~ and k~
+    const uint32_t c0 = seg * SEG + blk * 8;
+    tmem_ld8(acc_dq + c0, dq);
+    tmem_ld8(acc_dk + c0, dk);
+    tmem_ld8(acc_dv + c0, dv);
+#pragma unroll
+    for (int u = 7; u >= 0; --u) {
+      const int i = (int)c0 + u;
+      if (i < r.len) {
+        if (out.dv) st_out(out.dv, (size_t)(i * out.dv_step), dv[u]);
+        if (on) {
+          const float q = __bfloat162float(r.q[i * r.pitch + col]), k = __bfloat162float(r.k[i * r.pitch + col]);
+          float gq = fast_exp(G - ref) * dq[u];
+          const float inter = fast_exp(s.total - G - refd) * dk[u];
+          float gk = 0.f;
+          const float ei = fast_exp(raw_gate<SCALAR>(r, i, col));
+          float w = ei;
+          for (int j = i - 1; j >= 0 && w != 0.f; --j) {
+            gq = fmaf(dA(i, j) * w, __bfloat162float(r.k[j * r.pitch + col]), gq);
+            w *= fast_exp(raw_gate<SCALAR>(r, j, col));
+          }
+          w = 1.f;
+          for (int j = i + 1; j < r.len && w != 0.f; ++j) {
+            w *= fast_exp(raw_gate<SCALAR>(r, j, col));
+            gk = fmaf(dA(j, i) * w, __bfloat162float(r.q[j * r.pitch + col]), gk);
+          }
+          // the pair (i, i) has no gate in it: its shares of q dq and k dk cancel, and under strong gates they are
+          // larger than all else by more than fp32 holds
+          res.run += q * gq - k * gk;
+          const float dii = dA(i, i);
+          gq = fmaf(dii, k, gq);
+          gk = fmaf(dii, q, gk) + inter;
+          kdk[blk * 8 + u] = k * inter;
+          G -= raw_gate<SCALAR>(r, i, col);
+          if (out.add_dq) {
+            gq += out.add_dq[i * out.add_step];
+            gk += out.add_dk[i * out.add_step];
+          }
+          st_out(reinterpret_cast<TG*>(out.dq), (size_t)(i * out.dqk_step), gq);
+          st_out(reinterpret_cast<TG*>(out.dk), (size_t)(i * out.dqk_step), gk);
+        }
+      }
+      scratch[i * D + col] = res.run;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < SEG; ++t) {
+    scratch[(seg * SEG + t) * D + col] += res.tail;
+    res.tail += kdk[t];
+  }
+  return res;
+}
 
 // Warp roles: warps 0-15 gate q and k of the next chunk and write the gradients of a chunk out of
 // tensor memory (thread = one channel, 16 time steps); warps 16-19 convert A and dA to bf16 operands
@@ -1270,7 +1539,7 @@ constexpr int BWD_EPI_THREADS = 512, BWD_GATE_THREADS = 128;
 // issued: every write-out warp cumulates the 64 gates of a chunk in registers (warp_cumulate) and hands the
 // factors exp(+-(G - mid)) of the time steps around by shuffles.  dg is summed over the key channels inside
 // the kernel and written as fp32 [B,T,H] (the scalar gate's gradient is the sum of the channels').
-template <typename TG, typename TD, bool SCALAR, bool GEN>
+template <typename TG, typename TD, bool SCALAR, bool GEN, bool WIDE>
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_constant__ BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -1295,11 +1564,22 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   __shared__ float dgk_s[2][C];       // SCALAR: dg of a chunk summed over the channels
   __shared__ float diag[1][GEN ? 8 * C : 1];   // GEN: partial q_i . k_i [8][64] of a chunk
   __shared__ volatile int abort_flag;
+  __shared__ int wide_list[WIDE ? kWideList : 1], wide_count;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // tensor-memory columns: the exponent tile E_mid is consumed by the gating before A and dA take its place
   constexpr uint32_t cEm = 0, cA = 0, cET = 128, cdq = 256, cdk1 = 320, cdk2 = 384, cdv = 448;
   constexpr uint32_t cdA = GEN ? cdk1 : 64;
-  const int nit = (p.total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  int nit = (p.total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  if constexpr (WIDE) {   // the wide ones of this block's chunks (the order does not matter), mostly none
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the launch before this one is over, its writes are visible
+    if (tid == 0) wide_count = 0;
+    __syncthreads();
+    for (int n = tid; n < nit; n += BWD_THREADS)
+      if (p.wide[blockIdx.x + n * gridDim.x]) wide_list[atomicAdd(&wide_count, 1)] = blockIdx.x + n * gridDim.x;
+    __syncthreads();
+    nit = wide_count;
+    if (nit == 0) return;
+  }
 
   const int K = GEN ? p.geo.K : D, V = GEN ? p.geo.V : D;
   const int yc = GEN ? p.vs * D : 0;   // first value channel of this launch's slice
@@ -1307,7 +1587,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
   auto chunk_rows = [&](int it, int& h, int& row, int& hrow) -> int {
     // heads vary fastest over the chunks in flight: together the blocks read and write whole
     // token rows of the [B,T,H,D] activations
-    const int cid = blockIdx.x + it * gridDim.x;
+    const int cid = WIDE ? wide_list[it] : blockIdx.x + it * gridDim.x;
     h = cid % p.H;
     if constexpr (GEN) {
       const int slot = cid / p.H;
@@ -1397,6 +1677,15 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       *reinterpret_cast<uint4*>(ks + off) = mine ? kh : none;
       *reinterpret_cast<uint4*>(ks + TILE64 + off) = mine ? kl : none;
     };
+    auto raw_chunk = [&](int it) {   // GEN
+      int h, row, hrow;
+      const int len = chunk_rows(it, h, row, hrow);
+      const size_t at = (size_t)row * p.qk_pitch + (size_t)h * K;
+      RawChunk r{p.q + at, p.k + at, nullptr, p.qk_pitch, 0, p.gamma ? p.gamma[h] : 0.f, K, len};
+      if (!SCALAR) { r.g = p.g + ((size_t)row * p.H + h) * K; r.gstep = (long long)p.H * K; }
+      else if (p.gscalar) { r.g = p.gscalar + (size_t)row * p.H + h; r.gstep = p.H; }
+      return r;
+    };
     // GEN: A and dA -> masked hi + lo operands, 16 columns of both per thread (rows of an M = 64 accumulator sit in
     // lanes 0..15 of each quarter)
     auto convert = [&](int it) -> bool {
@@ -1404,12 +1693,19 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       tc_fence_after();
       const int ri = 16 * q4 + lane;
       float a[16], da[16];
-      tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
+      if (!WIDE) tmem_ld16(tmem_addr(tm, lane_base, cA + seg * 16), a);
       tmem_ld16(tmem_addr(tm, lane_base, cdA + seg * 16), da);
       if (lane < 16) {
-        if (seg == q4) set_diagonal(a, diag[0], 8, ri, lane);
-        store_tril16_split(Ps, gs, ri, seg * 16, a, p.scale);
+        if (!WIDE) {
+          if (seg == q4) set_diagonal(a, diag[0], 8, ri, lane);
+          store_tril16_split(Ps, gs, ri, seg * 16, a, p.scale);
+        }
         store_tril16_split(dAs, gs + SLAB64, ri, seg * 16, da, p.scale);
+      }
+      if constexpr (WIDE) {
+        const RawChunk raw = raw_chunk(it);
+        wide_operands<SCALAR>(raw, nullptr, ks, ks + TILE64, col, seg);
+        wide_matrix<SCALAR>(raw, Ps, gs, p.scale, warp, lane);
       }
       fence_async_smem();
       tc_fence_before();
@@ -1520,9 +1816,20 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       if (GEN) vbase = (size_t)(row + seg * SEG) * vstride + (size_t)h * V + yc + col;
       const size_t obase4 = obase - (lane & 3) + (size_t)(lane & 3) * ostride;   // channel group, own time row
       float dgl[SEG];
-      float run = 0.f, tail = 0.f;
+      float run = 0.f, tail = 0.f, h_scale = 1.f;
+      float* const wide_sums_at = reinterpret_cast<float*>(qs);   // (q~ is of no use in a wide chunk)
+      if constexpr (WIDE) {
+          if (!wait(&conv_done, it & 1, 13)) break;   // (long done: this thread reads what the others converted)
+          const size_t first = (size_t)row * p.H * K + (size_t)h * K + col, at = (size_t)row * p.dqk_pitch + (size_t)h * K + col;
+          const WideChannel out{p.add_dq ? p.add_dq + first : nullptr, p.add_dk ? p.add_dk + first : nullptr, dq_out + at, dk_out + at,
+                                has_v ? p.dv + (size_t)row * vstride + (size_t)h * V + yc + col : nullptr, (long long)ostride, p.dqk_pitch,
+                                (long long)vstride};
+          const WideResult res = wide_gradients<TG, SCALAR>(raw_chunk(it), out, tmem_addr(tm, lane_base, cdq), tmem_addr(tm, lane_base, cdk2),
+                                                            tmem_addr(tm, lane_base, cdv), dAs, gs + SLAB64, wide_sums_at, col, seg);
+          run = res.run; tail = res.tail; h_scale = res.h_scale;
+      }
 #pragma unroll
-      for (int blk = 1; blk >= 0; --blk) {
+      for (int blk = WIDE ? -1 : 1; blk >= 0; --blk) {
         float et[8] = {}, dq[8], dk1[8], dk2[8], dv[8];
         const uint32_t c0 = seg * SEG + blk * 8;
         if (!SCALAR) tmem_ld8(tmem_addr(tm, lane_base, cET + 64 * sl + c0), et);
@@ -1575,9 +1882,17 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
       asm volatile("bar.sync 1, %0;" ::"n"(BWD_EPI_THREADS) : "memory");
       const float later = (seg < 1 ? sufsum[sl][1][col] : 0.f) + (seg < 2 ? sufsum[sl][2][col] : 0.f) +
                           (seg < 3 ? sufsum[sl][3][col] : 0.f);
-      const float cst = later + tails[sl][0][col] + tails[sl][1][col] + tails[sl][2][col] + tails[sl][3][col] +
-                        hdh_s[sl][col] / p.scale;
+      // (of a wide chunk the steps of the earlier segments only, see wide_gradients)
+      float cst;
+      if (WIDE) cst = later + (seg > 0 ? tails[sl][0][col] : 0.f) + (seg > 1 ? tails[sl][1][col] : 0.f) + (seg > 2 ? tails[sl][2][col] : 0.f) +
+                      hdh_s[sl][col] / p.scale * h_scale;
+      else cst = later + tails[sl][0][col] + tails[sl][1][col] + tails[sl][2][col] + tails[sl][3][col] + hdh_s[sl][col] / p.scale;
       // (exp(G_n) sum_v h dh = sum_v h' dh' / scale)
+      if (WIDE) {
+#pragma unroll
+        for (int t = 0; t < SEG; ++t) dgl[t] = wide_sums_at[(seg * SEG + t) * D + col];
+        fence_async_smem();
+      }
       mbar_arrive(&e_done[sl]);   // tensor memory, the q~ / k~ tiles and hdh_s of this chunk are free
       if constexpr (SCALAR) {
         // sum over the 128 channels: the lanes of a warp by a shuffle butterfly (lane t keeps the total of time
@@ -1787,22 +2102,34 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           __syncwarp();
           if (!waitw(&gated, it & 1, 12)) break;
           tc_fence_after();
-          if (lane == 0) {
-            mul_A(qta, kta, 0); mul_A(qta, kla, 1); mul_A(qla, kta, 1);
-            umma_commit(&bar_A);
+          // (WIDE: k~ comes with the converted operands, A, dq_intra, dk_intra are no products)
+          auto mul_dv_inter = [&]() {
 #pragma unroll
             for (int k0 = 0; k0 < D; k0 += 16)   // dv^T[v][j] = dh'^T k~^T
               umma_bf16(tm + cdv, desc_mnmajor(dha, 128, k0, 0), desc_kmajor(kta, 64, 0, k0), umma_idesc(128, 64, 1, 0), k0 > 0);
+            if (WIDE) {
+#pragma unroll
+              for (int k0 = 0; k0 < D; k0 += 16)
+                umma_bf16(tm + cdv, desc_mnmajor(dha, 128, k0, 0), desc_kmajor(kla, 64, 0, k0), umma_idesc(128, 64, 1, 0), 1);
+            }
             umma_commit(&bar_r2);   // dh' and v are dead
+          };
+          if (lane == 0) {
+            if (!WIDE) { mul_A(qta, kta, 0); mul_A(qta, kla, 1); mul_A(qla, kta, 1); }
+            umma_commit(&bar_A);
+            if (!WIDE) mul_dv_inter();
           }
           __syncwarp();
           if (!waitw(&conv_done, it & 1, 13)) break;
           tc_fence_after();
           if (lane == 0) {
+            if (WIDE) mul_dv_inter();
             mul_dv(pa); mul_dv(pla);
             umma_commit(&bar_r1);   // h' and do are dead
-            mul_dq(kta, daa); mul_dq(kta, dala); mul_dq(kla, daa);
-            mul_dk(qta, daa, 0); mul_dk(qta, dala, 1); mul_dk(qla, daa, 1);
+            if (!WIDE) {
+              mul_dq(kta, daa); mul_dq(kta, dala); mul_dq(kla, daa);
+              mul_dk(qta, daa, 0); mul_dk(qta, dala, 1); mul_dk(qla, daa, 1);
+            }
             umma_commit(&bar_main);
           }
           __syncwarp();
@@ -1892,8 +2219,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_bwd_main(const __grid_consta
           load_dhv(it + 1);
           if (!wait(&bar_r1, it & 1, 8)) break;
           load_hdo(it + 1);
-          if (!SCALAR) {   // (the gate tile held the lower halves of A and dA)
-            if (!wait(&bar_main, it & 1, 8)) break;
+          if (!SCALAR) {   // (the gate tile held the lower halves of A and dA; WIDE: the write-out reads dA)
+            if (!wait(&bar_main, it & 1, 8) || (WIDE && !wait(&e_done[it & 1], (it >> 1) & 1, 14))) break;
             load_g(it + 1);
           }
           if (!wait(&e_done[it & 1], (it >> 1) & 1, 14)) break;
@@ -2123,12 +2450,33 @@ bool bwd_dtypes_ok(const tops_chunk_bwd_params& p) {
 
 template <typename TG, typename TD, bool SCALAR = false, bool GEN = false>
 int launch_bwd_main(const BwdParams& bp, cudaStream_t st) {
-  int rc = opt_in_smem(k_bwd_main<TG, TD, SCALAR, GEN>, BWD_SMEM);
+  int rc = opt_in_smem(k_bwd_main<TG, TD, SCALAR, GEN, false>, BWD_SMEM);
   if (rc) return rc;
   const int grid = bp.total < sm_count() ? bp.total : sm_count();
-  KernelScope ks("sm100_bwd_main", st);
-  k_bwd_main<TG, TD, SCALAR, GEN><<<grid, BWD_THREADS, BWD_SMEM, st>>>(bp);
-  return post_launch();
+  {
+    KernelScope ks("sm100_bwd_main", st);
+    k_bwd_main<TG, TD, SCALAR, GEN, false><<<grid, BWD_THREADS, BWD_SMEM, st>>>(bp);
+    if ((rc = post_launch())) return rc;
+  }
+  if constexpr (GEN) {
+    if (!bp.gscalar && !bp.gamma && SCALAR) return TOPS_OK;   // no gate
+    // What the launch above left of wide chunks is written again.  A launch of its own: it finds nothing to do as a rule,
+    // and taken care of in the kernel above wide chunks cost the narrow ones registers, 354 -> 407 us at T = 16384 in 13
+    // documents, H = 16 (364 us as a function called at the kernel's end).  It may be scheduled while the launch before it
+    // drains (see the wait in the kernel).
+    if ((rc = opt_in_smem(k_bwd_main<TG, TD, SCALAR, GEN, true>, BWD_SMEM))) return rc;
+    const int blocks = cdiv(bp.total, kWideList);
+    KernelScope ks("sm100_bwd_wide", st);
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid > blocks ? grid : blocks); cfg.blockDim = dim3(BWD_THREADS); cfg.dynamicSmemBytes = BWD_SMEM; cfg.stream = st;
+    cfg.attrs = &early; cfg.numAttrs = 1;
+    TOPS_CUDA_OK(cudaLaunchKernelEx(&cfg, k_bwd_main<TG, TD, SCALAR, GEN, true>, bp));
+    return post_launch();
+  }
+  return TOPS_OK;
 }
 
 int chunk_bwd(const tops_chunk_bwd_params& p, void* ws, size_t, cudaStream_t st) {
@@ -2271,6 +2619,7 @@ struct GenPlan {
   size_t words() const { return nch.empty() ? 0 : 3 * (size_t)N + (size_t)align_up(N + 1, 4) + (3 * (size_t)N % 4 ? 4 - 3 * (size_t)N % 4 : 0) + 8 * (size_t)runs; }
   size_t table_bytes() const { return nch.empty() ? 0 : align_up(words() * 4) + align_up((size_t)total_chunks * sizeof(ChunkEntry)); }
   size_t state_bytes() const { return align_up((size_t)total_chunks * HV * D * D * 2); }
+  size_t wide_bytes() const { return align_up((size_t)total_chunks * (HV / geo.VS) * 4); }
   size_t seg_state() const { return (size_t)runs * (HV / geo.VS) * geo.K * geo.V; }
   // end states, entry states, summed gates of the runs
   size_t seg_bytes() const { return cut ? align_up((2 * seg_state() + (size_t)runs * (HV / geo.VS) * D) * sizeof(float)) : 0; }
@@ -2333,7 +2682,8 @@ bool scalar_kind(int kind) { return kind != TOPS_GATE_PER_CHANNEL; }
 // pitch: of x and y where they are q, k or v (x_pitch 0 and y_pitch 0: contiguous)
 struct XYPitch { int64_t x = 0, y = 0; };
 int run_scan_gen(bool bwd, bool sum, const tops_chunk_problem& pb, const GenPlan& g, const void* x, const void* gate, const void* y,
-                 XYPitch pitch, const float* s0, const float* s0_seg, void* states, float* s_final, float* gsum, cudaStream_t st) {
+                 XYPitch pitch, const float* s0, const float* s0_seg, void* states, float* s_final, float* gsum, cudaStream_t st,
+                 void* wide = nullptr) {
   ScanParams sp;
   const int BT = pb.B * pb.T;
   const bool scalar = scalar_kind(pb.gate_kind);
@@ -2345,6 +2695,7 @@ int run_scan_gen(bool bwd, bool sum, const tops_chunk_problem& pb, const GenPlan
   if (states && (rc = state_map(&sp.mst, states, (size_t)g.total_chunks * g.HV * D))) return rc;
   sp.s0 = s0; sp.s0_seg = s0_seg; sp.states = reinterpret_cast<__nv_bfloat16*>(states); sp.s_final = s_final; sp.gsum = gsum;
   sp.T = pb.T; sp.H = pb.H; sp.NT = 0; sp.nseg = 1; sp.scale = pb.scale; sp.geo = g.geo; sp.skip_xy = -1;
+  sp.wide = reinterpret_cast<uint8_t*>(wide);
   auto launch = [&](auto kernel, const char* label) {
     if ((rc = opt_in_smem(kernel, SCAN_SMEM))) return rc;
     KernelScope ks(label, st);
@@ -2440,6 +2791,8 @@ int gen_chunk_fwd(const tops_chunk_fwd_params& p, void* ws, cudaStream_t st) {
   }
   up.s0 = p.h0; up.s0_seg = sc.starts; up.s_final = p.ht; up.o = reinterpret_cast<__nv_bfloat16*>(p.o);
   up.T = pb.T; up.H = pb.H; up.NT = 0; up.nseg = 1; up.scale = pb.scale; up.geo = g.geo;
+  up.q = reinterpret_cast<const __nv_bfloat16*>(p.q); up.k = reinterpret_cast<const __nv_bfloat16*>(p.k);
+  up.g = reinterpret_cast<const __nv_bfloat16*>(p.g); up.qk_pitch = p.pitch ? p.pitch : (long long)pb.H * pb.K;
   if ((rc = opt_in_smem(k_fwd_fused<true, true>, FUSED_SMEM)) || (rc = opt_in_smem(k_fwd_fused<false, true>, FUSED_SMEM))) return rc;
   KernelScope ks("sm100_fwd_fused", st);
   if (scalar) k_fwd_fused<true, true><<<g.blocks(), FUSED_THREADS, FUSED_SMEM, st>>>(up);
@@ -2456,7 +2809,8 @@ static size_t gen_partial_floats(const tops_chunk_bwd_params& p) {
 
 size_t gen_bwd_workspace_bytes(const tops_chunk_bwd_params& p) {
   const GenPlan g(p.pb);
-  return g.table_bytes() + (p.h_saved ? 1 : 2) * g.state_bytes() + g.seg_bytes() + align_up(gen_partial_floats(p) * sizeof(float)) + 256;
+  return g.table_bytes() + (p.h_saved ? 1 : 2) * g.state_bytes() + g.seg_bytes() + g.wide_bytes() +
+         align_up(gen_partial_floats(p) * sizeof(float)) + 256;
 }
 
 int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
@@ -2477,6 +2831,7 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
   char* hw = nullptr;
   if (!h) { hw = wsp; wsp += g.state_bytes(); }
   const GenSegs sc(wsp, g); wsp += g.seg_bytes();
+  char* wide = wsp; wsp += g.wide_bytes();
   float* part = reinterpret_cast<float*>(wsp);
   if (!h) {
     const XYPitch kv{p.pitch, p.pitch};
@@ -2486,7 +2841,7 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
   }
   const XYPitch qdo{p.pitch, 0};
   if ((rc = gen_starts(true, pb, g, p.q, p.g, p.do_, qdo, p.dht, p.dh0, sc, st))) return rc;
-  if ((rc = run_scan_gen(true, false, pb, g, p.q, p.g, p.do_, qdo, p.dht, sc.starts, dh, p.dh0, nullptr, st))) return rc;
+  if ((rc = run_scan_gen(true, false, pb, g, p.q, p.g, p.do_, qdo, p.dht, sc.starts, dh, p.dh0, nullptr, st, wide))) return rc;
   BwdParams bp;
   const int BT = pb.B * pb.T;
   const size_t rows = (size_t)g.total_chunks * g.HV * D;
@@ -2499,6 +2854,9 @@ int gen_chunk_bwd(const tops_chunk_bwd_params& p, void* ws, cudaStream_t st) {
   bp.gscalar = pb.gate_kind == TOPS_GATE_SCALAR ? reinterpret_cast<const __nv_bfloat16*>(p.g) : nullptr;
   bp.gamma = pb.gate_kind == TOPS_GATE_GAMMA ? reinterpret_cast<const float*>(p.g) : nullptr;
   bp.dv = reinterpret_cast<__nv_bfloat16*>(p.dv);
+  bp.q = reinterpret_cast<const __nv_bfloat16*>(p.q); bp.k = reinterpret_cast<const __nv_bfloat16*>(p.k);
+  bp.g = reinterpret_cast<const __nv_bfloat16*>(p.g); bp.qk_pitch = p.pitch ? p.pitch : (long long)pb.H * pb.K;
+  bp.wide = reinterpret_cast<const int*>(wide);
   bp.T = pb.T; bp.H = pb.H; bp.NT = g.nch.empty() ? g.geo.NTseq : g.total_chunks; bp.scale = pb.scale; bp.geo = g.geo;
   bp.total = g.total_chunks * pb.H;
   const size_t n = (size_t)BT * pb.H;

@@ -10,12 +10,14 @@ from .. import _lib as L
 from .common import device_boundaries, make_problem, total_chunks
 
 
-def tensor_core_shape(q, v, gate, gate_kind):
-    """Whether the tcgen05 kernels take tensors like these (with chunks of 64, whatever T and the packing)."""
-    K, V = q.shape[-1], v.shape[-1]
-    return (q.dtype == torch.bfloat16
-            and (gate_kind in (L.GATE_NONE, L.GATE_GAMMA) or gate.dtype == torch.bfloat16)
-            and 32 <= K <= 128 and K % 8 == 0 and 32 <= V <= 1024 and V % 8 == 0)
+@L.on_tensor_device
+def kernel_chunk(q, v, gate, gate_kind, scale, cu_seqlens, chunk):
+    """64 where the tcgen05 kernels take the problem, else the length asked for."""
+    B, T, H, K = q.shape
+    keep = []
+    gate_dtype = L.F32 if gate is None or gate_kind == L.GATE_GAMMA else L.dtype_code(gate.dtype)
+    pb = make_problem(B, T, H, K, v.shape[-1], 64, L.dtype_code(q.dtype), gate_dtype, gate_kind, scale, cu_seqlens=cu_seqlens, keep=keep)
+    return 64 if L.lib.tops_b200_chunk_selected_impl(C.byref(pb)) == L.IMPL_SM100 else chunk
 
 
 @L.on_tensor_device

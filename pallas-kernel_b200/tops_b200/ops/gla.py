@@ -17,7 +17,7 @@ import torch
 
 from .. import _lib as L
 from .._lib import ops_ext as X
-from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
+from ._chunk import chunk_bwd_call, chunk_fwd_call
 
 
 def _check_qkvg(q, k, v, g, initial_state, cu_seqlens):
@@ -75,19 +75,13 @@ def chunk_gla_bwd(q, k, v, g, g_cumsum, scale, initial_state, h, A, do, dht, chu
                           torch.float32, True, initial_state is not None, _cu_list(cu_seqlens))
 
 
-def _kernel_chunk(q, v, g, cu_seqlens, chunk_size):
-    """Chunk length the kernels use for the differentiable op.  The op's results (o, final state,
-    gradients) do not depend on the chunk length beyond where bf16 roundings fall, so a problem the
-    tcgen05 kernels can take (bf16, K <= 128) runs with their chunk of
-    64 whatever `chunk_size` asks for (the reference's default is 16); everything else keeps the
-    requested length.  The orchestrators that return per-chunk intermediates never change it."""
+def _kernel_chunk(chunk_size):
+    """Chunk length for a problem the tcgen05 kernels do not take (the extension picks 64 for one they do).  The op's
+    results (o, final state, gradients) do not depend on it beyond where roundings fall: the kernels hold chunks of 16, 32
+    or 64 time steps, longer (or shorter) powers of two run with the nearest."""
     assert chunk_size >= 1 and (chunk_size & (chunk_size - 1)) == 0, \
         f"chunk_size must be a power of 2, got {chunk_size}"   # tops/ops/common/cumsum.py:506-508
-    if tensor_core_shape(q, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL):
-        return 64
-    # the kernels hold chunks of 16, 32 or 64 time steps; longer (or shorter) powers of two give the
-    # same results computed with the nearest length they hold
-    return min(max(chunk_size, 16), 64)
+    return min(max(int(chunk_size), 16), 64)
 
 
 def chunk_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, output_final_state=False,
@@ -107,7 +101,7 @@ def chunk_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, out
         gg = gg.view(1, 1, H, 1) if gg.ndim == 1 and gg.shape[0] == H else gg
         g = torch.broadcast_to(gg, (B, T, H, K)).contiguous()
     return X.chunk(q, k, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL, initial_state, float(scale),
-                   bool(output_final_state), _cu_list(cu_seqlens) or [], _kernel_chunk(q, v, g, cu_seqlens, chunk_size))
+                   bool(output_final_state), _cu_list(cu_seqlens) or [], _kernel_chunk(chunk_size))
 
 
 def fused_chunk_gla(q, k, v, g=None, scale=None, initial_state=None, output_final_state=False,

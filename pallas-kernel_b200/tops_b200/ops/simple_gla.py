@@ -12,7 +12,7 @@ import torch
 
 from .. import _lib as L
 from .._lib import ops_ext as X
-from ._chunk import chunk_bwd_call, chunk_fwd_call, tensor_core_shape
+from ._chunk import chunk_bwd_call, chunk_fwd_call, kernel_chunk
 from .gla import fused_recurrent_gla
 
 
@@ -65,9 +65,7 @@ def _kernel_chunk(chunk_size):
 def _fwd(q, k, v, g, g_gamma, scale, initial_state, output_final_state, chunk_size, cu_seqlens, want_saved):
     _check(q, k, v, g, g_gamma, initial_state, cu_seqlens)
     gate, kind = _gate(g, g_gamma)
-    chunk_size = _kernel_chunk(chunk_size)
-    if tensor_core_shape(q, v, gate, kind):
-        chunk_size = 64
+    chunk_size = kernel_chunk(q, v, gate, kind, scale, _cu(cu_seqlens), _kernel_chunk(chunk_size))
     o, ht, _, _, saved = chunk_fwd_call(q, k, v, gate, kind, scale, initial_state, output_final_state, chunk_size,
                                         _cu(cu_seqlens), want_saved=want_saved)
     return o, ht, saved
@@ -89,9 +87,7 @@ def chunk_simple_gla_bwd(q, k, v, g, g_gamma, initial_state, do, dht, scale, chu
     forward kept (None recomputes them, as the reference does)."""
     _check(q, k, v, g, g_gamma, initial_state, cu_seqlens)
     gate, kind = _gate(g, g_gamma)
-    chunk_size = _kernel_chunk(chunk_size)
-    if tensor_core_shape(q, v, gate, kind):
-        chunk_size = 64
+    chunk_size = kernel_chunk(q, v, gate, kind, scale, _cu(cu_seqlens), _kernel_chunk(chunk_size))
     return chunk_bwd_call(q, k, v, gate, kind, scale, initial_state, do, dht, chunk_size, q.dtype,
                           g is not None, initial_state is not None, _cu(cu_seqlens), h_saved=h_saved)
 
@@ -105,10 +101,8 @@ def chunk_simple_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=No
     if scale is None:
         scale = K ** -0.5
     gate, kind = _gate(g, g_gamma)
-    chunk_size = _kernel_chunk(chunk_size)
-    if tensor_core_shape(q, v, gate, kind):
-        chunk_size = 64
-    return X.chunk(q, k, v, gate, kind, initial_state, float(scale), bool(output_final_state), _cu(cu_seqlens) or [], chunk_size)
+    return X.chunk(q, k, v, gate, kind, initial_state, float(scale), bool(output_final_state), _cu(cu_seqlens) or [],
+                   _kernel_chunk(chunk_size))
 
 
 def fused_chunk_simple_gla(q, k, v, g_gamma=None, initial_state=None, scale=None, output_final_state=False,

@@ -90,7 +90,11 @@ std::tuple<Tensor, OptTensor> chunk(const Tensor& q, const Tensor& k, const Tens
   Tensor o = c.empty({B, T, H, V}, v.scalar_type()), ht, hs;
   if (want_ht) ht = c.empty({s.N, H, K, V}, at::kFloat);
   tops_chunk_fwd_params p{};
+  // the results do not depend on the chunk length beyond where roundings fall: a problem the tcgen05 kernels take runs
+  // with their 64, every other one with the length it asks for (the CUDA-core kernels lose strong gates in longer chunks)
+  s.chunk = 64;
   p.pb = chunk_problem(s, q, v, gc);
+  if (tops_b200_chunk_selected_impl(&p.pb) != TOPS_IMPL_SM100) p.pb.chunk = s.chunk = chunk_len;
   p.q = ptr(qc); p.k = ptr(kc); p.v = ptr(vc); p.g = ptr(gc); p.h0 = ptr<float>(h0c); p.o = ptr(o); p.ht = ptr<float>(ht);
   const bool keep = wants_grad(q, k, v, gate, h0);
   Tensor cu_dev;
