@@ -18,6 +18,7 @@ from torch import nn
 from ._lib import ops_ext as X
 from .ops.gate import gla_gate
 from .ops.gla import chunk_gla, fused_chunk_gla, fused_recurrent_gla
+from .ops._recorded import active as recorded
 from .ops.norm import FusedRMSNormGated
 
 # "gelu" is the tanh approximation: the reference's table holds jax.nn.gelu, whose default is approximate=True
@@ -144,7 +145,7 @@ class GatedLinearAttention(nn.Module):
         if not (self.use_output_gate and self.fuse_norm_and_gate) or self.use_short_conv or self.feature_map_fn is not None \
                 or self.num_kv_groups != 1 or torch.is_autocast_enabled():
             return None
-        if (torch._C._get_tracing_state() is not None or torch.nn.modules.module._has_any_global_hook() or not self._plain()):
+        if (recorded() or torch.nn.modules.module._has_any_global_hook() or not self._plain()):
             return None
         q_len = x.shape[1]
         recurrent = q_len <= 64 or self.mode == "fused_recurrent"

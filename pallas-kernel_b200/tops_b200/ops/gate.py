@@ -18,6 +18,7 @@ import torch
 
 from .. import _lib as L
 from .._lib import ops_ext as X
+from ._recorded import call
 
 
 def _fill(p, g, H, K, kind, A_log, dt_bias, lower_bound, normalizer, clamp_min, out_dtype):
@@ -98,7 +99,7 @@ def kda_gate_fwd(g, A_log, dt_bias=None, lower_bound=None, output_dtype=torch.fl
     _check_gate(g)
     H, K = g.shape[-2:]
     _check_params(A_log, dt_bias, H, K)
-    return X.gate(g, A_log, dt_bias, _kind(lower_bound), 0.0 if lower_bound is None else float(lower_bound), 1.0, None, output_dtype)
+    return call(X.gate, g, A_log, dt_bias, _kind(lower_bound), 0.0 if lower_bound is None else float(lower_bound), 1.0, None, output_dtype)
 
 
 fused_kda_gate = kda_gate_fwd
@@ -120,4 +121,4 @@ def gla_gate(g, gate_logit_normalizer=16.0, clamp_min=None):
     """`log_sigmoid(g) / gate_logit_normalizer`, clipped from below by `clamp_min` when given: the gate
     of the GLA layer (`tops/layers/gla.py:277-279`), in g's dtype.  Differentiable."""
     _check_gate(g)
-    return X.gate(g, None, None, L.GATE_ACT_LOG_SIGMOID, 0.0, float(gate_logit_normalizer), clamp_min, None)
+    return call(X.gate, g, None, None, L.GATE_ACT_LOG_SIGMOID, 0.0, float(gate_logit_normalizer), clamp_min, None)

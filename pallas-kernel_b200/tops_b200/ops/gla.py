@@ -18,6 +18,7 @@ import torch
 from .. import _lib as L
 from .._lib import ops_ext as X
 from ._chunk import chunk_bwd_call, chunk_fwd_call
+from ._recorded import call
 
 
 def _check_qkvg(q, k, v, g, initial_state, cu_seqlens):
@@ -100,7 +101,7 @@ def chunk_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=None, out
         gg = g_gamma.to(torch.float32)
         gg = gg.view(1, 1, H, 1) if gg.ndim == 1 and gg.shape[0] == H else gg
         g = torch.broadcast_to(gg, (B, T, H, K)).contiguous()
-    return X.chunk(q, k, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL, initial_state, float(scale),
+    return call(X.chunk, q, k, v, g, L.GATE_NONE if g is None else L.GATE_PER_CHANNEL, initial_state, float(scale),
                    bool(output_final_state), _cu_list(cu_seqlens) or [], _kernel_chunk(chunk_size))
 
 
@@ -218,7 +219,7 @@ def fused_recurrent_gla(q, k, v, gk=None, gv=None, scale=None, initial_state=Non
     if scale is None:
         scale = K ** -0.5
     assert gk is None or gv is None or gk.dtype == gv.dtype
-    return X.recurrent(q, k, v, gk, gv, float(scale), initial_state, bool(output_final_state), bool(reverse),
+    return call(X.recurrent, q, k, v, gk, gv, float(scale), initial_state, bool(output_final_state), bool(reverse),
                        _cu_list(cu_seqlens) or [])
 
 

@@ -18,6 +18,7 @@ import torch
 
 from .. import _lib as L
 from .._lib import ops_ext as X
+from ._recorded import call
 
 
 def _check(q, k, v, g, beta, initial_state):
@@ -224,7 +225,7 @@ def fused_recurrent_kda(q, k, v, g, beta, scale=None, initial_state=None, output
     B, T, H, K, V = _check(q, k, v, g, beta, initial_state)
     if scale is None:
         scale = K ** -0.5
-    return X.kda(q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), False)
+    return call(X.kda, q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), False)
 
 
 def fused_recurrent_kda_decode_(q, k, v, g, beta, state, scale=None):
@@ -249,4 +250,4 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
         scale = K ** -0.5
     # the result does not depend on the chunk length beyond where roundings fall: a problem the
     # tensor-core kernels take runs with their chunk of 64
-    return X.kda(q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), True)
+    return call(X.kda, q, k, v, g, beta, float(scale), initial_state, bool(output_final_state), True)

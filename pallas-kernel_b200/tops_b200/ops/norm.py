@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 
 from .._lib import ops_ext as X
+from ._recorded import call
 
 
 def _check(x):
@@ -23,7 +24,7 @@ def _check(x):
 def l2norm(x, eps=1e-6):
     """x / sqrt(sum(x^2, -1) + eps), in x's dtype (fp32 arithmetic)."""
     _check(x)
-    return X.l2norm(x, float(eps))
+    return call(X.l2norm, x, float(eps))
 
 
 def rmsnorm_gated(x, g, weight=None, eps=1e-5):
@@ -31,7 +32,7 @@ def rmsnorm_gated(x, g, weight=None, eps=1e-5):
     _check(x)
     assert g.shape == x.shape, f"g shape {tuple(g.shape)} != x shape {tuple(x.shape)}"
     assert weight is None or weight.numel() == x.shape[-1], f"weight shape {tuple(weight.shape)} != ({x.shape[-1]},)"
-    return X.rmsnorm_gated(x, g, weight, float(eps))
+    return call(X.rmsnorm_gated, x, g, weight, float(eps))
 
 
 class FusedRMSNormGated(torch.nn.Module):

@@ -13,6 +13,7 @@ import torch
 from .. import _lib as L
 from .._lib import ops_ext as X
 from ._chunk import chunk_bwd_call, chunk_fwd_call, kernel_chunk
+from ._recorded import call
 from .gla import fused_recurrent_gla
 
 
@@ -101,7 +102,7 @@ def chunk_simple_gla(q, k, v, g=None, g_gamma=None, scale=None, initial_state=No
     if scale is None:
         scale = K ** -0.5
     gate, kind = _gate(g, g_gamma)
-    return X.chunk(q, k, v, gate, kind, initial_state, float(scale), bool(output_final_state), _cu(cu_seqlens) or [],
+    return call(X.chunk, q, k, v, gate, kind, initial_state, float(scale), bool(output_final_state), _cu(cu_seqlens) or [],
                    _kernel_chunk(chunk_size))
 
 
