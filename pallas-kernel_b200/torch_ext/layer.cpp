@@ -259,7 +259,10 @@ std::tuple<Tensor, OptTensor> gla_layer(const Tensor& x_, const Tensor& Wq, cons
     check(tops_b200_chunk_gla_fwd(&p, ws.data_ptr(), (size_t)ws.numel(), c.stream()), "chunk_gla_fwd");
     on = c.empty({d.n, d.V}, at::kBFloat16);
     norm_fwd(c, d, l, o, ptr(g), 0, c.in(nw), on);
-    out = at::mm(on, Wo.t()).view({d.B, d.T, d.hid});
+    // (not a view: autograd refuses in-place operations on a view made without gradients)
+    out = c.empty({d.B, d.T, d.hid}, at::kBFloat16);
+    Tensor rows = out.view({d.n, d.hid});
+    at::mm_out(rows, on, Wo.t());
   }
   auto node = make_node<LayerNode>(x_, Wq, Wk, Wv, Wg, Wlow, Wgk, bgk, nw, Wo, h0);
   node->d = d; node->law = l; node->cu = std::move(cu);

@@ -138,3 +138,22 @@ def test_an_output_of_another_width(T):
         (o, _, _), labels = _labels(lambda: layer(x))
         want = copy.deepcopy(layer).float()(x.float())[0]
     assert o.shape == (2, T, 96) and "lowrank_gate_fwd" not in labels and rel_l2(o, want) <= 2e-2
+
+
+def test_in_place_operations_on_the_output():
+    """`o += residual`, in-place dropout or activation on a training step's output, as on a linear layer's."""
+    layer = _layer(512, 4)
+    x = torch.randn(2, 70, 512, device="cuda", dtype=torch.bfloat16)
+    grads = []
+    for inplace in (False, True):
+        leaf = x.clone().requires_grad_()
+        o = layer(leaf)[0]
+        assert o.grad_fn is not None and not o._is_view()
+        if inplace:
+            o += leaf
+            o.relu_()
+        else:
+            o = torch.relu(o + leaf)
+        grads.append(torch.autograd.grad(o, [leaf, *layer.parameters()], torch.ones_like(o)))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
