@@ -250,6 +250,14 @@ def ptr(t) -> int | None:
     return t.data_ptr()
 
 
+def dense(t):
+    """Contiguous, on a 16-byte boundary (a view into a larger tensor may be on none); None stays None."""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 

@@ -31,11 +31,9 @@ def chunk_fwd_call(q, k, v, gate, gate_kind, scale, h0, want_ht, chunk, cu_seqle
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    gate = None if gate is None else gate.contiguous()
-    if gate_kind == L.GATE_GAMMA:
-        gate = gate.float().contiguous()
-    h0 = None if h0 is None else h0.float().contiguous()
+    q, k, v = L.dense(q), L.dense(k), L.dense(v)
+    gate = L.dense(gate.float() if gate_kind == L.GATE_GAMMA else gate)
+    h0 = L.dense(None if h0 is None else h0.float())
     N = B if cu_seqlens is None else len(cu_seqlens) - 1
     o = torch.empty(B, T, H, V, dtype=v.dtype, device=dev)
     ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if want_ht else None
@@ -80,13 +78,11 @@ def chunk_bwd_call(q, k, v, gate, gate_kind, scale, h0, do, dht, chunk, grad_dty
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
-    q, k, v, do = q.contiguous(), k.contiguous(), v.contiguous(), do.contiguous()
+    q, k, v, do = L.dense(q), L.dense(k), L.dense(v), L.dense(do)
     assert do.dtype == q.dtype, "do must have the dtype of q/k/v"
-    gate = None if gate is None else gate.contiguous()
-    if gate_kind == L.GATE_GAMMA:
-        gate = gate.float().contiguous()
-    h0 = None if h0 is None else h0.float().contiguous()
-    dht = None if dht is None else dht.float().contiguous()
+    gate = L.dense(gate.float() if gate_kind == L.GATE_GAMMA else gate)
+    h0 = L.dense(None if h0 is None else h0.float())
+    dht = L.dense(None if dht is None else dht.float())
     N = B if cu_seqlens is None else len(cu_seqlens) - 1
     keep = []
     p = L.ChunkBwdParams()

@@ -109,9 +109,9 @@ def _chunk_fwd_call(q, k, v, g, beta, scale, initial_state, output_final_state, 
     `[B,T,H,C]` when `want_A`, and saved the opaque residuals for the backward when `want_saved`."""
     B, T, H, K, V = _check(q, k, v, g, beta, initial_state)
     dev = q.device
-    q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+    q, k, v, g = L.dense(q), L.dense(k), L.dense(v), L.dense(g)
     beta_c = beta.to(q.dtype).contiguous()
-    h0 = None if initial_state is None else initial_state.float().contiguous()
+    h0 = L.dense(None if initial_state is None else initial_state.float())
     o = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
     Aqk = torch.empty(B, T, H, chunk_size, dtype=torch.float32, device=dev) if want_A else None
@@ -157,10 +157,10 @@ def _chunk_bwd_call(q, k, v, g, beta, do, scale, dht, saved, want_dh0, grad_dtyp
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
-    q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+    q, k, v, g = L.dense(q), L.dense(k), L.dense(v), L.dense(g)
     beta_c = beta.to(q.dtype).contiguous()
-    do = do.to(q.dtype).contiguous()
-    dhtc = None if dht is None else dht.float().contiguous()
+    do = L.dense(do.to(q.dtype))
+    dhtc = L.dense(None if dht is None else dht.float())
     dq = torch.empty(B, T, H, K, dtype=grad_dtype, device=dev)
     dk, dg = torch.empty_like(dq), torch.empty_like(dq)
     dbeta = torch.empty(B, T, H, dtype=grad_dtype, device=dev)
@@ -186,10 +186,10 @@ def _chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved):
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
-    q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+    q, k, v, g = L.dense(q), L.dense(k), L.dense(v), L.dense(g)
     beta_c = beta.to(q.dtype).contiguous()
-    do = do.to(q.dtype).contiguous()
-    dhtc = None if dht is None else dht.float().contiguous()
+    do = L.dense(do.to(q.dtype))
+    dhtc = L.dense(None if dht is None else dht.float())
     dv = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
     dh0 = torch.empty(B, H, K, V, dtype=torch.float32, device=dev)
     p = L.ChunkKdaBwdParams()

@@ -90,10 +90,13 @@ struct Call {
     need_cuda(t);
     return t.data_ptr<float>();
   }
-  Tensor in(const Tensor& t) const {   // contiguous, on a GPU
+  // contiguous, on a GPU, on a 16-byte boundary (which a view into a larger tensor may not be, and what moves 16 bytes per
+  // access asks for)
+  Tensor in(const Tensor& t) const {
     if (!t.defined()) return t;
     need_cuda(t);
-    return t.is_contiguous() ? t : t.contiguous();
+    if (!t.is_contiguous()) return t.contiguous();
+    return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone();
   }
   Tensor in(const OptTensor& t) const { return t.has_value() ? in(*t) : Tensor(); }
   Tensor in_as(const Tensor& t, at::ScalarType type) const { return t.defined() ? in(t.scalar_type() == type ? t : t.to(type)) : t; }
