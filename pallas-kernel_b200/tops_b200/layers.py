@@ -6,8 +6,9 @@ optional causal depthwise short convolutions (`tops/modules/convolution.py`), th
 `log_sigmoid(gk) / gate_logit_normalizer` (`gla_gate`), `fused_recurrent_gla` for sequences of at most
 64 tokens and the configured mode otherwise (chunk_size 16 as upstream), the fused RMS-norm + swish gate
 on the output (`FusedRMSNormGated`) or the plain RMS norm followed by the gate activation, and the output
-projection.  The layer its constructor's defaults make runs as one call of the torch extension (`_forward_fused`).  The linear projections and the short convolution are torch's own (they are outside the path
-this package replaces); everything between them runs on this package's kernels.
+projection.  The layer its constructor's defaults make runs as one call of the torch extension (`_forward_fused`).
+The linear projections and the short convolution are torch's own (they are outside the path this package replaces);
+everything between them runs on this package's kernels.
 """
 from __future__ import annotations
 
@@ -130,13 +131,17 @@ class GatedLinearAttention(nn.Module):
         return x if groups == 1 else x.repeat_interleave(groups, dim=-2)
 
     def _plain(self):
-        """The projections are ordinary bf16 linears nobody watches: they may be computed without calling the modules."""
-        lin = (self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.gk_proj[0], self.gk_proj[1], self.o_proj)
-        for m in (*lin, self.gk_proj, self.g_norm_swish_gate):
-            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks):
+        """The submodules are the ones the constructor made and nobody watches or wraps them: what they hold may be used
+        without calling them."""
+        gate, norm = self.gk_proj, self.g_norm_swish_gate
+        if type(gate) is not nn.Sequential or len(gate) != 2 or type(norm) is not FusedRMSNormGated:
+            return False
+        low, gk = gate
+        lin = (self.q_proj, self.k_proj, self.v_proj, self.g_proj, low, gk, self.o_proj)
+        for m in (*lin, gate, norm):
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__):
                 return False
-        return all(type(m) is nn.Linear and m.weight.dtype == torch.bfloat16 and m.weight.is_contiguous()
-                   and (m.bias is None) == (m is not self.gk_proj[1]) for m in lin)
+        return all(type(m) is nn.Linear and (m.bias is None) == (m is not gk) for m in lin)
 
     def _forward_fused(self, x, past_key_values, use_cache, cu_seqlens):
         """The whole layer in one call of the torch extension, for the layer its constructor's defaults make: all

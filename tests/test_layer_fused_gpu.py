@@ -82,6 +82,41 @@ def test_watched_or_replaced_projections_are_called():
     assert seen and "lowrank_gate_fwd" not in labels
 
 
+@pytest.mark.parametrize("T", [1, 70])
+@pytest.mark.parametrize("change", ["norm", "gate", "one gate module", "forward", "norm forward", "norm hook"])
+def test_any_changed_submodule_is_called(T, change):
+    from torch import nn
+    layer = _layer(512, 4)
+    x = torch.randn(1, T, 512, device="cuda", dtype=torch.bfloat16)
+    seen = []
+
+    def wrap(m):
+        inner = m.forward
+        m.forward = lambda *a: seen.append(1) or inner(*a)
+
+    class Watch(nn.Module):
+        def __init__(self, inner=None):
+            super().__init__()
+            self.inner = inner
+
+        def forward(self, *a):
+            seen.append(1)
+            return a[0] if self.inner is None else self.inner(*a)
+    if change == "norm":
+        layer.g_norm_swish_gate = Watch(layer.g_norm_swish_gate)
+    elif change == "gate":
+        layer.gk_proj.append(Watch())
+    elif change == "one gate module":
+        layer.gk_proj = Watch(nn.Linear(512, 256, device="cuda", dtype=torch.bfloat16))
+    elif change == "norm hook":
+        layer.g_norm_swish_gate.register_forward_hook(lambda *a: seen.append(1))
+    else:
+        wrap(layer.o_proj if change == "forward" else layer.g_norm_swish_gate)
+    with torch.no_grad():
+        layer(x)
+    assert seen
+
+
 @pytest.mark.parametrize("rows", [1, 7, 8, 9, 16, 31, 33, 64])
 @pytest.mark.parametrize("K,Ns", [(32, (8,)), (96, (17, 16, 1)), (2048, (512, 40))])
 def test_skinny_linear(rows, K, Ns):
