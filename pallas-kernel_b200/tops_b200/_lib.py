@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import functools
 import os
+import sys
 
 import torch
 
@@ -291,7 +292,7 @@ def raise_on_device_error(what: str = "tops_b200") -> None:
 # TOPS_B200_CHECK_DEVICE=1 makes every differentiable op check the device error word after its
 # backward pass (one synchronisation per step); off by default, the word stays readable at any time.
 CHECK_DEVICE = os.environ.get("TOPS_B200_CHECK_DEVICE", "0") not in ("", "0")
-ops_ext.configure(TopsError, CHECK_DEVICE)
+ops_ext.configure(sys.modules[__name__])   # (TopsError, and CHECK_DEVICE as it stands when a backward pass ends)
 
 
 def on_tensor_device(fn):

@@ -5,6 +5,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -24,16 +25,24 @@ using OptTensor = std::optional<Tensor>;
 namespace tops_torch {
 
 
-inline PyObject* g_error_class = nullptr;   // tops_b200.TopsError
-inline bool g_check_device = false;         // read the device error word after every backward
+inline PyObject* g_module = nullptr;   // tops_b200._lib: TopsError, CHECK_DEVICE
 
-inline void raise_tops(const std::string& text) {
-  if (g_error_class && PyGILState_Check()) {
-    PyErr_SetString(g_error_class, text.c_str());
-    throw py::error_already_set();
-  }
-  TORCH_CHECK(false, text);
+// Raises a Python exception, also from a node that runs on an autograd thread without the GIL: the engine carries a
+// python_error over to the thread that called backward().
+[[noreturn]] inline void raise_py(PyObject* type, const std::string& text) {
+  const bool held = PyGILState_Check();
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(type, text.c_str());
+  if (held) throw py::error_already_set();
+  python_error e;
+  e.persist();
+  throw e;
 }
+[[noreturn]] inline void raise_tops(const std::string& text) {
+  py::gil_scoped_acquire gil;
+  raise_py(py::handle(g_module).attr("TopsError").ptr(), text);
+}
+[[noreturn]] inline void raise_assertion(const std::string& text) { raise_py(PyExc_AssertionError, text); }
 inline void check(int rc, const char* what) {
   if (rc == 0) return;
   std::string text = std::string(what) + ": " + tops_b200_strerror(rc) + " (code " + std::to_string(rc) + ")";
@@ -45,7 +54,10 @@ inline void check(int rc, const char* what) {
   raise_tops(text);
 }
 inline void check_device_word(const char* what) {
-  if (!g_check_device) return;
+  {
+    py::gil_scoped_acquire gil;
+    if (!py::handle(g_module).attr("CHECK_DEVICE").cast<bool>()) return;
+  }
   int code = 0;
   check(tops_b200_device_error(&code), "device_error");
   if (code == 0) return;
@@ -58,11 +70,7 @@ inline int code_of(at::ScalarType t) {
   if (t == at::kFloat) return TOPS_F32;
   if (t == at::kBFloat16) return TOPS_BF16;
   if (t == at::kHalf) return TOPS_F16;
-  if (PyGILState_Check()) {
-    PyErr_SetString(PyExc_AssertionError, "unsupported dtype (fp32, bf16, fp16 only)");
-    throw py::error_already_set();
-  }
-  TORCH_CHECK(false, "unsupported dtype (fp32, bf16, fp16 only)");
+  raise_assertion("unsupported dtype (fp32, bf16, fp16 only)");
 }
 inline int code_of(const Tensor& t) { return code_of(t.scalar_type()); }
 
@@ -72,13 +80,7 @@ struct Call {
   c10::cuda::CUDAGuard guard;
   explicit Call(const Tensor& t) : dev(t.device()), guard(need_cuda(t)) {}
   static c10::Device need_cuda(const Tensor& t) {
-    if (!t.is_cuda()) {
-      if (PyGILState_Check()) {
-        PyErr_SetString(PyExc_AssertionError, "tops_b200 ops take CUDA tensors; there is no CPU path");
-        throw py::error_already_set();
-      }
-      TORCH_CHECK(false, "tops_b200 ops take CUDA tensors; there is no CPU path");
-    }
+    if (!t.is_cuda()) raise_assertion("tops_b200 ops take CUDA tensors; there is no CPU path");
     return t.device();
   }
   void* stream() const { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }

@@ -256,7 +256,7 @@ struct KdaNode : public OpNode {
       check_device_word("chunk_kda backward");
       if (g.scalar_type() != type) dg = dg.to(g.scalar_type());
     } else {
-      TORCH_CHECK(q.size(3) <= 128 && v.size(3) <= 128, "the KDA backward kernel takes K, V <= 128");
+      if (q.size(3) > 128 || v.size(3) > 128) raise_assertion("the KDA backward kernel takes K, V <= 128");
       dg = c.empty_as(g);
       tops_kda_bwd_params p{};
       p.B = (int)q.size(0); p.T = (int)q.size(1); p.H = (int)q.size(2); p.K = (int)q.size(3); p.V = (int)v.size(3);
@@ -488,10 +488,7 @@ Tensor rmsnorm_gated(const Tensor& x, const Tensor& g, const OptTensor& w_, doub
 }  // namespace
 
 PYBIND11_MODULE(_torch_ops, m) {
-  m.def("configure", [](py::object error_class, bool check_device) {
-    g_error_class = error_class.inc_ref().ptr();
-    g_check_device = check_device;
-  });
+  m.def("configure", [](py::object module) { g_module = module.inc_ref().ptr(); });
   m.def("chunk", &chunk);
   m.def("recurrent", &recurrent);
   m.def("recurrent_decode", &recurrent_decode);
