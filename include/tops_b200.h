@@ -399,7 +399,7 @@ int tops_b200_chunk_kda_fwd(const tops_chunk_kda_fwd_params* p, void* stream);
  * `grad_dtype` (TOPS_F32 as the reference's orchestrator returns them, or TOPS_BF16); dv bf16;
  * dg is with respect to the natural-log gate; dh0 fp32 (NULL to skip).
  * State gradient only: with dq = dk = dg = dbeta = NULL the call runs the reverse scan alone and
- * writes dh0 (dv is left alone).  The state gradient entering a span of tokens depends on the one leaving it
+ * writes dh0, and dv where it is not NULL.  The state gradient entering a span of tokens depends on the one leaving it
  * linearly, dh_in = M^T dh_out + D; a call with dht = NULL gives D, the summary a rank needs when one
  * sequence is sharded over time (no counterpart in the reference, which has no multi-device path).
  * ------------------------------------------------------------------------ */

@@ -1319,7 +1319,7 @@ int kda_chunk_bwd(const tops_chunk_kda_bwd_params& p, void* ws, cudaStream_t st)
     if ((rc = post_launch())) return rc;
   }
   const bool state_gradient_only = !p.dq && !p.dk && !p.dg && !p.dbeta;
-  if (state_gradient_only) return TOPS_OK;
+  if (state_gradient_only && !p.dv) return TOPS_OK;
   {
     KdaIntraParams ip;
     if ((rc = act_map(&ip.mdo, p.do_, BT, p.H)) || (rc = act_map(&ip.mvn, vnsaved, BT, p.H)) ||
@@ -1333,6 +1333,7 @@ int kda_chunk_bwd(const tops_chunk_kda_bwd_params& p, void* ws, cudaStream_t st)
     k_kda_bwd_intra<<<dim3(p.H, NT, p.B), NTHREADS, KDA_INTRA_SMEM, st>>>(ip);
     if ((rc = post_launch())) return rc;
   }
+  if (state_gradient_only) return TOPS_OK;   // (dv = beta T^T dv' is the kernel's above)
   {
     KdaBwdOutParams op;
     if ((rc = act_map(&op.mq, p.q, BT, p.H)) || (rc = act_map(&op.mk, p.k, BT, p.H)) ||

@@ -573,10 +573,10 @@ extern "C" size_t tops_b200_chunk_kda_bwd_workspace_bytes(const tops_chunk_kda_b
 
 extern "C" int tops_b200_chunk_kda_bwd(const tops_chunk_kda_bwd_params* p, void* workspace, size_t workspace_bytes,
                                        void* stream) {
-  if (!p || !p->q || !p->k || !p->v || !p->g || !p->beta || !p->do_ || !p->saved || !p->dv) return TOPS_E_NULL;
-  {   // dq, dk, dg, dbeta: all four, or none (state gradient only, which must then be asked for)
+  if (!p || !p->q || !p->k || !p->v || !p->g || !p->beta || !p->do_ || !p->saved) return TOPS_E_NULL;
+  {   // dq, dk, dg, dbeta: all four and dv, or none (state gradient only, which must then be asked for)
     const int given = !!p->dq + !!p->dk + !!p->dg + !!p->dbeta;
-    if ((given != 0 && given != 4) || (given == 0 && !p->dh0)) return TOPS_E_NULL;
+    if ((given != 0 && given != 4) || (given == 0 && !p->dh0) || (given == 4 && !p->dv)) return TOPS_E_NULL;
   }
   if (p->B < 1 || p->T < 1 || p->H < 1 || p->K < 1 || p->V < 1) return TOPS_E_BAD_SHAPE;
   if (!valid_dtype(p->dtype) || !valid_dtype(p->gate_dtype) || !valid_dtype(p->grad_dtype)) return TOPS_E_BAD_DTYPE;

@@ -190,7 +190,6 @@ def _chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved):
     beta_c = beta.to(q.dtype).contiguous()
     do = L.dense(do.to(q.dtype))
     dhtc = L.dense(None if dht is None else dht.float())
-    dv = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
     dh0 = torch.empty(B, H, K, V, dtype=torch.float32, device=dev)
     p = L.ChunkKdaBwdParams()
     p.B, p.T, p.H, p.K, p.V, p.chunk = B, T, H, K, V, 64
@@ -198,7 +197,7 @@ def _chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved):
     p.q, p.k, p.v, p.g, p.beta, p.do_, p.dht = (L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(g), L.ptr(beta_c), L.ptr(do),
                                                 L.ptr(dhtc))
     p.saved = L.ptr(saved)
-    p.dv, p.dh0 = L.ptr(dv), L.ptr(dh0)
+    p.dh0 = L.ptr(dh0)
     p.grad_dtype = L.F32
     ws = L.workspace(L.lib.tops_b200_chunk_kda_bwd_workspace_bytes(C.byref(p)), dev)
     L.check(L.lib.tops_b200_chunk_kda_bwd(C.byref(p), ws.data_ptr(), ws.numel(), L.stream_ptr(dev)), "chunk_kda_bwd")

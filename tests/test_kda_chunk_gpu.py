@@ -197,3 +197,28 @@ def test_chunk_kda_bwd_unnormalised_inputs_and_strong_gates(h0):
         assert_close(name, a.float().cpu(), r.float(), BF16)
     if h0:
         assert_close("dh0", dh0.cpu(), ref[5], BF16)
+
+
+def test_state_gradient_only_writes_dv_where_it_is_asked_for():
+    import ctypes as C
+
+    from tops_b200 import _lib as L
+    from tops_b200.ops import kda as M
+    B, T, H = 1, 192, 3
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    q, k = (torch.nn.functional.normalize(r(B, T, H, 128), dim=-1).to(torch.bfloat16) for _ in range(2))
+    v, do, g, beta = r(B, T, H, 128).to(torch.bfloat16), r(B, T, H, 128).to(torch.bfloat16), -r(B, T, H, 128).abs().to(torch.bfloat16) / 16, \
+        r(B, T, H).sigmoid().to(torch.bfloat16)
+    dht, scale = r(B, H, 128, 128), 128 ** -0.5
+    saved = M._chunk_fwd_call(q, k, v, g, beta, scale, None, False, 64, False, True)[4]
+    _, _, dv, _, _, dh0 = M._chunk_bwd_call(q, k, v, g, beta, do, scale, dht, saved, True, torch.bfloat16)
+    p = L.ChunkKdaBwdParams()
+    p.B, p.T, p.H, p.K, p.V, p.chunk, p.dtype, p.gate_dtype, p.scale, p.grad_dtype = B, T, H, 128, 128, 64, L.BF16, L.BF16, scale, L.F32
+    p.q, p.k, p.v, p.g, p.beta, p.do_, p.dht, p.saved = (L.ptr(t) for t in (q, k, v, g, beta, do, dht, saved))
+    got_dv, got_dh0 = torch.zeros_like(v), torch.zeros_like(dht)
+    p.dv, p.dh0 = L.ptr(got_dv), L.ptr(got_dh0)
+    ws = L.workspace(L.lib.tops_b200_chunk_kda_bwd_workspace_bytes(C.byref(p)), q.device)
+    L.check(L.lib.tops_b200_chunk_kda_bwd(C.byref(p), ws.data_ptr(), ws.numel(), L.stream_ptr(q.device)), "chunk_kda_bwd")
+    assert torch.equal(got_dh0, dh0) and torch.equal(got_dv, dv)
+    assert torch.equal(M._chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved), dh0)
