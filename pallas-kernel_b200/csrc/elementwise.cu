@@ -110,7 +110,11 @@ __device__ __forceinline__ float rcp_unit(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float sigmoidf(float x) { return rcp_unit(1.f + exp_unit(-x)); }
+// EXACT: CUDA's division and log1pf.  For results that are kept in fp32, where what the units and the polynomial below leave
+// (2e-7) shows: gates and norms of fp32 tensors were 1 - 5 % further from fp64 with them.
+template <bool EXACT> __device__ __forceinline__ float reciprocal(float x) { return EXACT ? 1.f / x : rcp_unit(x); }
+template <bool EXACT> __device__ __forceinline__ float exponential(float x) { return EXACT ? __expf(x) : exp_unit(x); }
+template <bool EXACT> __device__ __forceinline__ float sigmoidf(float x) { return reciprocal<EXACT>(1.f + exponential<EXACT>(-x)); }
 // log(1 + t) for 0 <= t <= 1 as t times a polynomial, a Chebyshev fit of log(1 + t) / t on [0, 1]: relative error
 // below 2e-7 in fp32, no cancellation for small t, no division
 __device__ __forceinline__ float log1p_unit(float t) {
@@ -126,16 +130,33 @@ __device__ __forceinline__ float log1p_unit(float t) {
   return p * t;
 }
 // with t = exp(-|x|): softplus(x) = max(x, 0) + log(1 + t), sigmoid(x) = 1 / (1 + t) or t / (1 + t)
-__device__ __forceinline__ float softplusf(float x) { return fmaxf(x, 0.f) + log1p_unit(exp_unit(-fabsf(x))); }
-__device__ __forceinline__ void softplus_sigmoid(float x, float& sp, float& sg) {
-  const float t = exp_unit(-fabsf(x)), i1 = rcp_unit(1.f + t);
-  sp = fmaxf(x, 0.f) + log1p_unit(t);
-  sg = x >= 0.f ? i1 : t * i1;
+template <bool EXACT> __device__ __forceinline__ float softplusf(float x) {
+  const float t = exponential<EXACT>(-fabsf(x));
+  return fmaxf(x, 0.f) + (EXACT ? log1pf(t) : log1p_unit(t));
+}
+template <bool EXACT> __device__ __forceinline__ void softplus_sigmoid(float x, float& sp, float& sg) {
+  const float t = exponential<EXACT>(-fabsf(x)), i1 = reciprocal<EXACT>(1.f + t);
+  sp = fmaxf(x, 0.f) + (EXACT ? log1pf(t) : log1p_unit(t));
+  sg = EXACT ? sigmoidf<true>(x) : x >= 0.f ? i1 : t * i1;
 }
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
+}
+// sum of a thread's products; fp32 tensors: in two halves, whose rounding is what four elements at a time had
+template <class T, int VW>
+__device__ __forceinline__ float sum_products(const float (&v)[VW], const float (&w)[VW]) {
+  constexpr int N = std::is_same<T, float>::value && VW == 8 ? 4 : VW;
+  float s = 0.f;
+#pragma unroll
+  for (int c = 0; c < VW; c += N) {
+    float h = 0.f;
+#pragma unroll
+    for (int t = c; t < c + N; ++t) h = fmaf(v[t], w[t], h);
+    s += h;
+  }
+  return s;
 }
 // sum over the 2^LG neighbouring lanes that share a row
 template <int LG>   // log2 of the lanes
@@ -153,7 +174,7 @@ __device__ __forceinline__ float row_sum(float x) {
 struct GateConst {
   const float* A_log;    // [H] (KDA kinds)
   const float* dt_bias;  // [H*K] or null
-  float lower_bound, inv_normalizer, clamp_min;
+  float lower_bound, normalizer, inv_normalizer, clamp_min;
   int has_clamp;
 };
 struct GateThread { int col; size_t row, step; bool on; };
@@ -173,6 +194,7 @@ template <class TI, class TO, int KIND, int VW>
 __global__ void __launch_bounds__(256) k_gate_fwd(const TI* __restrict__ g, TO* __restrict__ out, size_t rows, int H, int K,
                                                   GateConst c) {
   constexpr int U = 4;
+  constexpr bool EXACT = std::is_same<TO, float>::value;
   const int HK = H * K;
   const GateThread th = gate_thread<VW>(HK);
   if (!th.on) return;
@@ -196,10 +218,10 @@ __global__ void __launch_bounds__(256) k_gate_fwd(const TI* __restrict__ g, TO* 
 #pragma unroll
       for (int t = 0; t < VW; ++t) {
         const float xb = x[t] + bias[t];
-        if (KIND == TOPS_GATE_ACT_KDA) y[t] = -eA * softplusf(xb);
-        else if (KIND == TOPS_GATE_ACT_KDA_LOWER_BOUND) y[t] = c.lower_bound * sigmoidf(eA * xb);
+        if (KIND == TOPS_GATE_ACT_KDA) y[t] = -eA * softplusf<EXACT>(xb);
+        else if (KIND == TOPS_GATE_ACT_KDA_LOWER_BOUND) y[t] = c.lower_bound * sigmoidf<EXACT>(eA * xb);
         else {
-          y[t] = -softplusf(-xb) * c.inv_normalizer;   // log_sigmoid(x) = -softplus(-x)
+          y[t] = EXACT ? -softplusf<true>(-xb) / c.normalizer : -softplusf<false>(-xb) * c.inv_normalizer;   // log_sigmoid(x) = -softplus(-x)
           if (c.has_clamp && y[t] < c.clamp_min) y[t] = c.clamp_min;
         }
       }
@@ -217,6 +239,8 @@ __global__ void __launch_bounds__(256) k_gate_bwd(const TI* __restrict__ g, cons
   // rows in flight, measured on [8, 4096, 16, 128] bf16: the KDA law 87 us with four and 104 with two, log-sigmoid 67
   // with two and 77 with four
   constexpr int U = KIND == TOPS_GATE_ACT_LOG_SIGMOID ? 2 : 4;
+  // (the lower-bound law's dA_log is a small rest of large terms)
+  constexpr bool EXACT = std::is_same<TI, float>::value || KIND == TOPS_GATE_ACT_KDA_LOWER_BOUND;
   const int HK = H * K;
   const GateThread th = gate_thread<VW>(HK);
   float bias[VW], sb[VW], sa[VW], eA = 0.f;
@@ -247,17 +271,17 @@ __global__ void __launch_bounds__(256) k_gate_bwd(const TI* __restrict__ g, cons
           const float xb = x[t] + bias[t];
           if (KIND == TOPS_GATE_ACT_KDA) {
             float sp, sg;
-            softplus_sigmoid(xb, sp, sg);
+            softplus_sigmoid<EXACT>(xb, sp, sg);
             const float ed = -eA * d[t];
             o[t] = ed * sg;
             sa[t] = fmaf(ed, sp, sa[t]);
           } else if (KIND == TOPS_GATE_ACT_KDA_LOWER_BOUND) {
-            const float s = sigmoidf(eA * xb);
+            const float s = sigmoidf<EXACT>(eA * xb);
             o[t] = d[t] * c.lower_bound * s * (1.f - s) * eA;
             sa[t] = fmaf(o[t], xb, sa[t]);
           } else {
             float sp, sg;
-            softplus_sigmoid(-xb, sp, sg);   // log_sigmoid(x) = -softplus(-x), 1 - sigmoid(x) = sigmoid(-x)
+            softplus_sigmoid<EXACT>(-xb, sp, sg);   // log_sigmoid(x) = -softplus(-x), 1 - sigmoid(x) = sigmoid(-x)
             o[t] = (c.has_clamp && -sp * c.inv_normalizer < c.clamp_min) ? 0.f : d[t] * sg * c.inv_normalizer;
           }
           sb[t] += o[t];
@@ -363,8 +387,7 @@ __global__ void __launch_bounds__(256) k_l2norm_fwd(const T* __restrict__ x, T* 
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
       Vec<T, VW>::widen(raw[u][n], v[n]);
-#pragma unroll
-      for (int t = 0; t < VW; ++t) ss = fmaf(v[n][t], v[n][t], ss);
+      ss += sum_products<T>(v[n], v[n]);
     }
     ss = row_sum<LG>(ss);
     const float r = rsqrtf(ss + eps);
@@ -411,11 +434,8 @@ __global__ void __launch_bounds__(256) k_l2norm_bwd(const T* __restrict__ x, con
     for (int n = 0; n < NV; ++n) {
       Vec<T, VW>::widen(rx[u][n], v[n]);
       Vec<T, VW>::widen(rd[u][n], d[n]);
-#pragma unroll
-      for (int t = 0; t < VW; ++t) {
-        ss = fmaf(v[n][t], v[n][t], ss);
-        dot = fmaf(v[n][t], d[n][t], dot);
-      }
+      ss += sum_products<T>(v[n], v[n]);
+      dot += sum_products<T>(v[n], d[n]);
     }
     ss = row_sum<LG>(ss);
     dot = row_sum<LG>(dot);
@@ -484,8 +504,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
       Vec<T, VW>::widen(rx[u][n], v[n]);
-#pragma unroll
-      for (int t = 0; t < VW; ++t) ss = fmaf(v[n][t], v[n][t], ss);
+      ss += sum_products<T>(v[n], v[n]);
     }
     ss = row_sum<LG>(ss);
     const float r = rsqrtf(fmaf(ss, invD, eps));
@@ -501,7 +520,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_fwd(const T* __restrict__
           for (int t = 0; t < VW; ++t) wv[t] = 1.f;
           if (w.p) w.load<VW>(c, wv);
 #pragma unroll
-          for (int t = 0; t < VW; ++t) o[t] = v[n][t] * r * wv[t] * (gv[t] * sigmoidf(gv[t]));
+          for (int t = 0; t < VW; ++t) o[t] = v[n][t] * r * wv[t] * (gv[t] * sigmoidf<std::is_same<T, float>::value>(gv[t]));
           Vec<T, VW>::store(y + row * D + c, o);
         }
       }
@@ -546,8 +565,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__
     for (int n = 0; n < NV; ++n) {
       Vec<T, VW>::widen(rx[n], v[n]);
       Vec<T, VW>::widen(rd[n], dv[n]);
-#pragma unroll
-      for (int t = 0; t < VW; ++t) ss = fmaf(v[n][t], v[n][t], ss);
+      ss += sum_products<T>(v[n], v[n]);
     }
     ss = row_sum<LG>(ss);
     const float r = rsqrtf(fmaf(ss, invD, eps));
@@ -562,7 +580,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_gated_bwd(const T* __restrict__
       if (w.p && c < D) w.load<VW>(c, wv);
 #pragma unroll
       for (int t = 0; t < VW; ++t) {
-        const float gg = gv[t], s = sigmoidf(gg), silu = gg * s, xn = v[n][t] * r, dwv = dv[n][t] * wv[t];
+        const float gg = gv[t], s = sigmoidf<std::is_same<T, float>::value>(gg), silu = gg * s, xn = v[n][t] * r, dwv = dv[n][t] * wv[t];
         og[t] = dwv * xn * (s * (1.f + gg * (1.f - s)));   // d silu / dg = s (1 + g (1 - s))
         dw[n][t] += dv[n][t] * xn * silu;
         dv[n][t] = dwv * silu;                              // d(normalised x)
@@ -607,7 +625,7 @@ int dispatch(int dtype, F f) {
 
 GateConst gate_const(const tops_gate_act_params& p) {
   GateConst c;
-  c.A_log = p.A_log; c.dt_bias = p.dt_bias; c.lower_bound = p.lower_bound; c.inv_normalizer = 1.f / p.normalizer;
+  c.A_log = p.A_log; c.dt_bias = p.dt_bias; c.lower_bound = p.lower_bound; c.normalizer = p.normalizer; c.inv_normalizer = 1.f / p.normalizer;
   c.clamp_min = p.clamp_min; c.has_clamp = p.has_clamp_min;
   return c;
 }
@@ -822,7 +840,7 @@ __global__ void __launch_bounds__(256) k_lowrank_gate(tops_lowrank_gate_params p
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           xr[j] = from_f<T>(acc[j][t]);
-          float y = -softplusf(-to_f(xr[j])) * inv;
+          float y = -softplusf<std::is_same<T, float>::value>(-to_f(xr[j])) * inv;
           if (p.has_clamp_min && y < p.clamp_min) y = p.clamp_min;
           yr[j] = from_f<T>(y);
         }

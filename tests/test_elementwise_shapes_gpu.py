@@ -62,3 +62,28 @@ def test_tensors_without_elements_are_refused(shape):
     for call in (lambda: l2norm(x), lambda: rmsnorm_gated(x, x), lambda: gla_gate(x), lambda: kda_gate_fwd(x, torch.zeros(3, device="cuda"))):
         with pytest.raises((AssertionError, TopsError)):
             call()
+
+
+def test_fp32_results_keep_fp32_precision():
+    """Against fp64, fp32 tensors.  The bars are what CUDA's division and log1pf leave on these inputs (results, gradients),
+    plus 1 %; the approximate reciprocal and the polynomial of the 16-bit kernels leave 1 - 5 % more."""
+    from tops_b200.ops.gate import gla_gate, kda_gate_fwd
+    from tops_b200.ops.norm import l2norm, rmsnorm_gated
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x, z, dy = (torch.randn(2, 1500, 8, 128, generator=gen, device="cuda") for _ in range(3))
+    A = torch.randn(8, generator=gen, device="cuda")
+    F = torch.nn.functional
+    e = A.double().exp()[:, None]
+    cases = [(lambda t: kda_gate_fwd(t, A, lower_bound=-5.0), lambda t: -5 * torch.sigmoid(e * t), 5.092e-8, 1.128e-7),
+             (lambda t: gla_gate(t), lambda t: F.logsigmoid(t) / 16, 3.208e-8, 5.525e-8),
+             (lambda t: kda_gate_fwd(t, A), lambda t: -e * F.softplus(t), 5.817e-8, 6.566e-8),
+             (lambda t: l2norm(t), lambda t: t * torch.rsqrt(t.square().sum(-1, keepdim=True) + 1e-6), 4.677e-8, 5.377e-8),
+             (lambda t: rmsnorm_gated(t, z), lambda t: t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-5) * F.silu(z.double()),
+              7.186e-8, 7.729e-8)]
+    for op, ref, *bars in cases:
+        leaf, exact = x.clone().requires_grad_(), x.double().requires_grad_()
+        y, want = op(leaf), ref(exact)
+        pairs = [(y, want), (torch.autograd.grad(y, leaf, dy)[0], torch.autograd.grad(want, exact, dy.double())[0])]
+        for (a, b), bar in zip(pairs, bars):
+            err = ((a.double() - b).norm() / b.norm()).item()
+            assert err <= 1.01 * bar, (err, bar)
