@@ -125,9 +125,10 @@ struct KdaPrepParams {
   CUtensorMap mq, mk, mg;
   const __nv_bfloat16* beta;    // [B,T,H]
   uint8_t* prep;                // [B*NT*H] x PREP_BYTES
+  int c0;                       // first chunk of the stretch
   float* Aqk_out;               // [B,T,H,64] fp32 or null
   float* Akk_out;               // [B,T,H,64] fp32 or null
-  int T, H, NT, total;          // total = B * H * NT chunks
+  int T, H, NT, total;          // NT: chunks of the stretch; total = B * H * NT chunks
   float scale;
 };
 struct KdaPrepShared {
@@ -171,14 +172,18 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_kda_prep(const __grid_constant_
   const uint32_t tm = sh.tmem_slot, lane_base = q4 * 32;
   const int ri = 16 * q4 + lane;   // row of an M = 64 accumulator held by lanes 0..15 of each quarter
   const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), kha = smem_u32(khs), ga = smem_u32(gs), ma = smem_u32(mt), tba = smem_u32(tb);
+  auto chunk_row = [&](int cid) {   // its first token
+    const int bc = cid / p.H, b = bc / p.NT;
+    return b * p.T + (p.c0 + bc - b * p.NT) * C;
+  };
   bool ok = true;
   int it = 0;
   for (int cid = blockIdx.x; cid < p.total; cid += gridDim.x, ++it) {
     const uint32_t ph = it & 1;
-    const int h = cid % p.H, row = (cid / p.H) * C;   // chunks are numbered (batch, chunk, head): token row = 64 x (batch, chunk)
+    const int h = cid % p.H, row = chunk_row(cid);   // chunks are numbered (batch, chunk, head)
     uint8_t* out = p.prep + (size_t)cid * PREP_BYTES;
     if (tid == 32 && cid + gridDim.x < p.total) {   // the tiles of this block's next chunk, on their way to L2
-      const int nc = cid + gridDim.x, nh = nc % p.H, nrow = (nc / p.H) * C;
+      const int nc = cid + gridDim.x, nh = nc % p.H, nrow = chunk_row(nc);
       tma_prefetch_l2_3d(&p.mg, 0, nh, nrow); tma_prefetch_l2_3d(&p.mg, 64, nh, nrow);
       tma_prefetch_l2_3d(&p.mq, 0, nh, nrow); tma_prefetch_l2_3d(&p.mq, 64, nh, nrow);
       tma_prefetch_l2_3d(&p.mk, 0, nh, nrow); tma_prefetch_l2_3d(&p.mk, 64, nh, nrow);
@@ -376,7 +381,7 @@ struct KdaScanFwdParams {
   float* s_final;               // [B,H,K,V] or null
   __nv_bfloat16* o;             // [B,T,H,V]
   int keep;                     // store h' and v'
-  int T, H, NT;
+  int T, H, NT, c0;             // NT, c0: chunks of the stretch, its first
 };
 struct KdaScanFwdShared {
   uint64_t full[2], hready, vbar, vready, sbar, obar[2], ofree[2];
@@ -491,7 +496,7 @@ __global__ void __launch_bounds__(KDA_SF_THREADS, 1) k_kda_scan_fwd(const __grid
     for (int c = 0; c < NT; ++c) {
       if (!wait(&sh.obar[c & 1], (c >> 1) & 1, 5)) break;
       tc_fence_after();
-      __nv_bfloat16* dst = p.o + ((size_t)(b * p.T + c * C + 16 * g4 + lane) * p.H + h) * D;
+      __nv_bfloat16* dst = p.o + ((size_t)(b * p.T + (p.c0 + c) * C + 16 * g4 + lane) * p.H + h) * D;
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         float a[32];
@@ -546,7 +551,7 @@ __global__ void __launch_bounds__(KDA_SF_THREADS, 1) k_kda_scan_fwd(const __grid
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 16)   // D[k][v] = sum_j k~[j][k] v'[j][v]
           umma_bf16(tm + cD, desc_mnmajor(ka, 64, k0, 0), desc_mnmajor(va, 64, k0, 0), umma_idesc(128, 128, 1, 1), k0 > 0);
-        if (p.keep) {
+        if (p.keep) {   // (then there is one stretch, c0 = 0)
           const int row = b * p.T + c * C;
           tma_store_3d(&p.mvn, vts, 0, h, row);
           tma_store_3d(&p.mvn, vts + SLAB64, 64, h, row);
@@ -572,7 +577,7 @@ __global__ void __launch_bounds__(KDA_SF_THREADS, 1) k_kda_scan_fwd(const __grid
         if (c >= 2 && !wait(&sh.obar[c & 1], ((c - 2) >> 1) & 1, 5)) break;
         uint64_t* bar = &sh.full[c & 1];
         uint8_t* dst = stage(c);
-        const int row = b * p.T + c * C;
+        const int row = b * p.T + (p.c0 + c) * C;
         mbar_expect_tx(bar, KDA_SF_STAGE);
         bulk_load(dst, p.prep + slot(c) * PREP_BYTES, PREP_FWD, bar);
         tma_load_3d(dst + PREP_FWD, &p.mv, bar, 0, h, row);
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(KDA_SF_THREADS, 1) k_kda_scan_fwd(const __grid
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && sh.abort_flag) {
-    poison(p.o + ((size_t)b * p.T * p.H + h) * D);
+    poison(p.o + ((size_t)(b * p.T + p.c0 * C) * p.H + h) * D);
     if (p.s_final) poison(p.s_final + (size_t)blockIdx.x * D * D);
   }
 }
@@ -1227,7 +1232,22 @@ static size_t activation_bytes(int B, int T, int H) { return align_up((size_t)B 
 size_t kda_chunk_saved_bytes(const tops_chunk_kda_fwd_params& p) {
   return prep_bytes(p.B, p.T, p.H) + chunk_state_bytes(p.B, p.T, p.H) + activation_bytes(p.B, p.T, p.H);
 }
-size_t kda_chunk_fwd_workspace_bytes(const tops_chunk_kda_fwd_params& p) { return p.saved ? 0 : prep_bytes(p.B, p.T, p.H); }
+// Without one the sequences are walked in stretches whose tiles take a gigabyte at most (the state between them in fp32):
+// the tiles are 4.5 times the size of q, and nothing but the scan that follows reads them.  Two stretches instead of one at
+// B = 4, T = 8192, H = 32.
+constexpr size_t kPrepScratch = 1ull << 30;
+static int stretch_chunks(const tops_chunk_kda_fwd_params& p) {
+  const int NT = p.T / C;
+  const size_t per = (size_t)p.B * p.H * PREP_BYTES, fit = kPrepScratch / per;
+  const int most = fit < 1 ? 1 : fit < (size_t)NT ? (int)fit : NT;
+  return (NT + (NT + most - 1) / most - 1) / ((NT + most - 1) / most);   // (stretches of about equal length)
+}
+static size_t boundary_state_bytes(const tops_chunk_kda_fwd_params& p) {
+  return stretch_chunks(p) < p.T / C ? align_up((size_t)p.B * p.H * D * D * 4) : 0;
+}
+size_t kda_chunk_fwd_workspace_bytes(const tops_chunk_kda_fwd_params& p) {
+  return p.saved ? 0 : prep_bytes(p.B, stretch_chunks(p) * C, p.H) + boundary_state_bytes(p);
+}
 
 int kda_chunk_fwd(const tops_chunk_kda_fwd_params& p, cudaStream_t st) {
   if (!aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !aligned16(p.g) || !aligned16(p.o) || !aligned16(p.h0) ||
@@ -1243,13 +1263,15 @@ int kda_chunk_fwd(const tops_chunk_kda_fwd_params& p, cudaStream_t st) {
     TOPS_CUDA_OK(cudaMallocAsync(&own, kda_chunk_fwd_workspace_bytes(p), st));
     prep = reinterpret_cast<uint8_t*>(own);
   }
-  auto run = [&]() -> int {
+  float* boundary = nullptr;   // the state between two stretches
+  if (!p.saved && boundary_state_bytes(p)) boundary = reinterpret_cast<float*>(prep + prep_bytes(p.B, stretch_chunks(p) * C, p.H));
+  auto run = [&](int c0, int nch) -> int {
     {
       KdaPrepParams pp;
       if ((rc = act_map(&pp.mq, p.q, BT, p.H)) || (rc = act_map(&pp.mk, p.k, BT, p.H)) || (rc = act_map(&pp.mg, p.g, BT, p.H))) return rc;
       pp.beta = reinterpret_cast<const __nv_bfloat16*>(p.beta);
       pp.prep = prep; pp.Aqk_out = p.Aqk_out; pp.Akk_out = p.Akk_out;
-      pp.T = p.T; pp.H = p.H; pp.NT = NT; pp.total = p.B * NT * p.H; pp.scale = p.scale;
+      pp.T = p.T; pp.H = p.H; pp.NT = nch; pp.c0 = c0; pp.total = p.B * nch * p.H; pp.scale = p.scale;
       if ((rc = opt_in_smem(k_kda_prep, KDA_PREP_SMEM))) return rc;
       const int grid = pp.total < 2 * sm_count() ? pp.total : 2 * sm_count();
       KernelScope ks("sm100_kda_prep", st);
@@ -1264,14 +1286,17 @@ int kda_chunk_fwd(const tops_chunk_kda_fwd_params& p, cudaStream_t st) {
       if ((rc = state_map(&sp.mst, h, (size_t)p.B * NT * p.H * D)) || (rc = act_map(&sp.mvn, h + chunk_state_bytes(p.B, p.T, p.H), BT, p.H)))
         return rc;
     }
-    sp.prep = prep; sp.s0 = p.h0; sp.s_final = p.ht; sp.o = reinterpret_cast<__nv_bfloat16*>(p.o);
-    sp.T = p.T; sp.H = p.H; sp.NT = NT;
+    // (a block reads the state it starts from before it writes the one it ends with)
+    sp.prep = prep; sp.s0 = c0 ? boundary : p.h0; sp.s_final = c0 + nch < NT ? boundary : p.ht; sp.o = reinterpret_cast<__nv_bfloat16*>(p.o);
+    sp.T = p.T; sp.H = p.H; sp.NT = nch; sp.c0 = c0;
     if ((rc = opt_in_smem(k_kda_scan_fwd, KDA_SF_SMEM))) return rc;
     KernelScope ks("sm100_kda_scan_fwd", st);
     k_kda_scan_fwd<<<p.B * p.H, KDA_SF_THREADS, KDA_SF_SMEM, st>>>(sp);
     return post_launch();
   };
-  rc = run();
+  const int stretch = p.saved ? NT : stretch_chunks(p);
+  rc = TOPS_OK;
+  for (int c0 = 0; rc == TOPS_OK && c0 < NT; c0 += stretch) rc = run(c0, NT - c0 < stretch ? NT - c0 : stretch);
   if (own && cudaFreeAsync(own, st) != cudaSuccess && rc == TOPS_OK) rc = TOPS_E_CUDA;
   return rc;
 }

@@ -222,3 +222,25 @@ def test_state_gradient_only_writes_dv_where_it_is_asked_for():
     L.check(L.lib.tops_b200_chunk_kda_bwd(C.byref(p), ws.data_ptr(), ws.numel(), L.stream_ptr(q.device)), "chunk_kda_bwd")
     assert torch.equal(got_dh0, dh0) and torch.equal(got_dv, dv)
     assert torch.equal(M._chunk_bwd_state_gradient(q, k, v, g, beta, do, scale, dht, saved), dh0)
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 64 * 1001, 16), (2, 64 * 450, 32)])
+def test_a_forward_in_stretches_is_the_forward(B, T, H):
+    """Without gradients the sequences are walked in stretches of bounded scratch; a training forward keeps all tiles and
+    walks them at once."""
+    import ctypes as C
+
+    from tops_b200 import _lib as L
+    from tops_b200.ops.kda import _chunk_params, chunk_kda
+    gen = torch.Generator(device="cuda").manual_seed(13)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda", dtype=torch.bfloat16)
+    q, k = (torch.nn.functional.normalize(r(B, T, H, 128), dim=-1) for _ in range(2))
+    v, g, beta, h0 = r(B, T, H, 128), -r(B, T, H, 128).abs() / 16, r(B, T, H).sigmoid(), torch.randn(B, H, 128, 128, generator=gen, device="cuda")
+    p = _chunk_params(q, k, v, g, beta, 1.0, 64)
+    need = L.lib.tops_b200_chunk_kda_fwd_workspace_bytes(C.byref(p))
+    assert need < (1 << 30) + 4 * h0.numel() + 512 < L.lib.tops_b200_chunk_kda_saved_bytes(C.byref(p))
+    with torch.no_grad():
+        o, ht = chunk_kda(q, k, v, g, beta, initial_state=h0, output_final_state=True)
+    want = chunk_kda(q, k, v.requires_grad_(), g, beta, initial_state=h0, output_final_state=True)
+    assert torch.equal(o, want[0]) and torch.equal(ht, want[1])
+    assert L.device_error() == 0
