@@ -138,3 +138,49 @@ def test_recurrent_cumsum_gate_and_norm_kernels_stay_inside_their_buffers(arena)
     gnorm = torch.randn(2, 21, 3, 24).cuda()
     norm.FusedRMSNormGated(24).cuda()(x["v"], gnorm)
     assert arena.check() >= 8
+
+
+@pytest.mark.parametrize("B,T,H,K,V,cu,strong", [
+    (1, 100, 2, 64, 64, None, False),                # general tcgen05 form: short last chunk, K and V below the tile
+    (2, 70, 3, 72, 328, None, False),                # three value slices
+    (1, 1000, 2, 128, 128, None, True),              # runs of a cut sequence, strong gates
+    (1, 300, 2, 128, 256, [0, 1, 64, 129, 300], True),
+])
+def test_general_gla_kernels_stay_inside_their_buffers(arena, B, T, H, K, V, cu, strong):
+    """The forward that keeps states and the backward that uses them, in the types of their inputs: what the differentiable
+    ops run (whose own buffers come from the extension, where the arena does not reach)."""
+    from tops_b200 import _lib as L
+    from tops_b200.ops._chunk import chunk_bwd_call, chunk_fwd_call
+    x = _cuda_inputs(55, B, T, H, K, V, torch.bfloat16)
+    g = x["g"] * 90 if strong else x["g"]
+    N = B if cu is None else len(cu) - 1
+    h0, dht = (torch.randn(N, H, K, V).cuda() for _ in range(2))
+    o, ht, _, _, hs = chunk_fwd_call(x["q"], x["k"], x["v"], g, L.GATE_PER_CHANNEL, 0.1, h0, True, 64, cu, want_saved=True)
+    for kept in (hs, None):
+        grads = chunk_bwd_call(x["q"], x["k"], x["v"], g, L.GATE_PER_CHANNEL, 0.1, h0, x["do"], dht, 64, torch.float32, True, True, cu,
+                               h_saved=kept, primal_dtypes=True)
+    assert hs is not None and all(torch.isfinite(t.float()).all() for t in (o, ht, *grads))
+    assert arena.check() >= 10
+
+
+@pytest.mark.parametrize("dtype,rows,D", [(torch.bfloat16, 37, 72), (torch.float32, 5, 1000), (torch.float16, 300, 8)])
+def test_norm_and_gate_gradients_stay_inside_their_buffers(arena, dtype, rows, D):
+    import ctypes as C
+
+    from tops_b200 import _lib as L
+    x, g, dy = (torch.randn(rows, D).cuda().to(dtype) for _ in range(3))
+    w = torch.randn(D).cuda()
+    st = L.stream_ptr(x.device)
+    y, dx, dg = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    dw = torch.empty(D, dtype=torch.float32, device="cuda")
+    p = L.NormParams()
+    p.rows, p.D, p.dtype, p.eps, p.heads = rows, D, L.dtype_code(dtype), 1e-5, 1
+    p.x, p.gate, p.weight, p.y, p.dy, p.dx, p.dgate, p.dweight = (L.ptr(t) for t in (x, g, w, y, dy, dx, dg, dw))
+    L.check(L.lib.tops_b200_rmsnorm_gated_fwd(C.byref(p), st), "fwd")
+    ws = L.workspace(L.lib.tops_b200_rmsnorm_gated_bwd_workspace_bytes(C.byref(p)), x.device)
+    L.check(L.lib.tops_b200_rmsnorm_gated_bwd(C.byref(p), ws.data_ptr(), ws.numel(), st), "bwd")
+    L.check(L.lib.tops_b200_l2norm_fwd(C.byref(p), st), "l2")
+    L.check(L.lib.tops_b200_l2norm_bwd(C.byref(p), st), "l2")
+    from tops_b200.ops.gate import kda_gate_bwd
+    kda_gate_bwd(x.view(rows, 2, D // 2), torch.zeros(2).cuda(), torch.zeros(D).cuda(), dy.view(rows, 2, D // 2))
+    assert arena.check() >= 7

@@ -47,9 +47,39 @@ def test_training_step(B, T, hidden, heads, cu):
     for n, a, b in zip(names, got, run(ref, torch.float32)):
         assert a.dtype == torch.bfloat16 and a.shape == b.shape
         # dq and dk (and so dx) of a sequence's first token are what is left of do . o / |o|^2 after the norm's
-        # projection: rounding noise of do, amplified; everything else keeps the bf16 bar
+        # projection: rounding noise of do, amplified; everything else keeps the bf16 bar (test_training_step_from_a_state
+        # holds these three to it too)
         bar = 0.2 if n in ("x", "q_proj.weight", "k_proj.weight") else 2e-2
         assert rel_l2(a, b) <= bar, (n, rel_l2(a, b))
+
+
+@pytest.mark.parametrize("T,kw,frozen", [(65, {}, ()), (130, {"clamp_min": -0.06}, ()), (100, {"elementwise_affine": False}, ()),
+                                         (70, {}, ("q_proj", "gk_proj.0", "o_proj")), (70, {}, ("k_proj", "gk_proj.1", "g_norm_swish_gate"))])
+def test_training_step_from_a_state(T, kw, frozen):
+    """Every gradient of the one-call layer, the initial state's among them, with a cotangent on the final state.  From a state
+    no output is a multiple of one token's v, so no gradient is noise and all keep the bf16 bar.  (The clip takes the tail of
+    the gates: one that took half of them would have many at its edge, where a rounding decides about a gradient.)"""
+    from tops_b200.layers import Cache
+    layer = _layer(512, 4, **kw)
+    for n, p in layer.named_parameters():
+        p.requires_grad_(not n.startswith(frozen) if frozen else True)
+    ref = copy.deepcopy(layer).float()
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(2, T, 512, generator=gen, device="cuda").to(torch.bfloat16)
+    do = torch.randn(2, T, 512, generator=gen, device="cuda").to(torch.bfloat16)
+    h0, dht = (torch.randn(2, 4, 64, 128, generator=gen, device="cuda") for _ in range(2))
+
+    def run(m, dt):
+        leaf, state, cache = x.to(dt).requires_grad_(), h0.clone().requires_grad_(), Cache()
+        cache.update(recurrent_state=state, layer_idx=0)
+        o, _, cache = m(leaf, past_key_values=cache, use_cache=True)
+        params = [p for p in m.parameters() if p.requires_grad]
+        return [o, cache[0]["recurrent_state"], *torch.autograd.grad([o, cache[0]["recurrent_state"]], [leaf, state, *params], [do.to(dt), dht])]
+    got, labels = _labels(lambda: run(layer, torch.bfloat16))
+    assert "lowrank_gate_fwd" in labels
+    names = ["o", "ht", "x", "h0", *(n for n, p in layer.named_parameters() if p.requires_grad)]
+    for n, a, b in zip(names, got, run(ref, torch.float32)):
+        assert a.shape == b.shape and rel_l2(a, b) <= 2e-2, (n, rel_l2(a, b))
 
 
 @pytest.mark.parametrize("T1", [1, 3, 64, 65, 130])

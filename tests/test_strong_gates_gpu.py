@@ -98,3 +98,35 @@ def test_a_layer_with_strong_gates():
     leaf = x.clone().requires_grad_()
     grads = torch.autograd.grad(layer(leaf)[0].float().square().sum(), [leaf, *layer.parameters()])
     assert all(torch.isfinite(t.float()).all() for t in grads)
+
+
+@pytest.mark.parametrize("level", [-0.05, -5.0])
+def test_a_captured_step(level):
+    """Forward + backward of a packed batch in a CUDA graph, replayed on other inputs."""
+    from tops_b200.ops.gla import chunk_gla
+    cu = [0, 70, 300]
+    x, _ = _inputs(93, 1, 300, 2, 128, 128, 2, level, False)
+    y, _ = _inputs(94, 1, 300, 2, 128, 128, 2, level, False)
+    names = ("q", "k", "v", "g", "h0")
+    c = {n: t.cuda() for n, t in x.items()}
+    leaves = [c[n].requires_grad_() for n in names]
+
+    def step():
+        o, ht = chunk_gla(*leaves[:4], initial_state=leaves[4], output_final_state=True, cu_seqlens=cu)
+        return [o, ht, *torch.autograd.grad([o, ht], leaves, [c["do"], c["dht"]])]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    with torch.no_grad():
+        for n in c:
+            c[n].copy_(y[n])
+    graph.replay()
+    torch.cuda.synchronize()
+    want = step()
+    for a, b in zip(captured, want):
+        assert torch.equal(a, b)
