@@ -208,9 +208,9 @@ __global__ void __launch_bounds__(NTH) k_state_scan(ScanArgs<T> a) {
 // ===========================================================================
 // The serial scan above walks a sequence with K/64 x V/64 blocks per (sequence, head) and pays a full load latency and
 // two barriers per chunk (3.6 us at C = 16): with few heads most of the GPU idles.  Here k_chunk_products computes all
-// chunks at once and k_chunk_states adds them up, one thread per four state elements, its loads independent of the sum.
+// chunks at once and k_chunk_states adds them up, one thread per state element, its loads independent of the sum.
 // It costs two more passes over the states, so it serves the problems whose serial scan would not fill the GPU.
-// fp32, B = 2, T = 512, H = 4, K = V = 64, C = 16: 117 -> PAR_US us for both kernels.
+// fp32, B = 2, T = 512, H = 4, K = V = 64, C = 16: 117 -> 23 us for both kernels.
 template <class T, int C, bool BWD>
 __global__ void __launch_bounds__(NTH) k_chunk_products(ScanArgs<T> a, float* __restrict__ D, float* __restrict__ decay) {
   __shared__ float xs[C * LD];

@@ -9,8 +9,8 @@
 // 64 tokens of a segment (storing the decayed states h'_t of that segment in scratch), and runs
 // the reverse recurrence over the segment with the state gradient in registers.
 // k_kda_fwd<RK> is the older block-wide forward, kept for 128 < K <= 256.
-// These kernels are the correctness path for KDA; the chunked WY / UT-transform
-// formulation on the tensor cores is not built.
+// A few tokens per call (decode) run in k_kda_step.  The chunked WY / UT-transform formulation on the tensor cores, for
+// bf16, K = V = 128 and whole chunks of 64, is kda_sm100.cu.
 #include "kda.cuh"
 
 namespace tops {
@@ -484,7 +484,7 @@ constexpr size_t BW_SMEM = sizeof(TokenTile) + (SEGMENT * 32 + 2 * 2 * 4 * 128 +
 // whose lanes are rows, reads 32-byte pieces V floats apart and reached 0.9 TB/s here).  With S' the decayed state
 //     p = k^T S',   r = q^T S',   e = beta (v - p),   o = scale (r + (q . k) e),   S = S' + k (x) e
 // both reductions over the keys come from one pass over the registers, so a token costs one exchange through shared
-// memory.  B = 16, H = 32, K = V = 128, one token: 73.6 -> 18.2 us (3.7 TB/s; B = 128: 93.6 us, 5.8 TB/s).
+// memory.  B = 16, H = 32, K = V = 128, one token: 73.6 -> 16.4 us (4.1 TB/s; B = 128: 93.6 us, 5.8 TB/s).
 template <int RK, bool VEC>   // VEC: the state's rows go as float4
 __global__ void __launch_bounds__(FW_THREADS) k_kda_step(tops_kda_fwd_params a) {
   __shared__ float qs[16 * RK], ks[16 * RK], egs[16 * RK];

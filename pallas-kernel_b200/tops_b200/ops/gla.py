@@ -115,7 +115,7 @@ def fused_chunk_gla(q, k, v, g=None, scale=None, initial_state=None, output_fina
 # token-serial recurrence
 # ---------------------------------------------------------------------------
 @L.on_tensor_device
-def _rec_fwd_call(q, k, v, gk, gv, scale, initial_state, want_state, reverse, cu, o_dtype, state_out=None):
+def _rec_fwd_call(q, k, v, gk, gv, scale, initial_state, want_state, reverse, cu, o_dtype):
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
@@ -128,8 +128,7 @@ def _rec_fwd_call(q, k, v, gk, gv, scale, initial_state, want_state, reverse, cu
     N = B if cu is None else len(cu) - 1
     h0 = None if initial_state is None else initial_state.float().contiguous()
     o = torch.empty(B, T, H, V, dtype=o_dtype, device=dev)
-    if state_out is None and want_state:
-        state_out = torch.empty(N, H, K, V, dtype=torch.float32, device=dev)
+    state_out = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if want_state else None
     cu_dev = None if cu is None else torch.tensor(cu, dtype=torch.int32, device=dev)
     p = L.RecurrentFwdParams()
     p.B, p.T, p.H, p.K, p.V = B, T, H, K, V
